@@ -1,4 +1,4 @@
-// Causal grouped-query attention over the paged cache, one warp per (token, head).
+// Causal grouped-query attention over the paged cache, one warp per (token, head), or several where there are few.
 //
 // Replaces the reference's paged_attention_decode_kernel (src/cuda/gemm_cuda.cu:
 // 304-429), which serves one query token, with a kernel for any number of new
@@ -52,35 +52,41 @@ __device__ __forceinline__ float row_dot(const float* __restrict__ q, const __nv
     return sum;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
+// PARTS warps of a block share one (token, head): warp w takes the chunks w, w + PARTS, ... of 32 keys, and the first
+// warp merges their softmaxes in order.  PARTS = 1: a block's warps serve ATT_WARPS (token, head) pairs.
+// Bound by a warp's chain of loads per chunk, not by bytes: a decode step of 3 sequences x 32 heads of 64 over 250 keys
+// took 65 us with one warp each and takes 11 with eight, one sequence over 2,000 keys 487 and 67, 40 sequences over 600
+// keys 168 and (four warps each) 107.
+template <typename T, int PARTS>
+__global__ void __launch_bounds__((PARTS == 1 ? ATT_WARPS : PARTS) * 32)
 attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                  const int* __restrict__ block_table, int table_width, const int* __restrict__ positions,
                  const int* __restrict__ token_seq, T* __restrict__ out, int n_tokens, int num_heads,
                  int num_kv_heads, int block_size, float scale, int window) {
-    __shared__ __align__(16) float q_smem[ATT_WARPS][HD];
+    __shared__ __align__(16) float q_smem[PARTS == 1 ? ATT_WARPS : 1][HD];
+    __shared__ float part_acc[PARTS][HD], part_max[PARTS], part_sum[PARTS];
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * ATT_WARPS + warp;
-    if (item >= (long long)n_tokens * num_heads) return;       // whole warps leave together
+    const long long item = PARTS == 1 ? (long long)blockIdx.x * ATT_WARPS + warp : (long long)blockIdx.x;
+    if (item >= (long long)n_tokens * num_heads) return;       // whole warps (with PARTS > 1: whole blocks) leave together
     const int t = (int)(item / num_heads), head = (int)(item % num_heads);
     const int kv_head = head / (num_heads / num_kv_heads);
     const int pos = positions[t];
     const int* table = block_table + (size_t)token_seq[t] * table_width;
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
 
-    float* qs = q_smem[warp];
+    float* qs = q_smem[PARTS == 1 ? warp : 0];
     const T* q_row = q + ((size_t)t * num_heads + head) * HD;
-    for (int d = lane; d < HD; d += 32) qs[d] = to_float(q_row[d]);
-    __syncwarp();
+    for (int d = PARTS == 1 ? lane : threadIdx.x; d < HD; d += PARTS * 32) qs[d] = to_float(q_row[d]);
+    if (PARTS == 1) __syncwarp(); else __syncthreads();
 
     float acc[DIMS_PER_LANE];
 #pragma unroll
     for (int i = 0; i < DIMS_PER_LANE; ++i) acc[i] = 0.0f;
     float running_max = -INFINITY, running_sum = 0.0f;
 
-    for (int j0 = lo; j0 <= pos; j0 += 32) {
+    for (int j0 = PARTS == 1 ? lo : lo + 32 * warp; j0 <= pos; j0 += 32 * PARTS) {
         const int j = j0 + lane;
         const bool valid = j <= pos;
         int row = 0;                                   // row index in units of HD elements
@@ -98,6 +104,7 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
 #pragma unroll
         for (int i = 0; i < DIMS_PER_LANE; ++i) acc[i] *= rescale;
         const int count = min(32, pos - j0 + 1);
+#pragma unroll 4
         for (int jj = 0; jj < count; ++jj) {
             const float pj = __shfl_sync(0xffffffffu, p, jj);
             const int rj = __shfl_sync(0xffffffffu, row, jj);
@@ -107,6 +114,28 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
                 const int d = lane + 32 * i;
                 if (d < HD) acc[i] = fmaf(pj, to_float(v_row[d]), acc[i]);
             }
+        }
+    }
+    if (PARTS > 1) {
+#pragma unroll
+        for (int i = 0; i < DIMS_PER_LANE; ++i)
+            if (lane + 32 * i < HD) part_acc[warp][lane + 32 * i] = acc[i];
+        if (lane == 0) { part_max[warp] = running_max; part_sum[warp] = running_sum; }
+        __syncthreads();
+        if (warp > 0) return;
+        // (the first part always has a key, so the maximum over the parts is finite; a part without keys weighs exp(-inf) = 0)
+        const float own_max = lane < PARTS ? part_max[lane] : -INFINITY;
+        const float top = warp_max(own_max);
+        const float weight = expf(own_max - top);
+        running_sum = warp_sum(lane < PARTS ? part_sum[lane] * weight : 0.0f);
+#pragma unroll
+        for (int i = 0; i < DIMS_PER_LANE; ++i) acc[i] = 0.0f;
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part) {
+            const float scale_part = __shfl_sync(0xffffffffu, weight, part);
+#pragma unroll
+            for (int i = 0; i < DIMS_PER_LANE; ++i)
+                if (lane + 32 * i < HD) acc[i] = fmaf(scale_part, part_acc[part][lane + 32 * i], acc[i]);
         }
     }
     T* out_row = out + ((size_t)t * num_heads + head) * HD;
@@ -132,9 +161,12 @@ SKV_EXPORT int skv_attention(const void* q, const void* k_cache, const void* v_c
         return fail("skv_attention", "heads must be a positive multiple of kv heads");
     if (block_size <= 0 || window < 0) return fail("skv_attention", "bad block size or window");
     const long long items = (long long)n_tokens * num_heads;
-    const long long blocks = (items + ATT_WARPS - 1) / ATT_WARPS;
-    if (blocks > 0x7fffffffLL) return fail("skv_attention", "too many tokens in one step");
-    return launch_pdl("skv_attention", attention_kernel<skv_t>, dim3((unsigned)blocks), dim3(ATT_WARPS * 32), 0,
+    if (items > 0x7fffffffLL) return fail("skv_attention", "too many tokens in one step");
+    // while a warp each leaves the GPU's 64 warps an SM idle, eight or four warps share a (token, head)
+    const int parts = items * 8 <= (long long)sm_count() * 64 ? 8 : items * 4 <= (long long)sm_count() * 64 ? 4 : 1;
+    const long long blocks = parts > 1 ? items : (items + ATT_WARPS - 1) / ATT_WARPS;
+    auto kernel = parts == 8 ? attention_kernel<skv_t, 8> : parts == 4 ? attention_kernel<skv_t, 4> : attention_kernel<skv_t, 1>;
+    return launch_pdl("skv_attention", kernel, dim3((unsigned)blocks), dim3((parts > 1 ? parts : ATT_WARPS) * 32), 0,
                       stream, (const skv_t*)q, (const skv_t*)k_cache, (const skv_t*)v_cache, block_table,
                       table_width, positions, token_seq, (skv_t*)out, n_tokens, num_heads, num_kv_heads,
                       block_size, scale, window);

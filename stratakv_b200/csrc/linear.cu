@@ -13,7 +13,8 @@
 //                8t..8t+7, rows 8-15 the matching up rows; out[M,N/2] =
 //                act(gate) * up in the compute dtype
 //
-// float build: a true 32-bit FMA tile kernel (no tensor cores, no TF32).
+// float build: true 32-bit FMA kernels (no tensor cores, no TF32), one that streams the weights for a few tokens and
+// a tiled one.
 // bfloat16 build: a weight-streaming kernel for any M that keeps 16 weight rows
 // per block and feeds tokens in groups of 8 through mma.sync m16n8k16 with float
 // accumulation.  Each lane loads 16 bytes (8 consecutive k) of a weight row and of
@@ -54,80 +55,351 @@ __device__ __forceinline__ void epilogue_store(void* out, int mode, int M, int N
 
 #if SKV_DTYPE == SKV_F32
 // ---------------------------------------------------------------------------
-// 64x64 output tile, K in steps of 16, 256 threads, 4 tokens x 4 columns each.
-// A thread's columns are {2j, 2j+1, 2j+8, 2j+9} of one 16-column group so that a
-// gate column and its up column meet in one thread.
-constexpr int FBM = 64, FBN = 64, FBK = 16;
+// Steps of at most 16 tokens: the weights stream by once.  A block serves one group of 16 weight rows (of a gated
+// matrix: 8 gate rows and their up rows).  Four row groups of four rows ({2j, 2j+1, 2j+8, 2j+9}, so that a gate row and
+// its up row meet in one warp) times KS parts of K are its warps; a lane reads 16 bytes of each of its four rows and
+// 16 bytes of every token, and the parts meet in shared memory in a fixed order.  The weights travel two rounds ahead in
+// registers, the tokens two rounds ahead into shared memory (loads of the tokens through L1 queue behind the weights'
+// misses).  Bound by HBM: the weights are the only traffic that counts.  KS fills the GPU where N is small: 2048 rows are
+// 128 blocks.  Measured (weights larger than L2) at 1 / 3 / 8 / 16 tokens: 11264 x 2048 15.8 / 19.6 / 27 / 48 us (5.9 to 1.9
+// TB/s), 2048 x 5632 10.5 / 12.5 / 15.5 / 24 us.  A 64 x 64 tile did this before, one token or sixteen alike: 335 and 640 us.
+constexpr int FEW_MAX = 16;
 
-__global__ void __launch_bounds__(256)
-linear_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, void* __restrict__ out,
-                  int M, int N, int K, int mode, act_t act) {
-    __shared__ float As[FBK][FBM + 4];
-    __shared__ float Ws[FBK][FBN + 4];
+// The four numbers at k..k+3 of a row of K numbers: one 16-byte load, or (WIDE off: any K, any alignment) one by one.
+template <bool WIDE>
+__device__ __forceinline__ float4 load_four(const float* row, int k, int K, bool live) {
+    if (!live) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (WIDE) return k < K ? *(const float4*)(row + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return make_float4(k < K ? row[k] : 0.0f, k + 1 < K ? row[k + 1] : 0.0f, k + 2 < K ? row[k + 2] : 0.0f,
+                       k + 3 < K ? row[k + 3] : 0.0f);
+}
+
+template <int MT, int KS, bool WIDE>
+__global__ void __launch_bounds__(128 * KS)
+linear_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, void* __restrict__ out,
+                      int M, int N, int K, int mode, act_t act) {
+    constexpr int STAGES = 3;
+    extern __shared__ __align__(16) float few_smem[];
+    float (*tokens)[MT][128] = (float (*)[MT][128])(few_smem + (size_t)(threadIdx.x >> 7) * STAGES * MT * 128);   // this part's [stage][token][128 k]
+    __shared__ float sums[KS][16][MT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = warp & 3, part = warp >> 2;
+    const int n0 = blockIdx.x * 16;
+    const int local[4] = {2 * group, 2 * group + 1, 2 * group + 8, 2 * group + 9};
+    const int per_part = ((K + KS * 128 - 1) / (KS * 128)) * 128;
+    const int k_begin = part * per_part + 4 * lane, k_end = min(K, (part + 1) * per_part);
+    const float* rows[4];
+    bool live[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        live[r] = n0 + local[r] < N;
+        rows[r] = W + (size_t)(live[r] ? n0 + local[r] : 0) * K;
+    }
+    float4 w[2][4];
+    // the weights do not depend on the kernel in front: their first loads are under way before it has finished
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) w[s][r] = load_four<WIDE>(rows[r], k_begin + 128 * s, k_end, live[r]);
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * FBM, n0 = blockIdx.x * FBN;
-    const int group = tx >> 2, j = tx & 3;
-    int cols[4] = {16 * group + 2 * j, 16 * group + 2 * j + 1, 16 * group + 2 * j + 8, 16 * group + 2 * j + 9};
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += FBK) {
+    auto fetch_tokens = [&](int stage, int k) {                    // the part's warps take every fourth token each
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int e = tid + i * 256;
-            const int row = e >> 4, k = e & 15;
-            const int gm = m0 + row, gn = n0 + row, gk = k0 + k;
-            As[k][row] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : 0.0f;
-            Ws[k][row] = (gn < N && gk < K) ? W[(size_t)gn * K + gk] : 0.0f;
+        for (int m = group; m < MT; m += 4) {
+            const float* row = A + (size_t)min(m, M - 1) * K;
+            if (WIDE) {
+                const int bytes = k < k_end ? 16 : 0;              // (zeros beyond the part's end)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(smem_u32(&tokens[stage][m][4 * lane])),
+                             "l"(row + (k < k_end ? k : 0)), "r"(bytes) : "memory");
+            } else {
+                *(float4*)&tokens[stage][m][4 * lane] = load_four<false>(row, k, k_end, true);
+            }
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch_tokens(0, k_begin);
+    fetch_tokens(1, k_begin + 128);
+    float acc[4][MT] = {};
+    int stage = 0, k = k_begin;
+    // one round: the numbers of round i are used, those of round i + 2 are asked for
+    auto round = [&](float4 (&wk)[4]) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" :: "r"(part + 1) : "memory");    // the part's warps: everybody's copies are in, and the
+        fetch_tokens(stage >= 1 ? stage - 1 : STAGES - 1, k + 256);      // stage of the round before is free again
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const float4 a = *(const float4*)&tokens[stage][m][4 * lane];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                acc[r][m] = fmaf(a.w, wk[r].w, fmaf(a.z, wk[r].z, fmaf(a.y, wk[r].y, fmaf(a.x, wk[r].x, acc[r][m]))));
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) wk[r] = load_four<WIDE>(rows[r], k + 256, k_end, live[r]);
+        stage = stage == STAGES - 1 ? 0 : stage + 1;
+        k += 128;
+    };
+    while (k - 4 * lane < k_end) {                                 // (a round beyond the end adds zeros)
+        round(w[0]);
+        round(w[1]);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const float v = warp_sum(acc[r][m]);
+            if (lane == 0) sums[part][local[r]][m] = v;
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 16 * MT; i += 128 * KS) {
+        const int n = i & 15, m = i >> 4;
+        float v = sums[0][n][m];
+#pragma unroll
+        for (int p = 1; p < KS; ++p) v += sums[p][n][m];
+        if (mode == MODE_GATED) {
+            if (n >= 8 || m >= M) continue;
+            float up = sums[0][n + 8][m];
+#pragma unroll
+            for (int p = 1; p < KS; ++p) up += sums[p][n + 8][m];
+            const int half_n = N >> 1, o = (n0 >> 1) + n;
+            if (o < half_n) ((float*)out)[(size_t)m * half_n + o] = gated_product(v, up, act);
+        } else {
+            epilogue_store<float>(out, mode, M, N, m, n0 + n, v, act);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// More tokens: BM x 128 output tiles, 2 BM threads with 8 x 8 outputs each, K in steps of 16 through two shared buffers
+// (the next step's numbers travel to registers while this one's are multiplied).  Bound by the FMA pipe.  Where the
+// tiles alone leave SMs idle, a cluster of up to 8 blocks shares K; each block then adds up a slice of the tile's rows
+// over the blocks' shared memory, in rank order.  The 64 x 64 tile with 4 x 4 outputs a thread that this replaces read
+// shared memory twice as often per product.  639 tokens: x 11264 x 2048 1,307 -> 658 us (45 TFLOP/s of the pipe's 74),
+// x 2048 x 5632 1,172 -> 383 us; 2,000 tokens x 11264 x 2048 4,088 -> 2,030 us; 60 tokens x 2048 x 2048 257 -> 41 us.
+// In shared memory a row of 16 k is stored k-major; A's row index is XORed with k's upper bits (a warp's stores then
+// hit 32 banks), W's columns are kept as 64 "gate" columns (n mod 16 < 8) and their 64 "up" columns (n + 8), so that a
+// thread holds both of a gated pair.
+constexpr int FBN = 128, FBK = 16;
+
+template <int BM, bool WIDE>
+__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 1)
+linear_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, void* __restrict__ out,
+                       int M, int N, int K, int mode, act_t act) {
+    constexpr int THREADS = 2 * BM, A_LOADS = 2, W_LOADS = FBN * FBK / 4 / THREADS;
+    extern __shared__ __align__(16) float smem[];
+    float (*As)[FBK][BM] = (float (*)[FBK][BM])smem;
+    float (*Ws)[FBK][FBN] = (float (*)[FBK][FBN])(smem + 2 * FBK * BM);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = lane & 7, ty = lane >> 3, wn = warp & 1, wm = warp >> 1;
+    const int splits = gridDim.z, split = blockIdx.z;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * FBN;
+    const int steps = (K + FBK - 1) / FBK;
+    const int first = (int)((long long)steps * split / splits), last = (int)((long long)steps * (split + 1) / splits);
+
+    float4 a_next[A_LOADS], w_next[W_LOADS];
+    auto fetch = [&](int step) {
+        const int k = step * FBK + 4 * (tid & 3);
+#pragma unroll
+        for (int i = 0; i < A_LOADS; ++i) {
+            const int row = m0 + (tid + i * THREADS) / 4;
+            a_next[i] = load_four<WIDE>(A + (size_t)min(row, M - 1) * K, k, K, row < M);
+        }
+#pragma unroll
+        for (int i = 0; i < W_LOADS; ++i) {
+            const int row = n0 + (tid + i * THREADS) / 4;
+            w_next[i] = load_four<WIDE>(W + (size_t)min(row, N - 1) * K, k, K, row < N);
+        }
+    };
+    auto keep = [&](int buffer) {
+        const int kq = tid & 3;
+#pragma unroll
+        for (int i = 0; i < A_LOADS; ++i) {
+            const int row = ((tid + i * THREADS) / 4) ^ (kq << 3);
+            const float4 v = a_next[i];
+            As[buffer][4 * kq][row] = v.x; As[buffer][4 * kq + 1][row] = v.y;
+            As[buffer][4 * kq + 2][row] = v.z; As[buffer][4 * kq + 3][row] = v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < W_LOADS; ++i) {
+            const int row = (tid + i * THREADS) / 4;
+            const int at = (((row & 8) << 3) | ((row >> 4) << 3) | (row & 7)) ^ (kq << 3);
+            const float4 v = w_next[i];
+            Ws[buffer][4 * kq][at] = v.x; Ws[buffer][4 * kq + 1][at] = v.y;
+            Ws[buffer][4 * kq + 2][at] = v.z; Ws[buffer][4 * kq + 3][at] = v.w;
+        }
+    };
+    unsigned long long pairs[8][4] = {};                  // two neighbouring columns each: one instruction multiplies both
+    if (first < last) {
+        fetch(first);
+        keep(0);
+    }
+    __syncthreads();
+    for (int step = first; step < last; ++step) {
+        const int buffer = (step - first) & 1;
+        if (step + 1 < last) fetch(step + 1);
 #pragma unroll
         for (int k = 0; k < FBK; ++k) {
-            float a[4], w[4];
+            const int turn = (k >> 2) << 3;
+            float a[8];
+            *(float4*)a = *(const float4*)&As[buffer][k][(wm * 32 + ty * 4) ^ turn];
+            *(float4*)(a + 4) = *(const float4*)&As[buffer][k][(wm * 32 + 16 + ty * 4) ^ turn];
+            const ulonglong2 w_gate = *(const ulonglong2*)&Ws[buffer][k][(wn * 32 + tx * 4) ^ turn];
+            const ulonglong2 w_up = *(const ulonglong2*)&Ws[buffer][k][(64 + wn * 32 + tx * 4) ^ turn];
+            const unsigned long long w[4] = {w_gate.x, w_gate.y, w_up.x, w_up.y};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
+            for (int i = 0; i < 8; ++i) {
+                unsigned long long both;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(both) : "f"(a[i]));
 #pragma unroll
-            for (int c = 0; c < 4; ++c) w[c] = Ws[k][cols[c]];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(a[i], w[c], acc[i][c]);
+                for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(pairs[i][j]) : "l"(both), "l"(w[j]));
+            }
         }
+        if (step + 1 < last) keep(buffer ^ 1);
         __syncthreads();
     }
+    float acc[8][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (mode == MODE_GATED) {
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[i][2 * j]), "=f"(acc[i][2 * j + 1]) : "l"(pairs[i][j]));
+    // column n0 + column(j), column(j + 4) = column(j) + 8
+    const int column = ((wn * 32 + tx * 4) >> 3) * 16 + ((tx * 4) & 7);
+    const int half_n = N >> 1;
+    if (splits == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int m = m0 + wm * 32 + ty * 4 + (i & 3) + (i >> 2) * 16;
             if (m >= M) continue;
-            const int half_n = N >> 1;
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int n = n0 + cols[c];            // a gate row of W; its up row is n + 8
-                if (n >= N) continue;
-                const int o = ((n >> 4) << 3) + (n & 7);
-                if (o < half_n)
-                    ((float*)out)[(size_t)m * half_n + o] = gated_product(acc[i][c], acc[i][c + 2], act);
+            for (int j = 0; j < 4; ++j) {
+                const int n = n0 + column + j;
+                if (mode == MODE_GATED) {
+                    if (n < N) ((float*)out)[(size_t)m * half_n + (n >> 4) * 8 + (n & 7)] = gated_product(acc[i][j], acc[i][j + 4], act);
+                } else {
+                    epilogue_store<float>(out, mode, M, N, m, n, acc[i][j], act);
+                    epilogue_store<float>(out, mode, M, N, m, n + 8, acc[i][j + 4], act);
+                }
             }
-        } else {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) epilogue_store<float>(out, mode, M, N, m, n0 + cols[c], acc[i][c], act);
         }
+        return;
     }
+    // every block of the cluster leaves its sums in its own shared memory and adds up its share of the rows
+    float (*tile)[FBN] = (float (*)[FBN])smem;             // (the last step's barrier is behind us: the buffers are free)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = wm * 32 + ty * 4 + (i & 3) + (i >> 2) * 16;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tile[row][column + (j & 3) + (j >> 2) * 8] = acc[i][j];
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int rows_each = (BM + splits - 1) / splits;
+    const uint32_t here = smem_u32(smem);
+    for (int at = tid; at < rows_each * FBN; at += THREADS) {
+        const int row = split * rows_each + at / FBN, c = at % FBN, m = m0 + row, n = n0 + c;
+        if (row >= BM || m >= M || n >= N || (mode == MODE_GATED && (c & 8))) continue;
+        float v = 0.0f, up = 0.0f;
+        for (int rank = 0; rank < splits; ++rank) {
+            uint32_t there;
+            float part;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here + (row * FBN + c) * 4), "r"(rank));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part) : "r"(there));
+            v += part;
+            if (mode == MODE_GATED) {
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part) : "r"(there + 32));
+                up += part;
+            }
+        }
+        if (mode == MODE_GATED) ((float*)out)[(size_t)m * half_n + (n >> 4) * 8 + (n & 7)] = gated_product(v, up, act);
+        else epilogue_store<float>(out, mode, M, N, m, n, v, act);
+    }
+    __syncwarp();
+    // no block leaves while another still reads its sums
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 struct NormArgs { const float* row_scale; const float* partials_in; int n_partials_in, stride_in; float eps_in;
                   const int* rows; float* partials; int partial_stride; unsigned int* counter;
                   const float* gamma_next; float eps_next; void* scaled_out; float* row_scale_out; };
 
+template <bool WIDE, int MT>
+static int launch_few_of(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
+    const dim3 grid((N + 15) / 16);
+    constexpr int stages_of_part = 3 * MT * 128 * 4;
+    static const cudaError_t ready = [] {
+        const cudaError_t four = cudaFuncSetAttribute(linear_f32_few_kernel<MT, 4, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * stages_of_part);
+        const cudaError_t two = cudaFuncSetAttribute(linear_f32_few_kernel<MT, 2, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * stages_of_part);
+        return four != cudaSuccess ? four : two;
+    }();
+    if (ready != cudaSuccess) return fail("skv_linear(float)", cudaGetErrorString(ready));
+    // four parts of K where every block has an SM to itself (16 warps, most of its registers), else two
+    if ((int)grid.x <= sm_count())
+        return launch_pdl("skv_linear(float)", linear_f32_few_kernel<MT, 4, WIDE>, grid, dim3(512), 4 * stages_of_part, stream, (const float*)a, (const float*)w, out, M, N, K, mode, act);
+    return launch_pdl("skv_linear(float)", linear_f32_few_kernel<MT, 2, WIDE>, grid, dim3(256), 2 * stages_of_part, stream, (const float*)a, (const float*)w, out, M, N, K, mode, act);
+}
+
+template <bool WIDE>
+static int launch_few(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
+    if (M == 1) return launch_few_of<WIDE, 1>(a, w, out, M, N, K, mode, act, stream);
+    if (M == 2) return launch_few_of<WIDE, 2>(a, w, out, M, N, K, mode, act, stream);
+    if (M <= 4) return launch_few_of<WIDE, 4>(a, w, out, M, N, K, mode, act, stream);
+    if (M <= 8) return launch_few_of<WIDE, 8>(a, w, out, M, N, K, mode, act, stream);
+    return launch_few_of<WIDE, 16>(a, w, out, M, N, K, mode, act, stream);
+}
+
+template <int BM, bool WIDE>
+static int launch_tile_of(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
+    constexpr size_t buffers = (size_t)2 * FBK * (BM + FBN) * 4, tile = (size_t)BM * FBN * 4;
+    const size_t smem = buffers > tile ? buffers : tile;
+    static const cudaError_t ready = cudaFuncSetAttribute(linear_f32_tile_kernel<BM, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ready != cudaSuccess) return fail("skv_linear(float)", cudaGetErrorString(ready));
+    const int tiles = ((N + FBN - 1) / FBN) * ((M + BM - 1) / BM);
+    // K is shared by as many blocks as keep the fullest SM's share smallest: its blocks run one after the other as far as
+    // the FMA pipe goes, each for its part of K and about 200 k more to start and to add up.  A lone block leaves a third
+    // of the pipe idle.  639 x 2048 x 5632 is 80 tiles on 148 SMs: 605 us as
+    // two parts of K (160 blocks: some SMs have two), 383 us as five (400 blocks: three on the fullest).
+    int splits = 1;
+    float best = 0.0f;
+    for (int s = 1; s <= 8 && (s == 1 || K >= 128 * s); ++s) {
+        const int rounds = (tiles * s + sm_count() - 1) / sm_count();
+        const float cost = (float)rounds * ((float)K / s + (s > 1 ? 200.0f : 100.0f)) * (rounds * BM < 256 ? 1.4f : 1.0f);
+        if (s == 1 || cost < best) { best = cost; splits = s; }
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((N + FBN - 1) / FBN, (M + BM - 1) / BM, splits);
+    config.blockDim = dim3(2 * BM);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = 1;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = splits;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t status = cudaLaunchKernelEx(&config, linear_f32_tile_kernel<BM, WIDE>, (const float*)a, (const float*)w, out, M, N, K, mode, act);
+    if (status != cudaSuccess) return fail("skv_linear(float)", cudaGetErrorString(status));
+    return 0;
+}
+
+template <bool WIDE>
+static int launch_tile(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
+    if (M <= 32) return launch_tile_of<32, WIDE>(a, w, out, M, N, K, mode, act, stream);
+    if (M <= 64 || (M + 63) / 64 % 2 == 1 && M <= 320) return launch_tile_of<64, WIDE>(a, w, out, M, N, K, mode, act, stream);
+    return launch_tile_of<128, WIDE>(a, w, out, M, N, K, mode, act, stream);
+}
+
 static int launch_linear(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act,
                          int* flag, const NormArgs& norm, cudaStream_t stream) {
     (void)flag;
     if (norm.row_scale || norm.partials_in || norm.partials) return fail("skv_linear(float)", "the norm-fused form exists in the bfloat16 build only");
-    dim3 grid((N + FBN - 1) / FBN, (M + FBM - 1) / FBM);
-    return launch_pdl("skv_linear(float)", linear_f32_kernel, grid, dim3(256), 0, stream, (const float*)a,
-                      (const float*)w, out, M, N, K, mode, act);
+    const bool wide = K % 4 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15);
+    if (M <= FEW_MAX)
+        return wide ? launch_few<true>(a, w, out, M, N, K, mode, act, stream) : launch_few<false>(a, w, out, M, N, K, mode, act, stream);
+    return wide ? launch_tile<true>(a, w, out, M, N, K, mode, act, stream) : launch_tile<false>(a, w, out, M, N, K, mode, act, stream);
 }
 
 #else  // bfloat16
