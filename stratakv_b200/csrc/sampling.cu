@@ -286,6 +286,165 @@ __device__ unsigned long long radix_select(const float* __restrict__ row, const 
     return prefix;
 }
 
+// A top-k of at most FEW_K: the row is walked twice and the rest happens on a short list.
+// The k-th largest of the threads' own maxima is a bound below which none of the k largest logits can lie (k threads
+// hold one that is not below it), so the second walk writes down what reaches the bound: about 43 elements for k = 40,
+// 253 for k = 200.  Their order, the top-p cut and the draw come from counting: a thread per element counts the keys
+// above its own.  The masses, the cuts and the drawn number are those of the general path, integer for integer.
+// Bound by the two walks (the row comes from L2 or HBM once each, 16 bytes a load, no division but for what reaches
+// the bound).  64 rows of 128,256 logits with k = 40, p = 0.95: the general path's fourteen passes took 389 us.
+// Returns false where the list would not hold the candidates (more than SAMPLE_THREADS equal values at the bound) or
+// where the quotients lie so near zero that they lose bits (then the bound on x says nothing about x / temperature).
+constexpr int FEW_K = 256;
+
+__device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out, int vocab, float temperature, int top_k, float top_p,
+                           unsigned long long seed, uint32_t stream, uint32_t counter, int* __restrict__ flag, unsigned char* smem) {
+    float* maxima = (float*)smem;                                                          // [threads]
+    unsigned long long* keys = (unsigned long long*)(smem + SAMPLE_THREADS * 4);            // [threads], in list order
+    unsigned long long* sorted = keys + SAMPLE_THREADS;                                     // [threads], largest first
+    unsigned long long* masses = sorted + SAMPLE_THREADS;                                   // [threads], largest key first
+    unsigned long long* drawn = masses + SAMPLE_THREADS;                                    // [FEW_K], by index
+    int* listed = (int*)(drawn + FEW_K);                                                    // [threads]
+    int* drawn_index = listed + SAMPLE_THREADS;                                             // [FEW_K]
+    __shared__ float bound, extent[2];                      // extent: the largest logit, and the largest magnitude
+    __shared__ int count, bad_row, kept;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) { count = 0; bad_row = 0; extent[0] = -INFINITY; extent[1] = 0.0f; }
+    const bool wide = ((uintptr_t)row & 15) == 0;
+    const int quads = wide ? vocab >> 2 : 0;
+    float most = -INFINITY, largest = 0.0f;
+    bool bad = false;
+    auto look = [&](float x) {
+        bad |= !isfinite(x);
+        most = fmaxf(most, x);
+        largest = fmaxf(largest, fabsf(x));
+    };
+    for (int q0 = tid; q0 < quads; q0 += 4 * SAMPLE_THREADS) {
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            x[u] = q0 + u * SAMPLE_THREADS < quads ? ((const float4*)row)[q0 + u * SAMPLE_THREADS] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (q0 + u * SAMPLE_THREADS < quads) { look(x[u].x); look(x[u].y); look(x[u].z); look(x[u].w); }
+    }
+    for (int i = 4 * quads + tid; i < vocab; i += SAMPLE_THREADS) look(row[i]);
+    maxima[tid] = most;
+    __syncthreads();
+    if (bad) bad_row = 1;
+    const float warp_largest = warp_max(largest);
+    if (lane == 0) atomicMax((unsigned int*)&extent[1], __float_as_uint(warp_largest));     // (not negative: ordered as integers)
+    // the k-th largest of the maxima
+    int above = 0, not_below = 0;
+    for (int i = 0; i < SAMPLE_THREADS; i += 4) {
+        const float4 o = *(const float4*)(maxima + i);
+        above += (o.x > most) + (o.y > most) + (o.z > most) + (o.w > most);
+        not_below += (o.x >= most) + (o.y >= most) + (o.z >= most) + (o.w >= most);
+    }
+    if (above < top_k && not_below >= top_k) bound = most;                                  // (all who write write the same)
+    if (above == 0) extent[0] = most;
+    __syncthreads();
+    if (bad_row || !isfinite(extent[1] / temperature)) {
+        if (tid == 0) { if (flag) atomicOr(flag, 2); *out = 0; }
+        return true;
+    }
+    const float max_value = extent[0] / temperature, x_bound = bound, v_bound = x_bound / temperature;
+    if (fabsf(v_bound) < 1e-30f) return false;
+    const float x_low = x_bound - fabsf(x_bound) * 9.5367431640625e-7f;                     // (2^-20: 16 roundings of a quotient)
+    auto collect = [&](float x, int i) {
+        if (x >= x_low && x / temperature >= v_bound) {
+            const int at = atomicAdd(&count, 1);
+            if (at < SAMPLE_THREADS) listed[at] = i;
+        }
+    };
+    for (int q0 = tid; q0 < quads; q0 += 4 * SAMPLE_THREADS) {
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            x[u] = q0 + u * SAMPLE_THREADS < quads ? ((const float4*)row)[q0 + u * SAMPLE_THREADS] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = 4 * (q0 + u * SAMPLE_THREADS);
+            if (i >= 4 * quads || fmaxf(fmaxf(x[u].x, x[u].y), fmaxf(x[u].z, x[u].w)) < x_low) continue;
+            collect(x[u].x, i); collect(x[u].y, i + 1); collect(x[u].z, i + 2); collect(x[u].w, i + 3);
+        }
+    }
+    for (int i = 4 * quads + tid; i < vocab; i += SAMPLE_THREADS) collect(row[i], i);
+    __syncthreads();
+    const int n = count;
+    if (n > SAMPLE_THREADS) return false;
+    unsigned long long key = 0ull, mass = 0ull;
+    if (tid < n) {
+        const int i = listed[tid];
+        const float v = row[i] / temperature;
+        key = sort_key(v, i);
+        mass = fixed_mass(v, max_value);
+        keys[tid] = key;
+    }
+    __syncthreads();
+    int rank = 0;
+    for (int i = 0; i < n; ++i) rank += keys[i] > key;
+    if (tid < n) { sorted[rank] = key; masses[rank] = mass; }
+    __syncthreads();
+    // the top-p cut: lane l of the first warp walks ranks 8l to 8l + 7
+    if (tid < 32) {
+        unsigned long long own = 0ull;
+#pragma unroll
+        for (int j = 0; j < FEW_K / 32; ++j) own += 8 * lane + j < top_k ? masses[8 * lane + j] : 0ull;
+        const unsigned long long total = warp_sum_u64(own);
+        unsigned long long upto = own;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const unsigned long long before = __shfl_up_sync(0xffffffffu, upto, offset);
+            if (lane >= offset) upto += before;
+        }
+        unsigned long long target = (unsigned long long)((double)top_p * (double)total);
+        if (target < 1ull) target = 1ull;
+        if (lane == 0) kept = top_k;
+        __syncwarp();
+        if (top_p < 1.0f && upto >= target && upto - own < target) {
+            unsigned long long run = upto - own;
+            for (int j = 0; j < FEW_K / 32; ++j) {
+                run += 8 * lane + j < top_k ? masses[8 * lane + j] : 0ull;
+                if (run >= target) { kept = 8 * lane + j + 1; break; }
+            }
+        }
+    }
+    __syncthreads();
+    // the survivors by index, and the draw
+    const int survivors = kept;
+    if (tid < n && rank < survivors) {
+        const uint32_t own = (uint32_t)key;                                                 // (the index, complemented)
+        int place = 0;
+        for (int i = 0; i < survivors; ++i) place += (uint32_t)sorted[i] > own;
+        drawn[place] = mass;
+        drawn_index[place] = (int)(0xFFFFFFFFu - own);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        unsigned long long own = 0ull;
+#pragma unroll
+        for (int j = 0; j < FEW_K / 32; ++j) own += 8 * lane + j < survivors ? drawn[8 * lane + j] : 0ull;
+        const unsigned long long total = warp_sum_u64(own);
+        unsigned long long upto = own;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const unsigned long long before = __shfl_up_sync(0xffffffffu, upto, offset);
+            if (lane >= offset) upto += before;
+        }
+        const uint32_t r = philox_first_word(seed, stream, counter);
+        const unsigned long long target = __umul64hi(total, (unsigned long long)r << 32);   // in [0, total)
+        if (upto > target && upto - own <= target) {
+            unsigned long long run = upto - own;
+            for (int j = 0; j < FEW_K / 32; ++j) {
+                run += 8 * lane + j < survivors ? drawn[8 * lane + j] : 0ull;
+                if (target < run) { *out = drawn_index[8 * lane + j]; break; }
+            }
+        }
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab, float temperature, int top_k,
               float top_p, unsigned long long seed, const int* __restrict__ streams,
@@ -307,6 +466,10 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     pdl_wait();
     const float* row = logits + (size_t)blockIdx.x * vocab;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (top_k > 0 && top_k < vocab && top_k <= FEW_K &&
+        sample_few(row, out + blockIdx.x, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[blockIdx.x],
+                   (uint32_t)counters[blockIdx.x], flag, sample_smem))
+        return;
     if (threadIdx.x == 0) bad_flag = 0;
     __syncthreads();
 

@@ -102,3 +102,48 @@ def test_long_rows_and_ties_take_the_other_paths_of_the_kernel():
     short = logits[:32000].copy()
     short[[7, 31000, 31999]] = [3.0, 2.5, 2.0]
     assert set(draw(short, 3000, 1.0, 3, 1.0)) == {7, 31000, 31999}
+
+
+@pytest.mark.parametrize("vocab,top_k,top_p", [(2, 1, 1.0), (37, 36, 0.9), (513, 40, 1.0), (32000, 40, 0.95), (32001, 200, 0.9), (50257, 256, 0.5),
+                                               (128256, 20, 0.95)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_a_short_list_draws_what_the_whole_row_draws(vocab, top_k, top_p, ties):
+    """A small top-k is chosen from a short list; a row whose other logits are sunk to where they weigh 2^-40 of the largest
+    goes through every element of the row and must give the same tokens.  With ties more values equal the bound than the
+    list holds in the long rows, and the lower indices win."""
+    rng = np.random.default_rng(vocab + top_k)
+    rows = 24
+    logits = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
+    if ties:
+        logits = np.round(logits)
+    order = np.argsort(-logits, axis=1, kind="stable")
+    sunk = np.full_like(logits, -1e4)
+    kept = []
+    for r in range(rows):
+        probabilities = plain_llama.sample_reference(logits[r], 0.8, top_k, 1.0)
+        cumulative = np.cumsum(probabilities[order[r]])
+        if top_p < 1.0 and np.abs(cumulative - top_p).min() < 1e-5:
+            continue                                       # the cut falls within rounding: either side is right
+        count = min(top_k, int(np.searchsorted(cumulative, top_p)) + 1) if top_p < 1.0 else top_k
+        sunk[r, order[r, :count]] = logits[r, order[r, :count]]
+        kept.append(r)
+    k, outs = kernels(), []
+    streams = torch.arange(rows, dtype=torch.int32, device="cuda")
+    for values, limit, mass in ((logits, top_k, top_p), (sunk, 0, 1.0)):
+        out = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+        k.sample(torch.tensor(values, device="cuda"), out, 0.8, limit, mass, 5, streams, streams)
+        outs.append(out.cpu().numpy())
+    # (a drawn number falls within the 2^-40 x vocab of the sunk logits about once in 10^7 rows)
+    assert kept and (outs[0][kept] == outs[1][kept]).all()
+
+
+def test_a_short_list_flags_what_is_not_finite():
+    k = kernels()
+    for bad in (float("nan"), float("inf"), float("-inf"), 3e38):
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        logits = torch.zeros(2, 1001, device="cuda")
+        logits[1, 777] = bad
+        out = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+        zeros = torch.zeros(2, dtype=torch.int32, device="cuda")
+        k.sample(logits, out, 0.5, 40, 0.9, 0, zeros, zeros, flag)      # (3e38 / 0.5 overflows)
+        assert int(flag) == 2 and int(out[1]) == 0
