@@ -284,6 +284,310 @@ static int launch_token_side(float* x, const int* ids, const void* table, int ta
                       norm_w, eps, next_gamma, next_eps, (skv_t*)next_out, n_tokens, hidden, branch, post_gamma, post_eps);
 }
 
+#if SKV_DTYPE == SKV_BF16
+// The token input on tensor cores.  Both products are small (dim x hidden and back) but every token needs all of both
+// weights, which is what bounds them: a cluster takes 16 * MT tokens and shares the columns of the stream, eight warps
+// a block and COLS columns a warp, so the weights are read once per 16 or 32 tokens and a token's chain of loads is short.
+//   gate: a warp multiplies its own columns (its part of the inner size); sums over warps, then over the cluster;
+//   projection: a warp makes its own columns, which stay in registers while the mean of squares goes round.
+// The stream and the gated values are float32 and stay so: each is split into three bfloat16 whose sum is the float to
+// its last bit (24 of 24), against weights that are bfloat16 anyway, so the products are exact and the sums float.
+// Few tokens (MT 1): the smallest COLS whose cluster is at most 8 blocks, and the weights are asked into L2 ahead of the
+// wait.  Width 64 on 2,048 at 8 / 300 / 3,874 tokens: 20 / 79 / 187 us before, 10 / 32 / 65; on 4,096: 37 / 136 / 581, 14 / 33 / 137.
+constexpr int SIDE_WARPS = 8;
+
+__device__ __forceinline__ void side_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Three bfloat16 that add up to each of two floats, as pairs.
+__device__ __forceinline__ void split_pair(float u, float v, uint32_t (&out)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 part = __floats2bfloat162_rn(u, v);
+        out[i] = *(const uint32_t*)&part;
+        const float2 back = __bfloat1622float2(part);
+        u -= back.x; v -= back.y;
+    }
+}
+
+__device__ __forceinline__ void side_cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float side_remote(const float* p, int rank) {
+    uint32_t there;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(there) : "memory");
+    return v;
+}
+
+template <int DIM, int COLS, int MT>
+__global__ void __launch_bounds__(SIDE_WARPS * 32)
+token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
+                      int table_stride, int offset, int vocab, const __nv_bfloat16* __restrict__ gate_w,
+                      const __nv_bfloat16* __restrict__ proj_t, const float* __restrict__ norm_w, float eps,
+                      const float* __restrict__ next_gamma, float next_eps, __nv_bfloat16* __restrict__ next_out,
+                      int n_tokens, int hidden, int ranks) {
+    constexpr int R = 16 * MT, CW = COLS < 64 ? COLS : 64, CHUNKS = COLS / CW, TILES = CW / 8, PITCH = DIM + 8;
+    extern __shared__ __align__(16) float side_smem[];
+    float* part = side_smem;                                          // [warps][R][DIM]
+    float* own = part + SIDE_WARPS * R * DIM;                         // [R][DIM], read by the cluster
+    float* squares = own + R * DIM;                                   // [warps][R]
+    float* own_squares = squares + SIDE_WARPS * R;                    // [2][R], read by the cluster
+    float* factor = own_squares + 2 * R;                              // [R]
+    __nv_bfloat16* gated = (__nv_bfloat16*)(factor + R);              // [3][R][PITCH]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * R;
+    const int block_col = rank * SIDE_WARPS * COLS, col0 = block_col + warp * COLS;
+    if (MT == 1) {
+        constexpr int LINES = SIDE_WARPS * COLS * 2 / 128;             // 128-byte lines of a weight row in this block's columns
+        for (int i = tid; i < 2 * DIM * LINES; i += SIDE_WARPS * 32) {
+            const int c = block_col + (i % LINES) * 64, row = (i / LINES) % DIM;
+            const __nv_bfloat16* at = (i < DIM * LINES ? gate_w : proj_t) + (size_t)row * hidden + c;
+            if (c < hidden) asm volatile("prefetch.global.L2 [%0];" :: "l"(at));
+        }
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    const float* rows[MT][2];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) rows[m][h] = x + (size_t)min(t0 + 16 * m + 8 * h + g, n_tokens - 1) * hidden;
+
+    // gate_w . x over this warp's columns: 32 at a time, eight neighbours a lane (the order of k inside the two products
+    // of 16 is the same for both operands)
+    {
+        float acc[MT][DIM / 8][4] = {};
+#pragma unroll (MT == 1 ? 2 : 1)
+        for (int c = 0; c < COLS; c += 32) {
+            const int k = col0 + c + 8 * t;
+            if (col0 + c >= hidden) break;
+            uint4 w[DIM / 8];
+#pragma unroll
+            for (int n = 0; n < DIM / 8; ++n) w[n] = *(const uint4*)(gate_w + (size_t)(8 * n + g) * hidden + k);
+            uint32_t a[3][MT][2][4];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 u = *(const float4*)(rows[m][h] + k), v = *(const float4*)(rows[m][h] + k + 4);
+                    uint32_t p[4][3];
+                    split_pair(u.x, u.y, p[0]); split_pair(u.z, u.w, p[1]);
+                    split_pair(v.x, v.y, p[2]); split_pair(v.z, v.w, p[3]);
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) {
+                        a[s][m][0][h] = p[0][s]; a[s][m][0][2 + h] = p[1][s];
+                        a[s][m][1][h] = p[2][s]; a[s][m][1][2 + h] = p[3][s];
+                    }
+                }
+#pragma unroll
+            for (int n = 0; n < DIM / 8; ++n)
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int s = 2; s >= 0; --s) {
+                        side_mma(acc[m][n], a[s][m][0], w[n].x, w[n].y);
+                        side_mma(acc[m][n], a[s][m][1], w[n].z, w[n].w);
+                    }
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < DIM / 8; ++n) {
+                float* at = part + ((size_t)warp * R + 16 * m + g) * DIM + 8 * n + 2 * t;
+                *(float2*)at = make_float2(acc[m][n][0], acc[m][n][1]);
+                *(float2*)(at + 8 * DIM) = make_float2(acc[m][n][2], acc[m][n][3]);
+            }
+    }
+    __syncthreads();
+    for (int i = tid; i < R * DIM; i += SIDE_WARPS * 32) {
+        float sum = part[i];
+#pragma unroll
+        for (int w = 1; w < SIDE_WARPS; ++w) sum += part[w * R * DIM + i];
+        own[i] = sum;
+    }
+    side_cluster_sync();
+    for (int i = tid; i < R * DIM; i += SIDE_WARPS * 32) {
+        const int row = i / DIM, j = i % DIM;
+        const int id = ids[min(t0 + row, n_tokens - 1)];
+        const bool known = id >= 0 && id < vocab;                     // (the embedding has flagged an id outside the table)
+        const float e = known ? __bfloat162float(table[(size_t)id * table_stride + offset + j]) : 0.0f;
+        float sum = 0.0f;
+        for (int r = 0; r < ranks; ++r) sum += side_remote(own + i, r);
+        float v = known ? gelu_tanh(sum) * e : 0.0f;
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            const __nv_bfloat16 b = __float2bfloat16_rn(v);
+            gated[(s * R + row) * PITCH + j] = b;
+            v -= __bfloat162float(b);
+        }
+    }
+    __syncthreads();
+
+    // proj . gated for this warp's columns: column n of tile j is TILES * n + j of a chunk of CW, so that a lane's loads
+    // of the four rows it needs and its results lie side by side
+    float y[CHUNKS][MT][TILES][4] = {};
+    float sums[MT][2] = {};
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+        if (col0 + c * CW >= hidden) continue;
+#pragma unroll
+        for (int k = 0; k < DIM; k += 16) {
+            uint32_t w[4][TILES / 2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat16* at = proj_t + (size_t)(k + 2 * t + (i & 1) + 8 * (i >> 1)) * hidden + col0 + c * CW + TILES * g;
+                if (TILES == 8) { const uint4 v = *(const uint4*)at; w[i][0] = v.x; w[i][1] = v.y; w[i][TILES / 2 - 2] = v.z; w[i][TILES / 2 - 1] = v.w; }
+                else { const uint2 v = *(const uint2*)at; w[i][0] = v.x; w[i][1] = v.y; }
+            }
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int s = 2; s >= 0; --s) {
+                    const __nv_bfloat16* at = gated + (s * R + 16 * m + g) * PITCH + k + 2 * t;
+                    const uint32_t a[4] = {*(const uint32_t*)at, *(const uint32_t*)(at + 8 * PITCH), *(const uint32_t*)(at + 8),
+                                           *(const uint32_t*)(at + 8 * PITCH + 8)};
+#pragma unroll
+                    for (int j = 0; j < TILES; ++j) {
+                        const uint32_t pick = j & 1 ? 0x7632 : 0x5410;
+                        side_mma(y[c][m][j], a, __byte_perm(w[0][j >> 1], w[1][j >> 1], pick), __byte_perm(w[2][j >> 1], w[3][j >> 1], pick));
+                    }
+                }
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int j = 0; j < TILES; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    sums[m][h] += y[c][m][j][2 * h] * y[c][m][j][2 * h] + y[c][m][j][2 * h + 1] * y[c][m][j][2 * h + 1];
+    }
+    // the rows' factor 1 / sqrt(mean of squares + eps) from this lane's sums: over the quad, the warps, the cluster
+    auto make_factor = [&](int which, float eps_of) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float v = sums[m][h];
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (t == 0) squares[warp * R + 16 * m + 8 * h + g] = v;
+            }
+        __syncthreads();
+        if (tid < R) {
+            float v = 0.0f;
+            for (int w = 0; w < SIDE_WARPS; ++w) v += squares[w * R + tid];
+            own_squares[which * R + tid] = v;
+        }
+        side_cluster_sync();
+        if (tid < R) {
+            float v = 0.0f;
+            for (int r = 0; r < ranks; ++r) v += side_remote(own_squares + which * R + tid, r);
+            factor[tid] = 1.0f / sqrtf(v / (float)hidden + eps_of);
+        }
+        __syncthreads();
+    };
+    make_factor(0, eps);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = 16 * m + 8 * h + g;
+            const float inverse = factor[row];
+            sums[m][h] = 0.0f;
+            if (t0 + row >= n_tokens) continue;
+#pragma unroll
+            for (int c = 0; c < CHUNKS; ++c) {
+                if (col0 + c * CW >= hidden) continue;
+                const int col = col0 + c * CW + 2 * TILES * t;
+                float* at = x + (size_t)(t0 + row) * hidden + col;
+#pragma unroll
+                for (int i = 0; i < 2 * TILES; i += 4) {
+                    float4 v = *(const float4*)(at + i);
+                    const float4 n = *(const float4*)(norm_w + col + i);
+                    const int half = i / TILES, j = i % TILES;
+                    v.x += y[c][m][j][2 * h + half] * inverse * n.x; v.y += y[c][m][j + 1][2 * h + half] * inverse * n.y;
+                    v.z += y[c][m][j + 2][2 * h + half] * inverse * n.z; v.w += y[c][m][j + 3][2 * h + half] * inverse * n.w;
+                    *(float4*)(at + i) = v;
+                    y[c][m][j][2 * h + half] = v.x; y[c][m][j + 1][2 * h + half] = v.y;
+                    y[c][m][j + 2][2 * h + half] = v.z; y[c][m][j + 3][2 * h + half] = v.w;
+                    sums[m][h] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                }
+            }
+        }
+    if (next_out) {
+        __syncthreads();                                              // (the factors have been read)
+        make_factor(1, next_eps);
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = 16 * m + 8 * h + g;
+                if (t0 + row >= n_tokens) continue;
+                const float inverse = factor[row];
+#pragma unroll
+                for (int c = 0; c < CHUNKS; ++c) {
+                    if (col0 + c * CW >= hidden) continue;
+                    const int col = col0 + c * CW + 2 * TILES * t;
+                    __nv_bfloat16* at = next_out + (size_t)(t0 + row) * hidden + col;
+#pragma unroll
+                    for (int i = 0; i < 2 * TILES; i += 8) {
+                        uint32_t packed[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int e = i + 2 * q, half = e / TILES, j = e % TILES;
+                            const float2 n = *(const float2*)(next_gamma + col + e);
+                            const __nv_bfloat162 v = __floats2bfloat162_rn(y[c][m][j][2 * h + half] * inverse * n.x,
+                                                                           y[c][m][j + 1][2 * h + half] * inverse * n.y);
+                            packed[q] = *(const uint32_t*)&v;
+                        }
+                        *(uint4*)(at + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    }
+                }
+            }
+    }
+    side_cluster_sync();                                              // no block leaves while another reads its sums
+}
+
+template <int DIM, int COLS, int MT>
+static int launch_token_side_mma(float* x, const int* ids, const void* table, int table_stride, int offset, int vocab,
+                                 const void* gate_w, const void* proj_t, const float* norm_w, float eps,
+                                 const float* next_gamma, float next_eps, void* next_out, int n_tokens, int hidden,
+                                 cudaStream_t stream) {
+    constexpr int R = 16 * MT;
+    constexpr size_t smem = (size_t)((SIDE_WARPS + 1) * R * DIM + (SIDE_WARPS + 3) * R) * 4 + (size_t)3 * R * (DIM + 8) * 2;
+    auto kernel = token_side_mma_kernel<DIM, COLS, MT>;
+    static const cudaError_t ready = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ready != cudaSuccess) return fail("skv_token_side", cudaGetErrorString(ready));
+    const int ranks = (hidden + SIDE_WARPS * COLS - 1) / (SIDE_WARPS * COLS);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)(ranks * ((n_tokens + R - 1) / R)));
+    config.blockDim = dim3(SIDE_WARPS * 32);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = ranks;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t status = cudaLaunchKernelEx(&config, kernel, x, ids, (const __nv_bfloat16*)table, table_stride, offset, vocab,
+                                                  (const __nv_bfloat16*)gate_w, (const __nv_bfloat16*)proj_t, norm_w, eps, next_gamma,
+                                                  next_eps, (__nv_bfloat16*)next_out, n_tokens, hidden, ranks);
+    if (status != cudaSuccess) return fail("skv_token_side", cudaGetErrorString(status));
+    return 0;
+}
+#endif
+
 }  // namespace skv
 
 using namespace skv;
@@ -323,6 +627,20 @@ SKV_EXPORT int skv_token_side(float* x, const int* ids, const void* table, int t
         return fail("skv_token_side", "the next norm needs its weight and a place for its result");
     if ((size_t)(((dim + 3) & ~3) + hidden) * sizeof(float) > 200 * 1024)
         return fail("skv_token_side", "the stream is too wide for one block's shared memory");
+#if SKV_DTYPE == SKV_BF16
+    // the tensor-core form: a gated width it is built for, columns in whole chunks of 64 for at most 8 blocks a cluster,
+    // 16-byte rows, nothing to add first
+    if (!branch && (dim == 16 || dim == 32 || dim == 64) && hidden % 64 == 0 && hidden <= 8 * SIDE_WARPS * 128 &&
+        (((uintptr_t)x | (uintptr_t)gate_w | (uintptr_t)proj_t | (uintptr_t)norm_w | (uintptr_t)next_gamma | (uintptr_t)next_out) & 15) == 0) {
+#define SKV_SIDE_MMA(DIM, COLS, MT) launch_token_side_mma<DIM, COLS, MT>(x, ids, table, table_stride, offset, vocab, gate_w, proj_t, norm_w, \
+                                                                       eps, next_gamma, next_eps, next_out, n_tokens, hidden, stream)
+#define SKV_SIDE_DIM(DIM) (n_tokens > 256 ? SKV_SIDE_MMA(DIM, 128, 2) : hidden <= 8 * SIDE_WARPS * 32 ? SKV_SIDE_MMA(DIM, 32, 1) : \
+                           hidden <= 8 * SIDE_WARPS * 64 ? SKV_SIDE_MMA(DIM, 64, 1) : SKV_SIDE_MMA(DIM, 128, 1))
+        return dim == 64 ? SKV_SIDE_DIM(64) : dim == 32 ? SKV_SIDE_DIM(32) : SKV_SIDE_DIM(16);
+#undef SKV_SIDE_DIM
+#undef SKV_SIDE_MMA
+    }
+#endif
     const bool vec = hidden % 4 == 0 && (((uintptr_t)x | (uintptr_t)gate_w) & 15) == 0 && sizeof(skv_t) * hidden % 8 == 0;
     // eight tokens a block where their projected rows fit its shared memory, else four, else one; one token a block
     // where tokens are few, so that the step has blocks enough
