@@ -28,8 +28,7 @@
 namespace skv {
 
 constexpr int GEN_WARPS = 4;
-constexpr int GEN_MAX_VDIM = 512;
-constexpr int GEN_MERGE_ACC = GEN_MAX_VDIM / 32;   // what a lane of the merge keeps of a row of values                 // a lane keeps vdim / 32 accumulators: 8 up to 256, else 16
+constexpr int GEN_MAX_VDIM = 512;             // a lane keeps vdim / 32 accumulators: 8 up to 256, else 16
 
 constexpr int FINISH_WARPS = 8;
 
@@ -314,65 +313,227 @@ attention_general_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
         for (int c = num_heads * vdim + lane; c < out_stride; c += 32) out[(size_t)t * out_stride + c] = from_float<T>(0.0f);
 }
 
-// The parts of a (token, head) that attention_general_kernel left with splits > 1, put together: the largest maximum,
-// the sums and outputs brought to it, the sink, the gate.  A warp per (token, head).
+// The parts of a (token, head) that attention_general_kernel or latent_attention_kernel left with splits > 1, put together:
+// the largest maximum, the sums and outputs brought to it, the sink, the gate.  A block per (token, head): the first warp
+// makes the parts' weights, then a thread adds up its numbers of the parts with four loads on their way.  (A warp per
+// (token, head) that walked the parts one after the other took 20 us for 256 of them over 16 parts of 256 numbers,
+// with this one and the kernel below a decode step of 8 sequences over 780 cached rows takes 15 us in place of 69.)
+constexpr int MERGE_THREADS = 128, MERGE_MAX_SPLITS = 1024;
 template <typename T>
-__global__ void __launch_bounds__(GEN_WARPS * 32)
+__global__ void __launch_bounds__(MERGE_THREADS)
 attention_general_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
                                T* __restrict__ out, int n_tokens, int num_heads, int vdim, int splits,
                                const float* __restrict__ gate, int gate_stride, int out_stride, int gate_per_element,
                                const float* __restrict__ sink) {
+    __shared__ float weights[MERGE_MAX_SPLITS];
     pdl_launch_dependents();
     pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * GEN_WARPS + warp;
-    if (item >= (long long)n_tokens * num_heads) return;
+    const long long item = blockIdx.x;
     const int t = (int)(item / num_heads), head = (int)(item % num_heads);
-    const float* ml = partial_ml + (size_t)item * splits * 2;
-    // lane s (and s + 32, ...) holds part s's maximum and sum; the weights exp(max_s - top) are made once
-    float top = -INFINITY;
-    for (int s = lane; s < splits; s += 32) top = fmaxf(top, ml[2 * s]);      // (the first part always has the first key)
-    top = warp_max(top);
-    float total = 0.0f;
-    for (int s = lane; s < splits; s += 32) total += ml[2 * s] == -INFINITY ? 0.0f : ml[2 * s + 1] * expf(ml[2 * s] - top);
-    total = warp_sum(total);
-    if (sink) total += expf(sink[head] - top);
-    float factor = 1.0f / total;
-    if (gate && !gate_per_element) factor *= 1.0f / (1.0f + expf(-gate[(size_t)t * gate_stride + head]));
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const float* ml = partial_ml + (size_t)item * splits * 2;
+        float top = -INFINITY;
+        for (int s = lane; s < splits; s += 32) top = fmaxf(top, ml[2 * s]);      // (the first part always has the first key)
+        top = warp_max(top);
+        float total = 0.0f;
+        for (int s = lane; s < splits; s += 32) {
+            const float m = ml[2 * s], w = m == -INFINITY ? 0.0f : expf(m - top);
+            weights[s] = w;
+            if (w != 0.0f) total += ml[2 * s + 1] * w;
+        }
+        total = warp_sum(total);
+        if (sink) total += expf(sink[head] - top);
+        float factor = 1.0f / total;
+        if (gate && !gate_per_element) factor *= 1.0f / (1.0f + expf(-gate[(size_t)t * gate_stride + head]));
+        for (int s = lane; s < splits; s += 32) weights[s] *= factor;
+    }
+    __syncthreads();
     const float* gate_row = gate && gate_per_element ? gate + (size_t)t * gate_stride + (size_t)head * vdim : nullptr;
     T* out_row = out + (size_t)t * out_stride + (size_t)head * vdim;
     const float* o_parts = partial_o + (size_t)item * splits * vdim;
-    float value[GEN_MERGE_ACC];
+    for (int d = threadIdx.x; d < vdim; d += MERGE_THREADS) {
+        float value = 0.0f;
+        for (int s0 = 0; s0 < splits; s0 += 4) {
+            float part[4], w[4];
 #pragma unroll
-    for (int i = 0; i < GEN_MERGE_ACC; ++i) value[i] = 0.0f;
-    for (int s0 = 0; s0 < splits; s0 += 32) {
-        const int mine = s0 + lane;
-        const float m = mine < splits ? ml[2 * mine] : -INFINITY;
-        const float weight = m == -INFINITY ? 0.0f : expf(m - top) * factor;
-        const int count = min(32, splits - s0);
-        for (int j = 0; j < count; ++j) {
-            const float w = __shfl_sync(0xffffffffu, weight, j);
-            if (w == 0.0f) continue;                                   // (a part without keys left nothing to read)
-            const float* part = o_parts + (size_t)(s0 + j) * vdim;
-#pragma unroll
-            for (int i = 0; i < GEN_MERGE_ACC; ++i) {
-                const int d = lane + 32 * i;
-                if (d < vdim) value[i] = fmaf(part[d], w, value[i]);
+            for (int u = 0; u < 4; ++u) {                              // (a part without keys left nothing to read)
+                w[u] = s0 + u < splits ? weights[s0 + u] : 0.0f;
+                part[u] = w[u] != 0.0f ? o_parts[(size_t)(s0 + u) * vdim + d] : 0.0f;
             }
-        }
-    }
 #pragma unroll
-    for (int i = 0; i < GEN_MERGE_ACC; ++i) {
-        const int d = lane + 32 * i;
-        if (d < vdim) {
-            float v = value[i];
-            if (gate_row) v *= 1.0f / (1.0f + expf(-gate_row[d]));
-            out_row[d] = from_float<T>(v);
+            for (int u = 0; u < 4; ++u) value = fmaf(part[u], w[u], value);
         }
+        if (gate_row) value *= 1.0f / (1.0f + expf(-gate_row[d]));
+        out_row[d] = from_float<T>(value);
     }
     if (head == num_heads - 1)
-        for (int c = num_heads * vdim + lane; c < out_stride; c += 32) out[(size_t)t * out_stride + c] = from_float<T>(0.0f);
+        for (int c = num_heads * vdim + threadIdx.x; c < out_stride; c += MERGE_THREADS) out[(size_t)t * out_stride + c] = from_float<T>(0.0f);
 }
+
+#if SKV_DTYPE == SKV_BF16
+// Part of the keys of one token for 32 of its query heads on tensor cores, where all heads share one cached row of `dim`
+// numbers whose first `vdim` are the value (a latent with a rotated part behind it).  Tiles of 64 keys go through shared
+// memory once for all heads (cp.async, two stages); eight warps make the scores (16 heads x 16 keys each), then four rows
+// of the softmax each, then 16 heads x 64 numbers of the output each.  Scores, softmax and sums are float; a probability
+// is split into three bfloat16 that add up to it, against values that are bfloat16 anyway, so nothing is rounded that
+// attention_general_kernel kept.  That kernel, a warp per (token, head, part), read every key once per head:
+// with its merge 8 sequences x 32 heads over 780 rows of 272
+// numbers took 69 us and take 15, 1 sequence over 8,000 rows 150 and 29, 64 over 500 187 and 29.
+constexpr int LAT_KEYS = 64, LAT_HEADS = 32, LAT_MAX_DIM = 320, LAT_MAX_VDIM = 256, LAT_S_PITCH = LAT_KEYS + 4, LAT_P_PITCH = LAT_KEYS + 8;
+
+__device__ __forceinline__ void lat_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void lat_ldmatrix(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void lat_ldmatrix_trans(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+
+__global__ void __launch_bounds__(256)
+latent_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
+                        int table_width, const int* __restrict__ positions, const int* __restrict__ token_seq, int num_heads, int dim,
+                        int vdim, int block_size, float scale, int splits, float* __restrict__ partial_o, float* __restrict__ partial_ml) {
+    extern __shared__ __align__(16) unsigned char lat_smem[];
+    const int pitch = dim + 8;                                          // rows 16 bytes apart modulo 128: eight of them hit all banks
+    __nv_bfloat16* qs = (__nv_bfloat16*)lat_smem;                       // [LAT_HEADS][pitch]
+    __nv_bfloat16* keys = qs + LAT_HEADS * pitch;                       // [2][LAT_KEYS][pitch]
+    __nv_bfloat16* probs = keys + 2 * LAT_KEYS * pitch;                 // [3][LAT_HEADS][LAT_P_PITCH]
+    float* scores = (float*)(probs + 3 * LAT_HEADS * LAT_P_PITCH);      // [LAT_HEADS][LAT_S_PITCH]
+    float* rescale = scores + LAT_HEADS * LAT_S_PITCH;                  // [LAT_HEADS]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x / splits, split = blockIdx.x % splits, head0 = blockIdx.y * LAT_HEADS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, quad = lane & 3;
+    const int count = positions[t] + 1, tiles = (count + LAT_KEYS - 1) / LAT_KEYS, per_split = (tiles + splits - 1) / splits;
+    const int first = split * per_split, last = min(tiles, first + per_split);
+    const int live_heads = min(LAT_HEADS, num_heads - head0);
+    const size_t item0 = (size_t)t * num_heads + head0;
+    if (first >= last) {
+        if (tid < live_heads) {
+            partial_ml[((item0 + tid) * splits + split) * 2] = -INFINITY;
+            partial_ml[((item0 + tid) * splits + split) * 2 + 1] = 0.0f;
+        }
+        return;
+    }
+    const int* table = block_table + (size_t)token_seq[t] * table_width;
+    const int pieces = dim / 8;                                         // 16-byte pieces of a row
+    auto fetch = [&](int tile, int stage) {
+        for (int i = tid; i < LAT_KEYS * pieces; i += 256) {
+            const int row = i / pieces, piece = i - row * pieces, j = tile * LAT_KEYS + row;
+            const bool live = j < count;                                // (rows beyond the last key are zeros: stale ones may hold anything)
+            const int safe = live ? j : 0;
+            const __nv_bfloat16* from = cache + ((size_t)table[safe / block_size] * block_size + safe % block_size) * dim + 8 * piece;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(smem_u32(keys + ((size_t)stage * LAT_KEYS + row) * pitch + 8 * piece)),
+                         "l"(from), "r"(live ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(first, 0);
+    for (int i = tid; i < LAT_HEADS * pieces; i += 256) {
+        const int row = i / pieces, piece = i - row * pieces;
+        *(uint4*)(qs + row * pitch + 8 * piece) = row < live_heads ? *(const uint4*)(q + (item0 + row) * dim + 8 * piece) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const int m_tile = warp & 1, part = warp >> 1;                      // 16 heads; 16 keys of the scores, 64 numbers of the output
+    float acc[8][4] = {};
+    float running_max[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, running_sum[4] = {};
+    for (int tile = first; tile < last; ++tile) {
+        const int stage = (tile - first) & 1;
+        if (tile + 1 < last) {
+            fetch(tile + 1, stage ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const __nv_bfloat16* k_tile = keys + (size_t)stage * LAT_KEYS * pitch;
+        {
+            float s[2][4] = {};
+            const __nv_bfloat16* q_at = qs + (16 * m_tile + (lane & 15)) * pitch + 8 * (lane >> 4);
+            const __nv_bfloat16* k_at = k_tile + (16 * part + (lane & 7) + 8 * (lane >> 4)) * pitch + 8 * ((lane >> 3) & 1);
+            for (int d = 0; d < dim; d += 16) {
+                uint32_t a[4], b[4];
+                lat_ldmatrix(a, q_at + d);
+                lat_ldmatrix(b, k_at + d);
+                lat_mma(s[0], a, b[0], b[1]);
+                lat_mma(s[1], a, b[2], b[3]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = 16 * m_tile + g + 8 * (e >> 1), key = 16 * part + 8 * n + 2 * quad + (e & 1);
+                    scores[row * LAT_S_PITCH + key] = tile * LAT_KEYS + key < count ? s[n][e] * scale : -INFINITY;
+                }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = 4 * warp + i;
+            const float2 s = *(const float2*)(scores + row * LAT_S_PITCH + 2 * lane);
+            const float new_max = fmaxf(running_max[i], warp_max(fmaxf(s.x, s.y)));
+            float p[2] = {expf(s.x - new_max), expf(s.y - new_max)};
+            const float factor = expf(running_max[i] - new_max);        // 0 on the first tile
+            running_sum[i] = running_sum[i] * factor + warp_sum(p[0] + p[1]);
+            running_max[i] = new_max;
+            if (lane == 0) rescale[row] = factor;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const __nv_bfloat162 pair = __floats2bfloat162_rn(p[0], p[1]);
+                *(__nv_bfloat162*)(probs + (k * LAT_HEADS + row) * LAT_P_PITCH + 2 * lane) = pair;
+                const float2 back = __bfloat1622float2(pair);
+                p[0] -= back.x; p[1] -= back.y;
+            }
+        }
+        __syncthreads();
+        const float low = rescale[16 * m_tile + g], high = rescale[16 * m_tile + g + 8];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) { acc[n][0] *= low; acc[n][1] *= low; acc[n][2] *= high; acc[n][3] *= high; }
+#pragma unroll
+        for (int k = 0; k < LAT_KEYS; k += 16) {
+            uint32_t a[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) lat_ldmatrix(a[p], probs + (p * LAT_HEADS + 16 * m_tile + (lane & 15)) * LAT_P_PITCH + k + 8 * (lane >> 4));
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                const int c = 64 * part + 8 * n;
+                if (c >= vdim) continue;
+                uint32_t b[4];
+                lat_ldmatrix_trans(b, k_tile + (k + (lane & 15)) * pitch + c + 8 * (lane >> 4));
+#pragma unroll
+                for (int p = 2; p >= 0; --p) {
+                    lat_mma(acc[n], a[p], b[0], b[1]);
+                    lat_mma(acc[n + 1], a[p], b[2], b[3]);
+                }
+            }
+        }
+        __syncthreads();                                                // (the stage, the scores and the probabilities are free again)
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int row = 16 * m_tile + g + 8 * h;
+        if (row >= live_heads) continue;
+        float* o_part = partial_o + ((item0 + row) * splits + split) * vdim;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int c = 64 * part + 8 * n + 2 * quad;
+            if (c < vdim) *(float2*)(o_part + c) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (4 * warp + i < live_heads) {
+                partial_ml[((item0 + 4 * warp + i) * splits + split) * 2] = running_max[i];
+                partial_ml[((item0 + 4 * warp + i) * splits + split) * 2 + 1] = running_sum[i];
+            }
+    }
+}
+#endif
 
 }  // namespace skv
 
@@ -446,6 +607,28 @@ SKV_EXPORT int skv_attention_general(const void* q, const void* k_cache, const v
     const long long items = (long long)n_tokens * num_heads;
     const long long blocks = (items * splits + GEN_WARPS - 1) / GEN_WARPS;
     if (blocks > 0x7fffffffLL) return fail("skv_attention_general", "too many tokens in one step");
+#if SKV_DTYPE == SKV_BF16
+    // One cached row for all heads whose head is the value, in parts, with nothing that changes a score: the tensor-core
+    // form (rows in whole steps of 16 numbers that fit its tiles, the partial outputs' rows 8-byte aligned)
+    const bool latent = splits > 1 && num_kv_heads == 1 && k_cache == v_cache && value_stride == dim && dim % 16 == 0 && dim <= LAT_MAX_DIM &&
+                        vdim % 16 == 0 && vdim <= LAT_MAX_VDIM && vdim <= dim && window == 0 && !r1 && softcap == 0.0f &&
+                        items * splits <= 0x7fffffffLL && (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)partial_o) & 15) == 0;
+    if (latent) {
+        const size_t room = (size_t)((LAT_HEADS + 2 * LAT_KEYS) * (dim + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + (size_t)LAT_HEADS * (LAT_S_PITCH + 1) * 4;
+        static const cudaError_t ready = cudaFuncSetAttribute(latent_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            (int)(((LAT_HEADS + 2 * LAT_KEYS) * (LAT_MAX_DIM + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + LAT_HEADS * (LAT_S_PITCH + 1) * 4));
+        if (ready != cudaSuccess) return fail("skv_attention_general", cudaGetErrorString(ready));
+        if (int code = launch_pdl("skv_attention_general(latent)", latent_attention_kernel,
+                                  dim3((unsigned)(n_tokens * splits), (unsigned)((num_heads + LAT_HEADS - 1) / LAT_HEADS)), dim3(256), room, stream,
+                                  (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, block_table, table_width, positions, token_seq,
+                                  num_heads, dim, vdim, block_size, scale, splits, partial_o, partial_ml))
+            return code;
+        return launch_pdl("skv_attention_general(merge)", attention_general_merge_kernel<skv_t>,
+                          dim3((unsigned)items), dim3(MERGE_THREADS), 0, stream,
+                          (const float*)partial_o, (const float*)partial_ml, (skv_t*)out, n_tokens, num_heads, vdim, splits,
+                          gate, gate_stride, out_stride, gate_per_element, sink);
+    }
+#endif
     auto kernel = vdim <= 256 ? attention_general_kernel<skv_t, 8> : attention_general_kernel<skv_t, 16>;
     if (int code = launch_pdl("skv_attention_general", kernel, dim3((unsigned)blocks),
                               dim3(GEN_WARPS * 32), smem, stream, (const skv_t*)q, (const skv_t*)k_cache,
@@ -455,7 +638,7 @@ SKV_EXPORT int skv_attention_general(const void* q, const void* k_cache, const v
         return code;
     if (splits == 1) return 0;
     return launch_pdl("skv_attention_general(merge)", attention_general_merge_kernel<skv_t>,
-                      dim3((unsigned)((items + GEN_WARPS - 1) / GEN_WARPS)), dim3(GEN_WARPS * 32), 0, stream,
+                      dim3((unsigned)items), dim3(MERGE_THREADS), 0, stream,
                       (const float*)partial_o, (const float*)partial_ml, (skv_t*)out, n_tokens, num_heads, vdim, splits,
                       gate, gate_stride, out_stride, gate_per_element, sink);
 }

@@ -188,7 +188,8 @@ class LatentAttention(Mixer):
         # run side by side, enough to give every SM thirty-odd warps (a part is at least 64 keys)
         splits, scratch_o, scratch_ml = 1, None, None
         if step.is_decode and rt.device.type == "cuda":
-            splits = max(1, min(-(-rt.sm_count * 32 // (n * s.num_heads)), -(-step.max_ctx // 64), 64))
+            # (the bfloat16 kernel for parts of a latent's keys is worth the merge even in two)
+            splits = max(2 if rt.dtype == torch.bfloat16 else 1, min(-(-rt.sm_count * 32 // (n * s.num_heads)), -(-step.max_ctx // 64), 64))
             if splits > 1:
                 scratch_o = rt.workspace.get("attn_split_o", (n * s.num_heads * splits * s.latent_dim,), torch.float32)
                 scratch_ml = rt.workspace.get("attn_split_ml", (n * s.num_heads * splits * 2,), torch.float32)

@@ -45,3 +45,41 @@ def test_headwise_projection_keeps_an_infinity():
     out = torch.empty(2, 8, device="cuda")
     k.headwise_linear(x, w, out, 1)
     assert (out[0] == 64).all() and torch.isinf(out[1]).all()
+
+
+# rows with and without a part that is no value, one and several groups of 32 heads (the last not full), contexts that end at a
+# tile's and a part's edge, blocks smaller than a tile, more parts than tiles
+@pytest.mark.parametrize("heads,dim,vdim", [(32, 272, 256), (24, 288, 256), (3, 48, 32), (40, 320, 208), (16, 64, 64)])
+@pytest.mark.parametrize("lengths", [(1,), (63, 64, 65), (128, 129, 700), (2000, 3)])
+@pytest.mark.parametrize("block,splits", [(16, 2), (64, 7), (64, 40)])
+def test_attention_over_one_cached_row(heads, dim, vdim, lengths, block, splits):
+    k = lib()
+    n, width = len(lengths), -(-max(lengths) // block)
+    q = torch.randn(n, heads * dim, device="cuda").bfloat16()
+    cache = torch.full((n * width + 1, 1, block, dim), float("nan"), device="cuda").bfloat16()
+    table = torch.randperm(n * width, device="cuda").int().view(n, width)
+    kept = []
+    for i, length in enumerate(lengths):                    # (what lies beyond a sequence's end is not a number)
+        rows = torch.randn(length, dim, device="cuda").bfloat16()
+        kept.append(rows)
+        for j in range(0, length, block):
+            cache[table[i, j // block].long(), 0, :len(rows[j:j + block])] = rows[j:j + block]
+    positions = torch.tensor([length - 1 for length in lengths], dtype=torch.int32, device="cuda")
+    seqs = torch.arange(n, dtype=torch.int32, device="cuda")
+    gate, sink = torch.randn(n, heads + 3, device="cuda"), torch.randn(heads, device="cuda")
+    out = torch.full((n, heads * vdim), float("nan"), device="cuda").bfloat16()
+    scratch_o, scratch_ml = (torch.full((n * heads * splits * size,), float("nan"), device="cuda") for size in (vdim, 2))
+    k.attention_general(q, cache, cache, table, positions, seqs, out, heads, 1, dim, vdim, block, dim ** -0.5, gate=gate, gate_stride=heads + 3,
+                        sink=sink, value_stride=dim, splits=splits, scratch_o=scratch_o, scratch_ml=scratch_ml)
+    for i, rows in enumerate(kept):
+        scores = q[i].double().view(heads, dim) @ rows.double().T * dim ** -0.5
+        whole = torch.softmax(torch.cat([scores, sink.double()[:, None]], dim=1), dim=1)[:, :-1]
+        ref = whole @ rows.double()[:, :vdim] * torch.sigmoid(gate[i, :heads].double())[:, None]
+        # float throughout (a probability rounded to bfloat16 would show as 1e-3 in the partial sums), then one rounding
+        assert ((out[i].double().view(heads, vdim) - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()
+        merged = scratch_o.view(n, heads, splits, vdim)[i].double()
+        ml = scratch_ml.view(n, heads, splits, 2)[i].double()
+        live = ml[..., 0] > -math.inf
+        weight = torch.where(live, torch.exp(ml[..., 0] - ml[..., 0].max(dim=1, keepdim=True).values), 0.0)
+        total = (weight[..., None] * torch.where(live[..., None], merged, 0.0)).sum(1) / (weight * torch.where(live, ml[..., 1], 0.0)).sum(1)[:, None]
+        assert (total - torch.softmax(scores, dim=1) @ rows.double()[:, :vdim]).abs().max() <= 1e-5
