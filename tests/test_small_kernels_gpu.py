@@ -1,0 +1,46 @@
+"""Row kernels in their wide forms against float64: the norm of few rows, the embedding, the per-channel
+decay on tensor cores."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def lib(dtype=torch.bfloat16):
+    from stratakv_b200.ops import kernels_for
+    return kernels_for(dtype, 64, verbose=False)
+
+
+# widths of one quad, of part of a block, of several quads a thread, of all a block holds and one beyond; rows below and above the
+# count where a warp takes a row; parts of a row; chosen rows; a width that is no multiple of 4
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width,groups", [(4, 1), (130, 1), (500, 2), (2048, 1), (3076, 1), (4096, 2), (8192, 1), (8196, 1)])
+@pytest.mark.parametrize("n,chosen", [(1, False), (7, True), (1030, False)])
+def test_rmsnorm_forms(dtype, width, groups, n, chosen):
+    k = lib(dtype)
+    x, gamma = 3 * torch.randn(n, width, device="cuda"), 1 + 0.1 * torch.randn(width, device="cuda")
+    rows = torch.randint(0, n, (2 * n,), device="cuda").int() if chosen else None
+    out = torch.full((2 * n if chosen else n, width), float("nan"), device="cuda").to(dtype)
+    k.rmsnorm(x, gamma, 1e-5, out, rows, groups=groups)
+    source = x.double()[rows.long()] if chosen else x.double()
+    parts = source.view(len(out), groups, -1)
+    ref = (parts * torch.rsqrt((parts * parts).mean(-1, keepdim=True) + 1e-5)).view(len(out), width) * gamma.double()
+    assert ((out.double() - ref).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2e-6) * ref.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("hidden", [4, 260, 2048, 2052, 8192, 30])
+def test_embedding_with_a_folded_norm(hidden):
+    from types import SimpleNamespace
+    from stratakv_b200.residual import ResidualStats
+    k = lib()
+    ids = torch.tensor([3, 0, 12, 99, -1], dtype=torch.int32, device="cuda")
+    table, gamma = torch.randn(13, hidden, device="cuda").bfloat16(), 1 + 0.1 * torch.randn(hidden, device="cuda")
+    nan = lambda *shape: torch.full(shape, float("nan"), device="cuda")
+    stats = ResidualStats(nan(5, hidden).bfloat16(), nan(5), nan(5, -(-hidden // 16) + 4), torch.zeros(1, device="cuda", dtype=torch.int32))
+    stats.expect(SimpleNamespace(gamma=gamma, spec=SimpleNamespace(eps=1e-5)))
+    out, flag = nan(5, hidden), torch.zeros(1, dtype=torch.int32, device="cuda")
+    k.embed(table, ids, out, flag, stats=stats)
+    ref = torch.cat([table[ids[:3].long()].float(), torch.zeros(2, hidden, device="cuda")])
+    assert torch.equal(out, ref) and int(flag) == 1
+    assert torch.equal(stats.scaled, (ref * gamma).bfloat16())
+    torch.testing.assert_close(stats.partials[:, :1].double().sum(-1), (ref.double() ** 2).sum(-1), rtol=1e-5, atol=1e-9)
