@@ -1,5 +1,7 @@
 """Row kernels in their wide forms against float64: the norm of few rows, the embedding, the per-channel
 decay on tensor cores."""
+import math
+
 import pytest
 import torch
 
@@ -44,3 +46,15 @@ def test_embedding_with_a_folded_norm(hidden):
     assert torch.equal(out, ref) and int(flag) == 1
     assert torch.equal(stats.scaled, (ref * gamma).bfloat16())
     torch.testing.assert_close(stats.partials[:, :1].double().sum(-1), (ref.double() ** 2).sum(-1), rtol=1e-5, atol=1e-9)
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 40])
+@pytest.mark.parametrize("rank,channels", [(16, 64), (64, 576), (128, 2048), (24, 64), (64, 100)])
+def test_decay_per_channel(n, rank, channels):
+    k = lib()
+    lora, w2t, w0 = torch.randn(n, rank + 8, device="cuda"), (torch.randn(rank, channels, device="cuda") / math.sqrt(rank)).bfloat16(), torch.randn(channels, device="cuda") - 2
+    out = torch.full((n, channels), float("nan"), device="cuda")
+    k.time_mix_decay(lora, rank, w2t, w0, out)
+    z = torch.tanh(lora[:, :rank].double()) @ w2t.double() + w0.double()
+    # float throughout: exp(-exp(z)) has a slope of at most 0.37 in z, whose sum errs by a few 2^-24 of its terms
+    assert (out.double() - torch.exp(-torch.exp(z))).abs().max() <= 1.5e-6
