@@ -19,6 +19,15 @@ constexpr int ROUTE_THREADS = 256;
 constexpr int ROUTE_MAX_EXPERTS = 1024;
 constexpr int ROUTE_MAX_TOP = 16;
 
+#if SKV_DTYPE == SKV_BF16
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+#endif
+
 // The dot product of a weight row and a float row in shared memory, a warp's share of it: VEC, sixteen bytes of the weight
 // at a time (rows of whole 16 bytes).
 template <bool VEC>
@@ -354,6 +363,99 @@ expert_linear_kernel(const TIn* __restrict__ a, int a_stride, const int* __restr
     }
 }
 
+#if SKV_DTYPE == SKV_BF16
+// ---- projections of few pairs ----------------------------------------------------------------------------------------
+// A block owns 16 weight rows of one expert and streams them once for up to 8 of its rows (the tokens of the mma
+// m16n8k16; more rows go round again, with the weights from L2).  Rows are read where the tokens lie (rows: the token of
+// each sorted pair), with their weight where `weigh` says so: weights[pair] of the pair that place[] put at this row, on
+// the input rounded as scatter_rows rounds it.  A round's loads are all on their way at once: eight steps of 32 k a warp,
+// the rows' first, since loads return in the order they were asked for.
+// Bound by HBM: the chosen experts' weights.  The 128-row tiles of the tensor-memory form read the same bytes at half
+// the rate when a tile holds one to four rows, and need the rows gathered first.  Up and down projection of 8 gated experts of
+// 2816 x 2048, gathering included: 1 token x 2 26 + 18 -> 10 + 5 us, 4 tokens 49 + 34 -> 22 + 14, 16 tokens 45 + 23 -> 31 + 20;
+// of 7168 x 4096, 16 tokens: 190 + 90 -> 138 + 74 us (6.8 TB/s).
+constexpr int FEW_WARPS = 8, FEW_STEPS = 8;
+struct FewWeigh { const int* place; const float* weights; int top; };
+
+template <bool GATED, bool FLOAT_OUT>
+__global__ void __launch_bounds__(FEW_WARPS * 32, 2)
+expert_few_kernel(const __nv_bfloat16* __restrict__ a, int a_stride, const int* __restrict__ rows, const __nv_bfloat16* __restrict__ w,
+                  const int* __restrict__ offsets, void* __restrict__ out, int N, int K, act_t act_word, const FewWeigh weigh) {
+    __shared__ float part[FEW_WARPS][16][9];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int expert = blockIdx.y, lo = offsets[expert], hi = offsets[expert + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int n_rows = GATED ? 2 * N : N, n0 = blockIdx.x * 16, steps = (K + 31) >> 5;
+    const __nv_bfloat16* w_e = w + (size_t)expert * n_rows * K + 8 * t;
+    const __nv_bfloat16 *wa_row = w_e + (size_t)min(n0 + g, n_rows - 1) * K, *wb_row = w_e + (size_t)min(n0 + g + 8, n_rows - 1) * K;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int first = lo; first < hi; first += 8) {
+        const int p = first + g;
+        const bool has = p < hi;
+        const int source = has && rows ? rows[p] : p;
+        const __nv_bfloat16* x_row = a + (size_t)(has ? source : 0) * a_stride + 8 * t;
+        float factor = 1.0f;
+        if (weigh.place && has)
+            for (int k = 0; k < weigh.top; ++k)
+                if (weigh.place[source * weigh.top + k] == p) factor = weigh.weights[source * weigh.top + k];
+        float acc[4] = {};
+        for (int s0 = warp; s0 < steps; s0 += FEW_WARPS * FEW_STEPS) {
+            uint4 x[FEW_STEPS], wa[FEW_STEPS], wb[FEW_STEPS];
+#pragma unroll
+            for (int u = 0; u < FEW_STEPS; ++u) {
+                const int k = (s0 + u * FEW_WARPS) * 32;
+                x[u] = has && k + 8 * t < K ? *(const uint4*)(x_row + k) : zero;
+            }
+#pragma unroll
+            for (int u = 0; u < FEW_STEPS; ++u) {
+                const int k = (s0 + u * FEW_WARPS) * 32;
+                wa[u] = k + 8 * t < K ? __ldg((const uint4*)(wa_row + k)) : zero;
+                wb[u] = k + 8 * t < K ? __ldg((const uint4*)(wb_row + k)) : zero;
+            }
+#pragma unroll
+            for (int u = 0; u < FEW_STEPS; ++u) {
+                if (weigh.place) {
+                    __nv_bfloat162* pairs = (__nv_bfloat162*)&x[u];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __bfloat1622float2(pairs[i]);
+                        pairs[i] = __floats2bfloat162_rn(f.x * factor, f.y * factor);
+                    }
+                }
+                mma_bf16_16816(acc, wa[u].x, wb[u].x, wa[u].y, wb[u].y, x[u].x, x[u].y);
+                mma_bf16_16816(acc, wa[u].z, wb[u].z, wa[u].w, wb[u].w, x[u].z, x[u].w);
+            }
+        }
+        part[warp][g][2 * t] = acc[0]; part[warp][g][2 * t + 1] = acc[1];
+        part[warp][g + 8][2 * t] = acc[2]; part[warp][g + 8][2 * t + 1] = acc[3];
+        __syncthreads();
+        for (int i = threadIdx.x; i < (GATED ? 64 : 128); i += FEW_WARPS * 32) {
+            const int r = GATED ? i & 7 : i & 15, m = GATED ? i >> 3 : i >> 4, o = GATED ? (n0 >> 1) + r : n0 + r;
+            if (first + m >= hi || o >= N) continue;
+            float v = 0.0f, up = 0.0f;
+#pragma unroll
+            for (int q = 0; q < FEW_WARPS; ++q) {
+                v += part[q][r][m];
+                if (GATED) up += part[q][r + 8][m];
+            }
+            const int act = act_word < 0 ? -1 : (int)(act_word & 0xff);
+            if (GATED && act == ACT_SWIGLU_CLAMP) {
+                v = clamped_swiglu(v, up, act_param(act_word));
+            } else {
+                if (act == ACT_RELU2) v = relu_squared(v);
+                else if (act == ACT_GELU_TANH) v = gelu_tanh(v);
+                else if (act == ACT_SILU) v = v / (1.0f + expf(-v));
+                if (GATED) v *= up;
+            }
+            if (FLOAT_OUT) ((float*)out)[(size_t)(first + m) * N + o] = v;
+            else ((__nv_bfloat16*)out)[(size_t)(first + m) * N + o] = __float2bfloat16_rn(v);
+        }
+        __syncthreads();
+    }
+}
+#endif
+
 // ---- rows in sorted order --------------------------------------------------------------------------------------------
 // out[p] = a[rows[p]] for every sorted pair p: the tensor-core projection reads whole tiles of neighbouring rows.
 // Rows are K numbers, K * sizeof(T) a multiple of 16 bytes; a warp copies a row.
@@ -498,15 +600,42 @@ SKV_EXPORT int skv_sort_by_expert(const int* chosen, int pairs, int top, int exp
 // gated: w is [experts, 2 N, K], tiles of 8 gate rows and their 8 up rows; out = act(gate . a) * (up . a).
 // In bfloat16, rows that lie in sorted order already (rows null, a_stride = K) with K a multiple of 8 go to the
 // tensor-memory GEMM's grouped form; `flag` is where its bounded waits report that they gave up.
+// Few pairs in bfloat16 (skv_expert_few_serves) read each chosen expert's weights once, wherever the rows lie; `place`
+// [tokens, top] and `weights` [tokens, top] (both or neither; with rows) multiply each row by its pair's weight first.
+SKV_EXPORT int skv_expert_few_serves(int pairs, int experts, int K) {
+#if SKV_DTYPE == SKV_BF16
+    // up to four rows an expert on average: 16 tokens x 2 of 8 experts of 7168 x 4096 take 138 + 74 us here and 190 + 90 in the
+    // tensor-memory form's tiles, 1 token 42 + 22 and 87 + 62.  Short rows leave a block little to stream (64 experts, rows of
+    // 512: 64 pairs 41 us against 46, 128 pairs 52 against 46): they come here up to a pair an expert
+    return pairs <= (K >= 1024 ? 4 : 1) * experts && K % 8 == 0;
+#else
+    return 0;
+#endif
+}
+
 SKV_EXPORT int skv_expert_linear(const void* a, int a_stride, int a_rows, const int* rows, const void* w,
                                  const int* offsets, void* out, int out_is_float, int pairs, int experts, int N, int K,
-                                 act_t act, int gated, int* flag, cudaStream_t stream) {
+                                 act_t act, int gated, const int* place, const float* weights, int top, int* flag,
+                                 cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (experts <= 0 || experts > ROUTE_MAX_EXPERTS || N <= 0 || K <= 0 || a_stride < K || a_rows <= 0)
         return fail("skv_expert_linear", "sizes do not agree");
     if (!a || !w || !offsets || !out) return fail("skv_expert_linear", "rows, weights, offsets and a place for the result are needed");
     if (act >= 0 && (act & 0xff) >= (gated ? ACT_COUNT : ACT_SWIGLU_CLAMP)) return fail("skv_expert_linear", "this activation is not served");
     if (gated && (act < 0 || N % 8 != 0)) return fail("skv_expert_linear", "a gated weight needs an activation and whole tiles of 8 rows");
+    if ((place == nullptr) != (weights == nullptr) || (place && (!rows || top <= 0 || pairs % top)))
+        return fail("skv_expert_linear", "weighted rows need their tokens, places and weights");
+#if SKV_DTYPE == SKV_BF16
+    if (skv_expert_few_serves(pairs, experts, K) && a_stride % 8 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15)) {
+        const dim3 grid(((gated ? 2 * N : N) + 15) / 16, experts);
+        const FewWeigh weigh = {place, weights, top};
+        auto kernel = gated ? (out_is_float ? expert_few_kernel<true, true> : expert_few_kernel<true, false>)
+                            : (out_is_float ? expert_few_kernel<false, true> : expert_few_kernel<false, false>);
+        return launch_pdl("skv_expert_linear", kernel, grid, dim3(FEW_WARPS * 32), 0, stream, (const __nv_bfloat16*)a, a_stride, rows,
+                          (const __nv_bfloat16*)w, offsets, out, N, K, act, weigh);
+    }
+#endif
+    if (place) return fail("skv_expert_linear", "rows are weighted on their way in only for few pairs in bfloat16");
 #if SKV_DTYPE == SKV_BF16
     if (!rows && a_stride == K && K % 8 == 0 && a_rows >= pairs && !(((uintptr_t)a | (uintptr_t)w) & 15) &&
         (!gated || (!out_is_float && (act & 0xff) != ACT_RELU2)))

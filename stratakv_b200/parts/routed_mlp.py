@@ -133,7 +133,11 @@ class RoutedMlp(FeedForward):
         ops.sort_by_expert(chosen, s.experts, offsets, order, place)
         hidden = get("routed_hidden", (pairs, self.padded), rt.dtype)
         gate = dict(activation=s.activation, gated=self.gated, activation_param=getattr(s, "activation_param", 0.0))
-        if self.weigh_input:
+        if rt.device.type == "cuda" and ops.expert_few(pairs, s.experts, s.hidden_size):
+            # few pairs: each chosen expert's weights are streamed once, its rows read where the tokens lie
+            ops.expert_linear(h, self.w_up, offsets, hidden, rows=order, **gate,
+                              **(dict(place=place, weights=weights) if self.weigh_input else {}))
+        elif self.weigh_input:
             rows = get("routed_rows", (pairs, s.hidden_size), rt.dtype)
             ops.scatter_rows(h, place, weights, rows)
             ops.expert_linear(rows, self.w_up, offsets, hidden, **gate)
