@@ -33,8 +33,7 @@ namespace skv {
 
 constexpr int FHD = SKV_HEAD_DIM;
 constexpr int FKSTEPS = FHD / 16, FOTILES = FHD / 8;
-constexpr int FWARPS = 8, FTHREADS = FWARPS * 32;
-constexpr int FCHUNK = FWARPS * 16;                 // keys per stage: one group of 16 per warp
+constexpr int FWIDE = 8, FNARROW = 4;               // warps of a block's two forms (see the launch)
 constexpr int FMAX_STAGES = 4;                      // stages per launch: 2 .. FMAX_STAGES (see the launch below)
 // Staged rows: ldmatrix reads 16 bytes of each of 8 neighbouring rows at once, which must fall on different banks.
 // Rows of whole 128-byte multiples are stored with their 16-byte pieces exchanged (piece ^ (row & 7)), at no cost
@@ -46,7 +45,7 @@ __device__ __forceinline__ uint32_t f_staged(int row, int piece) {          // b
     return (uint32_t)(row * FROW + ((FSWIZZLED ? piece ^ (row & 7) : piece) << 4));
 }
 constexpr int FPIECES = FHD / 8;                    // 16-byte pieces per row
-constexpr int FSTAGE_BYTES = 2 * FCHUNK * FROW;     // keys, then values
+constexpr int FWARP_BYTES = 2 * 16 * FROW;            // what 16 keys and 16 values, one group per warp, take of a stage
 constexpr int FPITCH = FHD + 2;                     // floats per partial row: outputs, max, sum
 constexpr int FINBOX_ROWS = 24;                     // >= ceil(16 / blocks) * blocks for 1..8 blocks
 
@@ -59,8 +58,8 @@ constexpr int FTABLE = 512;                                         // entries o
 constexpr int F_TABLE_AT = F_INBOX_AT + FINBOX_ROWS * FPITCH * 4;   // [FTABLE] ints
 constexpr int F_STAGES_AT = (F_TABLE_AT + FTABLE * 4 + 127) / 128 * 128;   // also the warps' merge area after the loop
 constexpr int F_SMEM_LIMIT = 227 * 1024;
-static_assert(FWARPS * 16 * FPITCH * 4 <= 2 * FSTAGE_BYTES, "the merge area reuses the stages");
-static_assert(F_STAGES_AT + 2 * FSTAGE_BYTES <= F_SMEM_LIMIT, "shared memory");
+static_assert(16 * FPITCH * 4 <= 2 * FWARP_BYTES, "the merge area reuses the stages");
+static_assert(F_STAGES_AT + 2 * FWIDE * FWARP_BYTES <= F_SMEM_LIMIT, "shared memory");
 
 __device__ __forceinline__ void f_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                       uint32_t b0, uint32_t b1) {
@@ -135,8 +134,9 @@ __device__ __forceinline__ float4 f_add4(float4 a, const float* bias) {
 
 // EXTRAS false: the instantiation without any of the optional steps (nothing of them is compiled in, so the plain
 // rotary decoder runs the code it ran before they existed).
-template <bool EXTRAS>
-__global__ void __launch_bounds__(FTHREADS, FHD <= 64 ? 2 : 1)
+// FWARPS: 8, or 4 where blocks of a wide head outnumber the SMs.
+template <bool EXTRAS, int FWARPS>
+__global__ void __launch_bounds__(FWARPS * 32, FHD <= 64 || FWARPS == FNARROW ? 2 : 1)
 decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __restrict__ cos_sin,
                               __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
                               const int* __restrict__ block_table, int table_width,
@@ -145,7 +145,8 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
                               int write_kv, int block_shift, int stages, const NewTokenFinish finish,
                               const AttentionExtras extras) {
     extern __shared__ __align__(128) unsigned char fused_smem[];
-    constexpr int HALF = FHD / 2;
+    constexpr int HALF = FHD / 2, FTHREADS = FWARPS * 32;
+    constexpr int FCHUNK = FWARPS * 16, FSTAGE_BYTES = FWARPS * FWARP_BYTES;       // keys per stage
     pdl_launch_dependents();
     f_cluster_arrive();                               // "this block is running": waited for before the first remote store
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -534,26 +535,35 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
         if (cudaGetDevice(&device) != cudaSuccess ||
             cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count <= 0)
             return fail("skv_attention_decode_fused", "cannot read the number of SMs");
-        for (auto kernel : {decode_attention_fused_kernel<false>, decode_attention_fused_kernel<true>}) {
+        for (auto kernel : {decode_attention_fused_kernel<false, FWIDE>, decode_attention_fused_kernel<true, FWIDE>,
+                            decode_attention_fused_kernel<false, FNARROW>, decode_attention_fused_kernel<true, FNARROW>}) {
             const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM_LIMIT);
             if (status != cudaSuccess) return fail("skv_attention_decode_fused", cudaGetErrorString(status));
         }
         sm_count = count;
     }
-    // Two stages of 128 keys let two blocks share an SM.  A block that has an SM to itself, and whose piece of
-    // the longest context is at most four stages, fetches the whole piece ahead instead (measured: batch 8 at
-    // 2,048 keys gains 3 % that way, while deeper staging of longer pieces loses 10 %).
+    // Two stages of 128 keys let two blocks of head size 64 share an SM.  A block that has an SM to itself, and whose
+    // piece of the longest context is at most four stages, fetches the whole piece ahead instead (measured: batch 8 at
+    // 2,048 keys gains 3 % that way, while deeper staging of longer pieces loses 10 %).  Above head size 64 a block of
+    // eight warps fills an SM, and where there are more blocks than SMs each wave's start and end lie bare: blocks of
+    // four warps on stages of 64 keys share an SM in twos (head size 128: 8 sequences x 24 key heads over 430 keys
+    // 21 -> 16 us, 64 x 8 over 390 keys 48 -> 35, 64 x 32 over 1,000 keys 277 -> 225).  Long pieces are bound by bytes, so
+    // that a last wave of twos that is half empty costs more than it hides (16 x 24 over 1,000 keys: 384 blocks are three
+    // waves of one and four halves of two, 58 us against 63): there the eight warps stay.
     const long long blocks = (long long)n_seqs * num_kv_heads * m_tiles * splits;
-    const long long piece_chunks = ((long long)table_width * block_size / splits + FCHUNK - 1) / FCHUNK;
-    const int room = (F_SMEM_LIMIT - F_STAGES_AT) / FSTAGE_BYTES;
+    const long long waves = (blocks + sm_count - 1) / sm_count, pairs = 2 * ((blocks + 2 * sm_count - 1) / (2 * sm_count));
+    const bool narrow = FHD > 64 && blocks > sm_count && (10 * pairs <= 11 * waves || (long long)table_width * block_size <= 512 * splits);
+    const int warps = narrow ? FNARROW : FWIDE, stage_bytes = warps * FWARP_BYTES;
+    const long long piece_chunks = ((long long)table_width * block_size / splits + warps * 16 - 1) / (warps * 16);
+    const int room = (F_SMEM_LIMIT - F_STAGES_AT) / stage_bytes;
     // (a third stage for longer pieces, which two blocks of head size 64 could still share an SM with, measured
     // 7-12 % slower in the step at 8,100 and 16,200 keys)
     int stages = 2;
     if (blocks <= sm_count && piece_chunks <= FMAX_STAGES && piece_chunks <= room) stages = (int)(piece_chunks < 2 ? 2 : piece_chunks);
-    const size_t smem = (size_t)F_STAGES_AT + (size_t)stages * FSTAGE_BYTES;
+    const size_t smem = (size_t)F_STAGES_AT + (size_t)stages * stage_bytes;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(n_seqs, num_kv_heads * m_tiles, splits);
-    config.blockDim = dim3(FTHREADS);
+    config.blockDim = dim3(warps * 32);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attributes[2];
@@ -567,8 +577,10 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
     config.numAttrs = pdl_enabled() ? 2 : 1;
     const bool any_extras = q_bias || k_bias || v_bias || value_norm || bias || gate || row_stride != row_floats ||
                             qk_norm || q_temp_every > 0 || softcap > 0.0f;
+    auto kernel = narrow ? (any_extras ? decode_attention_fused_kernel<true, FNARROW> : decode_attention_fused_kernel<false, FNARROW>)
+                         : (any_extras ? decode_attention_fused_kernel<true, FWIDE> : decode_attention_fused_kernel<false, FWIDE>);
     const cudaError_t status = cudaLaunchKernelEx(
-        &config, any_extras ? decode_attention_fused_kernel<true> : decode_attention_fused_kernel<false>, qkv, (const float2*)cos_sin, (__nv_bfloat16*)k_cache,
+        &config, kernel, qkv, (const float2*)cos_sin, (__nv_bfloat16*)k_cache,
         (__nv_bfloat16*)v_cache, block_table, table_width, ctx_after, (__nv_bfloat16*)out, num_heads, num_kv_heads,
         block_size, scale, window, splits, m_tiles, write_kv, block_shift, stages, finish, extras);
     if (status != cudaSuccess) return fail("skv_attention_decode_fused", cudaGetErrorString(status));
