@@ -377,6 +377,39 @@ retention_chunk_output_kernel(const float* __restrict__ fused, const float* __re
     }
 }
 
+// Heads of whole 64 numbers: retention is linear_state.cu's recurrence with a fixed decay per head on the rotated rows.  Its
+// kernels (chunks of 64, eight products for every 16-byte operand they read from shared memory; those above: four for
+// five 4-byte ones) make the outputs, o [n_tokens][H][dv] float, and this one norms and gates them, a warp per (token, head).
+// 2,048 tokens, 32 heads of 64: 263 -> 153 us; 24 heads of 128: 577 -> 279; 8 x 647 tokens, 32 heads of 64: 769 -> 372.
+template <typename T>
+__global__ void __launch_bounds__(RET_THREADS)
+retention_finish_kernel(const float* __restrict__ o, const float* __restrict__ fused, float eps, T* __restrict__ out, int out_stride,
+                        int n_tokens, const RetentionShape shape) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, H = shape.heads, dv = shape.vdim;
+    const long long item = (long long)blockIdx.x * RET_WARPS + (threadIdx.x >> 5);
+    if (item >= (long long)n_tokens * H) return;
+    const size_t t = (size_t)(item / H);
+    const int head = (int)(item % H);
+    const float* row = o + (size_t)item * dv;
+    const float* gate = fused + t * shape.row_stride + (size_t)2 * H * shape.dim + (size_t)H * dv + (size_t)head * dv;
+    float squares = 0.0f;
+    for (int e = 2 * lane; e < dv; e += 64) {
+        const float2 x = *(const float2*)(row + e);
+        squares = fmaf(x.x, x.x, fmaf(x.y, x.y, squares));
+    }
+    const float factor = 1.0f / sqrtf(warp_sum(squares) / (float)dv + eps);
+    T* out_row = out + t * out_stride + (size_t)head * dv;
+    for (int e = 2 * lane; e < dv; e += 64) {
+        const float2 x = *(const float2*)(row + e), g = *(const float2*)(gate + e);
+        out_row[e] = from_float<T>(x.x * factor * (g.x / (1.0f + expf(-g.x))));
+        out_row[e + 1] = from_float<T>(x.y * factor * (g.y / (1.0f + expf(-g.y))));
+    }
+    if (head == H - 1)
+        for (int col = H * dv + lane; col < out_stride; col += 32) out[t * out_stride + col] = from_float<T>(0.0f);
+}
+
 static int reserve_shared(const void* kernel, size_t bytes, const char* name) {
     if (bytes <= 48 * 1024) return 0;
     if (bytes > 200 * 1024) return fail(name, "the head sizes are too large for this kernel's shared memory");
@@ -389,11 +422,27 @@ static int reserve_shared(const void* kernel, size_t bytes, const char* name) {
 
 using namespace skv;
 
+// linear_state.cu
+extern "C" long long skv_linear_state_scratch(int n_seqs, int max_q_len, int heads, int dim, int vdim, int with_floor);
+extern "C" int skv_linear_state(const float* rows, int row_stride, int q_at, int k_at, int v_at, int silu, const float* decay,
+                                const float* log_decay, const float* key_scale, const float* skip, float out_scale,
+                                const float* floor, float floor_eps, float* out, float* scratch, int n_tokens, int n_seqs, int heads, int groups, int dim, int vdim,
+                                int max_q_len, const int* positions, const int* token_seq, const int* cu_q,
+                                const int* slot_ids, float* state, long long state_stride, long long state_offset, cudaStream_t stream);
+
+// Whether a longer step's recurrence runs on linear_state.cu's kernels: heads of whole tiles, in chunks of 64 tokens.
+static bool as_linear_state(int dim, int vdim) { return dim % 64 == 0 && dim <= 128 && vdim % 64 == 0; }
+
 // Floats of scratch that skv_retention needs for a step whose longest sequence brings max_q_len tokens (0 for one
 // token a sequence).
 SKV_EXPORT long long skv_retention_scratch(int n_seqs, int max_q_len, int heads, int dim, int vdim) {
     if (max_q_len <= 1) return 0;
-    return (long long)n_seqs * ((max_q_len + RET_CHUNK - 1) / RET_CHUNK) * heads * dim * vdim;
+    const long long own = (long long)n_seqs * ((max_q_len + RET_CHUNK - 1) / RET_CHUNK) * heads * dim * vdim;
+    if (!as_linear_state(dim, vdim)) return own;
+    // the outputs of every token, then the chunks' sums; rows that are no whole 16 bytes still need `own`
+    const long long outputs = (long long)n_seqs * max_q_len * heads * vdim;
+    const long long both = outputs + skv_linear_state_scratch(n_seqs, max_q_len, heads, dim, vdim, 0);
+    return own > both ? own : both;
 }
 
 // fused: float [n_tokens, row_stride], rows [q | k | v | gate]; queries and keys are rotated in place where a step
@@ -430,6 +479,17 @@ SKV_EXPORT int skv_retention(float* fused, int row_stride, const float* rotation
     if (int code = launch_pdl("skv_retention", retention_rotate_kernel, dim3(n_tokens), dim3(RET_THREADS), 0, stream,
                               fused, rotation, n_tokens, shape, positions))
         return code;
+    if (as_linear_state(dim, vdim) && row_stride % 4 == 0 && state_stride % 4 == 0 && (((uintptr_t)fused | (uintptr_t)scratch | (uintptr_t)state) & 15) == 0) {
+        float* o = scratch;
+        float* chunks = scratch + (size_t)n_tokens * heads * vdim;
+        if (int code = skv_linear_state(fused, row_stride, 0, heads * dim, 2 * heads * dim, 0, decay, nullptr, nullptr, nullptr, 1.0f, nullptr,
+                                        0.0f, o, chunks, n_tokens, n_seqs, heads, heads, dim, vdim, max_q_len, positions, token_seq, cu_q,
+                                        slot_ids, state, state_stride, 0, stream))
+            return code;
+        const long long items = (long long)n_tokens * heads;
+        return launch_pdl("skv_retention", retention_finish_kernel<skv_t>, dim3((unsigned)((items + RET_WARPS - 1) / RET_WARPS)), dim3(RET_THREADS),
+                          0, stream, (const float*)o, (const float*)fused, eps, (skv_t*)out, out_stride, n_tokens, shape);
+    }
     const size_t sum_smem = (size_t)RET_CHUNK * (dim + vdim) * sizeof(float);
     if (int code = reserve_shared((const void*)retention_chunk_sum_kernel, sum_smem, "skv_retention")) return code;
     if (int code = launch_pdl("skv_retention", retention_chunk_sum_kernel, dim3(max_chunks, heads, n_seqs),

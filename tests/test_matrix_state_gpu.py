@@ -1,0 +1,136 @@
+"""Matrix states with a decay per head at whole tiles of 64, several cells a thread in the walk over chunks, and retention
+on the same kernels, against the recurrence in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def recurrence(q, k, v, log_decay, S, n_state):
+    """float64: outputs [T, H, P], key-sum products [T, H] and the state after; q, k [T, H, N], v [T, H, P], log_decay [T, H]."""
+    out, dots = [], []
+    for t in range(len(q)):
+        d = torch.exp(log_decay[t])
+        S = d[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+        n_state = d[:, None] * n_state + k[t]
+        out.append((q[t][:, None, :] @ S)[:, 0])
+        dots.append((n_state * q[t]).sum(-1))
+    return torch.stack(out), torch.stack(dots), S, n_state
+
+
+# chunks of 64 that are full, end at a tile's edge of 16 or a token behind it, and are one token; states that go on; heads that
+# share keys; every mechanism of the float kernel
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(3, 3, 64, 64), (4, 2, 128, 64), (2, 1, 64, 128), (2, 2, 128, 128)])
+@pytest.mark.parametrize("form", ["fixed", "fixed_silu", "per_token", "forgets", "floor"])
+@pytest.mark.parametrize("portions", [((64, 1, 130), (17, 65, 2)), ((200, 16, 63),)])
+def test_linear_state_in_whole_tiles(dtype, heads, groups, dim, vdim, form, portions):
+    from stratakv_b200.ops import kernels_for
+    ops = kernels_for(dtype, 64, verbose=False)
+    generator = torch.Generator(device="cuda").manual_seed(heads * dim + vdim)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device="cuda")
+    total = [sum(p[i] for p in portions) for i in range(3)]
+    width = 2 * groups * dim + heads * vdim
+    rows = [normal(n, width + 4) for n in total]
+    decay = torch.tensor([0.9, 0.99, 0.999, 0.0], device="cuda")[:heads].contiguous()
+    if form.startswith("fixed"):
+        logs = [torch.log(decay.double()).expand(n, heads) for n in total]
+    else:
+        logs = [-torch.rand(n, heads, generator=generator, device="cuda") * 0.1 for n in total]
+        if form == "forgets":                                   # e^-60 now and then, and once everything
+            for l in logs:
+                l[::7] = -60.0
+                l[len(l) // 2] = -4000.0
+    scale, skip = [torch.rand(n, heads, generator=generator, device="cuda") for n in total], normal(heads)
+    floor = [0.5 + torch.rand(n, heads, generator=generator, device="cuda") for n in total]
+    per_half = heads * dim * (vdim + (form == "floor"))
+    offset = 8
+    state = torch.full((5, offset + 2 * per_half), 1e30, device="cuda")
+    slots, want = [3, 0, 4], []
+    for i in range(3):
+        r = rows[i].double()
+        act = torch.nn.functional.silu if form == "fixed_silu" else (lambda z: z)
+        spread = lambda z: act(z).view(-1, groups, dim).repeat_interleave(heads // groups, dim=1)
+        q, k, v = spread(r[:, :groups * dim]), spread(r[:, groups * dim:2 * groups * dim]), act(r[:, 2 * groups * dim:width]).view(-1, heads, vdim)
+        if not form.startswith("fixed"):
+            k = k * scale[i].double()[:, :, None]
+        zeros = k.new_zeros(heads, dim, vdim)
+        o, dots, S, n_state = recurrence(q, k, v, logs[i].double(), zeros, zeros[:, :, 0])
+        # the sum of the magnitudes that a float sum's error is a fraction of
+        mass = recurrence(q.abs(), k.abs(), v.abs(), logs[i].double(), zeros, zeros[:, :, 0])[0]
+        if form == "floor":
+            weight = torch.maximum((0.5 * dots).abs(), floor[i].double()) + 1e-6
+            o, mass = 0.5 * o / weight[:, :, None], 0.5 * mass / weight[:, :, None] * 3
+        elif not form.startswith("fixed"):
+            o, mass = o + skip.double()[:, None] * v, mass + (skip.double()[:, None] * v).abs()
+        want.append((o, mass, S))
+    got, at = [[], [], []], [0, 0, 0]
+    for portion in portions:
+        cu = torch.tensor([0] + list(torch.tensor(portion).cumsum(0)), dtype=torch.int32, device="cuda")
+        positions = torch.cat([torch.arange(at[i], at[i] + portion[i], dtype=torch.int32) for i in range(3)]).cuda()
+        seqs = torch.repeat_interleave(torch.arange(3, dtype=torch.int32), torch.tensor(portion)).cuda()
+        meta = (positions, seqs, cu, torch.tensor(slots, dtype=torch.int32, device="cuda"))
+        pick = lambda parts: torch.cat([parts[i][at[i]:at[i] + portion[i]] for i in range(3)]).contiguous()
+        more = dict(decay=decay, silu=form == "fixed_silu") if form.startswith("fixed") else dict(log_decay=pick(logs), key_scale=pick(scale))
+        if form == "floor":
+            more.update(floor=pick(floor), floor_eps=1e-6, out_scale=0.5)
+        elif not form.startswith("fixed"):
+            more.update(skip=skip)
+        need = ops.linear_state_scratch(3, max(portion), heads, dim, vdim, form == "floor")
+        out = torch.full((sum(portion), heads * vdim), float("nan"), device="cuda")
+        ops.linear_state(pick(rows), 0, groups * dim, 2 * groups * dim, out, state, meta, heads, groups, dim, vdim, max(portion),
+                         scratch=torch.full((need,), float("nan"), device="cuda"), state_offset=offset, **more)
+        for i, part in enumerate(out.split(list(portion))):
+            got[i].append(part)
+            at[i] += portion[i]
+    for i in range(3):
+        o, mass, S = want[i]
+        # sums of up to a few hundred products in float: a few 2^-24 of their magnitudes' sum (operands rounded to bfloat16 or to
+        # sixteen bits anywhere would be off by 2^-9 or 2^-17 of a product)
+        assert ((torch.cat(got[i]).double().view(-1, heads, vdim) - o).abs() <= 3e-6 * mass + 1e-6).all()
+        last = state[slots[i], offset + ((total[i] - 1) & 1) * per_half:][:heads * dim * vdim].view(heads, dim, vdim)
+        assert (last.double() - S).abs().max() <= 3e-6 * (S.abs().max() + 10)
+    assert (state[[1, 2]] == 1e30).all() and (state[:, :offset] == 1e30).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,dim,vdim,rotated,spare", [(3, 64, 64, 32, 0), (2, 128, 64, 128, 8), (2, 64, 128, 0, 1), (2, 192, 64, 64, 0)])
+def test_retention_in_whole_tiles(dtype, heads, dim, vdim, rotated, spare):
+    """A head size of 192 and rows that are no whole 16 bytes stay on retention's own kernels."""
+    from stratakv_b200.ops import kernels_for
+    from stratakv_b200.parts.position import rope_table
+    ops = kernels_for(dtype, 64, verbose=False)
+    generator = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    lengths, eps = (130, 1, 64), 1e-5
+    width = 2 * heads * (dim + vdim) + spare
+    rows = [torch.randn(n, width, generator=generator, device="cuda") for n in lengths]
+    decay = torch.tensor([0.9, 0.999, 1.0], device="cuda")[:heads].contiguous()
+    table = torch.from_numpy(rope_table(rotated, 10000.0, 256)).cuda() if rotated else None
+    state = torch.full((4, 2 * heads * dim * vdim), 1e30, device="cuda")
+    slots = [2, 0, 3]
+    want = []
+    for r in rows:
+        n = len(r)
+        turn = lambda z: z
+        if rotated:
+            cos, sin = (table[:n, :, i].double()[:, None] for i in (0, 1))
+            half = rotated // 2
+            turn = lambda z: torch.cat([z[..., :half] * cos - z[..., half:rotated] * sin, z[..., half:rotated] * cos + z[..., :half] * sin, z[..., rotated:]], -1)
+        q, k = (turn(r[:, i * heads * dim:(i + 1) * heads * dim].double().view(n, heads, dim)) for i in (0, 1))
+        v = r[:, 2 * heads * dim:][:, :heads * vdim].double().view(n, heads, vdim)
+        gate = r[:, 2 * heads * dim + heads * vdim:][:, :heads * vdim].double()
+        run = lambda q, k, v: recurrence(q, k, v, torch.log(decay.double()).expand(n, heads), v.new_zeros(heads, dim, vdim), v.new_zeros(heads, dim))[0]
+        o, mass = run(q, k * dim ** -0.5, v), run(q.abs(), k.abs() * dim ** -0.5, v.abs())
+        factor = torch.rsqrt((o * o).mean(-1, keepdim=True) + eps)
+        act = torch.nn.functional.silu(gate)
+        want.append(((o * factor).reshape(n, -1) * act, (mass * factor).reshape(n, -1) * act.abs()))
+    cu = torch.tensor([0, 130, 131, 195], dtype=torch.int32, device="cuda")
+    positions = torch.cat([torch.arange(n, dtype=torch.int32) for n in lengths]).cuda()
+    meta = (positions, torch.repeat_interleave(torch.arange(3), torch.tensor(lengths)).int().cuda(), cu, torch.tensor(slots, dtype=torch.int32, device="cuda"))
+    out = torch.full((195, heads * vdim + 8), float("nan"), device="cuda").to(dtype)
+    scratch = torch.full((ops.retention_scratch(3, 130, heads, dim, vdim),), float("nan"), device="cuda")
+    ops.retention(torch.cat(rows).contiguous(), table, rotated, decay, eps, out, state, meta, heads, dim, vdim, 130, scratch)
+    ref, mass = (torch.cat(parts) for parts in zip(*want))
+    assert (out[:, heads * vdim:] == 0).all()
+    # a few 2^-24 of what the float sums' terms add up to, divided by the head's root mean square as they are
+    assert ((out[:, :heads * vdim].double() - ref).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * ref.abs() + 4e-6 * mass + 1e-6).all()
