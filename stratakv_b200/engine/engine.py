@@ -167,9 +167,6 @@ class Engine:
             if len(e.tokens) == 0:
                 raise StepError(f"slot {e.slot}: a step needs at least one token per sequence")
             tokens = _token_array(e.tokens)
-            if int(tokens.min()) < 0 or int(tokens.max()) >= vocab:
-                outside = np.flatnonzero((tokens < 0) | (tokens >= vocab))
-                raise StepError(f"slot {e.slot}: token id {int(tokens[outside[0]])} is outside the vocabulary of {vocab}")
             for w in e.want:
                 if not (0 <= int(w) < len(e.tokens)):
                     raise StepError(f"slot {e.slot}: wanted place {w} is outside this step's {len(e.tokens)} tokens")
@@ -179,6 +176,12 @@ class Engine:
             q_lens.append(len(e.tokens))
             ctx_before.append(before)
             wanted[e.slot] = before + len(e.tokens)
+        token_ids = np.concatenate(token_arrays) if len(token_arrays) > 1 else token_arrays[0]
+        if int(token_ids.min()) < 0 or int(token_ids.max()) >= vocab:        # (one look at all of them; who it was, only then)
+            for e, tokens in zip(entries, token_arrays):
+                outside = np.flatnonzero((tokens < 0) | (tokens >= vocab))
+                if outside.size:
+                    raise StepError(f"slot {e.slot}: token id {int(tokens[outside[0]])} is outside the vocabulary of {vocab}")
         self.cache.reserve(wanted)              # CacheFull leaves everything as it was
 
         n, total = len(entries), sum(q_lens)
@@ -204,9 +207,10 @@ class Engine:
             start, count = offsets[key]
             host[start:start + count] = values
 
-        put("token_ids", np.concatenate(token_arrays) if n > 1 else token_arrays[0])
-        put("positions", np.concatenate([np.arange(b, b + q) for b, q in zip(ctx_before, q_lens)]))
-        put("token_seq", np.repeat(np.arange(n), q_lens))
+        token_seq = np.repeat(np.arange(n), q_lens)
+        put("token_ids", token_ids)
+        put("positions", np.arange(total) + (np.array(ctx_before) - cu_q[:-1])[token_seq])
+        put("token_seq", token_seq)
         put("cu_q", cu_q)
         put("ctx_after", [wanted[slot] for slot in slots])
         put("slot_ids", slots)

@@ -12,14 +12,20 @@ class Workspace:
     def __init__(self, device):
         self.device = torch.device(device)
         self._buffers: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        # the view last handed out of each buffer: a step asks for the same one layer after layer, and making it (a slice,
+        # then a view) costs the host as much as the launch it is for
+        self._views: Dict[Tuple[str, torch.dtype], Tuple[tuple, torch.Tensor]] = {}
         self.generation = 0          # bumped whenever a buffer is reallocated
 
     def get(self, name: str, shape, dtype: torch.dtype, zero: bool = False) -> torch.Tensor:
         """``zero``: the buffer is zero when it is first handed out (and after it had to grow)."""
+        key = (name, dtype)
+        last = self._views.get(key)
+        if last is not None and last[0] == shape:
+            return last[1]
         count = 1
         for d in shape:
             count *= int(d)
-        key = (name, dtype)
         buffer = self._buffers.get(key)
         if buffer is None or buffer.numel() < count:
             capacity = max(count, 1)
@@ -28,4 +34,6 @@ class Workspace:
             buffer = (torch.zeros if zero else torch.empty)(capacity, dtype=dtype, device=self.device)
             self._buffers[key] = buffer
             self.generation += 1
-        return buffer[:count].view(*shape)
+        view = buffer[:count].view(*shape)
+        self._views[key] = (tuple(shape), view)
+        return view
