@@ -58,3 +58,34 @@ def test_experts_of_few_pairs(n, top, experts, N, K, form, crowded):
         ref = torch.relu(z) ** 2 if form == "relu2" else z
     # float sums of products that add up to order one, then one rounding to bfloat16
     assert ((out.double() - ref).abs() <= (2.0 ** -8 if form != "float" else 0.0) * ref.abs() + 2e-5 * (1 + ref.abs())).all()
+
+
+# tokens at a block's edges; dot products of one, two and several tiles and beyond a round of them, with and without the shared gate;
+# rows of one step, of fewer steps than warps, of several rounds, and of a width that is no multiple of 32 (a block a token)
+@pytest.mark.parametrize("n", [1, 16, 17, 40])
+@pytest.mark.parametrize("experts,shared,groups", [(1, True, 0), (8, False, 2), (8, True, 0), (15, True, 0), (17, False, 0), (70, True, 7), (1024, False, 0)])
+@pytest.mark.parametrize("hidden", [32, 480, 2080, 4096, 72])
+@pytest.mark.parametrize("softmax", [False, True])
+def test_router(n, experts, shared, groups, hidden, softmax):
+    k, top = lib(), min(2, experts)
+    h, w = torch.randn(n, hidden, device="cuda").bfloat16(), (torch.randn(experts, hidden, device="cuda") / math.sqrt(hidden)).bfloat16()
+    correction, gate = torch.randn(experts, device="cuda"), torch.randn(hidden, device="cuda").bfloat16() if shared else None
+    share = torch.full((n,), float("nan"), device="cuda") if shared else None
+    chosen, weights = torch.full((n, top), -1, dtype=torch.int32, device="cuda"), torch.full((n, top), float("nan"), device="cuda")
+    keep = groups // 2 if groups else 0
+    k.route_tokens(h, w, correction, top, 1.5, True, chosen, weights, gate, share, softmax=softmax, groups=groups, keep=keep)
+    z = h.double() @ w.double().T
+    score = torch.softmax(z, -1) if softmax else torch.sigmoid(z)
+    choice = score + correction.double()
+    if groups:
+        best = choice.view(n, groups, -1).amax(-1)
+        kept = torch.zeros_like(best).scatter_(1, best.topk(keep, -1).indices, 1.0).repeat_interleave(experts // groups, -1)
+        choice = torch.where(kept > 0, choice, -math.inf)
+    want = choice.topk(top, -1)
+    got = choice.gather(1, chosen.long())
+    # a float sum of products of order one errs by a few 1e-7: only scores that close may change places
+    assert (got - want.values).abs().max() <= 1e-5 and all(len(set(row)) == top for row in chosen.tolist())
+    picked = score.gather(1, chosen.long())
+    torch.testing.assert_close(weights.double(), 1.5 * picked / picked.sum(-1, keepdim=True), rtol=1e-5, atol=1e-7)
+    if shared:
+        torch.testing.assert_close(share.double(), torch.sigmoid(h.double() @ gate.double()), rtol=2e-5, atol=1e-6)
