@@ -27,3 +27,20 @@ def test_more_blocks_than_sms(heads, kv_heads, head_dim, block_size, lengths, wi
                              torch.tensor(lengths, dtype=torch.int32, device="cuda"), out, heads, kv_heads, head_dim,
                              block_size, scale, window, splits, True)
     close(out, attention_reference(setup, dtype, heads, kv_heads, scale, window).view(n, -1), dtype)
+
+
+@pytest.mark.parametrize("heads,kv_heads,lengths,window,reach,splits", [(160, 160, [130], 0, 200, 1), (160, 160, [700], 90, 90, 1),
+                                                                       (24, 24, [700, 1, 64, 333] * 2, 0, 400, 1), (40, 2, [520, 77], 0, 600, 8)])
+def test_bias_by_distance(heads, kv_heads, lengths, window, reach, splits):
+    """Against the split kernel, which reads the bias score by score: pieces whose distances end beyond the table."""
+    dtype, n, head_dim, scale = torch.bfloat16, len(lengths), 128, 0.04
+    k = lib(dtype, head_dim)
+    setup, qkv, table, _ = _fused_decode_case(dtype, lengths, heads, kv_heads, head_dim, 64, seed=heads)
+    bias = torch.rand(heads, reach, device="cuda") * 4
+    ctx = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    out, other = (torch.full((n, heads * head_dim), float("nan"), device="cuda").to(dtype) for _ in range(2))
+    k.attention_decode_fused(qkv, table, setup["k_cache"], setup["v_cache"], setup["table"], ctx, out, heads, kv_heads, head_dim, 64, scale,
+                             window, splits, True, bias=bias)
+    k.attention_decode(setup["q"].view(n, -1), setup["k_cache"], setup["v_cache"], setup["table"], ctx, other, heads, kv_heads, head_dim, 64,
+                       scale, window, 1, bias=bias)
+    close(out, other, dtype)
