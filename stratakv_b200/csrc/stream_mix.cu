@@ -8,7 +8,7 @@
 //   sum     (sum_out):                   sum_out[w] = sum_t x_t
 //
 // Everything is float; only normed_out is rounded to the compute dtype.  A block owns one token row; u is kept in
-// shared memory between the pass that makes it and the pass that scales it.
+// shared memory (or, in the wide form, in registers) between the pass that makes it and the pass that scales it.
 #include "common.cuh"
 
 namespace skv {
@@ -83,10 +83,126 @@ stream_mix_kernel(float* __restrict__ streams, const float* __restrict__ source,
         normed_out[base + w] = from_float<T>(stream_mix_u[w] * factor * gamma[w]);
 }
 
+// The same with a thread's share of the row, WIDE_QUADS (1 or 2) times four neighbouring numbers, in registers throughout
+// (hidden a multiple of 4 and at most 4,096, rows 16-byte aligned): every load of a thread is on its way at once, where the
+// kernel above waits for its row number by number, and the weights come ahead of the wait.  Few tokens are bound by that
+// chain, many by their bytes.  8 / 500 / 5,180 tokens, two streams of 2,048: 4.7 / 6.1 / 53 us above, 1.9 / 4.5 / 37 here; two of
+// 4,096: 6.7 / 14 / 98 and 2.4 / 7.9 / 70; four of 2,048: 4.9 / 9.9 / 87 and 2.5 / 7.9 / 72.
+constexpr int WIDE_THREADS = 512;
+
+template <typename T, int S, int WIDE_QUADS>
+__global__ void __launch_bounds__(WIDE_THREADS)
+stream_mix_wide_kernel(float* __restrict__ streams, const float* __restrict__ source, const float* __restrict__ branch,
+                       const float* __restrict__ mix, const float* __restrict__ write, const float* __restrict__ read,
+                       const float* __restrict__ gamma, float eps, T* __restrict__ normed_out, float* __restrict__ sum_out,
+                       int n_tokens, int hidden) {
+    __shared__ float c_mix[S * S], c_write[S], c_read[S];
+    __shared__ float reduce[33];
+    if (threadIdx.x < S * S) c_mix[threadIdx.x] = mix ? mix[threadIdx.x] : 0.0f;
+    if (threadIdx.x < S) {
+        c_write[threadIdx.x] = write ? write[threadIdx.x] : 0.0f;
+        c_read[threadIdx.x] = read ? read[threadIdx.x] : 0.0f;
+    }
+    float4 weight[WIDE_QUADS], u[WIDE_QUADS];
+#pragma unroll
+    for (int q = 0; q < WIDE_QUADS; ++q) {
+        const int w = 4 * (threadIdx.x + q * WIDE_THREADS);
+        weight[q] = u[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (gamma && w < hidden) weight[q] = *(const float4*)(gamma + w);
+    }
+    pdl_launch_dependents();
+    __syncthreads();
+    pdl_wait();
+    const size_t plane = (size_t)n_tokens * hidden, base = (size_t)blockIdx.x * hidden;
+    float squares = 0.0f;
+    float x[WIDE_QUADS][S][4], y[WIDE_QUADS][4];
+#pragma unroll
+    for (int q = 0; q < WIDE_QUADS; ++q) {
+        const int w = 4 * (threadIdx.x + q * WIDE_THREADS);
+        if (w >= hidden) continue;
+        if (source) {
+            const float4 v = *(const float4*)(source + base + w);
+#pragma unroll
+            for (int s = 0; s < S; ++s) { x[q][s][0] = v.x; x[q][s][1] = v.y; x[q][s][2] = v.z; x[q][s][3] = v.w; }
+        } else {
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const float4 v = *(const float4*)(streams + (size_t)s * plane + base + w);
+                x[q][s][0] = v.x; x[q][s][1] = v.y; x[q][s][2] = v.z; x[q][s][3] = v.w;
+            }
+        }
+        if (branch) {
+            const float4 v = *(const float4*)(branch + base + w);
+            y[q][0] = v.x; y[q][1] = v.y; y[q][2] = v.z; y[q][3] = v.w;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < WIDE_QUADS; ++q) {
+        const int w = 4 * (threadIdx.x + q * WIDE_THREADS);
+        if (w >= hidden) continue;
+        if (branch) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float fresh[S];
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+                    float acc = 0.0f;
+#pragma unroll
+                    for (int s = 0; s < S; ++s) acc = fmaf(c_mix[s * S + r], x[q][s][i], acc);
+                    fresh[r] = fmaf(c_write[r], y[q][i], acc);
+                }
+#pragma unroll
+                for (int r = 0; r < S; ++r) x[q][r][i] = fresh[r];
+            }
+#pragma unroll
+            for (int r = 0; r < S; ++r)
+                *(float4*)(streams + (size_t)r * plane + base + w) = make_float4(x[q][r][0], x[q][r][1], x[q][r][2], x[q][r][3]);
+        }
+        if (normed_out) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[i] = 0.0f;
+#pragma unroll
+                for (int s = 0; s < S; ++s) v[i] = fmaf(c_read[s], x[q][s][i], v[i]);
+                squares = fmaf(v[i], v[i], squares);
+            }
+            u[q] = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        if (sum_out) {
+            float total[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                total[i] = 0.0f;
+#pragma unroll
+                for (int s = 0; s < S; ++s) total[i] += x[q][s][i];
+            }
+            *(float4*)(sum_out + base + w) = make_float4(total[0], total[1], total[2], total[3]);
+        }
+    }
+    if (!normed_out) return;
+    const float total = block_sum(squares, reduce);
+    const float factor = 1.0f / sqrtf(total / (float)hidden + eps);
+#pragma unroll
+    for (int q = 0; q < WIDE_QUADS; ++q) {
+        const int w = 4 * (threadIdx.x + q * WIDE_THREADS);
+        if (w >= hidden) continue;
+        alignas(16) T out[4] = {from_float<T>(u[q].x * factor * weight[q].x), from_float<T>(u[q].y * factor * weight[q].y),
+                    from_float<T>(u[q].z * factor * weight[q].z), from_float<T>(u[q].w * factor * weight[q].w)};
+        if (sizeof(T) == 4) *(uint4*)(normed_out + base + w) = *(const uint4*)out;
+        else *(uint2*)(normed_out + base + w) = *(const uint2*)out;
+    }
+}
+
 template <int S>
 static int launch_stream_mix(float* streams, const float* source, const float* branch, const float* mix,
                              const float* write, const float* read, const float* gamma, float eps, void* normed_out,
                              float* sum_out, int n_tokens, int hidden, cudaStream_t stream) {
+    const uintptr_t places = (uintptr_t)streams | (uintptr_t)source | (uintptr_t)branch | (uintptr_t)gamma |
+                             (uintptr_t)normed_out | (uintptr_t)sum_out;
+    if (hidden % 4 == 0 && hidden <= 8 * WIDE_THREADS && (places & 15) == 0)
+        return launch_pdl("skv_stream_mix", hidden <= 4 * WIDE_THREADS ? stream_mix_wide_kernel<skv_t, S, 1> : stream_mix_wide_kernel<skv_t, S, 2>, dim3(n_tokens), dim3(WIDE_THREADS), 0, stream, streams,
+                          source, branch, mix, write, read, gamma, eps, (skv_t*)normed_out, sum_out, n_tokens, hidden);
     const size_t smem = normed_out ? (size_t)hidden * sizeof(float) : 0;
     auto kernel = stream_mix_kernel<skv_t, S>;
     if (smem > 48 * 1024) {

@@ -58,3 +58,22 @@ def test_decay_per_channel(n, rank, channels):
     z = torch.tanh(lora[:, :rank].double()) @ w2t.double() + w0.double()
     # float throughout: exp(-exp(z)) has a slope of at most 0.37 in z, whose sum errs by a few 2^-24 of its terms
     assert (out.double() - torch.exp(-torch.exp(z))).abs().max() <= 1.5e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hidden", [4, 2048, 2052, 4096, 4100, 30])
+@pytest.mark.parametrize("count", [1, 2, 8])
+def test_streams_of_wide_rows(dtype, hidden, count):
+    k, n = lib(dtype), 5
+    streams, branch = torch.randn(count, n, hidden, device="cuda"), torch.randn(n, hidden, device="cuda")
+    mix, write, read = torch.randn(count, count, device="cuda") / count, torch.randn(count, device="cuda"), torch.randn(count, device="cuda")
+    gamma = 1 + 0.1 * torch.randn(hidden, device="cuda")
+    want = torch.einsum("st,snw->tnw", mix.double(), streams.double()) + write.double()[:, None, None] * branch.double()
+    u = torch.einsum("s,snw->nw", read.double(), want)
+    normed = (u * torch.rsqrt((u * u).mean(-1, keepdim=True) + 1e-5)) * gamma.double()
+    out, total = torch.full((n, hidden), float("nan"), device="cuda").to(dtype), torch.full((n, hidden), float("nan"), device="cuda")
+    k.stream_mix(streams, count, branch=branch, mix=mix.reshape(-1), write=write, read=read, gamma=gamma, eps=1e-5, normed_out=out, sum_out=total)
+    # float sums of at most nine products of order one, twice over
+    assert (streams.double() - want).abs().max() <= 2e-6 * (1 + want.abs().max())
+    assert (total.double() - want.sum(0)).abs().max() <= 4e-6 * (1 + want.abs().max())
+    assert ((out.double() - normed).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * normed.abs() + 1e-5 * (1 + normed.abs().max())).all()
