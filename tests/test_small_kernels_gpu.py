@@ -60,6 +60,33 @@ def test_decay_per_channel(n, rank, channels):
     assert (out.double() - torch.exp(-torch.exp(z))).abs().max() <= 1.5e-6
 
 
+# widths of one quad, of a block's first round and beyond it, and no multiple of 4
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hidden", [4, 516, 2052, 4096, 30])
+@pytest.mark.parametrize("pairs,places", [(True, True), (True, False), (False, True)])
+def test_embedding_sum(dtype, hidden, pairs, places):
+    k = lib(dtype)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    ids, positions = i32([3, 0, 12, 5, 13, 7]), i32([0, 1, 2, 9, 0, 20])            # three sequences; an id and a place too far
+    seq, cu, slots = i32([0, 0, 0, 1, 2, 2]), i32([0, 3, 4, 6]), i32([2, 0, 1])
+    table, pair, place = (torch.randn(rows, hidden, device="cuda").to(dtype) for rows in (13, 8, 15))
+    last = i32([6, 4, 0, 0, 0, 0])
+    out, flag = torch.full((6, hidden), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    k.embed_sum(table, ids, out, positions, seq, cu, slots, flag, pair_table=pair if pairs else None, last_ids=last if pairs else None, mul_prev=5,
+                mul_cur=3, position_table=place if places else None, position_scale=0.5)
+    previous = [None, 3, 0, 6, None, None]                                          # position 9 reads the entry of even places
+    for t, (id, position) in enumerate(zip(ids.tolist(), positions.tolist())):
+        want = table[id].float() if id < 13 else torch.zeros(hidden, device="cuda")
+        if pairs and id < 13:
+            before = 13 if t == 5 else previous[t]
+            want = want + pair[7 if position == 0 else (before * 5 + id * 3) % 7].float()
+        if places and position < 15:
+            want = want + place[position].float() * 0.5
+        torch.testing.assert_close(out[t], want, rtol=1e-6, atol=1e-6)
+    assert int(flag) == (9 if places else 1)
+    assert not pairs or last.tolist() == [6, 5, 7, 0, 12, 0]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("hidden", [4, 2048, 2052, 4096, 4100, 30])
 @pytest.mark.parametrize("count", [1, 2, 8])
