@@ -43,6 +43,45 @@ projection_norm_kernel(float* __restrict__ rows, int row_stride, float eps, cons
         x[c] = (x[c] + (seg.bias ? seg.bias[c] : 0.0f)) * factor * seg.weight[c];
 }
 
+// The same with a thread's share of a segment, QUADS times four neighbouring numbers at most, in registers between the sum and the
+// scaling (segments of whole 16 bytes and at most 4,096 numbers); bias and weight come ahead of the wait.  The kernel above reads
+// a segment twice, number by number.  Segments of 2,048 and 256, 4 / 3,900 tokens: 4.5 / 28 us above, 1.6 / 25 here; of 4,096 and
+// 1,024: 7.8 / 59 and 1.8 / 32.
+constexpr int NORM_THREADS = 512, NORM_QUADS = 2;
+__global__ void __launch_bounds__(NORM_THREADS)
+projection_norm_wide_kernel(float* __restrict__ rows, int row_stride, float eps, const NormSegment first, const NormSegment second) {
+    __shared__ float scratch[33];
+    const NormSegment seg = blockIdx.y == 0 ? first : second;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 weight[NORM_QUADS], v[NORM_QUADS];
+#pragma unroll
+    for (int q = 0; q < NORM_QUADS; ++q) {
+        const int c = 4 * (threadIdx.x + q * NORM_THREADS);
+        weight[q] = c < seg.width ? *(const float4*)(seg.weight + c) : zero;
+        v[q] = seg.bias && c < seg.width ? *(const float4*)(seg.bias + c) : zero;
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    float* x = rows + (size_t)blockIdx.x * row_stride + seg.offset;
+    float squares = 0.0f;
+#pragma unroll
+    for (int q = 0; q < NORM_QUADS; ++q) {
+        const int c = 4 * (threadIdx.x + q * NORM_THREADS);
+        if (c >= seg.width) continue;
+        const float4 u = *(const float4*)(x + c);
+        v[q].x += u.x; v[q].y += u.y; v[q].z += u.z; v[q].w += u.w;
+        squares = fmaf(v[q].x, v[q].x, fmaf(v[q].y, v[q].y, fmaf(v[q].z, v[q].z, fmaf(v[q].w, v[q].w, squares))));
+    }
+    const float factor = 1.0f / sqrtf(block_sum(squares, scratch) / (float)seg.width + eps);
+#pragma unroll
+    for (int q = 0; q < NORM_QUADS; ++q) {
+        const int c = 4 * (threadIdx.x + q * NORM_THREADS);
+        if (c < seg.width)
+            *(float4*)(x + c) = make_float4(v[q].x * factor * weight[q].x, v[q].y * factor * weight[q].y, v[q].z * factor * weight[q].z,
+                                            v[q].w * factor * weight[q].w);
+    }
+}
+
 struct ConvBatch {
     const int* positions;      // [tokens]
     const int* token_seq;      // [tokens]
@@ -159,6 +198,78 @@ short_conv_rotary_kernel(const float* __restrict__ rows, int row_stride, const f
     }
 }
 
+// The same for four taps, pairs (2i, 2i + 1), four neighbouring channels and TOK tokens a thread (head sizes and the rotated part
+// multiples of 4, rows 16-byte aligned): a row is read once for its four uses, the weights once for TOK tokens.  Bound by bytes
+// for many tokens, where a warp per (token, head) waited on two numbers a load.  36 heads of 64, 4 / 3,600 tokens: 3.4 / 59 us there, 3.1 / 22 here; 40 of 128: 5.2 / 114 and 3.2 / 42.
+template <typename T, int TOK>
+__global__ void __launch_bounds__(128)
+short_conv_rotary_wide_kernel(const float* __restrict__ rows, int row_stride, const float* __restrict__ bias,
+                              const float* __restrict__ conv_w, const float2* __restrict__ cos_sin, int rotated,
+                              const int* __restrict__ block_table, int table_width, T* __restrict__ q_out,
+                              T* __restrict__ k_cache, T* __restrict__ v_cache, int n_tokens, int num_heads, int num_kv_heads,
+                              int dim, int block_size, int write_kv, const ConvBatch batch) {
+    const int channels = (num_heads + num_kv_heads) * dim, q_width = num_heads * dim;
+    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x), t0 = blockIdx.y * TOK;
+    if (c >= channels || (c >= q_width && !write_kv)) return;
+    const float4 b = bias ? *(const float4*)(bias + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(conv_w + 4 * (size_t)(c + i));
+    pdl_launch_dependents();
+    pdl_wait();
+    float4 x[TOK + 3];
+#pragma unroll
+    for (int i = 0; i < TOK + 3; ++i) {
+        const int t = min(max(t0 + i - 3, 0), n_tokens - 1);
+        const float4 v = *(const float4*)(rows + (size_t)t * row_stride + c);
+        x[i] = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    }
+    const int head = c / dim, d = c - head * dim, half = rotated >> 1;
+#pragma unroll
+    for (int i = 0; i < TOK; ++i) {
+        const int t = t0 + i;
+        if (t >= n_tokens) break;
+        const int p = batch.positions[t], s = batch.token_seq[t], first = batch.cu_q[s];
+        float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int back = 3 - k;
+            if (p - back < 0) continue;
+            float4 v = x[i + k];
+            if (t - back < first)
+                v = *(const float4*)(batch.state + (size_t)batch.slot_ids[s] * batch.state_stride + batch.state_offset +
+                                     (size_t)((p - back) & 3) * channels + c);
+            sum.x = fmaf(k == 0 ? w[0].x : k == 1 ? w[0].y : k == 2 ? w[0].z : w[0].w, v.x, sum.x);
+            sum.y = fmaf(k == 0 ? w[1].x : k == 1 ? w[1].y : k == 2 ? w[1].z : w[1].w, v.y, sum.y);
+            sum.z = fmaf(k == 0 ? w[2].x : k == 1 ? w[2].y : k == 2 ? w[2].z : w[2].w, v.z, sum.z);
+            sum.w = fmaf(k == 0 ? w[3].x : k == 1 ? w[3].y : k == 2 ? w[3].z : w[3].w, v.w, sum.w);
+        }
+        float4 turned = sum;
+        if (d < rotated) {
+            const float4 cs = *(const float4*)(cos_sin + (size_t)p * half + (d >> 1));
+            turned = make_float4(sum.x * cs.x - sum.y * cs.y, sum.y * cs.x + sum.x * cs.y, sum.z * cs.z - sum.w * cs.w,
+                                 sum.w * cs.z + sum.z * cs.w);
+        }
+        alignas(16) const T result[4] = {from_float<T>(turned.x), from_float<T>(turned.y), from_float<T>(turned.z), from_float<T>(turned.w)};
+        alignas(16) const T before[4] = {from_float<T>(sum.x), from_float<T>(sum.y), from_float<T>(sum.z), from_float<T>(sum.w)};
+        T* out = q_out + (size_t)t * q_width + c;
+        T* plain = nullptr;
+        if (c >= q_width) {
+            const int block = block_table[(size_t)s * table_width + p / block_size];
+            const size_t at = (((size_t)block * num_kv_heads + head - num_heads) * block_size + (p % block_size)) * dim + d;
+            out = k_cache + at;
+            if (v_cache) plain = v_cache + at;
+        }
+        if (sizeof(T) == 4) {
+            *(uint4*)out = *(const uint4*)result;
+            if (plain) *(uint4*)plain = *(const uint4*)before;
+        } else {
+            *(uint2*)out = *(const uint2*)result;
+            if (plain) *(uint2*)plain = *(const uint2*)before;
+        }
+    }
+}
+
 // grid (sequences, channel chunks): rows of the ring for the step's last taps - 1 positions of every sequence.
 __global__ void __launch_bounds__(256)
 short_conv_remember_kernel(const float* __restrict__ rows, int row_stride, const float* __restrict__ bias, int channels,
@@ -188,6 +299,11 @@ SKV_EXPORT int skv_projection_norm(float* rows, int row_stride, int n, float eps
         (width_b > 0 && (!weight_b || offset_b < 0 || offset_b + width_b > row_stride)))
         return fail("skv_projection_norm", "segments must lie inside a row and have weights");
     const NormSegment first{offset_a, width_a, bias_a, weight_a}, second{offset_b, width_b, bias_b, weight_b};
+    const uintptr_t places = (uintptr_t)rows | (uintptr_t)bias_a | (uintptr_t)weight_a | (uintptr_t)bias_b | (uintptr_t)weight_b;
+    if (((row_stride | offset_a | width_a | (width_b > 0 ? offset_b | width_b : 0)) & 3) == 0 && (places & 15) == 0 &&
+        max(width_a, width_b) <= 4 * NORM_THREADS * NORM_QUADS)
+        return launch_pdl("skv_projection_norm", projection_norm_wide_kernel, dim3(n, width_b > 0 ? 2 : 1), dim3(NORM_THREADS), 0,
+                          stream, rows, row_stride, eps, first, second);
     return launch_pdl("skv_projection_norm", projection_norm_kernel, dim3(n, width_b > 0 ? 2 : 1), dim3(256), 0, stream,
                       rows, row_stride, eps, first, second);
 }
@@ -215,6 +331,18 @@ SKV_EXPORT int skv_short_conv_rotary(const float* rows, int row_stride, const fl
         return fail("skv_short_conv_rotary", "sizes do not agree");
     if (!rows || !q_out || !k_cache || !block_table || (taps > 0 && !conv_w) || (taps > 1 && !state) || (rotated > 0 && !cos_sin))
         return fail("skv_short_conv_rotary", "a pointer is missing");
+    const uintptr_t places = (uintptr_t)rows | (uintptr_t)bias | (uintptr_t)conv_w | (uintptr_t)cos_sin | (uintptr_t)q_out | (uintptr_t)k_cache |
+                             (uintptr_t)v_cache | (uintptr_t)state;
+    const int each = n >= 8 * sm_count() ? 8 : 1;                     // tokens a thread, once there are tokens for all threads
+    if (taps == 4 && (interleaved || rotated == 0) && ((dim | rotated | row_stride | state_stride | state_offset) & 3) == 0 && (places & 15) == 0 &&
+        (n + each - 1) / each <= 65535) {
+        const int quads = (num_heads + num_kv_heads) * dim / 4;
+        return launch_pdl("skv_short_conv_rotary", each == 8 ? short_conv_rotary_wide_kernel<skv_t, 8> : short_conv_rotary_wide_kernel<skv_t, 1>,
+                          dim3((quads + 127) / 128, (n + each - 1) / each), dim3(128), 0, stream, rows, row_stride, bias, conv_w,
+                          (const float2*)cos_sin, rotated, block_table, table_width, (skv_t*)q_out, (skv_t*)k_cache, (skv_t*)v_cache, n,
+                          num_heads, num_kv_heads, dim, block_size, write_kv,
+                          conv_batch(positions, token_seq, cu_q, slot_ids, state, state_stride, state_offset));
+    }
     const long long items = (long long)n * (num_heads + num_kv_heads);
     return launch_pdl("skv_short_conv_rotary", short_conv_rotary_kernel<skv_t>, dim3((unsigned)((items + 7) / 8)), dim3(256),
                       0, stream, rows, row_stride, bias, conv_w, taps, (const float2*)cos_sin, rotated, interleaved,

@@ -104,3 +104,56 @@ def test_streams_of_wide_rows(dtype, hidden, count):
     assert (streams.double() - want).abs().max() <= 2e-6 * (1 + want.abs().max())
     assert (total.double() - want.sum(0)).abs().max() <= 4e-6 * (1 + want.abs().max())
     assert ((out.double() - normed).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * normed.abs() + 1e-5 * (1 + normed.abs().max())).all()
+
+
+# segments inside a row, of one quad, of a block's first round and beyond it, of more than a block holds, and off 16 bytes
+@pytest.mark.parametrize("segments", [[(4, 4, True), (8, 516, False)], [(0, 2052, False), (2052, 256, True)], [(0, 4096, True)], [(0, 4100, False), (4100, 8, False)],
+                                      [(2, 256, True)], [(0, 30, False), (32, 64, True)]])
+@pytest.mark.parametrize("n", [1, 9])
+def test_norm_of_segments(n, segments):
+    k = lib()
+    rows = torch.randn(n, max(o + w for o, w, _ in segments) + 4 & ~3, device="cuda")
+    want, given = rows.double(), []
+    for offset, width, biased in segments:
+        bias, weight = torch.randn(width, device="cuda") if biased else None, torch.randn(width, device="cuda")
+        x = want[:, offset:offset + width] + (bias.double() if biased else 0.0)
+        want[:, offset:offset + width] = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * weight.double()
+        given.append((offset, width, bias, weight))
+    k.projection_norm(rows, 1e-5, given)
+    assert ((rows.double() - want).abs() <= 2e-6 * want.abs() + 1e-6).all()
+
+
+def packed(lengths, starts, slots):
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    cu = [0]
+    for length in lengths:
+        cu.append(cu[-1] + length)
+    return cu[-1], (i32([p + i for p, length in zip(starts, lengths) for i in range(length)]), i32([s for s, length in enumerate(lengths) for _ in range(length)]),
+                    i32(cu), i32(slots))
+
+
+STEPS = [([1, 1, 1], [0, 2, 9]), ([5, 1, 2, 70], [0, 1, 3, 0]), ([700, 3, 600, 1, 2], [0, 0, 5, 2, 1])]      # the last: eight tokens a thread
+
+
+# the forms of four channels a thread against the general ones, which a state (or row) off 16 bytes takes; the sums have one order
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,kv_heads,dim,rotated,aliased", [(32, 4, 64, 64, True), (3, 1, 20, 12, False), (2, 2, 4, 0, True)])
+@pytest.mark.parametrize("lengths,starts", STEPS)
+@pytest.mark.parametrize("biased,write", [(True, True), (False, False)])
+def test_short_convolution_forms(dtype, heads, kv_heads, dim, rotated, aliased, lengths, starts, biased, write):
+    k, channels, slots = lib(dtype), (heads + kv_heads) * dim, list(range(len(lengths), 0, -1))
+    n, meta = packed(lengths, starts, slots)
+    rows, conv_w = torch.randn(n, channels + 4, device="cuda"), torch.randn(channels, 4, device="cuda")
+    bias, rotation = torch.randn(channels, device="cuda") if biased else None, torch.randn(800, rotated // 2, 2, device="cuda") if rotated else None
+    ring, table = torch.randn(len(lengths) + 1, 4 * channels, device="cuda"), torch.randperm(50 * len(lengths), device="cuda").int().view(len(lengths), 50)
+    results = []
+    for offset in (4, 3):
+        state = torch.zeros(len(lengths) + 1, 4 * channels + 4, device="cuda")
+        state[:, offset:offset + 4 * channels] = ring
+        q = torch.full((n, heads * dim), 7.0, device="cuda").to(dtype)
+        caches = [torch.full((50 * len(lengths), kv_heads, 16, dim), 7.0, device="cuda").to(dtype) for _ in range(2)]
+        k.short_conv_rotary(rows, bias, conv_w, 4, rotation, rotated, True, table, q, caches[0], caches[1] if aliased else None, heads, kv_heads, dim, 16,
+                            write, meta, state, offset)
+        results.append([q] + caches)
+    for got, want in zip(*results):
+        torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-6, atol=2e-6)
