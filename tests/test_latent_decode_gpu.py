@@ -83,3 +83,51 @@ def test_attention_over_one_cached_row(heads, dim, vdim, lengths, block, splits)
         weight = torch.where(live, torch.exp(ml[..., 0] - ml[..., 0].max(dim=1, keepdim=True).values), 0.0)
         total = (weight[..., None] * torch.where(live[..., None], merged, 0.0)).sum(1) / (weight * torch.where(live, ml[..., 1], 0.0)).sum(1)[:, None]
         assert (total - torch.softmax(scores, dim=1) @ rows.double()[:, :vdim]).abs().max() <= 1e-5
+
+
+# every size in quads, tokens few (a token's queries in slices) and many, and sizes that are not
+@pytest.mark.parametrize("heads,dim,rope,latent,rotated", [(32, 96, 32, 256, 32), (2, 8, 12, 1028, 8), (9, 4, 8, 4, 0), (4, 48, 16, 64, 12), (3, 5, 6, 10, 4)])
+@pytest.mark.parametrize("n", [1, 7, 320])
+@pytest.mark.parametrize("whole", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_latent_finish(heads, dim, rope, latent, rotated, n, whole, dtype):
+    from stratakv_b200.ops import kernels_for
+    k, q_head, block_size = kernels_for(dtype, 64, verbose=False), dim + rope, 16
+    at = -(-heads * q_head // 4) * 4
+    fused = torch.randn(n, -(-(at + latent + rope) // 4) * 4 + 4, device="cuda")
+    positions = (torch.arange(n, device="cuda") * 7 % 48).int()
+    table = torch.randperm(n * 3, device="cuda").int().view(n, 3)
+    rotation = torch.randn(48, rotated // 2, 2, device="cuda") if rotated else None
+    gamma = torch.rand(latent, device="cuda") + 0.5
+    nan = lambda *shape: torch.full(shape, float("nan"), device="cuda").to(dtype)
+    plain, folded, together, cache = nan(n, heads * dim), nan(n, heads * (latent + rope)), nan(n, heads * q_head), nan(n * 3, 1, block_size, latent + rope)
+    for write in (True, False):
+        k.latent_finish(fused, None if whole else plain, None if whole else folded, cache, positions, torch.arange(n, device="cuda").int(), table, heads, dim,
+                        rope, latent, block_size, rotation, rotated, at, gamma, 1e-5, write, q_whole=together if whole else None)
+        kept = cache.clone() if write else kept
+
+    def turn(x):
+        if not rotated:
+            return x
+        c, s = rotation.double()[positions.long()].unbind(-1)
+        while c.dim() < x.dim():
+            c, s = c[:, None], s[:, None]
+        u, v = x[..., :rotated // 2], x[..., rotated // 2:rotated]
+        return torch.cat([u * c - v * s, v * c + u * s, x[..., rotated:]], -1)
+
+    rows = fused.double()
+    queries = rows[:, :heads * q_head].view(n, heads, q_head)
+    queries = torch.cat([queries[..., :dim], turn(queries[..., dim:])], -1)
+    vector = rows[:, at:at + latent]
+    vector = vector * torch.rsqrt((vector * vector).mean(-1, keepdim=True) + 1e-5) * gamma.double()
+    want = torch.cat([vector, turn(rows[:, at + latent:at + latent + rope])], -1)
+    error = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-6                 # one rounding, or a few of float
+    near = lambda got, ref: ((got.double() - ref).abs() <= error * ref.abs() + 4e-6).all()
+    if whole:
+        assert near(together.view(n, heads, q_head), queries)
+    else:
+        assert near(plain.view(n, heads, dim), queries[..., :dim])
+        assert near(folded.view(n, heads, -1)[..., latent:], queries[..., dim:]) and torch.isnan(folded.view(n, heads, -1)[..., :latent]).all()
+    blocks = table[torch.arange(n, device="cuda"), (positions // block_size).long()].long()
+    assert near(cache[blocks, 0, (positions % block_size).long()], want)
+    assert int((~torch.isnan(cache)).sum()) == n * (latent + rope) and torch.equal(cache.nan_to_num(), kept.nan_to_num())
