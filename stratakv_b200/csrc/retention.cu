@@ -12,7 +12,8 @@
 // step that runs twice (a graph's capture after its warm-up) computes the same thing both times.
 //
 // One token a sequence: one kernel, a block per (head, sequence), does all of it.  Longer steps: queries and keys are
-// rotated in place, then the sequence's tokens are cut into chunks of 32.  With S the state before a chunk of L tokens,
+// rotated in place, then the sequence's tokens are cut into chunks: on the kernels of the decayed matrix state
+// (linear_state.cu) where heads are whole tiles of 64, else, here, of 32 tokens.  With S the state before a chunk of L tokens,
 //   o_i    = a^(i+1) S^T q_i + sum_(j<=i) a^(i-j) (q_i . k_j) v_j             (i, j count within the chunk)
 //   S_next = a^L S + sum_j a^(L-1-j) k_j v_j^T
 // so a first kernel leaves every chunk's own sum (the second term of S_next), a second walks the chunks of a sequence
@@ -109,6 +110,90 @@ retention_decode_kernel(const float* __restrict__ fused, const float* __restrict
         float o = 0.0f;
 #pragma unroll
         for (int w = 0; w < RET_WARPS; ++w) o += partial[w * dv + e];
+        v[e] = o;                              // (each thread replaces the values it alone reads from here on)
+        squares = fmaf(o, o, squares);
+    }
+    const float factor = 1.0f / sqrtf(block_sum(squares, reduce) / (float)dv + eps);
+    const float* gate = row + (size_t)2 * H * d + (size_t)H * dv + (size_t)head * dv;
+    T* out_row = out + (size_t)t * out_stride + (size_t)head * dv;
+    for (int e = threadIdx.x; e < dv; e += RET_THREADS) {
+        const float g = gate[e];
+        out_row[e] = from_float<T>(v[e] * factor * (g / (1.0f + expf(-g))));
+    }
+    if (head == H - 1)
+        for (int c = H * dv + threadIdx.x; c < out_stride; c += RET_THREADS) out[(size_t)t * out_stride + c] = from_float<T>(0.0f);
+}
+
+// The same with a thread on four neighbouring value columns (dv a multiple of 4 that divides 1,024, the state on 16 bytes): the
+// state, which lies in HBM, is asked for as soon as its slot is known, eight rows of a thread at once, and q, k and v are made
+// while it comes; the kernel above waits for each row it has stored before it asks for the next.  8 sequences, 32 heads of 64 / 24 of 128: 12 / 36 us there, 4.6 / 9.0 here (2.6 / 5.8 of
+// them the state's bytes).
+template <typename T>
+__global__ void __launch_bounds__(RET_THREADS)
+retention_decode_wide_kernel(const float* __restrict__ fused, const float* __restrict__ rotation,
+                             const float* __restrict__ decay, float eps, T* __restrict__ out, int out_stride,
+                             const RetentionShape shape, const RetentionBatch batch) {
+    constexpr int AHEAD = 8;
+    extern __shared__ __align__(16) float ret_smem[];
+    const int H = shape.heads, d = shape.dim, dv = shape.vdim;
+    const int quads = dv / 4, stripes = RET_THREADS / quads;      // threads of a state row; rows at a time
+    float* partial = ret_smem;                // [stripes][dv]: 1,024 floats
+    float* v = partial + 4 * RET_THREADS;     // [dv]
+    float* q = v + dv;                        // [d]
+    float* k = q + d;                         // [d]
+    __shared__ float reduce[33];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.x, s = blockIdx.y;
+    const int t = batch.cu_q[s];
+    const int p = batch.positions[t];
+    const size_t half_size = (size_t)H * d * dv;
+    float* slot = batch.state + (size_t)batch.slot_ids[s] * batch.state_stride;
+    const int e4 = 4 * (threadIdx.x % quads), first = threadIdx.x / quads;
+    const float* before = slot + (size_t)((p - 1) & 1) * half_size + (size_t)head * d * dv + e4;
+    float* after = slot + (size_t)(p & 1) * half_size + (size_t)head * d * dv + e4;
+    float4 S[AHEAD];
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int j = j0 + u * stripes;
+            S[u] = p > 0 && j < d ? *(const float4*)(before + (size_t)j * dv) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    load(first);
+    const float* row = fused + (size_t)t * shape.row_stride;
+    const float* cos_sin = rotation ? rotation + (size_t)min(p, shape.table_len - 1) * shape.rotated : nullptr;
+    const int turn = rotation ? shape.rotated : 0;
+    const float key_scale = 1.0f / sqrtf((float)d);
+    for (int j = threadIdx.x; j < 2 * d + dv; j += RET_THREADS) {
+        if (j < d) q[j] = rotated_value(row + (size_t)head * d, j, turn, cos_sin);
+        else if (j < 2 * d) k[j - d] = rotated_value(row + (size_t)(H + head) * d, j - d, turn, cos_sin) * key_scale;
+        else v[j - 2 * d] = row[(size_t)2 * H * d + (size_t)head * dv + j - 2 * d];
+    }
+    __syncthreads();
+    const float a = decay[head];
+    const float4 ve = *(const float4*)(v + e4);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int j0 = first; j0 < d; j0 += AHEAD * stripes) {
+        if (j0 != first) load(j0);
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int j = j0 + u * stripes;
+            if (j >= d) break;
+            const float kj = k[j], qj = q[j];
+            const float4 fresh = make_float4(fmaf(a, S[u].x, kj * ve.x), fmaf(a, S[u].y, kj * ve.y), fmaf(a, S[u].z, kj * ve.z),
+                                             fmaf(a, S[u].w, kj * ve.w));
+            *(float4*)(after + (size_t)j * dv) = fresh;
+            acc.x = fmaf(fresh.x, qj, acc.x); acc.y = fmaf(fresh.y, qj, acc.y);
+            acc.z = fmaf(fresh.z, qj, acc.z); acc.w = fmaf(fresh.w, qj, acc.w);
+        }
+    }
+    *(float4*)(partial + first * dv + e4) = acc;
+    __syncthreads();
+    float squares = 0.0f;
+    for (int e = threadIdx.x; e < dv; e += RET_THREADS) {
+        float o = 0.0f;
+        for (int w = 0; w < stripes; ++w) o += partial[w * dv + e];
         v[e] = o;                              // (each thread replaces the values it alone reads from here on)
         squares = fmaf(o, o, squares);
     }
@@ -467,8 +552,9 @@ SKV_EXPORT int skv_retention(float* fused, int row_stride, const float* rotation
     const RetentionBatch batch = {positions, token_seq, cu_q, slot_ids, state, state_stride};
     if (max_q_len == 1) {
         if (n_tokens != n_seqs) return fail("skv_retention", "one token a sequence means as many tokens as sequences");
-        const size_t smem = (size_t)(2 * dim + vdim + RET_WARPS * vdim) * sizeof(float);
-        auto kernel = retention_decode_kernel<skv_t>;
+        const bool wide = vdim % 4 == 0 && (4 * RET_THREADS) % vdim == 0 && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
+        const size_t smem = (size_t)(2 * dim + vdim + (wide ? 4 * RET_THREADS : RET_WARPS * vdim)) * sizeof(float);
+        auto kernel = wide ? retention_decode_wide_kernel<skv_t> : retention_decode_kernel<skv_t>;
         if (int code = reserve_shared((const void*)kernel, smem, "skv_retention")) return code;
         return launch_pdl("skv_retention", kernel, dim3(heads, n_seqs), dim3(RET_THREADS), smem, stream,
                           (const float*)fused, rotation, decay, eps, (skv_t*)out, out_stride, shape, batch);
