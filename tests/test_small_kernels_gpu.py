@@ -157,3 +157,26 @@ def test_short_convolution_forms(dtype, heads, kv_heads, dim, rotated, aliased, 
         results.append([q] + caches)
     for got, want in zip(*results):
         torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-6, atol=2e-6)
+
+
+@pytest.mark.parametrize("channels,part", [(2048, 64), (260, 20), (4, 4)])
+@pytest.mark.parametrize("lengths,starts", STEPS)
+def test_recurrent_unit_forms(channels, part, lengths, starts):
+    k, slots = lib(), list(range(len(lengths), 0, -1))
+    n, meta = packed(lengths, starts, slots)
+    yx, conv_w = torch.randn(n, 2 * channels, device="cuda"), torch.randn(channels, 4, device="cuda")
+    x_bias, conv_b, y_bias, r_bias, i_bias, rate = (torch.randn(channels, device="cuda") for _ in range(6))
+    gates, kept = torch.randn(n, 2 * channels, device="cuda"), torch.randn(len(lengths) + 1, 6 * channels, device="cuda")
+    results = []
+    for spare in (0, 1):
+        state = torch.zeros(len(lengths) + 1, 6 * channels + spare, device="cuda")
+        state[:, :6 * channels] = kept
+        u = torch.full((n, channels), float("nan"), device="cuda")
+        k.rglru_conv(yx, channels, x_bias, conv_w, conv_b, u, meta, state)
+        # (the general form of the gates: rows that begin off 16 bytes)
+        mine = torch.zeros(n * 2 * channels + spare, device="cuda")[spare:].view(n, 2 * channels).copy_(gates)
+        y = yx.clone()
+        k.rglru_gates(mine, u, y, y_bias, r_bias, i_bias, rate.abs(), part)
+        results.append((u, mine.clone(), y))
+    for got, want in zip(*results):
+        torch.testing.assert_close(got, want, rtol=2e-6, atol=2e-6)
