@@ -360,6 +360,173 @@ time_mix_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, c
     }
 }
 
+// The recurrence for heads of 64 or 128 numbers in rows of whole 16 bytes.  A thread keeps a tile of the state, four key channels
+// by four value columns, so a token's r, k and w come from shared memory once for four columns; two channels ride in one
+// packed multiply-add.  o = S r + v (r u . k), the bracket once for all columns.  The columns' sums over the DIM / 4 lanes of
+// a head's channels wait for four tokens: the sixteen of them are halved from lane to lane, 15 shuffles in place of 64.
+// Bound by issue (the kernel above: a column a thread, 95 instructions a token for what 55 do here, its copies four bytes at a time).
+// 32 heads of 64, 4 sequences of 1,024 tokens 445 us there, 200 here, 2,000 tokens alone 560 and 199, 16 of 200 348 and 106, 4 of one 8.0 and 4.3; 24 of
+// 128, 16 of 200 1,094 and 310.
+constexpr __host__ __device__ int tm_tile_tokens(int dim) { return dim <= 64 ? 16 : 8; }          // two staged sets within 48 KB
+
+__device__ __forceinline__ uint64_t tm_pair(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 tm_unpair(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ uint64_t tm_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ uint64_t tm_mul2(uint64_t a, uint64_t b) {
+    uint64_t v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+
+__device__ __forceinline__ void tm_copy16_async(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+template <typename T, int DIM>
+__global__ void __launch_bounds__(256)
+time_mix_scan_tile_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v,
+                          const float* __restrict__ decay, int stride, const float* __restrict__ bonus,
+                          float* __restrict__ out, const T* __restrict__ h, int hidden, int heads, int cols,
+                          const TimeMixBatch batch) {
+    constexpr int PARTS = DIM / 4, QUADS = DIM / 4, TM_TILE_TOKENS = tm_tile_tokens(DIM);
+    extern __shared__ __align__(16) float tm_stage[];     // two sets of [tokens][DIM] r, k, w and [tokens][cols] v
+    const int head = blockIdx.y, col0 = blockIdx.z * cols;
+    const int part = threadIdx.x % PARTS, group = threadIdx.x / PARTS;
+    const float4 u = *(const float4*)(bonus + (size_t)head * DIM + 4 * part);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int seq = blockIdx.x;
+    const int first = batch.cu_q[seq], n = batch.cu_q[seq + 1] - first;
+    if (n <= 0) return;
+    const size_t at_head = (size_t)first * stride + (size_t)head * DIM;
+    const int set = TM_TILE_TOKENS * (3 * DIM + cols);
+    auto stage = [&](int which, int t0) {
+        float* sr = tm_stage + which * set;
+        const int m = min(TM_TILE_TOKENS, n - t0);
+        for (int idx = threadIdx.x; idx < m * QUADS; idx += blockDim.x) {
+            const int tok = idx / QUADS, i = 4 * (idx % QUADS);
+            const size_t at = at_head + (size_t)(t0 + tok) * stride + i;
+            float* to = sr + tok * DIM + i;
+            tm_copy16_async(to, r + at);
+            tm_copy16_async(to + TM_TILE_TOKENS * DIM, k + at);
+            tm_copy16_async(to + 2 * TM_TILE_TOKENS * DIM, decay + at);
+        }
+        const int v_quads = cols / 4;
+        for (int idx = threadIdx.x; idx < m * v_quads; idx += blockDim.x) {
+            const int tok = idx / v_quads, i = 4 * (idx - tok * v_quads);
+            tm_copy16_async(sr + 3 * TM_TILE_TOKENS * DIM + tok * cols + i, v + at_head + (size_t)(t0 + tok) * stride + col0 + i);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0, 0);
+
+    const int p0 = batch.positions[first];
+    float* slot_state = batch.state + (size_t)batch.slot_ids[seq] * batch.state_stride + batch.state_offset;
+    const size_t half = (size_t)heads * DIM * DIM, mine = ((size_t)head * DIM + 4 * part) * DIM + col0 + 4 * group;
+    const float* s_read = slot_state + (size_t)((p0 - 1) & 1) * half + mine;
+    float* s_write = slot_state + (size_t)((p0 + n - 1) & 1) * half + mine;
+    uint64_t S[2][4];                                     // [channels 0, 1 and 2, 3][column]
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        if (p0 > 0) { lo = *(const float4*)(s_read + (2 * a) * DIM); hi = *(const float4*)(s_read + (2 * a + 1) * DIM); }
+        S[a][0] = tm_pair(lo.x, hi.x); S[a][1] = tm_pair(lo.y, hi.y); S[a][2] = tm_pair(lo.z, hi.z); S[a][3] = tm_pair(lo.w, hi.w);
+    }
+    const uint64_t u01 = tm_pair(u.x, u.y), u23 = tm_pair(u.z, u.w);
+
+    int which = 0;
+    for (int t0 = 0; t0 < n; t0 += TM_TILE_TOKENS, which ^= 1) {
+        if (t0 + TM_TILE_TOKENS < n) {
+            stage(which ^ 1, t0 + TM_TILE_TOKENS);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const float* sr = tm_stage + which * set + 4 * part;
+        const float* sv = tm_stage + which * set + 3 * TM_TILE_TOKENS * DIM + 4 * group;
+        const int m = min(TM_TILE_TOKENS, n - t0);
+        // one token: what it gives this thread's four columns, and the new S
+        auto work = [&](int tok, float* sum) {
+            const ulonglong2 r2 = *(const ulonglong2*)(sr + tok * DIM);
+            const ulonglong2 k2 = *(const ulonglong2*)(sr + (TM_TILE_TOKENS + tok) * DIM);
+            const ulonglong2 w2 = *(const ulonglong2*)(sr + (2 * TM_TILE_TOKENS + tok) * DIM);
+            const float4 v4 = *(const float4*)(sv + tok * cols);
+            const float2 own = tm_unpair(tm_fma2(tm_mul2(r2.y, u23), k2.y, tm_mul2(tm_mul2(r2.x, u01), k2.x)));
+            const float bracket = own.x + own.y;
+            const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const uint64_t vv = tm_pair(vs[b], vs[b]);
+                const float2 before = tm_unpair(tm_fma2(r2.y, S[1][b], tm_mul2(r2.x, S[0][b])));
+                S[0][b] = tm_fma2(w2.x, S[0][b], tm_mul2(k2.x, vv));
+                S[1][b] = tm_fma2(w2.y, S[1][b], tm_mul2(k2.y, vv));
+                sum[b] = fmaf(bracket, vs[b], before.x + before.y);
+            }
+        };
+        float* to = out + at_head + (size_t)t0 * stride + col0 + 4 * group;
+        int tok0 = 0;
+        for (; tok0 + 4 <= m; tok0 += 4) {
+            float sum[16];                                // [token][column]
+#pragma unroll
+            for (int q = 0; q < 4; ++q) work(tok0 + q, sum + 4 * q);
+            // each step a lane keeps the half of its sums that its bit of `part` names and gives the other half away
+            int kept = 16;
+#pragma unroll
+            for (int offset = PARTS / 2; offset > 0; offset >>= 1) {
+                if (kept > 1) {
+                    kept >>= 1;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (j >= kept) continue;
+                        const bool upper = part & offset;
+                        const float give = upper ? sum[j] : sum[kept + j];
+                        sum[j] = (upper ? sum[kept + j] : sum[j]) + __shfl_xor_sync(0xffffffffu, give, offset);
+                    }
+                } else {
+                    sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], offset);
+                }
+            }
+            const int which_sum = part / (PARTS / 16);
+            if (part % (PARTS / 16) == 0) to[(size_t)(tok0 + (which_sum >> 2)) * stride + (which_sum & 3)] = sum[0];
+        }
+#pragma unroll 1
+        for (; tok0 < m; ++tok0) {                        // the tokens behind the last four (a step of one token: all)
+            float sum[4];
+            work(tok0, sum);
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int offset = PARTS / 2; offset > 0; offset >>= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], offset);
+            if (part == 0) *(float4*)(to + (size_t)tok0 * stride) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        }
+        __syncthreads();                                  // before the next round's copies land in this set
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        const float2 c0 = tm_unpair(S[a][0]), c1 = tm_unpair(S[a][1]), c2 = tm_unpair(S[a][2]), c3 = tm_unpair(S[a][3]);
+        *(float4*)(s_write + (2 * a) * DIM) = make_float4(c0.x, c1.x, c2.x, c3.x);
+        *(float4*)(s_write + (2 * a + 1) * DIM) = make_float4(c0.y, c1.y, c2.y, c3.y);
+    }
+    // the mixer's input at the sequence's last token: a share of it from each of the sequence's blocks
+    float* kept = slot_state + 2 * half + (size_t)((p0 + n - 1) & 1) * hidden;
+    const T* last = h + (size_t)(first + n - 1) * hidden;
+    for (int w = (head * gridDim.z + blockIdx.z) * blockDim.x + threadIdx.x; w < hidden; w += gridDim.y * gridDim.z * blockDim.x)
+        kept[w] = to_float(last[w]);
+}
+
 // out[t][head] = o / rms(o) * norm * silu(gate) * out_scale; a warp per (token, head).
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -384,6 +551,48 @@ time_mix_finish_kernel(const float* __restrict__ o, const float* __restrict__ ga
     }
     if (head == heads - 1)                              // columns that pad the row to whole 16 bytes
         for (int d = heads * dim + lane; d < out_stride; d += 32) out[(size_t)t * out_stride + d] = from_float<T>(0.0f);
+}
+
+// The same for heads of 16, 32, 64 or 128 numbers (rows 16-byte aligned): a warp takes 512 neighbouring numbers of a token, four
+// loads of 16 bytes of each operand on their way a lane, and a head's numbers lie in dim / 4 neighbouring lanes.  Bound by bytes;
+// the kernel above has two numbers of either on their way: 3,600 tokens of 32 heads of 64 45 us there, 18 here.
+template <typename T>
+__global__ void __launch_bounds__(256)
+time_mix_finish_wide_kernel(const float* __restrict__ o, const float* __restrict__ gate, int stride,
+                            const float* __restrict__ norm, float eps, float out_scale, T* __restrict__ out, int out_stride,
+                            int n_tokens, int heads, int dim) {
+    const int lane = threadIdx.x & 31, width = heads * dim, per_token = (width + 511) / 512;
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int t = (int)(item / per_token), c0 = 512 * (int)(item - (long long)t * per_token) + 4 * lane;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 w[4], x[4], z[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = c0 + 128 * i < width ? *(const float4*)(norm + c0 + 128 * i) : zero;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (t >= n_tokens) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool inside = c0 + 128 * i < width;
+        x[i] = inside ? *(const float4*)(o + (size_t)t * stride + c0 + 128 * i) : zero;
+        z[i] = inside ? *(const float4*)(gate + (size_t)t * stride + c0 + 128 * i) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float squares = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
+        for (int offset = dim >> 3; offset > 0; offset >>= 1) squares += __shfl_xor_sync(0xffffffffu, squares, offset);
+        const float factor = out_scale / sqrtf(squares / (float)dim + eps);
+        if (c0 + 128 * i >= width) continue;
+        const float v[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, g[4] = {z[i].x, z[i].y, z[i].z, z[i].w}, n[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+        alignas(16) T result[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) result[e] = from_float<T>(v[e] * factor * n[e] * (g[e] / (1.0f + expf(-g[e]))));
+        T* to = out + (size_t)t * out_stride + c0 + 128 * i;
+        if (sizeof(T) == 4) *(uint4*)to = *(const uint4*)result;
+        else *(uint2*)to = *(const uint2*)result;
+    }
+    if (c0 == 4 * lane)                                 // columns that pad the row to whole 16 bytes
+        for (int d = width + lane; d < out_stride; d += 32) out[(size_t)t * out_stride + d] = from_float<T>(0.0f);
 }
 
 }  // namespace skv
@@ -453,9 +662,22 @@ SKV_EXPORT int skv_time_mix_scan(const float* r, const float* k, const float* v,
     if (heads <= 0 || dim <= 0 || dim > 32 * TM_REGS || heads > 65535)
         return fail("skv_time_mix_scan", "heads of 1 to 512 numbers are served");
     if (!r || !k || !v || !decay || !bonus || !out || !h || !state) return fail("skv_time_mix_scan", "a pointer is missing");
+    const long long blocks = (long long)n_seqs * heads;
+    const uintptr_t places = (uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)decay | (uintptr_t)bonus | (uintptr_t)state |
+                             (uintptr_t)out;
+    if ((dim == 64 || dim == 128) && (places & 15) == 0 && ((stride | state_stride | state_offset) & 3) == 0) {
+        // a block of at most 256 threads, with fewer columns (each block of a head stages all its r, k and w again) until there
+        // are two blocks an SM
+        int cols = 4 * 256 / (dim / 4);
+        while (cols > 16 && blocks * (dim / cols) < 2 * sm_count()) cols /= 2;
+        const size_t smem = 2 * (size_t)tm_tile_tokens(dim) * (3 * dim + cols) * sizeof(float);
+        const TimeMixBatch batch = time_mix_batch(positions, token_seq, cu_q, slot_ids, state, state_stride, state_offset);
+        return launch_pdl("skv_time_mix_scan", dim == 64 ? time_mix_scan_tile_kernel<skv_t, 64> : time_mix_scan_tile_kernel<skv_t, 128>,
+                          dim3(n_seqs, heads, dim / cols), dim3(cols / 4 * (dim / 4)), smem, stream, r, k, v, decay, stride, bonus, out,
+                          (const skv_t*)h, hidden, heads, cols, batch);
+    }
     // Few blocks (one prompt alone): four key channels a thread, so that a head's work spreads over four times the
     // threads; else sixteen.
-    const long long blocks = (long long)n_seqs * heads;
     const int regs = blocks * 4 <= sm_count() * 2 && dim <= 128 ? 4 : TM_REGS;
     int key_split = 1;
     while (key_split * regs < dim) key_split *= 2;
@@ -491,6 +713,13 @@ SKV_EXPORT int skv_time_mix_finish(const float* o, const float* gate, int stride
     if (heads <= 0 || dim <= 0 || out_stride < heads * dim) return fail("skv_time_mix_finish", "sizes do not agree");
     if (!o || !gate || !norm || !out) return fail("skv_time_mix_finish", "a pointer is missing");
     const long long items = (long long)n * heads;
+    const uintptr_t places = (uintptr_t)o | (uintptr_t)gate | (uintptr_t)norm | (uintptr_t)out;
+    // (few tokens: a warp a head has the shorter chain, 4 of 32 heads of 64 2.5 us against 3.3)
+    if (n >= 2 * sm_count() && (dim == 16 || dim == 32 || dim == 64 || dim == 128) && ((stride | out_stride) & 3) == 0 && (places & 15) == 0) {
+        const long long warps = (long long)n * ((heads * dim + 511) / 512);
+        return launch_pdl("skv_time_mix_finish", time_mix_finish_wide_kernel<skv_t>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0,
+                          stream, o, gate, stride, norm, eps, out_scale, (skv_t*)out, out_stride, n, heads, dim);
+    }
     return launch_pdl("skv_time_mix_finish", time_mix_finish_kernel<skv_t>, dim3((unsigned)((items + 7) / 8)), dim3(256), 0,
                       stream, o, gate, stride, norm, eps, out_scale, (skv_t*)out, out_stride, n, heads, dim);
 }

@@ -106,6 +106,51 @@ def test_streams_of_wide_rows(dtype, hidden, count):
     assert ((out.double() - normed).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * normed.abs() + 1e-5 * (1 + normed.abs().max())).all()
 
 
+# lengths below, at and beyond four tokens and a staged set of sixteen; a state to go on from and none; steps of few sequences (a
+# head's columns in slices) and of many; a state that does not lie on 16 bytes (the form of other head sizes)
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("lengths,heads", [([1], 2), ([35], 3), ([16, 1, 4, 33, 2, 17], 2), ([5] * 40, 8)])
+@pytest.mark.parametrize("offset", [0, 4, 2])
+def test_time_mix_scan(dim, lengths, heads, offset):
+    k = lib()
+    n, inner, hidden, seqs = sum(lengths), heads * dim, 24, len(lengths)
+    starts = [0 if s % 2 == 0 else 3 + s for s in range(seqs)]
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    cu = [0]
+    for length in lengths:
+        cu.append(cu[-1] + length)
+    slots = list(range(seqs, 0, -1))
+    meta = (i32([p + i for p, length in zip(starts, lengths) for i in range(length)]), i32([s for s, length in enumerate(lengths) for _ in range(length)]),
+            i32(cu), i32(slots))
+    rows = torch.randn(4, n, inner, device="cuda")
+    r, key, value = rows[0], rows[1] / 8, rows[2]
+    decay, bonus = torch.rand(n, inner, device="cuda"), torch.rand(inner, device="cuda")
+    floats = k.time_mix_state_floats(hidden, heads, dim)
+    state = torch.randn(seqs + 1, 4 + -(-floats // 4) * 4, device="cuda")
+    before, half = state.double(), heads * dim * dim
+    out, h = torch.full((n, inner), float("nan"), device="cuda"), torch.randn(n, hidden, device="cuda").bfloat16()
+    k.time_mix_scan(r, key, value, decay, bonus, out, h, seqs, heads, dim, meta, state, offset)
+    per_head = lambda t: t.double().view(-1, heads, dim)
+    for s in range(seqs):
+        p0, last = starts[s], starts[s] + lengths[s] - 1
+        S = torch.zeros(heads, dim, dim, device="cuda", dtype=torch.float64)
+        if p0 > 0:
+            S = before[slots[s], offset + ((p0 - 1) & 1) * half:][:half].view(heads, dim, dim).clone()
+        size = torch.ones_like(S)
+        for t in range(cu[s], cu[s + 1]):
+            rt, kt, vt, wt = (per_head(a[t])[0] for a in (r, key, value, decay))
+            kv = kt[:, :, None] * vt[:, None, :]
+            want = torch.einsum("hi,hij->hj", rt, S + bonus.double().view(heads, dim, 1) * kv)
+            mass = torch.einsum("hi,hij->hj", rt.abs(), S.abs() + kv.abs())
+            S = wt[:, :, None] * S + kv
+            # float sums of dim products, each with a few roundings behind it
+            assert ((per_head(out[t])[0] - want).abs() <= 1e-6 * mass + 1e-6).all()
+        got = state[slots[s], offset + (last & 1) * half:][:half].double().view(heads, dim, dim)
+        assert ((got - S).abs() <= 2e-6 * (1 + S.abs())).all()
+        kept = state[slots[s], offset + 2 * half + (last & 1) * hidden:][:hidden]
+        assert torch.equal(kept, h[cu[s + 1] - 1].float())
+
+
 # segments inside a row, of one quad, of a block's first round and beyond it, of more than a block holds, and off 16 bytes
 @pytest.mark.parametrize("segments", [[(4, 4, True), (8, 516, False)], [(0, 2052, False), (2052, 256, True)], [(0, 4096, True)], [(0, 4100, False), (4100, 8, False)],
                                       [(2, 256, True)], [(0, 30, False), (32, 64, True)]])
@@ -180,3 +225,17 @@ def test_recurrent_unit_forms(channels, part, lengths, starts):
         results.append((u, mine.clone(), y))
     for got, want in zip(*results):
         torch.testing.assert_close(got, want, rtol=2e-6, atol=2e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,dim", [(32, 64), (3, 128), (5, 16), (1, 32), (4, 48)])
+@pytest.mark.parametrize("n", [1, 9])
+def test_time_mix_finish(dtype, heads, dim, n):
+    k, width = lib(dtype), heads * dim
+    o, gate, norm = torch.randn(n, width, device="cuda"), torch.randn(n, width, device="cuda"), torch.rand(width, device="cuda") + 0.5
+    out = torch.full((n, width + 8), float("nan"), device="cuda").to(dtype)
+    k.time_mix_finish(o, gate, norm, 1e-5, 1.3, out, heads, dim)
+    x = o.double().view(n, heads, dim)
+    want = (x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5)).view(n, width) * norm.double() * 1.3 * torch.nn.functional.silu(gate.double())
+    assert ((out[:, :width].double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 3e-6) * want.abs() + 1e-6).all()
+    assert (out[:, width:] == 0).all()
