@@ -417,7 +417,7 @@ linear_state_carry_kernel(float* __restrict__ sums, const float* __restrict__ fa
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i)
             if (c0 + i < chunks) {
-                store(cell + (size_t)(c0 + i) * half_size, S);
+                if (c0 + i > 0 || p_first > 0) store(cell + (size_t)(c0 + i) * half_size, S);      // (nobody reads the zeros before a first token)
 #pragma unroll
                 for (int v = 0; v < V; ++v) S[v] = fmaf(f[i], S[v], own[i][v]);
             }
@@ -464,11 +464,13 @@ __device__ __forceinline__ void load_transposed(float* to, const float* __restri
 
 // The outputs of one chunk of one head; sums holds the state before every chunk (what linear_state_carry_kernel left).
 // Threads in 16 x 16, each with CH / 16 tokens and four columns.  n_pad: dim rounded up to a multiple of 4.
-template <int CH>
-__global__ void __launch_bounds__(LS_THREADS)
+// HEADS neighbouring heads a block, which share their queries and keys: those are read, and their products made, once (16 sequences of
+// about 150 tokens, 128 heads of 128 x 64 in 8 groups: all three kernels 975 us before, 714 so).  The first chunk of a sequence without a state skips the state.
+template <int CH, int HEADS>
+__global__ void __launch_bounds__(LS_THREADS, CH == 64 ? 2 : 1)
 linear_state_output_kernel(const float* __restrict__ rows, const float* __restrict__ sums, float* __restrict__ out,
                            int max_chunks, int n_pad, const LinearStateShape shape, const LinearStateDecay decay,
-                           const int* __restrict__ cu_q) {
+                           const int* __restrict__ cu_q, const int* __restrict__ positions) {
     extern __shared__ __align__(16) float ls_smem[];
     constexpr int LD = CH + 4, RI = CH / 16;              // a thread's tokens, and its keys in the scores
     const int H = shape.heads, N = shape.dim, P = shape.vdim;
@@ -484,201 +486,212 @@ linear_state_output_kernel(const float* __restrict__ rows, const float* __restri
     float* factor = spans + 16;                           // [CH]: what a token's output is multiplied by
     pdl_launch_dependents();
     pdl_wait();
-    const int chunk = blockIdx.x, head = blockIdx.y, s = blockIdx.z, g = head / (H / shape.groups);
+    const int chunk = blockIdx.x, s = blockIdx.z, g = blockIdx.y * HEADS / (H / shape.groups);
     const int first = cu_q[s] + chunk * CH, L = min(CH, cu_q[s + 1] - first);
     if (L <= 0) return;
+    const bool fresh = chunk == 0 && positions[first] == 0;          // no state before this chunk
     const bool vec_qk = ((shape.row_stride | shape.q_at | shape.k_at | N) & 3) == 0;
     const bool vec_v = ((shape.row_stride | shape.v_at | P) & 3) == 0 && (!decay.floor || ((H * N) & 3) == 0);
     const float* base = rows + (size_t)first * shape.row_stride;
-    if (threadIdx.x < 32) {
-        chunk_exponents<CH>(l, c, up_to, behind, decay, H, head, first, L);
-        __syncwarp();
-        if (threadIdx.x < 16) {
-            float sum = 0.0f;
-#pragma unroll
-            for (int x = 0; x < RI; ++x) sum += l[threadIdx.x * RI + x];
-            spans[threadIdx.x] = sum;
-        }
-    }
-    load_transposed<CH, LD>(qT, base + shape.q_at + g * N, shape.row_stride, N, n_pad, L, shape.silu, vec_qk);
-    load_transposed<CH, LD>(kT, base + shape.k_at + g * N, shape.row_stride, N, n_pad, L, shape.silu, vec_qk);
-    __syncthreads();
     const bool constant = decay.decay != nullptr;
     const int tx = tile_x(), ty = tile_y();
     const int i0 = ty * RI, j0 = tx * RI;
-    {
-        float acc[RI][RI];
+    float score[RI][RI];                                  // the queries' products with the keys, which all the block's heads share
 #pragma unroll
-        for (int a = 0; a < RI; ++a)
+    for (int a = 0; a < RI; ++a)
 #pragma unroll
-            for (int b = 0; b < RI; ++b) acc[a][b] = 0.0f;
-        if (j0 <= i0) {
+        for (int b = 0; b < RI; ++b) score[a][b] = 0.0f;
+#pragma unroll 1
+    for (int which = 0; which < HEADS; ++which) {
+        const int head = blockIdx.y * HEADS + which;
+        if (which > 0) __syncthreads();                   // the head before is through with shared memory
+        if (threadIdx.x < 32) {
+            chunk_exponents<CH>(l, c, up_to, behind, decay, H, head, first, L);
+            __syncwarp();
+            if (threadIdx.x < 16) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int x = 0; x < RI; ++x) sum += l[threadIdx.x * RI + x];
+                spans[threadIdx.x] = sum;
+            }
+        }
+        if (which == 0) {
+            load_transposed<CH, LD>(qT, base + shape.q_at + g * N, shape.row_stride, N, n_pad, L, shape.silu, vec_qk);
+            load_transposed<CH, LD>(kT, base + shape.k_at + g * N, shape.row_stride, N, n_pad, L, shape.silu, vec_qk);
+        }
+        __syncthreads();
+        {
+            if (which == 0 && j0 <= i0) {
 #pragma unroll 4
-            for (int n = 0; n < n_pad; ++n) {
-                float qi[RI], kj[RI];
-                if (RI == 4) {
-                    const float4 a = *(const float4*)(qT + n * LD + i0), b = *(const float4*)(kT + n * LD + j0);
-                    qi[0] = a.x; qi[1 % RI] = a.y; qi[2 % RI] = a.z; qi[3 % RI] = a.w;
-                    kj[0] = b.x; kj[1 % RI] = b.y; kj[2 % RI] = b.z; kj[3 % RI] = b.w;
-                } else {
+                for (int n = 0; n < n_pad; ++n) {
+                    float qi[RI], kj[RI];
+                    if (RI == 4) {
+                        const float4 a = *(const float4*)(qT + n * LD + i0), b = *(const float4*)(kT + n * LD + j0);
+                        qi[0] = a.x; qi[1 % RI] = a.y; qi[2 % RI] = a.z; qi[3 % RI] = a.w;
+                        kj[0] = b.x; kj[1 % RI] = b.y; kj[2 % RI] = b.z; kj[3 % RI] = b.w;
+                    } else {
 #pragma unroll
-                    for (int a = 0; a < RI; ++a) { qi[a] = qT[n * LD + i0 + a]; kj[a] = kT[n * LD + j0 + a]; }
+                        for (int a = 0; a < RI; ++a) { qi[a] = qT[n * LD + i0 + a]; kj[a] = kT[n * LD + j0 + a]; }
+                    }
+#pragma unroll
+                    for (int a = 0; a < RI; ++a)
+#pragma unroll
+                        for (int b = 0; b < RI; ++b) score[a][b] = fmaf(qi[a], kj[b], score[a][b]);
+                }
+            }
+            // the exponents between: what lies between the two tiles, then the tokens inside either
+            float between = 0.0f;
+            if (!constant && j0 < i0) {
+                for (int x = tx + 1; x < ty; ++x) between += spans[x];
+                between += l[i0];
+            }
+#pragma unroll
+            for (int b = 0; b < RI; ++b) {
+                const int j = j0 + b;
+                float sum = between;
+                if (j0 < i0) {
+#pragma unroll
+                    for (int x = RI - 1; x > 0; --x)
+                        if (x > b) sum += l[j0 + x];
                 }
 #pragma unroll
-                for (int a = 0; a < RI; ++a)
-#pragma unroll
-                    for (int b = 0; b < RI; ++b) acc[a][b] = fmaf(qi[a], kj[b], acc[a][b]);
+                for (int a = 0; a < RI; ++a) {
+                    const int i = i0 + a;
+                    float weight = 0.0f;
+                    if (j <= i && i < L) {
+                        float exponent;
+                        if (constant) {
+                            exponent = i == j ? 0.0f : (float)(i - j) * l[0];
+                        } else if (j0 < i0) {
+                            if (a > 0) sum += l[i];
+                            exponent = sum;
+                        } else {
+                            exponent = 0.0f;
+                            for (int x = j + 1; x <= i; ++x) exponent += l[x];
+                        }
+                        weight = score[a][b] * expf(exponent) * c[j];
+                    }
+                    wT[j * LD + i] = weight;
+                }
             }
         }
-        // the exponents between: what lies between the two tiles, then the tokens inside either
-        float between = 0.0f;
-        if (!constant && j0 < i0) {
-            for (int x = tx + 1; x < ty; ++x) between += spans[x];
-            between += l[i0];
-        }
+        float carry[RI];
 #pragma unroll
-        for (int b = 0; b < RI; ++b) {
-            const int j = j0 + b;
-            float sum = between;
-            if (j0 < i0) {
-#pragma unroll
-                for (int x = RI - 1; x > 0; --x)
-                    if (x > b) sum += l[j0 + x];
+        for (int a = 0; a < RI; ++a) carry[a] = i0 + a < L ? up_to[i0 + a] : 0.0f;
+        const float skip = decay.skip ? decay.skip[head] : 0.0f;
+        const float* chunk_before = sums + ((size_t)s * max_chunks + chunk) * ls_half(shape, decay);
+        const float* before = chunk_before + (size_t)head * N * P;
+        if (decay.floor) {
+            __syncthreads();                                  // (the scores are in place)
+            if (threadIdx.x < 4 * CH) {
+                const float* n_before = chunk_before + (size_t)H * N * P + (size_t)head * N;
+                const int i = threadIdx.x >> 2, part = threadIdx.x & 3;
+                float dot = 0.0f, own = 0.0f;
+                if (!fresh)
+                    for (int n = part; n < N; n += 4) dot = fmaf(qT[n * LD + i], n_before[n], dot);
+                for (int j = part; j <= i; j += 4) own += wT[j * LD + i];
+                dot = i < L ? fmaf(dot, up_to[i], own) : 0.0f;
+                dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+                dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+                if (part == 0)
+                    factor[i] = i < L ? decay.out_scale / (fmaxf(fabsf(dot * decay.out_scale), decay.floor[(size_t)(first + i) * H + head]) + decay.floor_eps) : 0.0f;
             }
+        } else if (threadIdx.x < CH) {
+            factor[threadIdx.x] = decay.out_scale;
+        }
+        float* st = kT;
+        const int j_end = min(L, ((ty | 3) + 1) * RI);        // (the four rows of threads of a warp walk the same keys)
+        for (int e0 = 0; e0 < P; e0 += 64) {
+            __syncthreads();                                  // the scores are in place; the tiles before have been read
+            if (vec_v) {
+#pragma unroll
+                for (int idx = threadIdx.x; idx < CH * 16; idx += LS_THREADS) {
+                    const int j = idx >> 4, e = (idx & 15) * 4;
+                    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (j < L && e0 + e < P) {
+                        x = *(const float4*)(base + (size_t)j * shape.row_stride + shape.v_at + head * P + e0 + e);
+                        if (shape.silu) x = make_float4(ls_silu(x.x), ls_silu(x.y), ls_silu(x.z), ls_silu(x.w));
+                    }
+                    *(float4*)(vs + j * 64 + e) = x;
+                }
+                const int state_quads = fresh ? 0 : N * 16;
+#pragma unroll 8
+                for (int idx = threadIdx.x; idx < state_quads; idx += LS_THREADS) {
+                    const int n = idx >> 4, e = (idx & 15) * 4;
+                    *(float4*)(st + n * 64 + e) = e0 + e < P ? *(const float4*)(before + (size_t)n * P + e0 + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            } else {
+                for (int idx = threadIdx.x; idx < CH * 64; idx += LS_THREADS) {
+                    const int j = idx >> 6, e = idx & 63;
+                    vs[idx] = j < L && e0 + e < P ? ls_read(base + (size_t)j * shape.row_stride + shape.v_at + head * P + e0 + e, shape.silu) : 0.0f;
+                }
+                for (int idx = threadIdx.x; idx < (fresh ? 0 : N * 64); idx += LS_THREADS) {
+                    const int n = idx >> 6, e = idx & 63;
+                    st[idx] = e0 + e < P ? before[(size_t)n * P + e0 + e] : 0.0f;
+                }
+            }
+            __syncthreads();
+            float acc[RI][4];
+#pragma unroll
+            for (int a = 0; a < RI; ++a)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[a][e] = 0.0f;
+            if (!fresh)
+#pragma unroll 4
+            for (int n = 0; n < N; ++n) {                     // what the state before the chunk gives
+                const float4 sv = *(const float4*)(st + n * 64 + tx * 4);
+                float qi[RI];
+                if (RI == 4) {
+                    const float4 a = *(const float4*)(qT + n * LD + i0);
+                    qi[0] = a.x; qi[1 % RI] = a.y; qi[2 % RI] = a.z; qi[3 % RI] = a.w;
+                } else {
+#pragma unroll
+                    for (int a = 0; a < RI; ++a) qi[a] = qT[n * LD + i0 + a];
+                }
+#pragma unroll
+                for (int a = 0; a < RI; ++a) {
+                    acc[a][0] = fmaf(qi[a], sv.x, acc[a][0]); acc[a][1] = fmaf(qi[a], sv.y, acc[a][1]);
+                    acc[a][2] = fmaf(qi[a], sv.z, acc[a][2]); acc[a][3] = fmaf(qi[a], sv.w, acc[a][3]);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < RI; ++a)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[a][e] *= carry[a];
+#pragma unroll 4
+            for (int j = 0; j < j_end; ++j) {                 // what the chunk's own tokens give
+                const float4 ve = *(const float4*)(vs + j * 64 + tx * 4);
+                float wi[RI];
+                if (RI == 4) {
+                    const float4 a = *(const float4*)(wT + j * LD + i0);
+                    wi[0] = a.x; wi[1 % RI] = a.y; wi[2 % RI] = a.z; wi[3 % RI] = a.w;
+                } else {
+#pragma unroll
+                    for (int a = 0; a < RI; ++a) wi[a] = wT[j * LD + i0 + a];
+                }
+#pragma unroll
+                for (int a = 0; a < RI; ++a) {
+                    acc[a][0] = fmaf(wi[a], ve.x, acc[a][0]); acc[a][1] = fmaf(wi[a], ve.y, acc[a][1]);
+                    acc[a][2] = fmaf(wi[a], ve.z, acc[a][2]); acc[a][3] = fmaf(wi[a], ve.w, acc[a][3]);
+                }
+            }
+            const int e = e0 + tx * 4;
 #pragma unroll
             for (int a = 0; a < RI; ++a) {
                 const int i = i0 + a;
-                float weight = 0.0f;
-                if (j <= i && i < L) {
-                    float exponent;
-                    if (constant) {
-                        exponent = i == j ? 0.0f : (float)(i - j) * l[0];
-                    } else if (j0 < i0) {
-                        if (a > 0) sum += l[i];
-                        exponent = sum;
-                    } else {
-                        exponent = 0.0f;
-                        for (int x = j + 1; x <= i; ++x) exponent += l[x];
-                    }
-                    weight = acc[a][b] * expf(exponent) * c[j];
+                if (i >= L || e >= P) continue;
+                const float4 own = *(const float4*)(vs + i * 64 + tx * 4);
+                const float f = factor[i];
+                const float o[4] = {fmaf(skip, own.x, acc[a][0] * f), fmaf(skip, own.y, acc[a][1] * f), fmaf(skip, own.z, acc[a][2] * f),
+                                    fmaf(skip, own.w, acc[a][3] * f)};
+                float* to = out + ((size_t)(first + i) * H + head) * P + e;
+                if ((P & 3) == 0) {
+                    *(float4*)to = make_float4(o[0], o[1], o[2], o[3]);
+                } else {
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                        if (e + x < P) to[x] = o[x];
                 }
-                wT[j * LD + i] = weight;
-            }
-        }
-    }
-    float carry[RI];
-#pragma unroll
-    for (int a = 0; a < RI; ++a) carry[a] = i0 + a < L ? up_to[i0 + a] : 0.0f;
-    const float skip = decay.skip ? decay.skip[head] : 0.0f;
-    const float* chunk_before = sums + ((size_t)s * max_chunks + chunk) * ls_half(shape, decay);
-    const float* before = chunk_before + (size_t)head * N * P;
-    if (decay.floor) {
-        __syncthreads();                                  // (the scores are in place)
-        if (threadIdx.x < 4 * CH) {
-            const float* n_before = chunk_before + (size_t)H * N * P + (size_t)head * N;
-            const int i = threadIdx.x >> 2, part = threadIdx.x & 3;
-            float dot = 0.0f, own = 0.0f;
-            for (int n = part; n < N; n += 4) dot = fmaf(qT[n * LD + i], n_before[n], dot);
-            for (int j = part; j <= i; j += 4) own += wT[j * LD + i];
-            dot = i < L ? fmaf(dot, up_to[i], own) : 0.0f;
-            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            if (part == 0)
-                factor[i] = i < L ? decay.out_scale / (fmaxf(fabsf(dot * decay.out_scale), decay.floor[(size_t)(first + i) * H + head]) + decay.floor_eps) : 0.0f;
-        }
-    } else if (threadIdx.x < CH) {
-        factor[threadIdx.x] = decay.out_scale;
-    }
-    float* st = kT;
-    const int j_end = min(L, ((ty | 3) + 1) * RI);        // (the four rows of threads of a warp walk the same keys)
-    for (int e0 = 0; e0 < P; e0 += 64) {
-        __syncthreads();                                  // the scores are in place; the tiles before have been read
-        if (vec_v) {
-#pragma unroll
-            for (int idx = threadIdx.x; idx < CH * 16; idx += LS_THREADS) {
-                const int j = idx >> 4, e = (idx & 15) * 4;
-                float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (j < L && e0 + e < P) {
-                    x = *(const float4*)(base + (size_t)j * shape.row_stride + shape.v_at + head * P + e0 + e);
-                    if (shape.silu) x = make_float4(ls_silu(x.x), ls_silu(x.y), ls_silu(x.z), ls_silu(x.w));
-                }
-                *(float4*)(vs + j * 64 + e) = x;
-            }
-#pragma unroll 8
-            for (int idx = threadIdx.x; idx < N * 16; idx += LS_THREADS) {
-                const int n = idx >> 4, e = (idx & 15) * 4;
-                *(float4*)(st + n * 64 + e) = e0 + e < P ? *(const float4*)(before + (size_t)n * P + e0 + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < CH * 64; idx += LS_THREADS) {
-                const int j = idx >> 6, e = idx & 63;
-                vs[idx] = j < L && e0 + e < P ? ls_read(base + (size_t)j * shape.row_stride + shape.v_at + head * P + e0 + e, shape.silu) : 0.0f;
-            }
-            for (int idx = threadIdx.x; idx < N * 64; idx += LS_THREADS) {
-                const int n = idx >> 6, e = idx & 63;
-                st[idx] = e0 + e < P ? before[(size_t)n * P + e0 + e] : 0.0f;
-            }
-        }
-        __syncthreads();
-        float acc[RI][4];
-#pragma unroll
-        for (int a = 0; a < RI; ++a)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[a][e] = 0.0f;
-#pragma unroll 4
-        for (int n = 0; n < N; ++n) {                     // what the state before the chunk gives
-            const float4 sv = *(const float4*)(st + n * 64 + tx * 4);
-            float qi[RI];
-            if (RI == 4) {
-                const float4 a = *(const float4*)(qT + n * LD + i0);
-                qi[0] = a.x; qi[1 % RI] = a.y; qi[2 % RI] = a.z; qi[3 % RI] = a.w;
-            } else {
-#pragma unroll
-                for (int a = 0; a < RI; ++a) qi[a] = qT[n * LD + i0 + a];
-            }
-#pragma unroll
-            for (int a = 0; a < RI; ++a) {
-                acc[a][0] = fmaf(qi[a], sv.x, acc[a][0]); acc[a][1] = fmaf(qi[a], sv.y, acc[a][1]);
-                acc[a][2] = fmaf(qi[a], sv.z, acc[a][2]); acc[a][3] = fmaf(qi[a], sv.w, acc[a][3]);
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < RI; ++a)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[a][e] *= carry[a];
-#pragma unroll 4
-        for (int j = 0; j < j_end; ++j) {                 // what the chunk's own tokens give
-            const float4 ve = *(const float4*)(vs + j * 64 + tx * 4);
-            float wi[RI];
-            if (RI == 4) {
-                const float4 a = *(const float4*)(wT + j * LD + i0);
-                wi[0] = a.x; wi[1 % RI] = a.y; wi[2 % RI] = a.z; wi[3 % RI] = a.w;
-            } else {
-#pragma unroll
-                for (int a = 0; a < RI; ++a) wi[a] = wT[j * LD + i0 + a];
-            }
-#pragma unroll
-            for (int a = 0; a < RI; ++a) {
-                acc[a][0] = fmaf(wi[a], ve.x, acc[a][0]); acc[a][1] = fmaf(wi[a], ve.y, acc[a][1]);
-                acc[a][2] = fmaf(wi[a], ve.z, acc[a][2]); acc[a][3] = fmaf(wi[a], ve.w, acc[a][3]);
-            }
-        }
-        const int e = e0 + tx * 4;
-#pragma unroll
-        for (int a = 0; a < RI; ++a) {
-            const int i = i0 + a;
-            if (i >= L || e >= P) continue;
-            const float4 own = *(const float4*)(vs + i * 64 + tx * 4);
-            const float f = factor[i];
-            const float o[4] = {fmaf(skip, own.x, acc[a][0] * f), fmaf(skip, own.y, acc[a][1] * f), fmaf(skip, own.z, acc[a][2] * f),
-                                fmaf(skip, own.w, acc[a][3] * f)};
-            float* to = out + ((size_t)(first + i) * H + head) * P + e;
-            if ((P & 3) == 0) {
-                *(float4*)to = make_float4(o[0], o[1], o[2], o[3]);
-            } else {
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    if (e + x < P) to[x] = o[x];
             }
         }
     }
@@ -1064,10 +1077,13 @@ SKV_EXPORT int skv_linear_state(const float* rows, int row_stride, int q_at, int
                               dim3((dim * per_key + cells_each - 1) / cells_each, heads, n_seqs), dim3(LS_THREADS), 0, stream, sums, (const float*)factors, max_chunks, ch, shape, decays, batch))
         return code;
     const size_t smem = ls_output_smem(ch, dim);
-    auto kernel = ch == 64 ? linear_state_output_kernel<64> : (ch == 32 ? linear_state_output_kernel<32> : linear_state_output_kernel<16>);
+    // heads of one group share a block where that leaves blocks for two rounds of two an SM
+    const int shared = ch == 64 && heads / groups % 4 == 0 && (long long)max_chunks * (heads / 4) * n_seqs >= 4LL * sm_count() ? 4 : 1;
+    auto kernel = ch == 64 ? (shared == 4 ? linear_state_output_kernel<64, 4> : linear_state_output_kernel<64, 1>)
+                           : (ch == 32 ? linear_state_output_kernel<32, 1> : linear_state_output_kernel<16, 1>);
     if (int code = ls_reserve((const void*)kernel, smem, name)) return code;
-    return launch_pdl(name, kernel, grid, dim3(LS_THREADS), smem, stream, rows, (const float*)sums, out, max_chunks,
-                      (dim + 3) & ~3, shape, decays, cu_q);
+    return launch_pdl(name, kernel, dim3(grid.x, grid.y / shared, grid.z), dim3(LS_THREADS), smem, stream, rows, (const float*)sums, out,
+                      max_chunks, (dim + 3) & ~3, shape, decays, cu_q, positions);
 }
 
 // One token a sequence of a Mamba-2 mixer, in one kernel: rows float [n_seqs, row_stride] hold the input projection with

@@ -199,3 +199,40 @@ def test_retention_of_one_token(dim, vdim, dtype):
         error = 1e-6 * (mass + mass.amax(-1, keepdim=True) * o.abs() * scale.abs().clamp(max=1)) * scale.abs()
         assert ((out[s, :heads * vdim].double().view(heads, vdim) - o * scale).abs() <= error + (2.0 ** -8 if dtype == torch.bfloat16 else 2e-6) * (o * scale).abs() + 1e-6).all()
     assert (out[:, heads * vdim:] == 0).all()
+
+
+# heads of a group in one block (enough blocks of them) against a sequence at a time, which has a block a head
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(64, 2, 128, 64), (64, 16, 64, 128)])
+@pytest.mark.parametrize("floor", [False, True])
+def test_heads_of_a_group_share_their_scores(heads, groups, dim, vdim, floor):
+    from stratakv_b200.ops import kernels_for
+    ops = kernels_for(torch.bfloat16, 64, verbose=False)
+    lengths, i32 = [130, 64, 1, 65, 20] * 4, lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    n, seqs = sum(lengths), len(lengths)
+    starts = [0 if s % 3 else 7 for s in range(seqs)]
+    rows = torch.randn(n, 2 * groups * dim + heads * vdim, device="cuda")
+    logs, scale, least = -torch.rand(n, heads, device="cuda") * 0.1, torch.rand(n, heads, device="cuda"), 0.5 + torch.rand(n, heads, device="cuda")
+    half = heads * dim * (vdim + floor)
+    kept = torch.randn(seqs, 2 * half, device="cuda")
+
+    def run(first, count):
+        span, base = lengths[first:first + count], sum(lengths[:first])
+        cu = [0]
+        for length in span:
+            cu.append(cu[-1] + length)
+        meta = (i32([starts[first + s] + i for s, length in enumerate(span) for i in range(length)]), i32([s for s, length in enumerate(span) for _ in range(length)]),
+                i32(cu), i32(range(first, first + count)))
+        out, part = torch.full((cu[-1], heads * vdim), float("nan"), device="cuda"), slice(base, base + cu[-1])
+        more = dict(floor=least[part].contiguous(), floor_eps=1e-6, out_scale=0.5) if floor else {}
+        need = ops.linear_state_scratch(count, max(span), heads, dim, vdim, floor)
+        ops.linear_state(rows[part].contiguous(), 0, groups * dim, 2 * groups * dim, out, state, meta, heads, groups, dim, vdim, max(span),
+                         scratch=torch.full((need,), float("nan"), device="cuda"), log_decay=logs[part].contiguous(), key_scale=scale[part].contiguous(), **more)
+        return out
+
+    state = kept.clone()
+    together, after = run(0, seqs), state
+    state = kept.clone()
+    apart = torch.cat([run(s, 1) for s in range(seqs)])
+    # (a sequence of one token alone is a step of another kernel: its sums have another order)
+    torch.testing.assert_close(together, apart, rtol=2e-5, atol=2e-5 * float(apart.abs().max()))
+    torch.testing.assert_close(after, state, rtol=1e-5, atol=1e-5)
