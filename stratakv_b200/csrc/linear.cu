@@ -446,54 +446,9 @@ struct NormArgs {
     float* row_scale_out;          // with counter: [M] = 1 / sqrt(mean(updated out[m, :]^2) + eps_next)
 };
 
-// One block owns 16 rows of W and one chunk of 8*TG tokens.  Its warps take the
-// 32-wide k steps round robin, then their partial tiles are summed in shared
-// memory in warp order (a fixed order: results do not depend on timing).
-// Weights do not depend on the kernel before this one, so the first batch of
-// weight loads is issued before pdl_wait(): it overlaps the predecessor's tail.
-template <int TG, int U, bool STREAM, int MAX_WARPS>
-__global__ void __launch_bounds__(MAX_WARPS * 32, MAX_WARPS == 4 ? (TG == 1 ? 5 : (TG == 2 ? 5 : 2)) : (MAX_WARPS == 8 && TG <= 2 ? 2 : 1))
-skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
-                          void* __restrict__ out, int M, int N, int K, int mode, act_t act, const NormArgs norm) {
-    extern __shared__ float red[];                 // [warps][16][8*TG + 1], [8*TG] factors, [8*TG][n_partials_in] partial sums
-    constexpr int COLS = 8 * TG, PITCH = COLS + 1;
-    pdl_launch_dependents();
-    const int warps = blockDim.x >> 5;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, tig = lane & 3;
-    const int n0 = blockIdx.x * 16, m0 = blockIdx.y * COLS;
-    const int steps = (K + 31) >> 5;
-
-    const int row_a = min(n0 + g, N - 1), row_b = min(n0 + g + 8, N - 1);
-    const bool has_a = n0 + g < N, has_b = n0 + g + 8 < N;
-    const __nv_bfloat16* wa_ptr = W + (size_t)row_a * K + tig * 8;
-    const __nv_bfloat16* wb_ptr = W + (size_t)row_b * K + tig * 8;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-
-    uint4 wa[U], wb[U];
-    auto load_weights = [&](int s0) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = (s0 + u * warps) << 5;
-            const bool live = (s0 + u * warps) < steps && (k + tig * 8) < K;
-            wa[u] = (live && has_a) ? load_weight16<STREAM>((const uint4*)(wa_ptr + k)) : zero;
-            wb[u] = (live && has_b) ? load_weight16<STREAM>((const uint4*)(wb_ptr + k)) : zero;
-        }
-    };
-    load_weights(warp);
-    pdl_wait();                                    // activations (and the residual stream) are ready now
-
-    const __nv_bfloat16* x_ptr[TG];
-    bool has_x[TG];
-#pragma unroll
-    for (int t = 0; t < TG; ++t) {
-        const int m = m0 + t * 8 + g;
-        has_x[t] = m < M;
-        const int safe = min(m, M - 1);
-        x_ptr[t] = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K + tig * 8;
-    }
-    float* factor = red + (size_t)warps * 16 * PITCH;
-    float* staged = factor + COLS;
+// The three steps that the kernels below share.  First, what a folded norm's factors will be made from is sent for.
+template <int COLS>
+__device__ __forceinline__ void skinny_send_for_norm(float* staged, const NormArgs& norm, int m0, int M) {
     if (norm.partials_in) {
         // the partial sums are wanted after the main loop: they travel to shared memory meanwhile, 16 bytes
         // at a time where the rows allow it (the row in shared memory is `pitch` floats)
@@ -517,24 +472,11 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
         // the factors are wanted after the main loop: bring their lines close meanwhile
         asm volatile("prefetch.global.L1 [%0];" ::"l"(norm.row_scale + threadIdx.x * 32));
     }
-    float acc[TG][4];
-#pragma unroll
-    for (int t = 0; t < TG; ++t) { acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f; }
+}
 
-    for (int s0 = warp; s0 < steps; s0 += warps * U) {
-        if (s0 != warp) load_weights(s0);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = (s0 + u * warps) << 5;
-            const bool live = (s0 + u * warps) < steps && (k + tig * 8) < K;
-#pragma unroll
-            for (int t = 0; t < TG; ++t) {
-                const uint4 xv = (live && has_x[t]) ? *(const uint4*)(x_ptr[t] + k) : zero;
-                mma_bf16_16816(acc[t], wa[u].x, wb[u].x, wa[u].y, wb[u].y, xv.x, xv.y);
-                mma_bf16_16816(acc[t], wa[u].z, wb[u].z, wa[u].w, wb[u].w, xv.z, xv.w);
-            }
-        }
-    }
+// Then, after the main loop, the factors of the block's tokens.
+template <int COLS>
+__device__ __forceinline__ void skinny_norm_factors(float* factor, const float* staged, const NormArgs& norm, int K, int warps, int warp, int lane) {
     if (norm.partials_in) {
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
@@ -546,6 +488,14 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
             if (lane == 0) factor[m] = 1.0f / sqrtf(total / (float)K + norm.eps_in);
         }
     }
+}
+
+// Last, the warps' partial tiles are added up and the result stored, rows n0 .. n0 + 15 of the weight.
+template <int TG>
+__device__ __forceinline__ void skinny_store(float* red, const float* factor, const float (&acc)[TG][4], void* __restrict__ out, int M,
+                                             int N, int n0, int m0, int mode, act_t act, const NormArgs& norm, int warps, int warp, int lane) {
+    constexpr int COLS = 8 * TG, PITCH = COLS + 1;
+    const int g = lane >> 2, tig = lane & 3;
     float* mine = red + (size_t)warp * 16 * PITCH;
 #pragma unroll
     for (int t = 0; t < TG; ++t) {
@@ -617,6 +567,150 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
     }
 }
 
+// One block owns 16 rows of W and one chunk of 8*TG tokens.  Its warps take the
+// 32-wide k steps round robin, then their partial tiles are summed in shared
+// memory in warp order (a fixed order: results do not depend on timing).
+// Weights do not depend on the kernel before this one, so the first batch of
+// weight loads is issued before pdl_wait(): it overlaps the predecessor's tail.
+template <int TG, int U, bool STREAM, int MAX_WARPS>
+__global__ void __launch_bounds__(MAX_WARPS * 32, MAX_WARPS == 4 ? (TG == 1 ? 5 : (TG == 2 ? 5 : 2)) : (MAX_WARPS == 8 && TG <= 2 ? 2 : 1))
+skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
+                          void* __restrict__ out, int M, int N, int K, int mode, act_t act, const NormArgs norm) {
+    extern __shared__ float red[];                 // [warps][16][8*TG + 1], [8*TG] factors, [8*TG][n_partials_in] partial sums
+    constexpr int COLS = 8 * TG, PITCH = COLS + 1;
+    pdl_launch_dependents();
+    const int warps = blockDim.x >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, tig = lane & 3;
+    const int n0 = blockIdx.x * 16, m0 = blockIdx.y * COLS;
+    const int steps = (K + 31) >> 5;
+
+    const int row_a = min(n0 + g, N - 1), row_b = min(n0 + g + 8, N - 1);
+    const bool has_a = n0 + g < N, has_b = n0 + g + 8 < N;
+    const __nv_bfloat16* wa_ptr = W + (size_t)row_a * K + tig * 8;
+    const __nv_bfloat16* wb_ptr = W + (size_t)row_b * K + tig * 8;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+
+    uint4 wa[U], wb[U];
+    auto load_weights = [&](int s0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = (s0 + u * warps) << 5;
+            const bool live = (s0 + u * warps) < steps && (k + tig * 8) < K;
+            wa[u] = (live && has_a) ? load_weight16<STREAM>((const uint4*)(wa_ptr + k)) : zero;
+            wb[u] = (live && has_b) ? load_weight16<STREAM>((const uint4*)(wb_ptr + k)) : zero;
+        }
+    };
+    load_weights(warp);
+    pdl_wait();                                    // activations (and the residual stream) are ready now
+
+    const __nv_bfloat16* x_ptr[TG];
+    bool has_x[TG];
+#pragma unroll
+    for (int t = 0; t < TG; ++t) {
+        const int m = m0 + t * 8 + g;
+        has_x[t] = m < M;
+        const int safe = min(m, M - 1);
+        x_ptr[t] = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K + tig * 8;
+    }
+    float* factor = red + (size_t)warps * 16 * PITCH;
+    float* staged = factor + COLS;
+    skinny_send_for_norm<COLS>(staged, norm, m0, M);
+    float acc[TG][4];
+#pragma unroll
+    for (int t = 0; t < TG; ++t) { acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f; }
+
+    for (int s0 = warp; s0 < steps; s0 += warps * U) {
+        if (s0 != warp) load_weights(s0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = (s0 + u * warps) << 5;
+            const bool live = (s0 + u * warps) < steps && (k + tig * 8) < K;
+#pragma unroll
+            for (int t = 0; t < TG; ++t) {
+                const uint4 xv = (live && has_x[t]) ? *(const uint4*)(x_ptr[t] + k) : zero;
+                mma_bf16_16816(acc[t], wa[u].x, wb[u].x, wa[u].y, wb[u].y, xv.x, xv.y);
+                mma_bf16_16816(acc[t], wa[u].z, wb[u].z, wa[u].w, wb[u].w, xv.z, xv.w);
+            }
+        }
+    }
+    skinny_norm_factors<COLS>(factor, staged, norm, K, warps, warp, lane);
+    skinny_store<TG>(red, factor, acc, out, M, N, n0, m0, mode, act, norm, warps, warp, lane);
+}
+
+// The same for at most 8 tokens where the tiles outnumber what two blocks of 8 warps an SM hold and the inner size gives a warp
+// at most twelve steps: that many blocks walk the tiles, and a warp keeps eight steps of weights on their way in two halves.
+// As soon as one half is multiplied the next is asked for, into the block's next tile too, so that the tokens' loads, the sums
+// and the stores do not leave the memory idle, which blocks that come and go did for a third of their life.  8 tokens, 9,248
+// / 12,288 / 32,000 x 3,072: 13.1 / 17.8 / 40.8 us a block a tile, 11.0 / 15.2 / 34.8 so; 8,192 / 32,000 x 2,048 8.8 / 27.5 and
+// 7.1 / 23.6.  Longer inner sizes gain nothing (28,672 x 4,096 44.2 and 44.7), and fewer tiles lose by the smaller bursts (1 token, 3,072 x 12,288
+// 16.6 and 18.1).
+constexpr int WALK_WARPS = 8, WALK_HALF = 4;
+
+__global__ void __launch_bounds__(WALK_WARPS * 32, 2)
+skinny_walk_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
+                        void* __restrict__ out, int M, int N, int K, int mode, act_t act, const NormArgs norm) {
+    extern __shared__ float red[];                 // as above
+    constexpr int COLS = 8, PITCH = COLS + 1;
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, tig = lane & 3;
+    const int steps = (K + 31) >> 5, tiles = (N + 15) >> 4;
+    const int halves = ((steps + WALK_WARPS - 1) / WALK_WARPS + WALK_HALF - 1) / WALK_HALF;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+
+    uint4 wa[2][WALK_HALF], wb[2][WALK_HALF];
+    int asked_tile = blockIdx.x, asked = 0;        // the next half to ask for
+    auto load_weights = [&](uint4 (&a)[WALK_HALF], uint4 (&b)[WALK_HALF]) {
+        if (asked_tile >= tiles) return;
+        const int row_a = asked_tile * 16 + g, row_b = row_a + 8;
+        const __nv_bfloat16* a_ptr = W + (size_t)min(row_a, N - 1) * K + tig * 8;
+        const __nv_bfloat16* b_ptr = W + (size_t)min(row_b, N - 1) * K + tig * 8;
+#pragma unroll
+        for (int u = 0; u < WALK_HALF; ++u) {
+            const int step = warp + (asked * WALK_HALF + u) * WALK_WARPS, k = step << 5;
+            const bool live = step < steps && (k + tig * 8) < K;
+            a[u] = live && row_a < N ? load_weight16<true>((const uint4*)(a_ptr + k)) : zero;
+            b[u] = live && row_b < N ? load_weight16<true>((const uint4*)(b_ptr + k)) : zero;
+        }
+        if (++asked == halves) { asked = 0; asked_tile += gridDim.x; }
+    };
+    load_weights(wa[0], wb[0]);
+    load_weights(wa[1], wb[1]);
+    pdl_wait();                                    // activations (and the residual stream) are ready now
+
+    const bool has_x = g < M;
+    const int safe = min(g, M - 1);
+    const __nv_bfloat16* x_ptr = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K + tig * 8;
+    float* factor = red + (size_t)WALK_WARPS * 16 * PITCH;
+    float* staged = factor + COLS;
+    skinny_send_for_norm<COLS>(staged, norm, 0, M);
+    float acc[1][4] = {};
+    auto multiply = [&](const uint4 (&a)[WALK_HALF], const uint4 (&b)[WALK_HALF], int half) {
+#pragma unroll
+        for (int u = 0; u < WALK_HALF; ++u) {
+            const int step = warp + (half * WALK_HALF + u) * WALK_WARPS, k = step << 5;
+            const uint4 xv = has_x && step < steps && (k + tig * 8) < K ? *(const uint4*)(x_ptr + k) : zero;
+            mma_bf16_16816(acc[0], a[u].x, b[u].x, a[u].y, b[u].y, xv.x, xv.y);
+            mma_bf16_16816(acc[0], a[u].z, b[u].z, a[u].w, b[u].w, xv.z, xv.w);
+        }
+    };
+    int half = 0;
+    bool second = false;                           // which of the two halves in registers comes next
+    for (int tile = blockIdx.x; tile < tiles;) {
+        if (second) { multiply(wa[1], wb[1], half); load_weights(wa[1], wb[1]); }
+        else { multiply(wa[0], wb[0], half); load_weights(wa[0], wb[0]); }
+        second = !second;
+        if (++half < halves) continue;
+        if (tile == (int)blockIdx.x) skinny_norm_factors<COLS>(factor, staged, norm, K, WALK_WARPS, warp, lane);
+        else __syncthreads();                      // the tile before has been stored
+        skinny_store<1>(red, factor, acc, out, M, N, tile * 16, 0, mode, act, norm, WALK_WARPS, warp, lane);
+        acc[0][0] = acc[0][1] = acc[0][2] = acc[0][3] = 0.0f;
+        half = 0;
+        tile += gridDim.x;
+    }
+}
+
 template <int TG, int U, int MAX_WARPS>
 static int launch_skinny_as(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act,
                             int warps, const NormArgs& norm, cudaStream_t stream) {
@@ -631,6 +725,14 @@ static int launch_skinny_as(const void* a, const void* w, void* out, int M, int 
     return launch_pdl("skv_linear(bfloat16)", skinny_linear_bf16_kernel<TG, U, false, MAX_WARPS>, grid,
                       dim3(warps * 32), smem, stream, (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K,
                       mode, act, norm);
+}
+
+static int launch_walk(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, const NormArgs& norm,
+                       cudaStream_t stream) {
+    const size_t smem = ((size_t)WALK_WARPS * 16 * 9 + 8 + (size_t)8 * (norm.partials_in ? (norm.n_partials_in + 3) & ~3 : 0)) * sizeof(float);
+    if (smem > 48 * 1024) return fail("skv_linear(bfloat16)", "too many partial sums for the consumer to stage: let the producer finish them");
+    return launch_pdl("skv_linear(bfloat16)", skinny_walk_bf16_kernel, dim3(2 * sm_count()), dim3(WALK_WARPS * 32), smem, stream,
+                      (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K, mode, act, norm);
 }
 
 // Warps per block.  Four to five row tiles per SM: 4 warps, compiled to fit 5 blocks on an SM so that
@@ -653,6 +755,8 @@ static int launch_skinny(const void* a, const void* w, void* out, int M, int N, 
     if (warps == 8 && MAX_WARPS >= 16 && steps > 8 * U * 2 && blocks <= sms) warps = 16;   // (16 warps: one block per SM)
     if (warps > MAX_WARPS) warps = MAX_WARPS;
     while (warps > 1 && warps > steps) warps >>= 1;
+    if (TG == 1 && warps == WALK_WARPS && row_tiles > 2 * sms && chunks == 1 && steps <= 12 * WALK_WARPS && !norm.partials)
+        return launch_walk(a, w, out, M, N, K, mode, act, norm, stream);
     if (warps <= 4) return launch_skinny_as<TG, U, 4>(a, w, out, M, N, K, mode, act, warps, norm, stream);
     if (warps <= 8 || MAX_WARPS < 16) return launch_skinny_as<TG, U, 8>(a, w, out, M, N, K, mode, act, warps, norm, stream);
     return launch_skinny_as<TG, U, 16>(a, w, out, M, N, K, mode, act, warps, norm, stream);
@@ -671,7 +775,12 @@ static int launch_linear(const void* a, const void* w, void* out, int M, int N, 
     if ((norm.row_scale || norm.partials_in || norm.partials) && M > 64)
         return fail("skv_linear(bfloat16)", "the norm-fused form serves steps of at most 64 tokens");
     // above 16 tokens the tensor-memory kernels take over, unless a norm is folded into this projection
-    if (M > 16 && !norm.row_scale && !norm.partials_in && !norm.partials)
+    // (above 8 where the weights are 48 MB or more: sixteen tokens' fragments cost the streaming kernel 20 to 40 %, which its
+    // shorter start makes up for only on smaller ones: 16 tokens, 6,144 x 4,096 / 3,072 x 12,288 / 32,000 x 2,048 / 128,256 x 4,096
+    // 17.5 / 24 / 31 / 222 us there, 11.7 / 16 / 21 / 161 here; 4,096 x 4,096 10.2 and 11.1).
+    // (an activation in the epilogue stays here, with libm's exponential and a division)
+    const bool plain = mode != MODE_GATED && !(act & ACT_ON_STORE);
+    if ((M > 16 || (M > 8 && plain && (long long)N * K >= 24LL << 20)) && !norm.row_scale && !norm.partials_in && !norm.partials)
         return linear_tcgen05(a, w, out, M, N, K, mode, act, flag, stream);
     // at most 8 warps and under 100 registers a thread: two blocks fit on an SM, so the next
     // kernel's weight loads are in flight while this one finishes
