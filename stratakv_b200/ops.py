@@ -951,6 +951,8 @@ class Kernels:
         lays them out, and ``out[p] = act(gate_e . a) * (up_e . a)``.)
         ``out[p] = act(w[e] . a[row(p)])`` for every sorted pair p of expert e (``offsets`` from ``sort_by_expert``);
         ``w`` ``[experts, N, K]``; ``row(p) = rows[p]`` (the first projection gathers its input from the tokens) or p.
+        ``place`` and ``weights`` ``[tokens, top]`` (only where ``expert_few`` says so, with ``rows``): each pair's row is
+        multiplied by its weight first, rounded to the compute dtype.
         ``out`` ``[pairs, N]`` is the compute dtype (with ``activation``) or float32.  Sums are float32."""
         self._want(a, self.dtype, "a"); self._want(w, self.dtype, "w"); self._want(offsets, torch.int32, "offsets")
         if out.dtype not in (self.dtype, torch.float32) or not out.is_cuda or not out.is_contiguous():

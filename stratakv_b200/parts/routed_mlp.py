@@ -16,9 +16,10 @@ the dense gated feed-forward packs them.
 
 Kernels (``csrc/routed_mlp.cu``): the router (scores, choice, weights, the shared expert's gate), a counting sort of
 the (token, expert) pairs by expert, the two projections over the sorted pairs (each block of rows reads the
-weights of the one expert that its rows chose; the first gathers its rows from the tokens), and the weighted sum,
-which also adds the shared expert's result.  The shared expert's projections are the library's own.  Nothing is read
-back to the host, so a step can be captured in a graph.
+weights of the one expert that its rows chose; the first gathers its rows from the tokens; few pairs in bfloat16
+stream each chosen expert's weights once, whatever its rows), and the weighted sum, which also adds the shared
+expert's result.  The shared expert's projections are the library's own.  Nothing is read back to the host, so a
+step can be captured in a graph.
 """
 from __future__ import annotations
 

@@ -2,8 +2,8 @@
 
 One table ``[vocab, layers * dim]`` serves all layers; layer i reads the columns ``[i * dim, (i + 1) * dim)`` of the
 token's row: ``e``.  Then ``g = gelu_tanh(gate x) * e``, ``y = proj g`` and ``x += rmsnorm(y) * norm`` (a plain-weight
-RMS norm).  ``dim`` is small, so the whole thing is one kernel with a block per token (``csrc/stream_ops.cu``), which
-can also leave the next layer's first norm of the new stream.
+RMS norm).  ``dim`` is small, so the whole thing is one kernel (``csrc/stream_ops.cu``: in bfloat16 a cluster of blocks per
+16 or 32 tokens on tensor cores, else a block per token), which can also leave the next layer's first norm of the new stream.
 """
 from __future__ import annotations
 
@@ -32,8 +32,8 @@ class TokenSide(Part):
         self.gamma = self.rt.upload(tensors[s.norm_weight], torch.float32)
 
     # The kernel can first add a sublayer's branch through the norm after it (``forward``'s ``branch``, ``post_norm``),
-    # but measured slower than ``rmsnorm_add`` followed by this kernel (16,320 tokens of width 2,048: 931 us against
-    # 115 + 490 us; a decode step of 8 sequences 0.80 against 0.78 ms), so the arrangement is told not to ask for it.
+    # but only the block per token does that, and measured slower than ``rmsnorm_add`` followed by that same kernel (16,320
+    # tokens of width 2,048: 931 us against 115 + 490 us), so the arrangement is told not to ask for it.
     adds_branch = False
 
     def forward(self, step, x, next_norm=None, next_out=None, branch=None, post_norm=None) -> None:
