@@ -12,7 +12,7 @@
 //
 // Cache layout per entry: [block][kv_head][block_size][head_dim]; a token's keys
 // are found through block_table[seq][position / block_size].
-#include "common.cuh"
+#include "head_size.cuh"
 
 namespace skv {
 
@@ -150,6 +150,8 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
 }  // namespace skv
 
 using namespace skv;
+
+SKV_EXPORT int skv_library_head_dim() { return SKV_HEAD_DIM; }
 
 SKV_EXPORT int skv_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
                              int table_width, const int* positions, const int* token_seq, void* out,

@@ -17,7 +17,7 @@
 // products are unchanged.  For P.V a lane reads head_dim/8 consecutive elements of
 // four keys and pairs them across keys with byte permutes; tile j's column g is
 // then head-dim element g*head_dim/8 + j, undone when the output is written.
-#include "common.cuh"
+#include "head_size.cuh"
 
 #include <mutex>
 

@@ -21,7 +21,7 @@
 //    pushes its partial (max, sum, output) rows into the shared memory of the block that owns the
 //    row, one cluster barrier makes them visible, and the owner merges and writes the row.  No
 //    scratch in global memory, no second kernel, no barrier after the merge.
-#include "common.cuh"
+#include "head_size.cuh"
 
 
 // Two stages of 128 keys and values must fit one block's shared memory, which holds for head sizes up

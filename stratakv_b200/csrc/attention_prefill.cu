@@ -10,7 +10,7 @@
 // scores and the output accumulate in float in mma.sync m16n8k16 fragments with an
 // online softmax; the scale multiplies the finished dot product; a query at absolute
 // position p sees keys lo..p (lo = 0 or p - window + 1).
-#include "common.cuh"
+#include "head_size.cuh"
 
 #if SKV_DTYPE == SKV_BF16 && SKV_HEAD_DIM <= 128
 

@@ -23,7 +23,7 @@
 // The softmax is the long pole, so a block uses only half of the SM's tensor memory and shared
 // memory and (for head size 64) two blocks share an SM.  Every mbarrier
 // wait is bounded; on time-out bit 2 (value 4) of the flag word is raised and the block drains.
-#include "common.cuh"
+#include "head_size.cuh"
 
 #if SKV_DTYPE == SKV_BF16 && (SKV_HEAD_DIM == 64 || SKV_HEAD_DIM == 128)
 

@@ -16,12 +16,9 @@
 #define SKV_F32 0
 #define SKV_BF16 1
 
-// Each build of the library serves one compute dtype and one head size.
+// Each build of the library serves one compute dtype (and its attention files one head size: head_size.cuh).
 #ifndef SKV_DTYPE
 #error "compile with -DSKV_DTYPE=0 (float) or 1 (bfloat16)"
-#endif
-#ifndef SKV_HEAD_DIM
-#error "compile with -DSKV_HEAD_DIM=<head size, a multiple of 16>"
 #endif
 #if SKV_DTYPE == SKV_BF16
 typedef __nv_bfloat16 skv_t;
@@ -31,15 +28,14 @@ typedef float skv_t;
 
 #define SKV_EXPORT extern "C" __attribute__((visibility("default")))
 
+// This thread's last message, 512 bytes (elementwise.cu; the attention kernels' library takes it from there, so that
+// skv_last_error() answers for both).
+SKV_EXPORT char* skv_error_buffer();
+
 namespace skv {
 
-inline char* error_buffer() {
-    static thread_local char buffer[512] = {0};
-    return buffer;
-}
-
 inline int fail(const char* what, const char* detail = "") {
-    snprintf(error_buffer(), 512, "%s%s%s", what, detail[0] ? ": " : "", detail);
+    snprintf(skv_error_buffer(), 512, "%s%s%s", what, detail[0] ? ": " : "", detail);
     return 1;
 }
 

@@ -562,9 +562,12 @@ __global__ void scale_inplace_kernel(float* __restrict__ x, float factor, size_t
 
 using namespace skv;
 
-SKV_EXPORT const char* skv_last_error() { return error_buffer(); }
+SKV_EXPORT char* skv_error_buffer() {
+    static thread_local char buffer[512] = {0};
+    return buffer;
+}
+SKV_EXPORT const char* skv_last_error() { return skv_error_buffer(); }
 SKV_EXPORT int skv_library_dtype() { return SKV_DTYPE; }
-SKV_EXPORT int skv_library_head_dim() { return SKV_HEAD_DIM; }
 
 // Checkpoint tensors in the stored type -> the type a part computes in, on the device (the reference converts
 // FP32 weights to BF16 by dropping the low half, src/cuda/gemm_cuda.cu:74-83; here to nearest even).  Kinds: 0 float32,

@@ -31,7 +31,9 @@
  * [head_dim], int32 block_table [n_seqs, table_width], int32 ctx_after [n_seqs] (keys
  * cached for each sequence, the query's own included), bfloat16 out like q.  Returns 0, or
  * non-zero after recording a message that skv_last_error() returns.  Only the bfloat16
- * build of the library implements it, for the head size that build was compiled for.
+ * build of the library implements it, for the head size that build was compiled for
+ * (libstratakv_bf16_hd<size>_*.so, which needs the libstratakv_bf16_*.so of its build in the
+ * same folder).
  */
 #ifndef STRATAKV_NO_ALLOC_H
 #define STRATAKV_NO_ALLOC_H

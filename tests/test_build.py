@@ -1,0 +1,39 @@
+"""What is compiled per head size, and that the libraries of one dtype share the rest."""
+import ctypes
+import re
+
+import pytest
+
+from stratakv_b200.csrc import build
+
+
+def test_only_what_reads_the_head_size_is_compiled_per_head_size():
+    """Sixteen libraries of every kernel were 441 MB, too much to carry; only the attention files differ between them."""
+    sources = {path.name for path in build.CSRC.glob("*.cu")}
+    assert sources == set(build.HEAD_SOURCES) | set(build.COMMON_SOURCES) and not set(build.HEAD_SOURCES) & set(build.COMMON_SOURCES)
+    for name in sources:
+        text = (build.CSRC / name).read_text()
+        assert bool(re.search(r"\bSKV_HEAD_DIM\b", text)) == (name in build.HEAD_SOURCES), name
+        assert ('#include "head_size.cuh"' in text) == (name in build.HEAD_SOURCES), name
+    assert build.common_library_name("bfloat16") != build.common_library_name("float32")
+    assert build.library_name("bfloat16", 64) != build.library_name("bfloat16", 128)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_one_handle_has_both_libraries_and_one_message(dtype):
+    path = build.find_built(dtype, 64)
+    if path is None:
+        pytest.skip("not compiled yet")
+    common = path.parent / build.common_library_name(dtype)
+    assert path.stat().st_size < common.stat().st_size / 4
+    lib = ctypes.CDLL(str(path))
+    lib.skv_last_error.restype = ctypes.c_char_p
+    assert lib.skv_library_head_dim() == 64 and lib.skv_library_dtype() == build.DTYPE_CODES[dtype]
+    null = ctypes.c_void_p(0)
+    # a refusal of the attention library, then one of the common library: no kernel is reached
+    one = ctypes.c_int(1)
+    assert lib.skv_attention(null, null, null, null, one, null, null, null, one, one, one, ctypes.c_int(48), ctypes.c_int(16),
+                             ctypes.c_float(1.0), ctypes.c_int(0), null) != 0
+    assert lib.skv_last_error().startswith(b"skv_attention:")
+    assert lib.skv_rmsnorm(null, null, ctypes.c_float(1.0), null, null, one, ctypes.c_int(0), one, null) != 0
+    assert lib.skv_last_error().startswith(b"skv_rmsnorm:")
