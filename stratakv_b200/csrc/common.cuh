@@ -144,6 +144,42 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
     return __float2bfloat16_rn(v);
 }
 
+#if SKV_DTYPE == SKV_BF16
+// ---- mma.sync m16n8k16 -------------------------------------------------------
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// acc += a b for an operand of PARTS bfloat16 that add up to a float (PARTS 1: a bfloat16), the smallest part first.  The
+// tensor core cuts off what lies below its accumulator's last bit, always towards zero, so that a sum kept in it drifts by its
+// length: over 256 numbers it erred 3 times as much as a chain of float multiply-adds, over 4,000 15 times.  So only sixteen
+// products meet there, and the sums of sixteen are added by ordinary additions, which round.
+template <int PARTS>
+__device__ __forceinline__ void mma_bf16_add(float (&acc)[4], const uint32_t (&a)[PARTS][4], uint32_t b0, uint32_t b1) {
+    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int s = PARTS - 1; s >= 0; --s) mma_bf16(sum, a[s], b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] += sum[i];
+}
+
+// Three bfloat16 that add up to a float to its last bit (24 of 24), for two floats at once, u in the low halves.  Each part is the
+// upper half of what is left, so that a large float stays finite where rounding would make it infinite, and nothing is left of
+// an infinity.
+__device__ __forceinline__ void split3(float u, float v, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        const uint32_t a = __float_as_uint(u), b = __float_as_uint(v);
+        parts[s] = __byte_perm(a, b, 0x7632);
+        const float top_u = __uint_as_float(a & 0xffff0000u), top_v = __uint_as_float(b & 0xffff0000u);
+        u = u == top_u ? 0.0f : u - top_u;
+        v = v == top_v ? 0.0f : v - top_v;
+    }
+}
+#endif
+
 // Two optional terms of an attention kernel, both off when their pointer is null.
 //   bias:  a table [num_heads][bias_len]; bias[h][d] is taken off the score of a key at distance d from the
 //          query (a distance beyond the table reads its last entry).  The entries are in units of log2, that is the

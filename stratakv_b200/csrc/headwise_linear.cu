@@ -74,18 +74,14 @@ headwise_linear_kernel(const TIn* __restrict__ x, int x_stride, const TW* __rest
 // The same on tensor cores (mma.sync m16n8k16), for weights whose rows are whole 16 bytes: a warp makes 16 tokens x 8 NT
 // outputs of a head.  A lane reads eight neighbouring k of a row at a time, in the same order for both operands.  A float
 // input stays float: it is split into three bfloat16 that add up to it (24 of 24 bits), against weights that are
-// bfloat16 anyway, so every product is exact and the sums are float.
+// bfloat16 anyway, so every product is exact and the sums are float (mma_bf16_add: relative errors over an inner size of 256 of
+// 0.8e-7 to 0.9e-7 of a float input and 0.7e-7 of a bfloat16 one, where the FMA kernel's are 2.5e-7 to 2.9e-7 and 1.1e-7 to 1.5e-7
+// and sums left in the tensor core had up to 8.5e-7; that costs 0 to 10 % of a prompt's time and nothing of a few tokens').
 // A step of few tokens is bound by latency (a matrix of a MB over all heads): NT 2 gives warps enough, and the first
 // weights are under way before the wait.  A prompt is bound by the rows it reads and writes: NT 8 reads a float row once
-// per 64 outputs.  32 heads 64 -> 256 at 8 and 3,764 tokens: 6.2 -> 1.8 us and 216 -> 48; 256 -> 64: 17.7 -> 3.2 us and
-// 219 -> 34; float to float 64 -> 64: 5.1 -> 2.2 us and 57 -> 17.
+// per 64 outputs.  32 heads 64 -> 256 at 8 and 3,764 tokens: 6.2 -> 1.6 us and 216 -> 49; 256 -> 64: 17.7 -> 3.1 us and
+// 219 -> 37; float to float 64 -> 64: 5.1 -> 2.1 us and 57 -> 18.
 constexpr int HM_WARPS = 4;
-
-__device__ __forceinline__ void headwise_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // Eight numbers of a row as operand pairs: parts[s][i] holds numbers 2i and 2i + 1 (of a float row its s-th bfloat16).
 __device__ __forceinline__ void headwise_parts(const __nv_bfloat16* p, bool live, uint32_t (&parts)[1][4]) {
@@ -94,18 +90,14 @@ __device__ __forceinline__ void headwise_parts(const __nv_bfloat16* p, bool live
 }
 __device__ __forceinline__ void headwise_parts(const float* p, bool live, uint32_t (&parts)[3][4]) {
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f), lo = live ? *(const float4*)p : zero, hi = live ? *(const float4*)(p + 4) : zero;
-    float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-    for (int s = 0; s < 3; ++s)
+    for (int i = 0; i < 4; ++i) {
+        uint32_t pair[3];
+        split3(v[2 * i], v[2 * i + 1], pair);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            parts[s][i] = *(const uint32_t*)&pair;
-            const float2 back = __bfloat1622float2(pair);
-            // (what is left of an infinity is not a number: nothing, so that the first part says it alone)
-            v[2 * i] = isfinite(back.x) ? v[2 * i] - back.x : 0.0f;
-            v[2 * i + 1] = isfinite(back.y) ? v[2 * i + 1] - back.y : 0.0f;
-        }
+        for (int s = 0; s < 3; ++s) parts[s][i] = pair[s];
+    }
 }
 
 __device__ __forceinline__ void headwise_store(float* p, float u, float v) { *(float2*)p = make_float2(u, v); }
@@ -142,14 +134,15 @@ headwise_mma_kernel(const TIn* __restrict__ x, int x_stride, const __nv_bfloat16
 #pragma unroll
         for (int h = 0; h < 2; ++h) headwise_parts(rows[h] + k, k < in_dim, a[h]);
         if (k0 > 0) load_weights(k);
+        uint32_t first[PARTS][4], second[PARTS][4];
 #pragma unroll
-        for (int s = PARTS - 1; s >= 0; --s) {
-            const uint32_t first[4] = {a[0][s][0], a[1][s][0], a[0][s][1], a[1][s][1]}, second[4] = {a[0][s][2], a[1][s][2], a[0][s][3], a[1][s][3]};
+        for (int s = 0; s < PARTS; ++s)
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                headwise_mma(acc[n], first, weights[n].x, weights[n].y);
-                headwise_mma(acc[n], second, weights[n].z, weights[n].w);
-            }
+            for (int i = 0; i < 4; ++i) { first[s][i] = a[i & 1][s][i >> 1]; second[s][i] = a[i & 1][s][2 + (i >> 1)]; }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            mma_bf16_add<PARTS>(acc[n], first, weights[n].x, weights[n].y);
+            mma_bf16_add<PARTS>(acc[n], second, weights[n].z, weights[n].w);
         }
     }
 #pragma unroll

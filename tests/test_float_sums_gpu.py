@@ -1,0 +1,50 @@
+"""Float sums that tensor cores make err no more than the chain of float multiply-adds that they stand for."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def lib():
+    from stratakv_b200.ops import kernels_for
+    return kernels_for(torch.bfloat16, 64, verbose=False)
+
+
+def chain(x, w):
+    """[..., m, k] and [..., n, k] -> [..., m, n] in float32, one multiply-add after the other."""
+    total = torch.zeros(*x.shape[:-1], w.shape[-2], device=x.device)
+    for k in range(x.shape[-1]):
+        total = (total.double() + x[..., :, None, k].double() * w[..., None, :, k].double()).float()
+    return total
+
+
+def error(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+# (a sum of one sign is what drifts where it is cut off instead of rounded)
+@pytest.mark.parametrize("heads,in_dim,out_dim", [(32, 64, 64), (8, 256, 64), (2, 512, 96), (3, 2048, 40)])
+@pytest.mark.parametrize("n", [8, 100])
+@pytest.mark.parametrize("x_float", [False, True])
+@pytest.mark.parametrize("one_sign", [False, True])
+def test_headwise_projection(heads, in_dim, out_dim, n, x_float, one_sign):
+    x, w = torch.randn(n, heads * in_dim, device="cuda"), (torch.randn(heads, out_dim, in_dim, device="cuda") / math.sqrt(in_dim)).bfloat16()
+    x = x if x_float else x.bfloat16()
+    if one_sign:
+        x, w = x.abs(), w.abs()
+    out = torch.empty(n, heads * out_dim, device="cuda")
+    lib().headwise_linear(x, w, out, heads)
+    by_head = x.view(n, heads, in_dim).transpose(0, 1)
+    want = by_head.double() @ w.double().transpose(1, 2)
+    assert error(out.view(n, heads, out_dim).transpose(0, 1), want) <= error(chain(by_head, w), want)
+
+
+def test_headwise_projection_of_the_largest_floats():
+    """Beyond the largest bfloat16, short of the largest float: rounded to nearest, the first of its three parts was infinite."""
+    x, w = torch.ones(2, 64, device="cuda"), torch.ones(1, 8, 64, device="cuda").bfloat16()
+    x[1, 3], x[0, 5] = 3.4e38, -3.4e38
+    out = torch.empty(2, 8, device="cuda")
+    lib().headwise_linear(x, w, out, 1)
+    assert torch.equal(out, x.sum(-1, keepdim=True).expand(2, 8))
