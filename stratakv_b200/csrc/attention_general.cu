@@ -317,7 +317,7 @@ attention_general_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
 // the largest maximum, the sums and outputs brought to it, the sink, the gate.  A block per (token, head): the first warp
 // makes the parts' weights, then a thread adds up its numbers of the parts with four loads on their way.  (A warp per
 // (token, head) that walked the parts one after the other took 20 us for 256 of them over 16 parts of 256 numbers,
-// with this one and the kernel below a decode step of 8 sequences over 780 cached rows takes 15 us in place of 69.)
+// with this one and the kernel below a decode step of 8 sequences over 780 cached rows takes 14 us in place of 69.)
 constexpr int MERGE_THREADS = 128, MERGE_MAX_SPLITS = 1024;
 template <typename T>
 __global__ void __launch_bounds__(MERGE_THREADS)
@@ -377,16 +377,12 @@ attention_general_merge_kernel(const float* __restrict__ partial_o, const float*
 // memory once for all heads (cp.async, two stages); eight warps make the scores (16 heads x 16 keys each), then four rows
 // of the softmax each, then 16 heads x 64 numbers of the output each.  Scores, softmax and sums are float; a probability
 // is split into three bfloat16 that add up to it, against values that are bfloat16 anyway, so nothing is rounded that
-// attention_general_kernel kept.  That kernel, a warp per (token, head, part), read every key once per head:
-// with its merge 8 sequences x 32 heads over 780 rows of 272
-// numbers took 69 us and take 15, 1 sequence over 8,000 rows 150 and 29, 64 over 500 187 and 29.
+// attention_general_kernel kept, and sums are added by mma_bf16_add (relative errors before the output's rounding, rows of 288, two
+// parts of 8,000: 2.1e-7, that kernel 7.2e-7; sums left in the tensor core 110e-7, at 1 to 7 % less time).  That kernel, a warp
+// per (token, head, part), read every key once per head: with its merge 8 sequences x 32 heads over 780 rows of 272
+// numbers took 69 us and take 14, 1 sequence over 8,000 rows 150 and 30, 64 over 500 187 and 31.
 constexpr int LAT_KEYS = 64, LAT_HEADS = 32, LAT_MAX_DIM = 320, LAT_MAX_VDIM = 256, LAT_S_PITCH = LAT_KEYS + 4, LAT_P_PITCH = LAT_KEYS + 8;
 
-__device__ __forceinline__ void lat_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void lat_ldmatrix(uint32_t (&r)[4], const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
 }
@@ -456,11 +452,11 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
             const __nv_bfloat16* q_at = qs + (16 * m_tile + (lane & 15)) * pitch + 8 * (lane >> 4);
             const __nv_bfloat16* k_at = k_tile + (16 * part + (lane & 7) + 8 * (lane >> 4)) * pitch + 8 * ((lane >> 3) & 1);
             for (int d = 0; d < dim; d += 16) {
-                uint32_t a[4], b[4];
-                lat_ldmatrix(a, q_at + d);
+                uint32_t a[1][4], b[4];
+                lat_ldmatrix(a[0], q_at + d);
                 lat_ldmatrix(b, k_at + d);
-                lat_mma(s[0], a, b[0], b[1]);
-                lat_mma(s[1], a, b[2], b[3]);
+                mma_bf16_add<1>(s[0], a, b[0], b[1]);
+                mma_bf16_add<1>(s[1], a, b[2], b[3]);
             }
 #pragma unroll
             for (int n = 0; n < 2; ++n)
@@ -476,18 +472,15 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
             const int row = 4 * warp + i;
             const float2 s = *(const float2*)(scores + row * LAT_S_PITCH + 2 * lane);
             const float new_max = fmaxf(running_max[i], warp_max(fmaxf(s.x, s.y)));
-            float p[2] = {expf(s.x - new_max), expf(s.y - new_max)};
+            const float p[2] = {expf(s.x - new_max), expf(s.y - new_max)};
             const float factor = expf(running_max[i] - new_max);        // 0 on the first tile
             running_sum[i] = running_sum[i] * factor + warp_sum(p[0] + p[1]);
             running_max[i] = new_max;
             if (lane == 0) rescale[row] = factor;
+            uint32_t parts[3];
+            split3(p[0], p[1], parts);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const __nv_bfloat162 pair = __floats2bfloat162_rn(p[0], p[1]);
-                *(__nv_bfloat162*)(probs + (k * LAT_HEADS + row) * LAT_P_PITCH + 2 * lane) = pair;
-                const float2 back = __bfloat1622float2(pair);
-                p[0] -= back.x; p[1] -= back.y;
-            }
+            for (int k = 0; k < 3; ++k) *(uint32_t*)(probs + (k * LAT_HEADS + row) * LAT_P_PITCH + 2 * lane) = parts[k];
         }
         __syncthreads();
         const float low = rescale[16 * m_tile + g], high = rescale[16 * m_tile + g + 8];
@@ -504,11 +497,8 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
                 if (c >= vdim) continue;
                 uint32_t b[4];
                 lat_ldmatrix_trans(b, k_tile + (k + (lane & 15)) * pitch + c + 8 * (lane >> 4));
-#pragma unroll
-                for (int p = 2; p >= 0; --p) {
-                    lat_mma(acc[n], a[p], b[0], b[1]);
-                    lat_mma(acc[n + 1], a[p], b[2], b[3]);
-                }
+                mma_bf16_add<3>(acc[n], a, b[0], b[1]);
+                mma_bf16_add<3>(acc[n + 1], a, b[2], b[3]);
             }
         }
         __syncthreads();                                                // (the stage, the scores and the probabilities are free again)

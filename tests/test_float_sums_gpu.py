@@ -48,3 +48,34 @@ def test_headwise_projection_of_the_largest_floats():
     out = torch.empty(2, 8, device="cuda")
     lib().headwise_linear(x, w, out, 1)
     assert torch.equal(out, x.sum(-1, keepdim=True).expand(2, 8))
+
+
+# scores of rows that differ, and (queries of zero) means of values of one sign, whose sums are the longest
+@pytest.mark.parametrize("heads,dim,vdim,length,splits", [(32, 272, 256, 780, 2), (32, 288, 256, 8000, 2), (20, 320, 64, 3000, 3)])
+@pytest.mark.parametrize("means", [False, True])
+def test_attention_over_one_cached_row(heads, dim, vdim, length, splits, means):
+    """The parts before the merge (the merged output is rounded to bfloat16)."""
+    block, n = 64, 2
+    width = -(-length // block)
+    q = torch.randn(n, heads * dim, device="cuda").bfloat16() * (0 if means else 1)
+    cache = torch.randn(n * width, 1, block, dim, device="cuda").bfloat16()
+    cache = cache.abs() if means else cache
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    out = torch.empty(n, heads * vdim, device="cuda").bfloat16()
+    scratch_o, scratch_ml = (torch.empty(n * heads * splits * size, device="cuda") for size in (vdim, 2))
+    lib().attention_general(q, cache, cache, torch.arange(n * width, device="cuda").int().view(n, width), i32([length - 1] * n), i32(range(n)), out,
+                            heads, 1, dim, vdim, block, dim ** -0.5, value_stride=dim, splits=splits, scratch_o=scratch_o, scratch_ml=scratch_ml)
+    rows = cache.view(n, width * block, dim)[:, :length]
+    parts, (top, total) = scratch_o.view(n, heads, splits, vdim).double(), scratch_ml.view(n, heads, splits, 2).double().unbind(-1)
+    weight = torch.exp(top - top.amax(-1, keepdim=True))
+    got = (weight[..., None] * parts).sum(2) / (weight * total).sum(-1, keepdim=True)
+    scores = q.double().view(n, heads, dim) @ rows.double().transpose(1, 2) * dim ** -0.5
+    want = torch.softmax(scores, -1) @ rows.double()[..., :vdim]
+    # the same in float32, one multiply-add after the other in each part
+    tiles = -(-length // 64)
+    each = -(-tiles // splits) * 64
+    mine = chain(q.view(n, heads, dim), rows) * torch.tensor(dim ** -0.5, device="cuda")
+    p = torch.exp(mine - mine.amax(-1, keepdim=True))
+    plain = sum(chain(p[..., i:i + each], rows[:, i:i + each, :vdim].transpose(1, 2)).double() for i in range(0, length, each))
+    plain = plain / sum(chain(p[..., i:i + each], torch.ones(n, 1, min(each, length - i), device="cuda")).double() for i in range(0, length, each))
+    assert error(got, want) <= error(plain, want)
