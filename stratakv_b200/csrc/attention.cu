@@ -97,8 +97,9 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
             score = row_dot(qs, k_cache + (size_t)row * HD) * scale;
         }
         const float new_max = fmaxf(running_max, warp_max(score));
-        const float p = valid ? expf(score - new_max) : 0.0f;
-        const float rescale = expf(running_max - new_max);     // 0 on the first chunk
+        const float base = new_max == -INFINITY ? 0.0f : new_max;      // (a part whose scores so far are all -infinity weighs nothing)
+        const float p = valid ? expf(score - base) : 0.0f;
+        const float rescale = expf(running_max - base);        // 0 on the first chunk
         running_sum = running_sum * rescale + warp_sum(p);
         running_max = new_max;
 #pragma unroll
@@ -123,7 +124,7 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
         if (lane == 0) { part_max[warp] = running_max; part_sum[warp] = running_sum; }
         __syncthreads();
         if (warp > 0) return;
-        // (the first part always has a key, so the maximum over the parts is finite; a part without keys weighs exp(-inf) = 0)
+        // (a part without keys, or with scores of -infinity alone, weighs exp(-inf) = 0)
         const float own_max = lane < PARTS ? part_max[lane] : -INFINITY;
         const float top = warp_max(own_max);
         const float weight = expf(own_max - top);

@@ -74,3 +74,16 @@ def test_float_attention_over_parts_of_the_keys(lengths, heads, kv_heads, window
         ref = torch.einsum("hj,hjd->hd", torch.softmax(scores, dim=-1), V)
         # scores of up to about 10 carry 64 roundings of 2^-24 each, which the softmax turns into relative errors
         assert (out[i].double() - ref).abs().max() <= 2e-5
+
+
+def test_float_attention_over_a_part_that_weighs_nothing():
+    """Keys whose scores are all -infinity, a whole part of them: they take no share, as in a walk over all keys in turn."""
+    d, block, n, heads = 64, 16, 300, 4
+    keys, values = (torch.randn(19, 1, block, d, device="cuda") for _ in range(2))
+    keys[4:6] = -math.inf                                                  # keys 64 to 95: the third part's first
+    q, i32 = torch.rand(1, heads, d, device="cuda") + 0.1, lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    out = torch.full_like(q, float("nan"))
+    lib(d).attention(q, keys, values, i32([list(range(19))]), i32([n - 1]), i32([0]), out, heads, 1, d, block, d ** -0.5, 0)
+    scores = q[0].double() @ keys.view(-1, d)[:n].double().T * d ** -0.5
+    assert (scores[:, 64:96] == -math.inf).all()
+    assert (out[0].double() - torch.softmax(scores, -1) @ values.view(-1, d)[:n].double()).abs().max() <= 2e-5
