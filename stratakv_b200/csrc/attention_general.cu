@@ -472,8 +472,9 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
             const int row = 4 * warp + i;
             const float2 s = *(const float2*)(scores + row * LAT_S_PITCH + 2 * lane);
             const float new_max = fmaxf(running_max[i], warp_max(fmaxf(s.x, s.y)));
-            const float p[2] = {expf(s.x - new_max), expf(s.y - new_max)};
-            const float factor = expf(running_max[i] - new_max);        // 0 on the first tile
+            const float base = new_max == -INFINITY ? 0.0f : new_max;   // (scores that are all -infinity so far weigh nothing)
+            const float p[2] = {expf(s.x - base), expf(s.y - base)};
+            const float factor = expf(running_max[i] - base);           // 0 on the first tile
             running_sum[i] = running_sum[i] * factor + warp_sum(p[0] + p[1]);
             running_max[i] = new_max;
             if (lane == 0) rescale[row] = factor;

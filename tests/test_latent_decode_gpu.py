@@ -131,3 +131,19 @@ def test_latent_finish(heads, dim, rope, latent, rotated, n, whole, dtype):
     blocks = table[torch.arange(n, device="cuda"), (positions // block_size).long()].long()
     assert near(cache[blocks, 0, (positions % block_size).long()], want)
     assert int((~torch.isnan(cache)).sum()) == n * (latent + rope) and torch.equal(cache.nan_to_num(), kept.nan_to_num())
+
+
+def test_attention_over_one_cached_row_whose_scores_begin_at_minus_infinity():
+    """The first tile of the second part: its rows take no share."""
+    heads, dim, vdim, block, n = 4, 48, 32, 64, 256
+    cache, q = torch.randn(4, 1, block, dim, device="cuda").bfloat16(), (torch.rand(1, heads * dim, device="cuda") + 0.1).bfloat16()
+    cache[2, :, :, vdim:] = -math.inf
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    out, scratch_o, scratch_ml = torch.empty(1, heads * vdim, device="cuda").bfloat16(), torch.empty(heads * 2 * vdim, device="cuda"), torch.empty(heads * 4, device="cuda")
+    lib().attention_general(q, cache, cache, i32([list(range(4))]), i32([n - 1]), i32([0]), out, heads, 1, dim, vdim, block, dim ** -0.5,
+                            value_stride=dim, splits=2, scratch_o=scratch_o, scratch_ml=scratch_ml)
+    rows = cache.view(n, dim).double()
+    scores = q.double().view(heads, dim) @ rows.T * dim ** -0.5
+    assert (scores[:, 128:192] == -math.inf).all()
+    want = torch.softmax(scores, -1) @ rows[:, :vdim]
+    assert ((out.double().view(heads, vdim) - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5).all()
