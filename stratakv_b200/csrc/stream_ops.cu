@@ -291,27 +291,12 @@ static int launch_token_side(float* x, const int* ids, const void* table, int ta
 //   gate: a warp multiplies its own columns (its part of the inner size); sums over warps, then over the cluster;
 //   projection: a warp makes its own columns, which stay in registers while the mean of squares goes round.
 // The stream and the gated values are float32 and stay so: each is split into three bfloat16 whose sum is the float to
-// its last bit (24 of 24), against weights that are bfloat16 anyway, so the products are exact and the sums float.
+// its last bit (24 of 24), against weights that are bfloat16 anyway, so the products are exact and the sums float
+// (mma_bf16_add: what is added errs by 1.3e-7 to 1.5e-7 of itself, 1.8e-7 to 2.2e-7 in the block per token below; sums left in the
+// tensor core erred by 3.1e-7 with many tokens, at 2 to 8 % less time).
 // Few tokens (MT 1): the smallest COLS whose cluster is at most 8 blocks, and the weights are asked into L2 ahead of the
-// wait.  Width 64 on 2,048 at 8 / 300 / 3,874 tokens: 20 / 79 / 187 us before, 10 / 32 / 65; on 4,096: 37 / 136 / 581, 14 / 33 / 137.
+// wait.  Width 64 on 2,048 at 8 / 300 / 3,874 tokens: 20 / 79 / 187 us before, 10 / 35 / 71; on 4,096: 37 / 136 / 581, 14 / 36 / 147.
 constexpr int SIDE_WARPS = 8;
-
-__device__ __forceinline__ void side_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// Three bfloat16 that add up to each of two floats, as pairs.
-__device__ __forceinline__ void split_pair(float u, float v, uint32_t (&out)[3]) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const __nv_bfloat162 part = __floats2bfloat162_rn(u, v);
-        out[i] = *(const uint32_t*)&part;
-        const float2 back = __bfloat1622float2(part);
-        u -= back.x; v -= back.y;
-    }
-}
 
 __device__ __forceinline__ void side_cluster_sync() {
     __syncwarp();
@@ -371,30 +356,28 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
             uint4 w[DIM / 8];
 #pragma unroll
             for (int n = 0; n < DIM / 8; ++n) w[n] = *(const uint4*)(gate_w + (size_t)(8 * n + g) * hidden + k);
-            uint32_t a[3][MT][2][4];
+            uint32_t a[MT][2][3][4];
 #pragma unroll
             for (int m = 0; m < MT; ++m)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float4 u = *(const float4*)(rows[m][h] + k), v = *(const float4*)(rows[m][h] + k + 4);
                     uint32_t p[4][3];
-                    split_pair(u.x, u.y, p[0]); split_pair(u.z, u.w, p[1]);
-                    split_pair(v.x, v.y, p[2]); split_pair(v.z, v.w, p[3]);
+                    split3(u.x, u.y, p[0]); split3(u.z, u.w, p[1]);
+                    split3(v.x, v.y, p[2]); split3(v.z, v.w, p[3]);
 #pragma unroll
                     for (int s = 0; s < 3; ++s) {
-                        a[s][m][0][h] = p[0][s]; a[s][m][0][2 + h] = p[1][s];
-                        a[s][m][1][h] = p[2][s]; a[s][m][1][2 + h] = p[3][s];
+                        a[m][0][s][h] = p[0][s]; a[m][0][s][2 + h] = p[1][s];
+                        a[m][1][s][h] = p[2][s]; a[m][1][s][2 + h] = p[3][s];
                     }
                 }
 #pragma unroll
             for (int n = 0; n < DIM / 8; ++n)
 #pragma unroll
-                for (int m = 0; m < MT; ++m)
-#pragma unroll
-                    for (int s = 2; s >= 0; --s) {
-                        side_mma(acc[m][n], a[s][m][0], w[n].x, w[n].y);
-                        side_mma(acc[m][n], a[s][m][1], w[n].z, w[n].w);
-                    }
+                for (int m = 0; m < MT; ++m) {
+                    mma_bf16_add<3>(acc[m][n], a[m][0], w[n].x, w[n].y);
+                    mma_bf16_add<3>(acc[m][n], a[m][1], w[n].z, w[n].w);
+                }
         }
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -420,13 +403,10 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         const float e = known ? __bfloat162float(table[(size_t)id * table_stride + offset + j]) : 0.0f;
         float sum = 0.0f;
         for (int r = 0; r < ranks; ++r) sum += side_remote(own + i, r);
-        float v = known ? gelu_tanh(sum) * e : 0.0f;
+        uint32_t parts[3];
+        split3(known ? gelu_tanh(sum) * e : 0.0f, 0.0f, parts);
 #pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const __nv_bfloat16 b = __float2bfloat16_rn(v);
-            gated[(s * R + row) * PITCH + j] = b;
-            v -= __bfloat162float(b);
-        }
+        for (int s = 0; s < 3; ++s) gated[(s * R + row) * PITCH + j] = __ushort_as_bfloat16((unsigned short)parts[s]);
     }
     __syncthreads();
 
@@ -447,18 +427,20 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
                 else { const uint2 v = *(const uint2*)at; w[i][0] = v.x; w[i][1] = v.y; }
             }
 #pragma unroll
-            for (int m = 0; m < MT; ++m)
+            for (int m = 0; m < MT; ++m) {
+                uint32_t a[3][4];
 #pragma unroll
-                for (int s = 2; s >= 0; --s) {
+                for (int s = 0; s < 3; ++s) {
                     const __nv_bfloat16* at = gated + (s * R + 16 * m + g) * PITCH + k + 2 * t;
-                    const uint32_t a[4] = {*(const uint32_t*)at, *(const uint32_t*)(at + 8 * PITCH), *(const uint32_t*)(at + 8),
-                                           *(const uint32_t*)(at + 8 * PITCH + 8)};
-#pragma unroll
-                    for (int j = 0; j < TILES; ++j) {
-                        const uint32_t pick = j & 1 ? 0x7632 : 0x5410;
-                        side_mma(y[c][m][j], a, __byte_perm(w[0][j >> 1], w[1][j >> 1], pick), __byte_perm(w[2][j >> 1], w[3][j >> 1], pick));
-                    }
+                    a[s][0] = *(const uint32_t*)at; a[s][1] = *(const uint32_t*)(at + 8 * PITCH);
+                    a[s][2] = *(const uint32_t*)(at + 8); a[s][3] = *(const uint32_t*)(at + 8 * PITCH + 8);
                 }
+#pragma unroll
+                for (int j = 0; j < TILES; ++j) {
+                    const uint32_t pick = j & 1 ? 0x7632 : 0x5410;
+                    mma_bf16_add<3>(y[c][m][j], a, __byte_perm(w[0][j >> 1], w[1][j >> 1], pick), __byte_perm(w[2][j >> 1], w[3][j >> 1], pick));
+                }
+            }
         }
 #pragma unroll
         for (int m = 0; m < MT; ++m)

@@ -79,3 +79,29 @@ def test_attention_over_one_cached_row(heads, dim, vdim, length, splits, means):
     plain = sum(chain(p[..., i:i + each], rows[:, i:i + each, :vdim].transpose(1, 2)).double() for i in range(0, length, each))
     plain = plain / sum(chain(p[..., i:i + each], torch.ones(n, 1, min(each, length - i), device="cuda")).double() for i in range(0, length, each))
     assert error(got, want) <= error(plain, want)
+
+
+def warp_sum(x, w):
+    """``chain`` as a warp makes it: a lane takes four neighbouring numbers of every 128, then the lanes are added in pairs."""
+    lanes = lambda z: z.view(*z.shape[:-1], -1, 32, 4).transpose(-3, -2).flatten(-2).transpose(-3, -2)
+    parts = torch.stack([chain(a, b) for a, b in zip(lanes(x).unbind(-3), lanes(w).unbind(-3))])
+    while len(parts) > 1:
+        parts = parts[:len(parts) // 2] + parts[len(parts) // 2:]
+    return parts[0]
+
+
+# few tokens (a cluster of 16 tokens) and many (of 32)
+@pytest.mark.parametrize("dim,hidden", [(64, 2048), (32, 4096)])
+@pytest.mark.parametrize("n", [8, 300])
+def test_token_input(dim, hidden, n):
+    x, ids = 3 * torch.randn(n, hidden, device="cuda"), torch.randint(0, 50, (n,), device="cuda").int()
+    table, gate = torch.randn(50, dim, device="cuda").bfloat16(), (torch.randn(dim, hidden, device="cuda") / math.sqrt(hidden)).bfloat16()
+    proj, norm = torch.randn(dim, hidden, device="cuda").bfloat16(), 1 + 0.1 * torch.randn(hidden, device="cuda")
+    gelu = lambda z: torch.nn.functional.gelu(z, approximate="tanh")
+    unit = lambda y: y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-5)
+    want = unit((gelu(x.double() @ gate.double().T) * table[ids.long()].double()) @ proj.double()) * norm.double()
+    plain = x + unit(chain(gelu(warp_sum(x, gate.float())) * table[ids.long()].float(), proj.T)) * norm
+    got = x.clone()
+    lib().token_side(got, ids, table, 0, dim, gate, proj, norm, 1e-5)
+    before = x.double()
+    assert error(got.double() - before, want) <= error(plain.double() - before, want)
