@@ -775,12 +775,10 @@ static int launch_linear(const void* a, const void* w, void* out, int M, int N, 
     if ((norm.row_scale || norm.partials_in || norm.partials) && M > 64)
         return fail("skv_linear(bfloat16)", "the norm-fused form serves steps of at most 64 tokens");
     // above 16 tokens the tensor-memory kernels take over, unless a norm is folded into this projection
-    // (above 8 where the weights are 48 MB or more: sixteen tokens' fragments cost the streaming kernel 20 to 40 %, which its
-    // shorter start makes up for only on smaller ones: 16 tokens, 6,144 x 4,096 / 3,072 x 12,288 / 32,000 x 2,048 / 128,256 x 4,096
-    // 17.5 / 24 / 31 / 222 us there, 11.7 / 16 / 21 / 161 here; 4,096 x 4,096 10.2 and 11.1).
-    // (an activation in the epilogue stays here, with libm's exponential and a division)
-    const bool plain = mode != MODE_GATED && !(act & ACT_ON_STORE);
-    if ((M > 16 || (M > 8 && plain && (long long)N * K >= 24LL << 20)) && !norm.row_scale && !norm.partials_in && !norm.partials)
+    // (from 9 tokens on they are faster over large weights, 16 tokens, 6,144 x 4,096 / 128,256 x 4,096 11.7 / 161 us against 17.5 /
+    // 222, but tensor memory keeps a sum over the whole inner size and cuts it off at every step, where eight warps here sum an eighth
+    // each: relative to float64 21e-7 against 4.7e-7, and 21e-7 against 2.4e-7 with an inner size of 2,048)
+    if (M > 16 && !norm.row_scale && !norm.partials_in && !norm.partials)
         return linear_tcgen05(a, w, out, M, N, K, mode, act, flag, stream);
     // at most 8 warps and under 100 registers a thread: two blocks fit on an SM, so the next
     // kernel's weight loads are in flight while this one finishes

@@ -1,5 +1,5 @@
-"""Projections of at most 16 tokens where blocks walk the weight's tiles (at most 8 tokens) and where the tensor-memory kernel takes
-over (9 to 16 tokens, 48 MB of weights), against float64."""
+"""Projections of at most 16 tokens where blocks walk the weight's tiles (at most 8 tokens), and of 8 to 16 tokens over weights around
+48 MB, against float64."""
 import math
 
 import pytest
@@ -18,7 +18,7 @@ def test_tiles_are_walked(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(8, 6146, 4096), (9, 6144, 4096), (16, 6146, 4096), (16, 6142, 4096), (13, 3072, 12288), (12, 40000, 648)])
-def test_where_the_tensor_memory_kernel_takes_over(M, N, K):
+def test_up_to_sixteen_tokens_over_large_weights(M, N, K):
     check(M, N, K)
 
 

@@ -105,3 +105,13 @@ def test_token_input(dim, hidden, n):
     lib().token_side(got, ids, table, 0, dim, gate, proj, norm, 1e-5)
     before = x.double()
     assert error(got.double() - before, want) <= error(plain.double() - before, want)
+
+
+# nine to sixteen tokens, weights on both sides of 48 MB
+@pytest.mark.parametrize("M,N,K", [(9, 32000, 2048), (16, 6144, 4096), (12, 4096, 4096)])
+def test_projection_of_up_to_sixteen_tokens(M, N, K):
+    from stratakv_b200 import ops
+    a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
+    out, want = torch.empty(M, N, device="cuda"), a.double() @ w.double().T
+    lib().linear(a, w, out, ops.MODE_STORE_F32)
+    assert error(out, want) <= error(chain(a, w), want)
