@@ -115,3 +115,14 @@ def test_projection_of_up_to_sixteen_tokens(M, N, K):
     out, want = torch.empty(M, N, device="cuda"), a.double() @ w.double().T
     lib().linear(a, w, out, ops.MODE_STORE_F32)
     assert error(out, want) <= error(chain(a, w), want)
+
+
+@pytest.mark.parametrize("rank,channels", [(64, 2048), (256, 512), (480, 512)])
+@pytest.mark.parametrize("n", [4, 100])
+def test_decay_per_channel(rank, channels, n):
+    lora, w2, w0 = torch.randn(n, rank, device="cuda"), (torch.randn(rank, channels, device="cuda") / math.sqrt(rank)).bfloat16(), torch.randn(channels, device="cuda") - 2
+    out = torch.empty(n, channels, device="cuda")
+    lib().time_mix_decay(lora, rank, w2, w0, out)
+    want = torch.exp(-torch.exp(torch.tanh(lora.double()) @ w2.double() + w0.double()))
+    plain = torch.exp(-torch.exp(chain(torch.tanh(lora), w2.T) + w0))
+    assert error(out, want) <= error(plain, want)
