@@ -60,6 +60,8 @@ constexpr int F_STAGES_AT = (F_TABLE_AT + FTABLE * 4 + 127) / 128 * 128;   // al
 constexpr int F_SMEM_LIMIT = 227 * 1024;
 static_assert(16 * FPITCH * 4 <= 2 * FWARP_BYTES, "the merge area reuses the stages");
 static_assert(F_STAGES_AT + 2 * FWIDE * FWARP_BYTES <= F_SMEM_LIMIT, "shared memory");
+// Whether two blocks of four warps share an SM's 228 KB (each takes 1 KB besides its own): head sizes up to 160.
+constexpr bool FNARROW_PAIRS = 2 * (F_STAGES_AT + 2 * FNARROW * FWARP_BYTES + 1024) <= 228 * 1024;
 
 __device__ __forceinline__ void f_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                       uint32_t b0, uint32_t b1) {
@@ -130,6 +132,17 @@ struct NewTokenFinish {
 __device__ __forceinline__ float4 f_add4(float4 a, const float* bias) {
     const float4 b = *(const float4*)bias;
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// Warps of a block.  Above head size 64 a block of eight fills an SM, and where there are more blocks than SMs each wave's start
+// and end lie bare: blocks of four warps on stages of 64 keys share an SM in twos, where they fit (head size 128: 8 sequences x 24
+// key heads over 430 keys 21 -> 16 us, 64 x 8 over 390 keys 48 -> 35, 64 x 32 over 1,000 keys 277 -> 225; at 192, where one block
+// has the SM to itself, four warps lose: 8 x 24 over 430 keys 28 -> 36 us, 32 x 24 over 1,000 156 -> 226).  Long pieces are bound by bytes, so that a last wave of twos that is half empty
+// costs more than it hides (16 x 24 over 1,000 keys: 384 blocks are three waves of one and four halves of two, 58 us against 63):
+// there the eight warps stay.
+static int fused_warps(long long blocks, long long keys, int splits, int sms) {
+    const long long waves = (blocks + sms - 1) / sms, pairs = 2 * ((blocks + 2 * sms - 1) / (2 * sms));
+    return FNARROW_PAIRS && FHD > 64 && blocks > sms && (10 * pairs <= 11 * waves || keys <= 512 * splits) ? FNARROW : FWIDE;
 }
 
 // EXTRAS false: the instantiation without any of the optional steps (nothing of them is compiled in, so the plain
@@ -573,16 +586,10 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
     }
     // Two stages of 128 keys let two blocks of head size 64 share an SM.  A block that has an SM to itself, and whose
     // piece of the longest context is at most four stages, fetches the whole piece ahead instead (measured: batch 8 at
-    // 2,048 keys gains 3 % that way, while deeper staging of longer pieces loses 10 %).  Above head size 64 a block of
-    // eight warps fills an SM, and where there are more blocks than SMs each wave's start and end lie bare: blocks of
-    // four warps on stages of 64 keys share an SM in twos (head size 128: 8 sequences x 24 key heads over 430 keys
-    // 21 -> 16 us, 64 x 8 over 390 keys 48 -> 35, 64 x 32 over 1,000 keys 277 -> 225).  Long pieces are bound by bytes, so
-    // that a last wave of twos that is half empty costs more than it hides (16 x 24 over 1,000 keys: 384 blocks are three
-    // waves of one and four halves of two, 58 us against 63): there the eight warps stay.
+    // 2,048 keys gains 3 % that way, while deeper staging of longer pieces loses 10 %).
     const long long blocks = (long long)n_seqs * num_kv_heads * m_tiles * splits;
-    const long long waves = (blocks + sm_count - 1) / sm_count, pairs = 2 * ((blocks + 2 * sm_count - 1) / (2 * sm_count));
-    const bool narrow = FHD > 64 && blocks > sm_count && (10 * pairs <= 11 * waves || (long long)table_width * block_size <= 512 * splits);
-    const int warps = narrow ? FNARROW : FWIDE, stage_bytes = warps * FWARP_BYTES;
+    const int warps = fused_warps(blocks, (long long)table_width * block_size, splits, sm_count), stage_bytes = warps * FWARP_BYTES;
+    const bool narrow = warps == FNARROW;
     const long long piece_chunks = ((long long)table_width * block_size / splits + warps * 16 - 1) / (warps * 16);
     const int room = (F_SMEM_LIMIT - F_STAGES_AT) / stage_bytes;
     // (a third stage for longer pieces, which two blocks of head size 64 could still share an SM with, measured
@@ -629,6 +636,9 @@ SKV_EXPORT int skv_attention_decode_fused(const float* qkv, const float* cos_sin
 
 SKV_EXPORT int skv_has_attention_decode_fused() { return 1; }
 
+// Warps that a block of such a step takes on a GPU of `sms` SMs.
+SKV_EXPORT int skv_attention_decode_fused_warps(int blocks, int keys, int splits, int sms) { return fused_warps(blocks, keys, splits, sms); }
+
 #else
 
 SKV_EXPORT int skv_attention_decode_fused(const float*, const float*, void*, void*, const int*, int, const int*, void*,
@@ -646,5 +656,7 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float*, int, const float*
 }
 
 SKV_EXPORT int skv_has_attention_decode_fused() { return 0; }
+
+SKV_EXPORT int skv_attention_decode_fused_warps(int, int, int, int) { return 0; }
 
 #endif

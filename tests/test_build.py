@@ -37,3 +37,15 @@ def test_one_handle_has_both_libraries_and_one_message(dtype):
     assert lib.skv_last_error().startswith(b"skv_attention:")
     assert lib.skv_rmsnorm(null, null, ctypes.c_float(1.0), null, null, one, ctypes.c_int(0), one, null) != 0
     assert lib.skv_last_error().startswith(b"skv_rmsnorm:")
+
+
+# (blocks, keys, parts): more blocks than SMs, short pieces and long ones; as many blocks as SMs
+@pytest.mark.parametrize("head_dim,pairs", [(64, False), (80, True), (128, True), (192, False)])
+def test_narrow_blocks_of_fused_decode_where_two_share_an_sm(head_dim, pairs):
+    """At 192 two blocks of four warps take 250 KB, more than an SM has: they ran alone, with half the bytes on their way."""
+    path = build.find_built("bfloat16", head_dim)
+    if path is None:
+        pytest.skip("not compiled yet")
+    warps = ctypes.CDLL(str(path)).skv_attention_decode_fused_warps
+    assert warps(192, 448, 1, 148) == warps(2 * 148, 4096, 1, 148) == (4 if pairs else 8)
+    assert warps(148, 448, 1, 148) == 8 and warps(384, 1024, 1, 148) == 8
