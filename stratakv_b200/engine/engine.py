@@ -149,6 +149,13 @@ class Engine:
             self._pinned = torch.empty(capacity, dtype=torch.int32, pin_memory=pin)
         return self._pinned, self._meta
 
+    def _check_vocabulary(self, entries, token_arrays) -> None:
+        vocab = self.spec.vocab_size
+        for e, tokens in zip(entries, token_arrays):
+            outside = np.flatnonzero((tokens < 0) | (tokens >= vocab))
+            if outside.size:
+                raise StepError(f"slot {e.slot}: token id {int(tokens[outside[0]])} is outside the vocabulary of {vocab}")
+
     def prepare(self, entries: Sequence[StepEntry]):
         """Check a step, reserve its cache blocks, and upload its metadata.
         Returns ``(StepBatch, want_rows, n_want)``; nothing has run yet."""
@@ -161,27 +168,27 @@ class Engine:
         if len(entries) > self.config.slots:
             raise StepError(f"{len(entries)} sequences in one step; the engine holds {self.config.slots}")
         q_lens, ctx_before, wanted, token_arrays = [], [], {}, []
-        for e in entries:
-            if e.slot not in self.cache.sequences:
-                raise StepError(f"slot {e.slot} is not open")
-            if len(e.tokens) == 0:
-                raise StepError(f"slot {e.slot}: a step needs at least one token per sequence")
-            tokens = _token_array(e.tokens)
-            for w in e.want:
-                if not (0 <= int(w) < len(e.tokens)):
-                    raise StepError(f"slot {e.slot}: wanted place {w} is outside this step's {len(e.tokens)} tokens")
-            before = self.cache.length(e.slot)
-            self._check_context(e.slot, before + len(e.tokens))
-            token_arrays.append(tokens)
-            q_lens.append(len(e.tokens))
-            ctx_before.append(before)
-            wanted[e.slot] = before + len(e.tokens)
+        try:
+            for e in entries:
+                if e.slot not in self.cache.sequences:
+                    raise StepError(f"slot {e.slot} is not open")
+                if len(e.tokens) == 0:
+                    raise StepError(f"slot {e.slot}: a step needs at least one token per sequence")
+                token_arrays.append(_token_array(e.tokens))
+                for w in e.want:
+                    if not (0 <= int(w) < len(e.tokens)):
+                        raise StepError(f"slot {e.slot}: wanted place {w} is outside this step's {len(e.tokens)} tokens")
+                before = self.cache.length(e.slot)
+                self._check_context(e.slot, before + len(e.tokens))
+                q_lens.append(len(e.tokens))
+                ctx_before.append(before)
+                wanted[e.slot] = before + len(e.tokens)
+        except Exception:
+            self._check_vocabulary(entries, token_arrays)       # (a token id that came before what is wrong is named first)
+            raise
         token_ids = np.concatenate(token_arrays) if len(token_arrays) > 1 else token_arrays[0]
         if int(token_ids.min()) < 0 or int(token_ids.max()) >= vocab:        # (one look at all of them; who it was, only then)
-            for e, tokens in zip(entries, token_arrays):
-                outside = np.flatnonzero((tokens < 0) | (tokens >= vocab))
-                if outside.size:
-                    raise StepError(f"slot {e.slot}: token id {int(tokens[outside[0]])} is outside the vocabulary of {vocab}")
+            self._check_vocabulary(entries, token_arrays)
         self.cache.reserve(wanted)              # CacheFull leaves everything as it was
 
         n, total = len(entries), sum(q_lens)

@@ -66,6 +66,14 @@ def test_step_checks(tmp_path):
         probe = engine.open_sequence()
         assert engine.step([StepEntry(probe, ids, [1])]).shape == (1, 256)
         engine.close_sequence(probe)
+    # several things wrong: the first in the step's order is named
+    for later in (StepEntry(99, [1], []), StepEntry(engine.open_sequence(), [1, 2], [2]), StepEntry(engine.open_sequence(), [], [])):
+        with pytest.raises(StepError, match=f"slot {slot}: token id 256 is outside the vocabulary"):
+            engine.step([StepEntry(slot, [1, 256], [0]), later])
+        if later.slot != 99:
+            engine.close_sequence(later.slot)
+    with pytest.raises(StepError, match=f"slot {slot}: token id 256 is outside the vocabulary"):
+        engine.step([StepEntry(slot, [1, 256], [7])])
     with pytest.raises(StepError, match="at least one token"):
         engine.step([StepEntry(slot, [], [])])
     with pytest.raises(StepError, match="twice"):
