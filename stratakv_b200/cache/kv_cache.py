@@ -57,6 +57,10 @@ class SequenceRecord:
     dropped: Dict[int, int] = field(default_factory=dict)          # group -> leading logical blocks freed
 
 
+def _capturing(device) -> bool:
+    return device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+
+
 class KVCache:
     def __init__(self, requests: Sequence[CacheRequest], num_blocks: int, block_size: int,
                  max_slots: int, dtype: torch.dtype, device):
@@ -122,8 +126,10 @@ class KVCache:
 
     def state(self, entry: int) -> torch.Tensor:
         """``[max_slots + 1, state_bytes]`` bytes of per-sequence state of one cache entry (the last row is the
-        spare one of ``spare_slot``)."""
-        self._zero_new_rows()
+        spare one of ``spare_slot``).  While a step is captured as a graph nothing is zeroed here: its own slots' rows are
+        since ``reserve``, and a slot taken after that would be zeroed at every replay."""
+        if self._unzeroed and not _capturing(self.device):
+            self._zero_new_rows()
         return self._state[entry]
 
     def _zero_new_rows(self) -> None:

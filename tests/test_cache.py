@@ -112,6 +112,21 @@ def test_state_is_zeroed_when_a_slot_is_taken():
     assert again == slot and int(cache.state(0)[again].sum()) == 0
 
 
+def test_nothing_is_zeroed_while_a_graph_is_captured(monkeypatch):
+    """A launch recorded then would be repeated at every replay, over a live sequence's state."""
+    from stratakv_b200.cache import kv_cache
+    cache = KVCache([CacheRequest("none", state_bytes=8), CacheRequest("kv", 1, 16)], 4, 16, 2, torch.float32, "cpu")
+    captured = cache.acquire()
+    cache.reserve({captured: 1})
+    cache._state[0][:] = 7                             # (what an earlier sequence left)
+    later = cache.acquire()
+    with monkeypatch.context() as context:
+        context.setattr(kv_cache, "_capturing", lambda device: True)
+        assert (cache.state(0) == 7).all()
+    cache.reserve({later: 1})
+    assert (cache._state[0][later] == 0).all() and (cache._state[0][captured] == 7).all()
+
+
 def test_random_traffic_never_loses_a_block():
     rng = random.Random(0)
     cache = kv(entries=1, blocks=12, slots=5)
