@@ -570,6 +570,16 @@ SKV_EXPORT int skv_paged_gather(const void* cache, const int* block_table, int t
                       (const skv_t*)cache, block_table, table_width, positions, seqs, (skv_t*)out, n_rows, width, block_size);
 }
 
+// Whether attention over one cached row of `dim` numbers for all heads, the first `vdim` of them the value, has a tensor-core form
+// for parts of the keys: rows in whole steps of 16 numbers that fit its tiles.
+SKV_EXPORT int skv_attention_latent_serves(int dim, int vdim) {
+#if SKV_DTYPE == SKV_BF16
+    return dim % 16 == 0 && dim <= LAT_MAX_DIM && vdim % 16 == 0 && vdim <= LAT_MAX_VDIM && vdim <= dim;
+#else
+    return 0;
+#endif
+}
+
 // `r1`, `r2`: float [num_heads] or both null.  `gate`: float, the gate's logit of (token t, head h) at
 // gate[t * gate_stride + h], or null.  `out` rows are out_stride >= heads * vdim apart; what lies beyond a row's
 // heads is set to zero.  `sink`: float [num_heads] or null; exp(sink[h]) is added to the softmax's denominator.
@@ -600,10 +610,10 @@ SKV_EXPORT int skv_attention_general(const void* q, const void* k_cache, const v
     if (blocks > 0x7fffffffLL) return fail("skv_attention_general", "too many tokens in one step");
 #if SKV_DTYPE == SKV_BF16
     // One cached row for all heads whose head is the value, in parts, with nothing that changes a score: the tensor-core
-    // form (rows in whole steps of 16 numbers that fit its tiles, the partial outputs' rows 8-byte aligned)
-    const bool latent = splits > 1 && num_kv_heads == 1 && k_cache == v_cache && value_stride == dim && dim % 16 == 0 && dim <= LAT_MAX_DIM &&
-                        vdim % 16 == 0 && vdim <= LAT_MAX_VDIM && vdim <= dim && window == 0 && !r1 && softcap == 0.0f &&
-                        items * splits <= 0x7fffffffLL && (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)partial_o) & 15) == 0;
+    // form, where the sizes are its own and the partial outputs' rows 8-byte aligned
+    const bool latent = splits > 1 && num_kv_heads == 1 && k_cache == v_cache && value_stride == dim && skv_attention_latent_serves(dim, vdim) &&
+                        window == 0 && !r1 && softcap == 0.0f && items * splits <= 0x7fffffffLL &&
+                        (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)partial_o) & 15) == 0;
     if (latent) {
         const size_t room = (size_t)((LAT_HEADS + 2 * LAT_KEYS) * (dim + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + (size_t)LAT_HEADS * (LAT_S_PITCH + 1) * 4;
         static const cudaError_t ready = cudaFuncSetAttribute(latent_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

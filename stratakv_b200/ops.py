@@ -540,6 +540,11 @@ class Kernels:
             ctypes.c_float(qk_norm_eps), _ptr(k_norm_weight), ctypes.c_float(coef), int(every), int(key_dim),
             _stream()), "qkv_finish")
 
+    def attention_latent(self, dim: int, vdim: int) -> bool:
+        """True if ``attention_general`` has a tensor-core form for parts of the keys (``splits`` > 1) where all heads share one
+        cached row of ``dim`` numbers whose first ``vdim`` are the value."""
+        return bool(self.lib.skv_attention_latent_serves(int(dim), int(vdim)))
+
     def attention_general(self, q, k_cache, v_cache, block_table, positions, token_seq, out, num_heads: int,
                           num_kv_heads: int, dim: int, vdim: int, block_size: int, scale: float, window: int = 0,
                           r1=None, r2=None, gate=None, gate_stride: int = 0, softcap: float = 0.0,

@@ -41,6 +41,13 @@ def _extended(spec) -> bool:
                 or getattr(spec, "shares_kv", False))
 
 
+def decode_parts(pairs: int, max_ctx: int, sm_count: int, on_tensor_cores: bool) -> int:
+    """Parts that a decode step of so many (token, head) pairs cuts each pair's keys into: enough to give every SM thirty-odd
+    warps, of 64 keys at least; two at least where the kernel for parts runs on tensor cores (``Kernels.attention_latent``), which
+    is worth the merge."""
+    return max(2 if on_tensor_cores else 1, min(-(-sm_count * 32 // pairs), -(-max_ctx // 64), 64))
+
+
 class LatentAttention(Mixer):
     graph_safe = True
     stores_branch = True
@@ -185,11 +192,10 @@ class LatentAttention(Mixer):
         ops.headwise_linear(q_plain, self.w_k_up_t, q_folded, s.num_heads, out_head_stride=self.key_dim)
         mixed = rt.workspace.get("latent_ctx", (n, s.num_heads * s.latent_dim), rt.dtype)
         # one token a sequence: few (token, head) pairs over long contexts, so each pair's keys are cut into parts that
-        # run side by side, enough to give every SM thirty-odd warps (a part is at least 64 keys)
+        # run side by side, enough to give every SM thirty-odd warps
         splits, scratch_o, scratch_ml = 1, None, None
         if step.is_decode and rt.device.type == "cuda":
-            # (the bfloat16 kernel for parts of a latent's keys is worth the merge even in two)
-            splits = max(2 if rt.dtype == torch.bfloat16 else 1, min(-(-rt.sm_count * 32 // (n * s.num_heads)), -(-step.max_ctx // 64), 64))
+            splits = decode_parts(n * s.num_heads, step.max_ctx, rt.sm_count, ops.attention_latent(self.key_dim, s.latent_dim))
             if splits > 1:
                 scratch_o = rt.workspace.get("attn_split_o", (n * s.num_heads * splits * s.latent_dim,), torch.float32)
                 scratch_ml = rt.workspace.get("attn_split_ml", (n * s.num_heads * splits * 2,), torch.float32)
