@@ -208,7 +208,8 @@ route_tokens_kernel(const T* __restrict__ h, const T* __restrict__ router, const
 #if SKV_DTYPE == SKV_BF16
 // The same on tensor cores, for rows of whole 64 bytes: a block takes 16 tokens, its 16 warps share the hidden numbers out and
 // add up in shared memory, then each warp chooses for one token.  Rows and weights are bfloat16, so the products are exact;
-// every 32 of them are added to a float sum by an ordinary addition.  A block of one token's dot products (above) read
+// every 16 of them are added to a float sum by an ordinary addition (mma_bf16_add), and the warps' sums in pairs: weights of a softmax
+// err as the kernel above does (0.94 to 1.00 of it; 1.1 to 1.4 with 32 products at a time and the warps one after the other).  A block of one token's dot products (above) read
 // the router once a token and was a chain of waits: E 8 of 2,048, 8 / 300 / 5,180 tokens
 // 4.2 / 6.5 / 37 us, 3.6 / 4.5 / 12.5 here; 64 experts 16 / 32 / 208 and 8 / 9 / 29.
 // The first weights are in registers, and the others asked into L2, ahead of the wait: in a step of few tokens they come
@@ -265,11 +266,9 @@ route_tokens_mma_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16
                 if (s0 + ROUTE_MMA_WARPS * p >= steps) break;
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
-                    float c[4] = {};
-                    mma_bf16_16816(c, a[p][0].x, a[p][1].x, a[p][0].y, a[p][1].y, w[p][j].x, w[p][j].y);
-                    mma_bf16_16816(c, a[p][0].z, a[p][1].z, a[p][0].w, a[p][1].w, w[p][j].z, w[p][j].w);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[j][i] += c[i];
+                    const uint32_t first[1][4] = {{a[p][0].x, a[p][1].x, a[p][0].y, a[p][1].y}}, second[1][4] = {{a[p][0].z, a[p][1].z, a[p][0].w, a[p][1].w}};
+                    mma_bf16_add<1>(acc[j], first, w[p][j].x, w[p][j].y);
+                    mma_bf16_add<1>(acc[j], second, w[p][j].z, w[p][j].w);
                 }
             }
         }
@@ -283,9 +282,14 @@ route_tokens_mma_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16
         for (int i = threadIdx.x; i < ROUTE_ROWS * COLS; i += ROUTE_MMA_WARPS * 32) {
             const int row = i / COLS, e = n0 + i % COLS;
             if (e >= dots || t0 + row >= n_tokens) continue;
-            float sum = part[i];
+            float sums[ROUTE_MMA_WARPS];                              // (added in pairs: fewer roundings at the sum's full size)
 #pragma unroll
-            for (int k = 1; k < ROUTE_MMA_WARPS; ++k) sum += part[k * ROUTE_ROWS * COLS + i];
+            for (int k = 0; k < ROUTE_MMA_WARPS; ++k) sums[k] = part[k * ROUTE_ROWS * COLS + i];
+#pragma unroll
+            for (int half = ROUTE_MMA_WARPS / 2; half > 0; half /= 2)
+#pragma unroll
+                for (int k = 0; k < half; ++k) sums[k] += sums[k + half];
+            const float sum = sums[0];
             const float s = softmax && e < experts ? sum : 1.0f / (1.0f + expf(-sum));
             if (e < experts) {
                 score[row * experts + e] = s;

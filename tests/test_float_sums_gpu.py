@@ -126,3 +126,15 @@ def test_decay_per_channel(rank, channels, n):
     want = torch.exp(-torch.exp(torch.tanh(lora.double()) @ w2.double() + w0.double()))
     plain = torch.exp(-torch.exp(chain(torch.tanh(lora), w2.T) + w0))
     assert error(out, want) <= error(plain, want)
+
+
+# (a softmax of large scores: the error of a sum is the relative error of its weight)
+@pytest.mark.parametrize("experts,hidden", [(8, 2048), (64, 4096)])
+def test_router(experts, hidden, n=2000):
+    h, w = torch.randn(n, hidden, device="cuda").bfloat16(), (8 * torch.randn(experts, hidden, device="cuda") / math.sqrt(hidden)).bfloat16()
+    chosen, weights = torch.empty(n, 4, dtype=torch.int32, device="cuda"), torch.empty(n, 4, device="cuda")
+    lib().route_tokens(h, w, None, 4, 1.0, False, chosen, weights, softmax=True)
+    want = torch.softmax(h.double() @ w.double().T, -1).gather(1, chosen.long())
+    plain = torch.softmax(warp_sum(h.float(), w.float()).double(), -1).gather(1, chosen.long())
+    # (besides the sums' errors the kernel's weights have those of an exponential, a sum and a division: four units of 2^-24)
+    assert error(weights / want, torch.ones_like(want)) <= math.hypot(error(plain / want, torch.ones_like(want)), 4 * 2.0 ** -24)
