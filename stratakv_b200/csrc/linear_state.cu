@@ -654,10 +654,11 @@ linear_state_output_kernel(const float* __restrict__ rows, const float* __restri
                     acc[a][2] = fmaf(qi[a], sv.z, acc[a][2]); acc[a][3] = fmaf(qi[a], sv.w, acc[a][3]);
                 }
             }
+            float own_sum[RI][4];                             // (a sum of its own: its roundings are of its own size)
 #pragma unroll
             for (int a = 0; a < RI; ++a)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[a][e] *= carry[a];
+                for (int e = 0; e < 4; ++e) own_sum[a][e] = 0.0f;
 #pragma unroll 4
             for (int j = 0; j < j_end; ++j) {                 // what the chunk's own tokens give
                 const float4 ve = *(const float4*)(vs + j * 64 + tx * 4);
@@ -671,10 +672,14 @@ linear_state_output_kernel(const float* __restrict__ rows, const float* __restri
                 }
 #pragma unroll
                 for (int a = 0; a < RI; ++a) {
-                    acc[a][0] = fmaf(wi[a], ve.x, acc[a][0]); acc[a][1] = fmaf(wi[a], ve.y, acc[a][1]);
-                    acc[a][2] = fmaf(wi[a], ve.z, acc[a][2]); acc[a][3] = fmaf(wi[a], ve.w, acc[a][3]);
+                    own_sum[a][0] = fmaf(wi[a], ve.x, own_sum[a][0]); own_sum[a][1] = fmaf(wi[a], ve.y, own_sum[a][1]);
+                    own_sum[a][2] = fmaf(wi[a], ve.z, own_sum[a][2]); own_sum[a][3] = fmaf(wi[a], ve.w, own_sum[a][3]);
                 }
             }
+#pragma unroll
+            for (int a = 0; a < RI; ++a)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[a][e] = fmaf(acc[a][e], carry[a], own_sum[a][e]);
             const int e = e0 + tx * 4;
 #pragma unroll
             for (int a = 0; a < RI; ++a) {

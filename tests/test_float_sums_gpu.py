@@ -138,3 +138,33 @@ def test_router(experts, hidden, n=2000):
     plain = torch.softmax(warp_sum(h.float(), w.float()).double(), -1).gather(1, chosen.long())
     # (besides the sums' errors the kernel's weights have those of an exponential, a sum and a division: four units of 2^-24)
     assert error(weights / want, torch.ones_like(want)) <= math.hypot(error(plain / want, torch.ones_like(want)), 4 * 2.0 ** -24)
+
+
+# sequences of several chunks: what the state gives and what the chunk's own tokens give are sums of their own
+@pytest.mark.parametrize("heads,dim", [(8, 64), (4, 128)])
+def test_retention_of_prompts(heads, dim):
+    """Against the recurrence in float32, a multiply-add a product."""
+    from stratakv_b200.ops import kernels_for
+    k, length = kernels_for(torch.float32, 64, verbose=False), 500
+    fused = torch.randn(length, 4 * heads * dim, device="cuda")
+    decay = 1 - 2.0 ** -(5.0 + torch.arange(heads, device="cuda") % 4)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    state, out = torch.zeros(1, 2 * heads * dim * dim, device="cuda"), torch.empty(length, heads * dim, device="cuda")
+    scratch = torch.empty(k.retention_scratch(1, length, heads, dim, dim), device="cuda")
+    k.retention(fused.clone(), None, 0, decay, 1e-5, out, state, (i32(range(length)), i32([0] * length), i32([0, length]), i32([0])), heads, dim, dim,
+                length, scratch)
+    q, key, v, gate = fused.double().view(length, 4, heads, dim).unbind(1)
+
+    def run(round_it):
+        S, rows, scaled = torch.zeros(heads, dim, dim, device="cuda").double(), [], round_it(key * dim ** -0.5)
+        for t in range(length):
+            S = round_it(decay.double()[:, None, None] * S + round_it(scaled[t, :, :, None] * v[t, :, None, :]))
+            o = torch.zeros(heads, dim, device="cuda").double()
+            for d in range(dim):
+                o = round_it(o + q[t, :, d, None] * S[:, d])
+            rows.append(o)
+        o = torch.stack(rows)
+        return o * torch.rsqrt((o * o).mean(-1, keepdim=True) + 1e-5) * torch.nn.functional.silu(gate)
+
+    want = run(lambda z: z)
+    assert error(out.view(length, heads, dim), want) <= error(run(lambda z: z.float().double()), want)
