@@ -720,12 +720,17 @@ SKV_EXPORT int skv_sort_by_expert(const int* chosen, int pairs, int top, int exp
 // tensor-memory GEMM's grouped form; `flag` is where its bounded waits report that they gave up.
 // Few pairs in bfloat16 (skv_expert_few_serves) read each chosen expert's weights once, wherever the rows lie; `place`
 // [tokens, top] and `weights` [tokens, top] (both or neither; with rows) multiply each row by its pair's weight first.
-SKV_EXPORT int skv_expert_few_serves(int pairs, int experts, int K) {
+// `fullest`: the most rows one expert may have (as many as there are tokens), 0 where it is not known.
+SKV_EXPORT int skv_expert_few_serves(int pairs, int experts, int K, int fullest) {
 #if SKV_DTYPE == SKV_BF16
     // up to four rows an expert on average: 16 tokens x 2 of 8 experts of 7168 x 4096 take 138 + 74 us here and 190 + 90 in the
     // tensor-memory form's tiles, 1 token 42 + 22 and 87 + 62.  Short rows leave a block little to stream (64 experts, rows of
-    // 512: 64 pairs 41 us against 46, 128 pairs 52 against 46): they come here up to a pair an expert
-    return pairs <= (K >= 1024 ? 4 : 1) * experts && K % 8 == 0;
+    // 512: 64 pairs 41 us against 46, 128 pairs 52 against 46): they come here up to a pair an expert.
+    // Where all tokens choose the same experts these go over their rows eight a round: with 2 of 8 experts of 2816 x 2048 or 4 of 64
+    // of 1408 x 2048 chosen by all of 16 / 32 / 64 tokens 16 + 9 / - / - and 24 + 16 / 36 + 23 / 62 + 35 us, in tiles 17 + 14 / - / -
+    // and 16 + 11 / 16 + 11 / 16 + 12 (8 of 128 of 1024 x 2048, 16 tokens: 35 + 29 and 19 + 12).  So more than two rounds are not
+    // risked, though choices at random gain there too (4 of 64, 16 / 64 tokens: 83 + 51 / 121 + 71 against 110 + 63 / 150 + 81).
+    return pairs <= (K >= 1024 ? 4 : 1) * experts && K % 8 == 0 && fullest <= 16;
 #else
     return 0;
 #endif
@@ -733,8 +738,8 @@ SKV_EXPORT int skv_expert_few_serves(int pairs, int experts, int K) {
 
 SKV_EXPORT int skv_expert_linear(const void* a, int a_stride, int a_rows, const int* rows, const void* w,
                                  const int* offsets, void* out, int out_is_float, int pairs, int experts, int N, int K,
-                                 act_t act, int gated, const int* place, const float* weights, int top, int* flag,
-                                 cudaStream_t stream) {
+                                 act_t act, int gated, const int* place, const float* weights, int top, int fullest,
+                                 int* flag, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (experts <= 0 || experts > ROUTE_MAX_EXPERTS || N <= 0 || K <= 0 || a_stride < K || a_rows <= 0)
         return fail("skv_expert_linear", "sizes do not agree");
@@ -744,7 +749,7 @@ SKV_EXPORT int skv_expert_linear(const void* a, int a_stride, int a_rows, const 
     if ((place == nullptr) != (weights == nullptr) || (place && (!rows || top <= 0 || pairs % top)))
         return fail("skv_expert_linear", "weighted rows need their tokens, places and weights");
 #if SKV_DTYPE == SKV_BF16
-    if (skv_expert_few_serves(pairs, experts, K) && a_stride % 8 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15)) {
+    if (skv_expert_few_serves(pairs, experts, K, fullest) && a_stride % 8 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15)) {
         const dim3 grid(((gated ? 2 * N : N) + 15) / 16, experts);
         const FewWeigh weigh = {place, weights, top};
         auto kernel = gated ? (out_is_float ? expert_few_kernel<true, true> : expert_few_kernel<true, false>)

@@ -944,14 +944,16 @@ class Kernels:
         build's tensor-core form wants neighbouring rows of whole 16 bytes."""
         return self.dtype == torch.bfloat16 and hidden % 8 == 0
 
-    def expert_few(self, pairs: int, experts: int, hidden: int) -> bool:
+    def expert_few(self, pairs: int, experts: int, hidden: int, fullest: int = 0) -> bool:
         """True if ``expert_linear`` serves this many pairs with the kernel that streams each chosen expert's weights once
-        and reads its rows where the tokens lie (``rows``; weighted on the way with ``place`` and ``weights``)."""
-        return self.dtype == torch.bfloat16 and bool(self.lib.skv_expert_few_serves(int(pairs), int(experts), int(hidden)))
+        and reads its rows where the tokens lie (``rows``; weighted on the way with ``place`` and ``weights``).  ``fullest``:
+        the most rows one expert may have, where that is known (the tokens)."""
+        return self.dtype == torch.bfloat16 and bool(self.lib.skv_expert_few_serves(int(pairs), int(experts), int(hidden), int(fullest)))
 
     def expert_linear(self, a, w, offsets, out, rows=None, activation: Optional[str] = None, flag=None,
-                      gated: bool = False, activation_param: float = 0.0, place=None, weights=None):
-        """(``activation_param``: the number of a parametric activation, which gated experts may have.)
+                      gated: bool = False, activation_param: float = 0.0, place=None, weights=None, fullest: int = 0):
+        """(``fullest``: as in ``expert_few``.)
+        (``activation_param``: the number of a parametric activation, which gated experts may have.)
         (``gated``: ``w`` is ``[experts, 2 N, K]`` in tiles of 8 gate rows and their 8 up rows, as ``pack_gate_up``
         lays them out, and ``out[p] = act(gate_e . a) * (up_e . a)``.)
         ``out[p] = act(w[e] . a[row(p)])`` for every sorted pair p of expert e (``offsets`` from ``sort_by_expert``);
@@ -976,7 +978,7 @@ class Kernels:
                 raise KernelError("expert_linear: one row index per pair is needed")
         if place is not None:
             self._want(place, torch.int32, "place"); self._want(weights, torch.float32, "weights")
-            if rows is None or place.numel() != pairs or place.shape != weights.shape or not self.expert_few(pairs, experts, K):
+            if rows is None or place.numel() != pairs or place.shape != weights.shape or not self.expert_few(pairs, experts, K, fullest):
                 raise KernelError("expert_linear: rows are weighted on their way in for few pairs only, with a weight and a place each")
         if activation is not None and (activation not in ACTIVATIONS or (activation in PARAMETRIC_ACTIVATIONS and not gated)):
             raise KernelError(f"expert_linear: activation '{activation}' is not supported")
@@ -984,7 +986,7 @@ class Kernels:
             _ptr(a), a.stride(0), a.shape[0], _ptr(rows), _ptr(w), _ptr(offsets), _ptr(out),
             int(out.dtype == torch.float32), pairs, experts, N, K,
             activation_word(activation, activation_param) if activation is not None else ctypes.c_longlong(-1),
-            int(bool(gated)), _ptr(place), _ptr(weights), place.shape[-1] if place is not None else 0,
+            int(bool(gated)), _ptr(place), _ptr(weights), place.shape[-1] if place is not None else 0, int(fullest),
             _ptr(flag if flag is not None else self.error_flag), _stream()), "expert_linear")
 
     def combine_experts(self, results, place, weights, shared, share, x, add: bool = True):

@@ -134,23 +134,24 @@ class RoutedMlp(FeedForward):
         ops.sort_by_expert(chosen, s.experts, offsets, order, place)
         hidden = get("routed_hidden", (pairs, self.padded), rt.dtype)
         gate = dict(activation=s.activation, gated=self.gated, activation_param=getattr(s, "activation_param", 0.0))
-        if rt.device.type == "cuda" and ops.expert_few(pairs, s.experts, s.hidden_size):
+        fullest = dict(fullest=n) if rt.device.type == "cuda" else {}
+        if fullest and ops.expert_few(pairs, s.experts, s.hidden_size, **fullest):
             # few pairs: each chosen expert's weights are streamed once, its rows read where the tokens lie
-            ops.expert_linear(h, self.w_up, offsets, hidden, rows=order, **gate,
+            ops.expert_linear(h, self.w_up, offsets, hidden, rows=order, **gate, **fullest,
                               **(dict(place=place, weights=weights) if self.weigh_input else {}))
         elif self.weigh_input:
             rows = get("routed_rows", (pairs, s.hidden_size), rt.dtype)
             ops.scatter_rows(h, place, weights, rows)
-            ops.expert_linear(rows, self.w_up, offsets, hidden, **gate)
+            ops.expert_linear(rows, self.w_up, offsets, hidden, **gate, **fullest)
         elif ops.expert_rows_sorted_first(s.hidden_size):
             # the tensor-core projection reads tiles of neighbouring rows: bring the tokens' rows into sorted order first
             gathered = get("routed_rows", (pairs, s.hidden_size), rt.dtype)
             ops.gather_rows(h, order, gathered)
-            ops.expert_linear(gathered, self.w_up, offsets, hidden, **gate)
+            ops.expert_linear(gathered, self.w_up, offsets, hidden, **gate, **fullest)
         else:
-            ops.expert_linear(h, self.w_up, offsets, hidden, rows=order, **gate)
+            ops.expert_linear(h, self.w_up, offsets, hidden, rows=order, **gate, **fullest)
         results = get("routed_results", (pairs, s.hidden_size), torch.float32)
-        ops.expert_linear(hidden, self.w_down, offsets, results)
+        ops.expert_linear(hidden, self.w_down, offsets, results, **fullest)
         shared_out = None
         if self.shared_up is not None:
             z = get("ffn_hidden", (n, self.shared_padded), rt.dtype)

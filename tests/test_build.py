@@ -49,3 +49,14 @@ def test_narrow_blocks_of_fused_decode_where_two_share_an_sm(head_dim, pairs):
     warps = ctypes.CDLL(str(path)).skv_attention_decode_fused_warps
     assert warps(192, 448, 1, 148) == warps(2 * 148, 4096, 1, 148) == (4 if pairs else 8)
     assert warps(148, 448, 1, 148) == 8 and warps(384, 1024, 1, 148) == 8
+
+
+# (pairs, experts, inner size, the most rows an expert may have): spread over the experts, or perhaps all on a few of them
+@pytest.mark.parametrize("step,serves", [((32, 8, 2048, 16), True), ((32, 8, 2048, 0), True), ((33, 8, 2048, 0), False), ((64, 64, 512, 16), True),
+                                         ((256, 64, 2048, 0), True), ((256, 64, 2048, 128), False), ((68, 64, 2048, 17), False), ((4, 8, 2044, 2), False)])
+def test_experts_of_few_pairs_and_few_tokens(step, serves):
+    """128 tokens that all choose the same 2 of 64 experts were sixteen rounds over the same weights."""
+    path = build.find_built("bfloat16", 64)
+    if path is None:
+        pytest.skip("not compiled yet")
+    assert ctypes.CDLL(str(path)).skv_expert_few_serves(*step) == int(serves)
