@@ -616,9 +616,8 @@ SKV_EXPORT int skv_attention_general(const void* q, const void* k_cache, const v
                         (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)partial_o) & 15) == 0;
     if (latent) {
         const size_t room = (size_t)((LAT_HEADS + 2 * LAT_KEYS) * (dim + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + (size_t)LAT_HEADS * (LAT_S_PITCH + 1) * 4;
-        static const cudaError_t ready = cudaFuncSetAttribute(latent_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int)(((LAT_HEADS + 2 * LAT_KEYS) * (LAT_MAX_DIM + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + LAT_HEADS * (LAT_S_PITCH + 1) * 4));
-        if (ready != cudaSuccess) return fail("skv_attention_general", cudaGetErrorString(ready));
+        constexpr size_t most = (size_t)((LAT_HEADS + 2 * LAT_KEYS) * (LAT_MAX_DIM + 8) + 3 * LAT_HEADS * LAT_P_PITCH) * 2 + (size_t)LAT_HEADS * (LAT_S_PITCH + 1) * 4;
+        if (int code = reserve_shared_once<latent_attention_kernel>("skv_attention_general", most)) return code;
         if (int code = launch_pdl("skv_attention_general(latent)", latent_attention_kernel,
                                   dim3((unsigned)(n_tokens * splits), (unsigned)((num_heads + LAT_HEADS - 1) / LAT_HEADS)), dim3(256), room, stream,
                                   (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, block_table, table_width, positions, token_seq,

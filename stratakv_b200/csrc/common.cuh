@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -91,6 +92,20 @@ inline int sm_count() {
         return value;
     }();
     return count;
+}
+
+// Dynamic shared memory beyond 48 KB, at most `bytes` in any launch: asked for once per kernel and device.
+template <auto KERNEL>
+inline int reserve_shared_once(const char* name, size_t bytes) {
+    static std::atomic<unsigned long long> done{0};
+    int device = 0;
+    cudaError_t status = cudaGetDevice(&device);
+    const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
+    if (status == cudaSuccess && (done.load(std::memory_order_relaxed) & bit)) return 0;
+    if (status == cudaSuccess) status = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (status != cudaSuccess) return fail(name, cudaGetErrorString(status));
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return 0;
 }
 
 // Activations of a gated feed-forward's gate, chosen by the part's spec (ops.ACTIVATIONS has the names).

@@ -327,15 +327,12 @@ template <bool WIDE, int MT>
 static int launch_few_of(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
     const dim3 grid((N + 15) / 16);
     constexpr int stages_of_part = 3 * MT * 128 * 4;
-    static const cudaError_t ready = [] {
-        const cudaError_t four = cudaFuncSetAttribute(linear_f32_few_kernel<MT, 4, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * stages_of_part);
-        const cudaError_t two = cudaFuncSetAttribute(linear_f32_few_kernel<MT, 2, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * stages_of_part);
-        return four != cudaSuccess ? four : two;
-    }();
-    if (ready != cudaSuccess) return fail("skv_linear(float)", cudaGetErrorString(ready));
     // four parts of K where every block has an SM to itself (16 warps, most of its registers), else two
-    if ((int)grid.x <= sm_count())
+    if ((int)grid.x <= sm_count()) {
+        if (int code = reserve_shared_once<linear_f32_few_kernel<MT, 4, WIDE>>("skv_linear(float)", 4 * stages_of_part)) return code;
         return launch_pdl("skv_linear(float)", linear_f32_few_kernel<MT, 4, WIDE>, grid, dim3(512), 4 * stages_of_part, stream, (const float*)a, (const float*)w, out, M, N, K, mode, act);
+    }
+    if (int code = reserve_shared_once<linear_f32_few_kernel<MT, 2, WIDE>>("skv_linear(float)", 2 * stages_of_part)) return code;
     return launch_pdl("skv_linear(float)", linear_f32_few_kernel<MT, 2, WIDE>, grid, dim3(256), 2 * stages_of_part, stream, (const float*)a, (const float*)w, out, M, N, K, mode, act);
 }
 
@@ -352,8 +349,7 @@ template <int BM, bool WIDE>
 static int launch_tile_of(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, cudaStream_t stream) {
     constexpr size_t buffers = (size_t)2 * FBK * (BM + FBN) * 4, tile = (size_t)BM * FBN * 4;
     const size_t smem = buffers > tile ? buffers : tile;
-    static const cudaError_t ready = cudaFuncSetAttribute(linear_f32_tile_kernel<BM, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (ready != cudaSuccess) return fail("skv_linear(float)", cudaGetErrorString(ready));
+    if (int code = reserve_shared_once<linear_f32_tile_kernel<BM, WIDE>>("skv_linear(float)", smem)) return code;
     const int tiles = ((N + FBN - 1) / FBN) * ((M + BM - 1) / BM);
     // K is shared by as many blocks as keep the fullest SM's share smallest: its blocks run one after the other as far as
     // the FMA pipe goes, each for its part of K and about 200 k more to start and to add up.  A lone block leaves a third

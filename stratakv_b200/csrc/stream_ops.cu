@@ -545,8 +545,7 @@ static int launch_token_side_mma(float* x, const int* ids, const void* table, in
     constexpr int R = 16 * MT;
     constexpr size_t smem = (size_t)((SIDE_WARPS + 1) * R * DIM + (SIDE_WARPS + 3) * R) * 4 + (size_t)3 * R * (DIM + 8) * 2;
     auto kernel = token_side_mma_kernel<DIM, COLS, MT>;
-    static const cudaError_t ready = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (ready != cudaSuccess) return fail("skv_token_side", cudaGetErrorString(ready));
+    if (int code = reserve_shared_once<token_side_mma_kernel<DIM, COLS, MT>>("skv_token_side", smem)) return code;
     const int ranks = (hidden + SIDE_WARPS * COLS - 1) / (SIDE_WARPS * COLS);
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(ranks * ((n_tokens + R - 1) / R)));

@@ -39,6 +39,12 @@ def test_one_handle_has_both_libraries_and_one_message(dtype):
     assert lib.skv_last_error().startswith(b"skv_rmsnorm:")
 
 
+def test_shared_memory_is_asked_for_on_every_device():
+    """A kernel's limit belongs to a device: a status kept once per process left a second GPU's launches refused."""
+    for path in build.CSRC.glob("*.cu"):
+        assert "static const cudaError_t" not in path.read_text(), path.name
+
+
 # (blocks, keys, parts): more blocks than SMs, short pieces and long ones; as many blocks as SMs
 @pytest.mark.parametrize("head_dim,pairs", [(64, False), (80, True), (128, True), (192, False)])
 def test_narrow_blocks_of_fused_decode_where_two_share_an_sm(head_dim, pairs):
