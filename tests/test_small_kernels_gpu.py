@@ -229,8 +229,10 @@ def test_recurrent_unit_forms(channels, part, lengths, starts):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("heads,dim", [(32, 64), (3, 128), (5, 16), (1, 32), (4, 48)])
-@pytest.mark.parametrize("n", [1, 9])
+@pytest.mark.parametrize("n", [1, 9, "many", "many and five"])      # (the wide form: two tokens an SM and more)
 def test_time_mix_finish(dtype, heads, dim, n):
+    many = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = {"many": many, "many and five": many + 5}.get(n, n)
     k, width = lib(dtype), heads * dim
     o, gate, norm = torch.randn(n, width, device="cuda"), torch.randn(n, width, device="cuda"), torch.rand(width, device="cuda") + 0.5
     out = torch.full((n, width + 8), float("nan"), device="cuda").to(dtype)
