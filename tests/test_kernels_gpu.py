@@ -263,7 +263,9 @@ def _folded(stats, norm, rows=None):
 
 
 @pytest.mark.parametrize("M,N,K,hidden_out", [(1, 176, 64, 72), (5, 104, 80, 40), (8, 2560, 2048, 2048),
-                                              (16, 96, 1024, 1000), (33, 48, 96, 104), (64, 256, 4096, 512)])
+                                              (16, 96, 1024, 1000), (33, 48, 96, 104), (64, 256, 4096, 512),
+                                              # blocks that walk several tiles, the last not whole, with one tile's factors
+                                              (8, 9250, 2048, 64), (1, 9250, 3072, 64)])
 def test_linear_with_folded_norm(M, N, K, hidden_out):
     """RMSNorm folded into the projections around it: the kernel that writes the stream (the embedding,
     a residual-add projection) leaves the row times the norm's weight and the row's factor, the
