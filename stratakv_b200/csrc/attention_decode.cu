@@ -31,15 +31,6 @@ constexpr int OTILES = DHD / 8;           // n8 tiles of the output
 constexpr int VWORDS = DHD / 16;          // 32-bit words a lane reads per key for P.V
 constexpr int DEC_WARPS = 8;
 
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // 2^x by the special-function unit; scores are kept in units of log2 (see attention_prefill.cu).
 __device__ __forceinline__ float dec_exp2(float x) {
     float y;
@@ -130,7 +121,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 #pragma unroll
             for (int step = 0; step < KSTEPS; ++step) {
                 const uint2 kb = live ? *(const uint2*)(key_row + 16 * step) : make_uint2(0u, 0u);
-                mma16816(s[t], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb.x, kb.y);
+                mma_bf16_16816(s[t], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb.x, kb.y);
             }
         }
         // scale, mask, online softmax
@@ -182,9 +173,9 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 #pragma unroll
         for (int w = 0; w < VWORDS; ++w) {
             // low halves are element 2w of the lane's range, high halves element 2w+1
-            mma16816(o[2 * w], a0, a1, a2, a3, __byte_perm(vw[0][w], vw[1][w], 0x5410),
+            mma_bf16_16816(o[2 * w], a0, a1, a2, a3, __byte_perm(vw[0][w], vw[1][w], 0x5410),
                      __byte_perm(vw[2][w], vw[3][w], 0x5410));
-            mma16816(o[2 * w + 1], a0, a1, a2, a3, __byte_perm(vw[0][w], vw[1][w], 0x7632),
+            mma_bf16_16816(o[2 * w + 1], a0, a1, a2, a3, __byte_perm(vw[0][w], vw[1][w], 0x7632),
                      __byte_perm(vw[2][w], vw[3][w], 0x7632));
         }
     }

@@ -63,15 +63,6 @@ static_assert(F_STAGES_AT + 2 * FWIDE * FWARP_BYTES <= F_SMEM_LIMIT, "shared mem
 // Whether two blocks of four warps share an SM's 228 KB (each takes 1 KB besides its own): head sizes up to 160.
 constexpr bool FNARROW_PAIRS = 2 * (F_STAGES_AT + 2 * FNARROW * FWARP_BYTES + 1024) <= 228 * 1024;
 
-__device__ __forceinline__ void f_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                      uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 __device__ __forceinline__ void f_ldmatrix(uint32_t (&r)[4], uint32_t address) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(address));
@@ -394,8 +385,8 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
             for (int step = 0; step < FKSTEPS; ++step) {
                 uint32_t kb[4];                       // keys 0-7: dims 0-7, 8-15 of the step; keys 8-15 likewise
                 f_ldmatrix(kb, k_rows + f_staged((lane & 7) + (lane >> 4) * 8, 2 * step + ((lane >> 3) & 1)));
-                f_mma(s[0], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
-                f_mma(s[1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
+                mma_bf16_16816(s[0], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
+                mma_bf16_16816(s[1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
             }
             float tile_max[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -443,8 +434,8 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
             for (int j = 0; j < FOTILES; j += 2) {
                 uint32_t vb[4];                       // dims 8j..: keys 0-7, 8-15; dims 8j+8..: keys 0-7, 8-15
                 f_ldmatrix_trans(vb, v_rows + f_staged((lane & 7) + ((lane >> 3) & 1) * 8, j + (lane >> 4)));
-                f_mma(o[j], a0, a1, a2, a3, vb[0], vb[1]);
-                f_mma(o[j + 1], a0, a1, a2, a3, vb[2], vb[3]);
+                mma_bf16_16816(o[j], a0, a1, a2, a3, vb[0], vb[1]);
+                mma_bf16_16816(o[j + 1], a0, a1, a2, a3, vb[2], vb[3]);
             }
         }
         __syncthreads();                              // the stage is free

@@ -21,15 +21,6 @@ constexpr int PF_BM = 64, PF_BN = 64, PF_WARPS = 4;
 constexpr int PF_PITCH = PHD + 8;                 // elements; 16 bytes of padding per row
 constexpr int PF_KSTEPS = PHD / 16, PF_DTILES = PHD / 8;
 
-__device__ __forceinline__ void pf_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                       uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -155,8 +146,8 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
                     const __nv_bfloat16* src = k_tile + (16 * n2 + (id >> 1) * 8 + r) * PF_PITCH + 16 * step + (id & 1) * 8;
                     uint32_t kb[4];
                     ldmatrix_x4(kb, smem_u32(src));
-                    pf_mma(s[2 * n2], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
-                    pf_mma(s[2 * n2 + 1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
+                    mma_bf16_16816(s[2 * n2], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
+                    mma_bf16_16816(s[2 * n2 + 1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
                 }
             }
             // scale and mask
@@ -212,8 +203,8 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
                     const __nv_bfloat16* src = v_tile + (16 * ks + (id & 1) * 8 + r) * PF_PITCH + 16 * d2 + (id >> 1) * 8;
                     uint32_t vb[4];
                     ldmatrix_x4_trans(vb, smem_u32(src));
-                    pf_mma(o[2 * d2], a0, a1, a2, a3, vb[0], vb[1]);
-                    pf_mma(o[2 * d2 + 1], a0, a1, a2, a3, vb[2], vb[3]);
+                    mma_bf16_16816(o[2 * d2], a0, a1, a2, a3, vb[0], vb[1]);
+                    mma_bf16_16816(o[2 * d2 + 1], a0, a1, a2, a3, vb[2], vb[3]);
                 }
             }
         }

@@ -161,10 +161,11 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 
 #if SKV_DTYPE == SKV_BF16
 // ---- mma.sync m16n8k16 -------------------------------------------------------
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // acc += a b for an operand of PARTS bfloat16 that add up to a float (PARTS 1: a bfloat16), the smallest part first.  The
@@ -175,7 +176,7 @@ template <int PARTS>
 __device__ __forceinline__ void mma_bf16_add(float (&acc)[4], const uint32_t (&a)[PARTS][4], uint32_t b0, uint32_t b1) {
     float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int s = PARTS - 1; s >= 0; --s) mma_bf16(sum, a[s], b0, b1);
+    for (int s = PARTS - 1; s >= 0; --s) mma_bf16_16816(sum, a[s][0], a[s][1], a[s][2], a[s][3], b0, b1);
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] += sum[i];
 }

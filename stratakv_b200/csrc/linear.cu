@@ -400,15 +400,6 @@ static int launch_linear(const void* a, const void* w, void* out, int M, int N, 
 
 #else  // bfloat16
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                               uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 template <bool STREAM>
 __device__ __forceinline__ uint4 load_weight16(const uint4* p) {
     return STREAM ? __ldcs(p) : __ldg(p);

@@ -19,15 +19,6 @@ constexpr int ROUTE_THREADS = 256;
 constexpr int ROUTE_MAX_EXPERTS = 1024;
 constexpr int ROUTE_MAX_TOP = 16;
 
-#if SKV_DTYPE == SKV_BF16
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                               uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-#endif
-
 // The dot product of a weight row and a float row in shared memory, a warp's share of it: VEC, sixteen bytes of the weight
 // at a time (rows of whole 16 bytes).
 template <bool VEC>

@@ -292,7 +292,7 @@ static int launch_token_side(float* x, const int* ids, const void* table, int ta
 //   projection: a warp makes its own columns, which stay in registers while the mean of squares goes round.
 // The stream and the gated values are float32 and stay so: each is split into three bfloat16 whose sum is the float to
 // its last bit (24 of 24), against weights that are bfloat16 anyway, so the products are exact and the sums float
-// (mma_bf16_add: what is added errs by 1.3e-7 to 1.5e-7 of itself, 1.8e-7 to 2.2e-7 in the block per token below; sums left in the
+// (mma_bf16_add: what is added errs by 1.3e-7 to 1.5e-7 of itself, 1.8e-7 to 2.2e-7 in the block per token above; sums left in the
 // tensor core erred by 3.1e-7 with many tokens, at 2 to 8 % less time).
 // Few tokens (MT 1): the smallest COLS whose cluster is at most 8 blocks, and the weights are asked into L2 ahead of the
 // wait.  Width 64 on 2,048 at 8 / 300 / 3,874 tokens: 20 / 79 / 187 us before, 10 / 35 / 71; on 4,096: 37 / 136 / 581, 14 / 36 / 147.
