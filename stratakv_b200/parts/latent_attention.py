@@ -44,8 +44,8 @@ def _extended(spec) -> bool:
 def decode_parts(pairs: int, max_ctx: int, sm_count: int, on_tensor_cores: bool) -> int:
     """Parts that a decode step of so many (token, head) pairs cuts each pair's keys into: enough to give every SM thirty-odd
     warps, of 64 keys at least; two at least where the kernel for parts runs on tensor cores (``Kernels.attention_latent``), which
-    is worth the merge."""
-    return max(2 if on_tensor_cores else 1, min(-(-sm_count * 32 // pairs), -(-max_ctx // 64), 64))
+    is worth the merge from about 32 keys on (8 sequences x 32 heads over 5 / 20 / 64 rows of 272: 12 us in two parts, 7 / 9 / 18 in one)."""
+    return max(2 if on_tensor_cores and max_ctx > 32 else 1, min(-(-sm_count * 32 // pairs), -(-max_ctx // 64), 64))
 
 
 class LatentAttention(Mixer):

@@ -11,6 +11,8 @@ def test_two_parts_only_where_they_run_on_tensor_cores():
     """A latent of 512 with a rotated part of 64 in a large batch went through memory in two parts for a kernel that does not serve it."""
     assert decode_parts(64 * 128, 1000, 148, False) == 1 and decode_parts(64 * 128, 1000, 148, True) == 2
     assert decode_parts(8 * 32, 40, 148, False) == 1
+    # short contexts: the kernel for parts and the merge take longer than the walk over a few keys
+    assert decode_parts(8 * 32, 32, 148, True) == 1 and decode_parts(8 * 32, 33, 148, True) == 2
     assert decode_parts(8 * 32, 780, 148, False) == decode_parts(8 * 32, 780, 148, True) == 13
     assert decode_parts(4, 100000, 148, True) == 64
 
