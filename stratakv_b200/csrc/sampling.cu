@@ -298,6 +298,14 @@ __device__ unsigned long long radix_select(const float* __restrict__ row, const 
 constexpr int FEW_K = 256;
 constexpr int FEW_LOADS = 8;           // 16-byte loads a thread keeps on its way in a walk (4: 44 us for those 64 rows out of HBM, 8: 28)
 
+// The rows it is taken for: a thread walks four neighbouring logits at a time, so that rows shorter than 4 x top_k leave fewer maxima
+// than k and all of the row on the list, and counting costs more than passes over a short row: top-k 20 / 100 / 256 alone 13.5 / 15.6 /
+// 22 us over 1,000 logits here (11.3 in passes), 13.7 / 15.6 / 20 over 2,000 (13.9), 14.5 / 16.6 / 22 over 5,000 (22).  With a top-p the
+// passes go on for the cut: top-k 20 / 200 14 / 19 us over 1,000 (21 and 23), but 256 35 (23).
+__host__ __device__ inline bool sample_few_serves(int vocab, int top_k, float top_p) {
+    return top_k > 0 && top_k <= FEW_K && vocab >= (top_p < 1.0f ? 4 * top_k : 2000 + 10 * top_k);
+}
+
 __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out, int vocab, float temperature, int top_k, float top_p,
                            unsigned long long seed, uint32_t stream, uint32_t counter, int* __restrict__ flag, unsigned char* smem) {
     float* maxima = (float*)smem;                                                          // [threads]
@@ -467,7 +475,7 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     pdl_wait();
     const float* row = logits + (size_t)blockIdx.x * vocab;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (top_k > 0 && top_k < vocab && top_k <= FEW_K &&
+    if (sample_few_serves(vocab, top_k, top_p) &&
         sample_few(row, out + blockIdx.x, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[blockIdx.x],
                    (uint32_t)counters[blockIdx.x], flag, sample_smem))
         return;
@@ -588,6 +596,9 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
 }
 
 }  // namespace skv
+
+// Whether such a call chooses from a short list.
+SKV_EXPORT int skv_sample_few_serves(int vocab, int top_k, float top_p) { return sample_few_serves(vocab, top_k, top_p); }
 
 SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, float temperature, int top_k,
                           float top_p, unsigned long long seed, const int* streams, const int* counters,

@@ -66,3 +66,15 @@ def test_experts_of_few_pairs_and_few_tokens(step, serves):
     if path is None:
         pytest.skip("not compiled yet")
     assert ctypes.CDLL(str(path)).skv_expert_few_serves(*step) == int(serves)
+
+
+# (vocabulary, top-k, top-p): short rows, where passes over the row are faster, and long ones
+@pytest.mark.parametrize("call,serves", [((1000, 20, 1.0), False), ((1000, 20, 0.9), True), ((1000, 200, 0.9), True), ((1000, 256, 0.95), False),
+                                         ((2000, 200, 1.0), False), ((2200, 20, 1.0), True), ((32000, 256, 1.0), True), ((128256, 257, 0.9), False),
+                                         ((128256, 0, 0.9), False), ((1, 1, 0.9), False), ((2, 2, 0.5), False)])
+def test_rows_that_are_sampled_from_a_short_list(call, serves):
+    path = build.find_built("bfloat16", 64)
+    if path is None:
+        pytest.skip("not compiled yet")
+    vocab, top_k, top_p = call
+    assert bool(ctypes.CDLL(str(path)).skv_sample_few_serves(vocab, top_k, ctypes.c_float(top_p))) == serves

@@ -104,7 +104,7 @@ def test_long_rows_and_ties_take_the_other_paths_of_the_kernel():
     assert set(draw(short, 3000, 1.0, 3, 1.0)) == {7, 31000, 31999}
 
 
-@pytest.mark.parametrize("vocab,top_k,top_p", [(2, 1, 1.0), (37, 36, 0.9), (513, 40, 1.0), (32000, 40, 0.95), (32001, 200, 0.9), (50257, 256, 0.5),
+@pytest.mark.parametrize("vocab,top_k,top_p", [(2, 1, 1.0), (37, 36, 0.9), (513, 40, 1.0), (160, 40, 0.9), (1000, 200, 0.9), (2401, 40, 1.0), (32000, 40, 0.95), (32001, 200, 0.9), (50257, 256, 0.5),
                                                (128256, 20, 0.95)])
 @pytest.mark.parametrize("ties", [False, True])
 def test_a_short_list_draws_what_the_whole_row_draws(vocab, top_k, top_p, ties):
