@@ -130,8 +130,18 @@ def _build_once(target: Path, compile_it) -> None:
         try:
             if not target.is_file():
                 compile_it()
+                drop_older(target)
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
+
+
+def drop_older(target: Path) -> None:
+    """Libraries of the same dtype and head size, of other sources, go from the folder: nothing loads them again, and some tens of
+    megabytes for every change of a source add up."""
+    stem = target.name.rsplit("_", 1)[0]
+    for other in target.parent.glob(f"{stem}_*.so"):
+        if other != target and other.name.rsplit("_", 1)[0] == stem:
+            other.unlink(missing_ok=True)
 
 
 def _compile(nvcc: str, what: str, sources, defines, link_flags, target: Path, verbose: bool) -> None:

@@ -39,6 +39,17 @@ def test_one_handle_has_both_libraries_and_one_message(dtype):
     assert lib.skv_last_error().startswith(b"skv_rmsnorm:")
 
 
+def test_a_new_library_replaces_those_of_older_sources(tmp_path):
+    names = ["libstratakv_bf16_0123456789ab.so", "libstratakv_bf16_ba9876543210.so", "libstratakv_bf16_hd64_0123456789ab.so",
+             "libstratakv_bf16_hd64_ba9876543210.so", "libstratakv_bf16_hd6_0123456789ab.so", "libstratakv_f32_0123456789ab.so"]
+    for name in names:
+        (tmp_path / name).write_text("")
+    build.drop_older(tmp_path / names[0])
+    assert {path.name for path in tmp_path.iterdir()} == set(names) - {names[1]}
+    build.drop_older(tmp_path / names[2])
+    assert {path.name for path in tmp_path.iterdir()} == set(names) - {names[1], names[3]}
+
+
 def test_shared_memory_is_asked_for_on_every_device():
     """A kernel's limit belongs to a device: a status kept once per process left a second GPU's launches refused."""
     for path in build.CSRC.glob("*.cu"):
