@@ -454,7 +454,9 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
     return true;
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// Two blocks an SM, where their rows fit its shared memory: left to itself the short list takes 93 registers a thread, and with one
+// block an SM 296 rows of 50,257 logits with top-p alone took 710 us in place of 439.
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab, float temperature, int top_k,
               float top_p, unsigned long long seed, const int* __restrict__ streams,
               const int* __restrict__ counters, int* __restrict__ flag, int staged) {
@@ -600,6 +602,15 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
 // Whether such a call chooses from a short list.
 SKV_EXPORT int skv_sample_few_serves(int vocab, int top_k, float top_p) { return sample_few_serves(vocab, top_k, top_p); }
 
+// Blocks of the sampling kernel that an SM holds, with as much dynamic shared memory as rows too long to be staged take.
+SKV_EXPORT int skv_sample_blocks_per_sm() {
+    const size_t histograms = (size_t)SAMPLE_WARPS * 256 * (sizeof(unsigned long long) + sizeof(unsigned int)) + (size_t)SAMPLE_CANDIDATES * sizeof(int);
+    int blocks = 0;
+    if (cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(histograms + 152 * 1024)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, sample_kernel, SAMPLE_THREADS, histograms) != cudaSuccess) return -1;
+    return blocks;
+}
+
 SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, float temperature, int top_k,
                           float top_p, unsigned long long seed, const int* streams, const int* counters,
                           int* flag, cudaStream_t stream) {
@@ -621,6 +632,9 @@ SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, fl
         if (status != cudaSuccess) return fail("skv_sample", cudaGetErrorString(status));
         configured = true;
     }
-    return launch_pdl("skv_sample", sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), histograms + (staged ? row_bytes : 0), stream, logits, out,
+    // Rows that fit the GPU's SMs one by one take more than half of an SM's memory each: blocks of this launch that start while the one
+    // in front still runs would share SMs and leave others idle (128 rows of 50,257, top-k 40 and top-p 45 us, 36 so).
+    const size_t smem = histograms + (staged ? row_bytes : 0), alone = 116 * 1024;
+    return launch_pdl("skv_sample", sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), rows <= sm_count() && smem < alone ? alone : smem, stream, logits, out,
                       vocab, temperature, top_k, top_p, (unsigned long long)seed, streams, counters, flag, staged);
 }

@@ -147,3 +147,8 @@ def test_a_short_list_flags_what_is_not_finite():
         zeros = torch.zeros(2, dtype=torch.int32, device="cuda")
         k.sample(logits, out, 0.5, 40, 0.9, 0, zeros, zeros, flag)      # (3e38 / 0.5 overflows)
         assert int(flag) == 2 and int(out[1]) == 0
+
+
+def test_two_blocks_of_the_kernel_share_an_sm():
+    """More rows than SMs: with one block an SM they take half as long again."""
+    assert kernels().lib.skv_sample_blocks_per_sm() >= 2
