@@ -316,7 +316,7 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
     int* listed = (int*)(drawn + FEW_K);                                                    // [threads]
     int* drawn_index = listed + SAMPLE_THREADS;                                             // [FEW_K]
     __shared__ float bound, extent[2];                      // extent: the largest logit, and the largest magnitude
-    __shared__ int count, bad_row, kept;
+    __shared__ int count, bad_row, kept, at_bound;
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0) { count = 0; bad_row = 0; extent[0] = -INFINITY; extent[1] = 0.0f; }
     const bool wide = ((uintptr_t)row & 15) == 0;
@@ -350,7 +350,7 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
         above += (o.x > most) + (o.y > most) + (o.z > most) + (o.w > most);
         not_below += (o.x >= most) + (o.y >= most) + (o.z >= most) + (o.w >= most);
     }
-    if (above < top_k && not_below >= top_k) bound = most;                                  // (all who write write the same)
+    if (above < top_k && not_below >= top_k) { bound = most; at_bound = not_below - above; }    // (all who write write the same)
     if (above == 0) extent[0] = most;
     __syncthreads();
     if (bad_row || !isfinite(extent[1] / temperature)) {
@@ -359,6 +359,8 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
     }
     const float max_value = extent[0] / temperature, x_bound = bound, v_bound = x_bound / temperature;
     if (fabsf(v_bound) < 1e-30f) return false;
+    // equal values at the bound in three threads of four: fewer than k logits stand out of a row of the mask's value, say
+    if (at_bound > SAMPLE_THREADS / 4 * 3 && x_bound > -INFINITY) return false;
     const float x_low = x_bound - fabsf(x_bound) * 9.5367431640625e-7f;                     // (2^-20: 16 roundings of a quotient)
     auto collect = [&](float x, int i) {
         if (x >= x_low && x / temperature >= v_bound) {
@@ -366,7 +368,7 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
             if (at < SAMPLE_THREADS) listed[at] = i;
         }
     };
-    for (int q0 = tid; q0 < quads; q0 += FEW_LOADS * SAMPLE_THREADS) {
+    for (int q0 = tid; q0 < quads && *(volatile int*)&count <= SAMPLE_THREADS; q0 += FEW_LOADS * SAMPLE_THREADS) {   // (no further once it overflows)
         float4 x[FEW_LOADS];
 #pragma unroll
         for (int u = 0; u < FEW_LOADS; ++u)

@@ -149,6 +149,28 @@ def test_a_short_list_flags_what_is_not_finite():
         assert int(flag) == 2 and int(out[1]) == 0
 
 
+@pytest.mark.parametrize("vocab", [5000, 32000, 128256])
+@pytest.mark.parametrize("allowed", [3, 39, 41, 700])
+def test_masked_rows_with_few_logits_left(vocab, allowed):
+    """Fewer than top-k logits that are not the mask's: the others are equal, and the list cannot hold them."""
+    rng = np.random.default_rng(vocab + allowed)
+    rows = 8
+    logits = np.full((rows, vocab), -1e30, dtype=np.float32)
+    sunk = np.full((rows, vocab), -1e4, dtype=np.float32)
+    for r in range(rows):
+        places = rng.choice(vocab, allowed, replace=False)
+        logits[r, places] = rng.standard_normal(allowed) * 2
+        best = places[np.argsort(-logits[r, places], kind="stable")[:40]]
+        sunk[r, best] = logits[r, best]
+    k, outs = kernels(), []
+    streams = torch.arange(rows, dtype=torch.int32, device="cuda")
+    for values, limit in ((logits, 40), (sunk, 0)):
+        out = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+        k.sample(torch.tensor(values, device="cuda"), out, 1.0, limit, 1.0, 9, streams, streams)
+        outs.append(out.cpu().numpy())
+    assert (outs[0] == outs[1]).all()
+
+
 def test_two_blocks_of_the_kernel_share_an_sm():
     """More rows than SMs: with one block an SM they take half as long again."""
     assert kernels().lib.skv_sample_blocks_per_sm() >= 2
