@@ -31,9 +31,10 @@ class TokenSide(Part):
         self.w_proj_t = self.rt.upload(tensors[s.proj_weight]).t().contiguous()     # [dim, hidden]
         self.gamma = self.rt.upload(tensors[s.norm_weight], torch.float32)
 
-    # The kernel can first add a sublayer's branch through the norm after it (``forward``'s ``branch``, ``post_norm``),
-    # but only the block per token does that, and measured slower than ``rmsnorm_add`` followed by that same kernel (16,320
-    # tokens of width 2,048: 931 us against 115 + 490 us), so the arrangement is told not to ask for it.
+    # The kernel can first add a sublayer's branch through the norm after it (``forward``'s ``branch``, ``post_norm``), but
+    # only in its block per token, which serves float32 and other widths: that takes three times as long as the tensor-core
+    # form (3,900 tokens of width 2,048 187 us against 71), and with the branch longer than ``rmsnorm_add`` and itself apart (16,320
+    # tokens: 931 us against 115 + 490), so the arrangement is told not to ask for it.
     adds_branch = False
 
     def forward(self, step, x, next_norm=None, next_out=None, branch=None, post_norm=None) -> None:
