@@ -94,12 +94,14 @@ inline int sm_count() {
     return count;
 }
 
-// Dynamic shared memory beyond 48 KB, at most `bytes` in any launch: asked for once per kernel and device.
+// Dynamic shared memory beyond 48 KB, at most `bytes` in any launch: asked for once per kernel and device (which device is current is
+// only asked where there are several).
 template <auto KERNEL>
 inline int reserve_shared_once(const char* name, size_t bytes) {
     static std::atomic<unsigned long long> done{0};
+    static const int devices = [] { int count = 0; return cudaGetDeviceCount(&count) == cudaSuccess ? count : 0; }();
     int device = 0;
-    cudaError_t status = cudaGetDevice(&device);
+    cudaError_t status = devices == 1 ? cudaSuccess : cudaGetDevice(&device);
     const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
     if (status == cudaSuccess && (done.load(std::memory_order_relaxed) & bit)) return 0;
     if (status == cudaSuccess) status = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
