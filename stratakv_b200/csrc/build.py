@@ -136,8 +136,11 @@ def _build_once(target: Path, compile_it) -> None:
 
 
 def drop_older(target: Path) -> None:
-    """Libraries of the same dtype and head size, of other sources, go from the folder: nothing loads them again, and some tens of
-    megabytes for every change of a source add up."""
+    """Libraries of the same dtype and head size, of other sources, go from the package's own folder: nothing loads them again, and
+    some tens of megabytes for every change of a source add up.  The folder for temporary files is shared by every copy of the
+    package, each of which may be of other sources, so there they stay."""
+    if target.parent != CSRC / "_build":
+        return
     stem = target.name.rsplit("_", 1)[0]
     for other in target.parent.glob(f"{stem}_*.so"):
         if other != target and other.name.rsplit("_", 1)[0] == stem:

@@ -39,15 +39,20 @@ def test_one_handle_has_both_libraries_and_one_message(dtype):
     assert lib.skv_last_error().startswith(b"skv_rmsnorm:")
 
 
-def test_a_new_library_replaces_those_of_older_sources(tmp_path):
+# in the package's own folder; the one for temporary files is shared with other copies of the package
+@pytest.mark.parametrize("own", [True, False])
+def test_a_new_library_replaces_those_of_older_sources(own, tmp_path, monkeypatch):
+    monkeypatch.setattr(build, "CSRC", tmp_path if own else tmp_path / "elsewhere")
+    folder = tmp_path / "_build"
+    folder.mkdir()
     names = ["libstratakv_bf16_0123456789ab.so", "libstratakv_bf16_ba9876543210.so", "libstratakv_bf16_hd64_0123456789ab.so",
              "libstratakv_bf16_hd64_ba9876543210.so", "libstratakv_bf16_hd6_0123456789ab.so", "libstratakv_f32_0123456789ab.so"]
     for name in names:
-        (tmp_path / name).write_text("")
-    build.drop_older(tmp_path / names[0])
-    assert {path.name for path in tmp_path.iterdir()} == set(names) - {names[1]}
-    build.drop_older(tmp_path / names[2])
-    assert {path.name for path in tmp_path.iterdir()} == set(names) - {names[1], names[3]}
+        (folder / name).write_text("")
+    build.drop_older(folder / names[0])
+    assert {path.name for path in folder.iterdir()} == set(names) - ({names[1]} if own else set())
+    build.drop_older(folder / names[2])
+    assert {path.name for path in folder.iterdir()} == set(names) - ({names[1], names[3]} if own else set())
 
 
 def test_shared_memory_is_asked_for_on_every_device():
