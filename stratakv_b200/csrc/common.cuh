@@ -196,6 +196,20 @@ __device__ __forceinline__ void split3(float u, float v, uint32_t (&parts)[3]) {
         v = v == top_v ? 0.0f : v - top_v;
     }
 }
+
+// ---- weights on their way in shared memory ------------------------------------
+// 16 bytes into a slot of this lane's own (zeros where not live), read back by the same lane: no barrier, only its wait for its copies.
+__device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint4 ring_read(uint32_t at) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void ring_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
 #endif
 
 // Two optional terms of an attention kernel, both off when their pointer is null.

@@ -15,8 +15,8 @@
 //
 // float build: true 32-bit FMA kernels (no tensor cores, no TF32), one that streams the weights for a few tokens and
 // a tiled one.
-// bfloat16 build: a weight-streaming kernel for any M that keeps 16 weight rows
-// per block and feeds tokens in groups of 8 through mma.sync m16n8k16 with float
+// bfloat16 build: weight-streaming kernels for few tokens that take 16 weight rows
+// at a time and feed tokens in groups of 8 through mma.sync m16n8k16 with float
 // accumulation.  Each lane loads 16 bytes (8 consecutive k) of a weight row and of
 // a token row and issues two MMAs on them; the k order inside an MMA is permuted
 // the same way for both operands, which leaves the dot products unchanged.
@@ -400,11 +400,6 @@ static int launch_linear(const void* a, const void* w, void* out, int M, int N, 
 
 #else  // bfloat16
 // ---------------------------------------------------------------------------
-template <bool STREAM>
-__device__ __forceinline__ uint4 load_weight16(const uint4* p) {
-    return STREAM ? __ldcs(p) : __ldg(p);
-}
-
 // RMSNorm folded into the projections around it.  The kernel that updates the float residual stream
 // (residual-add mode) also leaves, per token, the updated row times the NEXT norm's weight in bfloat16
 // and the factor 1 / sqrt(mean(row^2) + eps); the projection after that norm takes those activations
@@ -477,6 +472,26 @@ __device__ __forceinline__ void skinny_norm_factors(float* factor, const float* 
     }
 }
 
+// The block that gets here last adds the partial sums of squares up and leaves the rows' factors.
+__device__ __forceinline__ void skinny_finish_partials(const NormArgs& norm, int M, int N, int partials, int warps, int warp, int lane) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(norm.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        for (int m = warp; m < M; m += warps) {
+            const float* partial = norm.partials + (size_t)m * norm.partial_stride;
+            float total = 0.0f;
+            for (int p = lane; p < partials; p += 32) total += __ldcg(partial + p);
+            total = warp_sum(total);
+            if (lane == 0) norm.row_scale_out[m] = 1.0f / sqrtf(total / (float)N + norm.eps_next);
+        }
+        if (threadIdx.x == 0) *norm.counter = 0u;
+    }
+}
+
 // Last, the warps' partial tiles are added up and the result stored, rows n0 .. n0 + 15 of the weight.
 template <int TG>
 __device__ __forceinline__ void skinny_store(float* red, const float* factor, const float (&acc)[TG][4], void* __restrict__ out, int M,
@@ -528,24 +543,7 @@ __device__ __forceinline__ void skinny_store(float* red, const float* factor, co
             for (int offset = 8; offset > 0; offset >>= 1) square += __shfl_xor_sync(0xffffffffu, square, offset);
             if (r == 0 && m0 + m < M) norm.partials[(size_t)(m0 + m) * norm.partial_stride + blockIdx.x] = square;
         }
-        if (!norm.counter) return;                  // the consumer adds the partial sums up
-        // the last block to get here adds them up (the grid has one chunk of tokens: M <= 8*TG)
-        __shared__ bool last;
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) last = atomicAdd(norm.counter, 1u) == gridDim.x - 1;
-        __syncthreads();
-        if (last) {
-            __threadfence();
-            for (int m = warp; m < M; m += warps) {
-                const float* partial = norm.partials + (size_t)m * norm.partial_stride;
-                float total = 0.0f;
-                for (int p = lane; p < (int)gridDim.x; p += 32) total += __ldcg(partial + p);
-                total = warp_sum(total);
-                if (lane == 0) norm.row_scale_out[m] = 1.0f / sqrtf(total / (float)N + norm.eps_next);
-            }
-            if (threadIdx.x == 0) *norm.counter = 0u;
-        }
+        if (norm.counter) skinny_finish_partials(norm, M, N, gridDim.x, warps, warp, lane);      // (one chunk of tokens: M <= 8*TG)
     } else {
         for (int idx = threadIdx.x; idx < 16 * COLS; idx += blockDim.x) {
             const int r = idx & 15, m = idx >> 4;
@@ -554,13 +552,13 @@ __device__ __forceinline__ void skinny_store(float* red, const float* factor, co
     }
 }
 
-// One block owns 16 rows of W and one chunk of 8*TG tokens.  Its warps take the
+// 17 to 64 tokens with a folded norm: one block owns 16 rows of W and every token (at most 8 TG).  Its warps take the
 // 32-wide k steps round robin, then their partial tiles are summed in shared
 // memory in warp order (a fixed order: results do not depend on timing).
 // Weights do not depend on the kernel before this one, so the first batch of
 // weight loads is issued before pdl_wait(): it overlaps the predecessor's tail.
-template <int TG, int U, bool STREAM, int MAX_WARPS>
-__global__ void __launch_bounds__(MAX_WARPS * 32, MAX_WARPS == 4 ? (TG == 1 ? 5 : (TG == 2 ? 5 : 2)) : (MAX_WARPS == 8 && TG <= 2 ? 2 : 1))
+template <int TG, int U>
+__global__ void __launch_bounds__(256)
 skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
                           void* __restrict__ out, int M, int N, int K, int mode, act_t act, const NormArgs norm) {
     extern __shared__ float red[];                 // [warps][16][8*TG + 1], [8*TG] factors, [8*TG][n_partials_in] partial sums
@@ -569,7 +567,7 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tig = lane & 3;
-    const int n0 = blockIdx.x * 16, m0 = blockIdx.y * COLS;
+    const int n0 = blockIdx.x * 16, m0 = 0;
     const int steps = (K + 31) >> 5;
 
     const int row_a = min(n0 + g, N - 1), row_b = min(n0 + g + 8, N - 1);
@@ -584,8 +582,8 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
         for (int u = 0; u < U; ++u) {
             const int k = (s0 + u * warps) << 5;
             const bool live = (s0 + u * warps) < steps && (k + tig * 8) < K;
-            wa[u] = (live && has_a) ? load_weight16<STREAM>((const uint4*)(wa_ptr + k)) : zero;
-            wb[u] = (live && has_b) ? load_weight16<STREAM>((const uint4*)(wb_ptr + k)) : zero;
+            wa[u] = (live && has_a) ? __ldcs((const uint4*)(wa_ptr + k)) : zero;
+            wb[u] = (live && has_b) ? __ldcs((const uint4*)(wb_ptr + k)) : zero;
         }
     };
     load_weights(warp);
@@ -625,128 +623,231 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
     skinny_store<TG>(red, factor, acc, out, M, N, n0, m0, mode, act, norm, warps, warp, lane);
 }
 
-// The same for at most 8 tokens where the tiles outnumber what two blocks of 8 warps an SM hold and the inner size gives a warp
-// at most twelve steps: that many blocks walk the tiles, and a warp keeps eight steps of weights on their way in two halves.
-// As soon as one half is multiplied the next is asked for, into the block's next tile too, so that the tokens' loads, the sums
-// and the stores do not leave the memory idle, which blocks that come and go did for a third of their life.  8 tokens, 9,248
-// / 12,288 / 32,000 x 3,072: 13.1 / 17.8 / 40.8 us a block a tile, 11.0 / 15.2 / 34.8 so; 8,192 / 32,000 x 2,048 8.8 / 27.5 and
-// 7.1 / 23.6.  Longer inner sizes gain nothing (28,672 x 4,096 44.2 and 44.7), and fewer tiles lose by the smaller bursts (1 token, 3,072 x 12,288
-// 16.6 and 18.1).
-constexpr int WALK_WARPS = 8, WALK_HALF = 4;
+// At most 16 tokens: the weights stream by once, and on their way they wait in shared memory.  Such a projection is bound by HBM
+// and, in a decode step's chain of dependent kernels, by how much of its weights is on the SMs before the kernel in front has
+// finished and how little must happen after that.  So:
+//  * A lane copies (cp.async) the very 16 bytes that it will multiply into slots of its own, DEPTH steps of its warp ahead: no
+//    registers for what is on its way, no barrier, and a wait for its own copies only.  The first DEPTH steps are asked for ahead
+//    of the wait for the kernel in front, and asking goes on into the block's next tile, through its sums and stores.  128 KB on
+//    its way an SM are needed: 64 KB a block and two blocks, or 96 to 144 KB in one.
+//  * 16 warps share a tile of 16 rows, which leaves a warp 4 or 8 steps of the common inner sizes: their activations are read
+//    once, all at the same time, and stay in registers for all of a block's tiles (XSTEPS).  Longer inner sizes bring theirs
+//    through the slots beside the weights.
+//  * A tile ends with one barrier; 128 threads per 8 tokens add the warps' sums up in warp order, and its gated pairs, squares and
+//    stores need no other.  What they add to was asked for a tile ahead.
+// Decode steps before (blocks of 4 to 16 warps that held the weights on their way in registers and came and went with the
+// tiles, or walked them) and now, in us: Llama 2,048 x 22, 1 / 8 tokens 713 / 815 and 543 / 626; 4 layers of 4,096 with 14,336 at 1 / 16
+// tokens 567 / 832 and 469 / 533; of 4,096 with 11,008 at 8 537 and 392; Zepavik 3,072 x 4 at 1 / 8 / 16 278 / 381 / 525 and 249 / 315 / 367.
+// The same walk with the weights on their way in registers (two blocks of 8 warps, or 16 warps): 563 / 693 for the first pair.
+constexpr int RING_WARPS = 16;
 
-__global__ void __launch_bounds__(WALK_WARPS * 32, 2)
-skinny_walk_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
+template <int TG, int XSTEPS, int DEPTH>
+constexpr int ring_smem() { return RING_WARPS * DEPTH * (1024 + (XSTEPS ? 0 : 512 * TG)) + 2 * RING_WARPS * 16 * (8 * TG + 1) * 4; }
+
+template <int TG, int XSTEPS, int DEPTH>
+__global__ void __launch_bounds__(RING_WARPS * 32, 2 * (ring_smem<TG, XSTEPS, DEPTH>() + 1024) <= 228 * 1024 ? 2 : 1)
+skinny_ring_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
                         void* __restrict__ out, int M, int N, int K, int mode, act_t act, const NormArgs norm) {
-    extern __shared__ float red[];                 // as above
-    constexpr int COLS = 8, PITCH = COLS + 1;
+    constexpr int PITCH = 8 * TG + 1, SLOT = 1024 + (XSTEPS ? 0 : 512 * TG);
+    extern __shared__ __align__(128) unsigned char ring_raw[];
+    float (*red)[RING_WARPS][16 * PITCH] = (float (*)[RING_WARPS][16 * PITCH])(ring_raw + RING_WARPS * DEPTH * SLOT);
+    __shared__ float factor[8 * TG];
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tig = lane & 3;
-    const int steps = (K + 31) >> 5, tiles = (N + 15) >> 4;
-    const int halves = ((steps + WALK_WARPS - 1) / WALK_WARPS + WALK_HALF - 1) / WALK_HALF;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const int tiles = (N + 15) >> 4, per_tile = (((K + 31) >> 5) + RING_WARPS - 1) / RING_WARPS;
+    const int k0 = warp * 32 + tig * 8;            // this lane's first k of a tile; a step further is RING_WARPS * 32 more
+    const uint32_t mine_at = smem_u32(ring_raw) + warp * DEPTH * SLOT + lane * 16;
 
-    uint4 wa[2][WALK_HALF], wb[2][WALK_HALF];
-    int asked_tile = blockIdx.x, asked = 0;        // the next half to ask for
-    auto load_weights = [&](uint4 (&a)[WALK_HALF], uint4 (&b)[WALK_HALF]) {
+    int asked_tile = blockIdx.x, asked = 0, asked_slot = 0;      // the next step to ask for
+    auto ask_weights = [&]() {
         if (asked_tile >= tiles) return;
-        const int row_a = asked_tile * 16 + g, row_b = row_a + 8;
-        const __nv_bfloat16* a_ptr = W + (size_t)min(row_a, N - 1) * K + tig * 8;
-        const __nv_bfloat16* b_ptr = W + (size_t)min(row_b, N - 1) * K + tig * 8;
-#pragma unroll
-        for (int u = 0; u < WALK_HALF; ++u) {
-            const int step = warp + (asked * WALK_HALF + u) * WALK_WARPS, k = step << 5;
-            const bool live = step < steps && (k + tig * 8) < K;
-            a[u] = live && row_a < N ? load_weight16<true>((const uint4*)(a_ptr + k)) : zero;
-            b[u] = live && row_b < N ? load_weight16<true>((const uint4*)(b_ptr + k)) : zero;
-        }
-        if (++asked == halves) { asked = 0; asked_tile += gridDim.x; }
+        const int row = asked_tile * 16 + g, k = k0 + asked * (RING_WARPS * 32);
+        const __nv_bfloat16* from = W + (size_t)row * K + k;
+        const bool has_a = k < K && row < N, has_b = k < K && row + 8 < N;
+        ring_copy(mine_at + asked_slot * SLOT, has_a ? from : W, has_a);
+        ring_copy(mine_at + asked_slot * SLOT + 512, has_b ? from + (size_t)8 * K : W, has_b);
     };
-    load_weights(wa[0], wb[0]);
-    load_weights(wa[1], wb[1]);
+    auto advance = [&]() {
+        ring_commit();
+        if (++asked_slot == DEPTH) asked_slot = 0;
+        if (++asked == per_tile) { asked = 0; asked_tile += gridDim.x; }
+    };
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) { ask_weights(); advance(); }
+    // the thread's output of a tile: column 16 tile + r of token m (the first 128 TG threads)
+    const int r = threadIdx.x & 15, m = threadIdx.x >> 4;
+    const bool stores = m < min(M, 8 * TG);
+    const bool keeps = mode == MODE_ADD_F32 && norm.partials;
+    int tile = blockIdx.x;
+    float gamma = keeps && stores && tile * 16 + r < N ? norm.gamma_next[tile * 16 + r] : 0.0f;
     pdl_wait();                                    // activations (and the residual stream) are ready now
 
-    const bool has_x = g < M;
-    const int safe = min(g, M - 1);
-    const __nv_bfloat16* x_ptr = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K + tig * 8;
-    float* factor = red + (size_t)WALK_WARPS * 16 * PITCH;
-    float* staged = factor + COLS;
-    skinny_send_for_norm<COLS>(staged, norm, 0, M);
-    float acc[1][4] = {};
-    auto multiply = [&](const uint4 (&a)[WALK_HALF], const uint4 (&b)[WALK_HALF], int half) {
+    const __nv_bfloat16* x_ptr[TG];
 #pragma unroll
-        for (int u = 0; u < WALK_HALF; ++u) {
-            const int step = warp + (half * WALK_HALF + u) * WALK_WARPS, k = step << 5;
-            const uint4 xv = has_x && step < steps && (k + tig * 8) < K ? *(const uint4*)(x_ptr + k) : zero;
-            mma_bf16_16816(acc[0], a[u].x, b[u].x, a[u].y, b[u].y, xv.x, xv.y);
-            mma_bf16_16816(acc[0], a[u].z, b[u].z, a[u].w, b[u].w, xv.z, xv.w);
+    for (int t = 0; t < TG; ++t) {
+        const int safe = min(t * 8 + g, M - 1);
+        x_ptr[t] = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K;
+    }
+    uint4 xv[XSTEPS ? XSTEPS : 1][TG];
+    auto ask_x = [&](int step, int slot) {
+        const int k = k0 + step * (RING_WARPS * 32);
+#pragma unroll
+        for (int t = 0; t < TG; ++t) {
+            const bool live = t * 8 + g < M && k < K;
+            ring_copy(mine_at + slot * SLOT + 1024 + 512 * t, live ? x_ptr[t] + k : X, live);
         }
     };
-    int half = 0;
-    bool second = false;                           // which of the two halves in registers comes next
-    for (int tile = blockIdx.x; tile < tiles;) {
-        if (second) { multiply(wa[1], wb[1], half); load_weights(wa[1], wb[1]); }
-        else { multiply(wa[0], wb[0], half); load_weights(wa[0], wb[0]); }
-        second = !second;
-        if (++half < halves) continue;
-        if (tile == (int)blockIdx.x) skinny_norm_factors<COLS>(factor, staged, norm, K, WALK_WARPS, warp, lane);
-        else __syncthreads();                      // the tile before has been stored
-        skinny_store<1>(red, factor, acc, out, M, N, tile * 16, 0, mode, act, norm, WALK_WARPS, warp, lane);
-        acc[0][0] = acc[0][1] = acc[0][2] = acc[0][3] = 0.0f;
-        half = 0;
-        tile += gridDim.x;
+    if (XSTEPS) {
+#pragma unroll
+        for (int s = 0; s < XSTEPS; ++s)
+#pragma unroll
+            for (int t = 0; t < TG; ++t) {
+                const int k = k0 + s * (RING_WARPS * 32);
+                xv[s][t] = t * 8 + g < M && k < K ? *(const uint4*)(x_ptr[t] + k) : make_uint4(0u, 0u, 0u, 0u);
+            }
+    } else {
+#pragma unroll
+        for (int i = 0; i < DEPTH; ++i) ask_x(i % per_tile, i);
+        ring_commit();
     }
+    float old = 0.0f;
+    if (mode == MODE_ADD_F32 && stores && tile * 16 + r < N) old = ((const float*)out)[(size_t)m * N + tile * 16 + r];
+    if (norm.partials_in) {
+        if (warp < M) {                            // a token a warp, lanes in a fixed order
+            const float* row = norm.partials_in + (size_t)(norm.rows ? norm.rows[warp] : warp) * norm.stride_in;
+            float total = 0.0f;
+#pragma unroll 4
+            for (int p = lane; p < norm.n_partials_in; p += 32) total += row[p];
+            total = warp_sum(total);
+            if (lane == 0) factor[warp] = 1.0f / sqrtf(total / (float)K + norm.eps_in);
+        }
+    } else if (norm.row_scale && threadIdx.x < M) {
+        factor[threadIdx.x] = norm.row_scale[norm.rows ? norm.rows[threadIdx.x] : threadIdx.x];
+    }
+    if (!XSTEPS) ring_wait<0>();
+
+    float acc[TG][4] = {};
+    int slot = 0, parity = 0;
+    auto step = [&](const uint4 (&kept)[TG]) {
+        ring_wait<DEPTH - 1>();
+        const uint32_t at = mine_at + slot * SLOT;
+        const uint4 a = ring_read(at), b = ring_read(at + 512);
+#pragma unroll
+        for (int t = 0; t < TG; ++t) {
+            const uint4 x = XSTEPS ? kept[t] : ring_read(at + 1024 + 512 * t);
+            mma_bf16_16816(acc[t], a.x, b.x, a.y, b.y, x.x, x.y);
+            mma_bf16_16816(acc[t], a.z, b.z, a.w, b.w, x.z, x.w);
+        }
+        // (the slot has been read: what the products needed is in registers)
+        ask_weights();
+        if (!XSTEPS && asked_tile < tiles) ask_x(asked, asked_slot);
+        advance();
+        if (++slot == DEPTH) slot = 0;
+    };
+    while (tile < tiles) {
+        if (XSTEPS) {
+#pragma unroll
+            for (int s = 0; s < XSTEPS; ++s)
+                if (s < per_tile) step(xv[s]);
+        } else {
+#pragma unroll 1
+            for (int s = 0; s < per_tile; ++s) step(xv[0]);
+        }
+        float* mine = red[parity][warp];
+#pragma unroll
+        for (int t = 0; t < TG; ++t) {
+            mine[g * PITCH + t * 8 + 2 * tig] = acc[t][0];
+            mine[g * PITCH + t * 8 + 2 * tig + 1] = acc[t][1];
+            mine[(g + 8) * PITCH + t * 8 + 2 * tig] = acc[t][2];
+            mine[(g + 8) * PITCH + t * 8 + 2 * tig + 1] = acc[t][3];
+            acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
+        }
+        __syncthreads();                           // (two buffers: the next tile's sums are written while this one's are read)
+        const int n = tile * 16 + r;
+        tile += gridDim.x;
+        if (threadIdx.x < 128 * TG) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < RING_WARPS; ++w) sum += red[parity][w][r * PITCH + m];       // in warp order, whatever the timing
+            if (norm.partials_in || norm.row_scale) sum *= factor[m];
+            const bool live = stores && n < N;
+            if (mode == MODE_GATED) {
+                const float up = __shfl_down_sync(0xffffffffu, sum, 8);
+                if (live && r < 8)
+                    ((__nv_bfloat16*)out)[(size_t)m * (N >> 1) + ((n >> 4) << 3) + r] = __float2bfloat16_rn(gated_product(sum, up, act));
+            } else if (mode == MODE_ADD_F32) {
+                const size_t at = (size_t)m * N + n;
+                const float updated = live ? old + sum : 0.0f;
+                if (live) ((float*)out)[at] = updated;
+                if (keeps) {
+                    // the updated row times the next norm's weight; its sum of squares over this tile's columns
+                    if (live) norm.scaled_out[at] = __float2bfloat16_rn(updated * gamma);
+                    float square = updated * updated;
+#pragma unroll
+                    for (int offset = 8; offset > 0; offset >>= 1) square += __shfl_xor_sync(0xffffffffu, square, offset);
+                    if (r == 0 && stores) norm.partials[(size_t)m * norm.partial_stride + (n >> 4)] = square;
+                }
+                if (tile < tiles && stores && tile * 16 + r < N) {
+                    old = ((const float*)out)[(size_t)m * N + tile * 16 + r];
+                    if (keeps) gamma = norm.gamma_next[tile * 16 + r];
+                }
+            } else if (live) {
+                epilogue_store<__nv_bfloat16>(out, mode, M, N, m, n, sum, act);
+            }
+        }
+        parity ^= 1;
+    }
+    if (keeps && norm.counter) skinny_finish_partials(norm, M, N, tiles, RING_WARPS, warp, lane);
 }
 
-template <int TG, int U, int MAX_WARPS>
-static int launch_skinny_as(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act,
-                            int warps, const NormArgs& norm, cudaStream_t stream) {
-    const int row_tiles = (N + 15) / 16, chunks = (M + 8 * TG - 1) / (8 * TG);
-    const size_t smem = ((size_t)warps * 16 * (8 * TG + 1) + 8 * TG + (size_t)8 * TG * (norm.partials_in ? (norm.n_partials_in + 3) & ~3 : 0)) * sizeof(float);
-    if (smem > 48 * 1024) return fail("skv_linear(bfloat16)", "too many partial sums for the consumer to stage: let the producer finish them");
-    dim3 grid(row_tiles, chunks);
-    if (chunks == 1)
-        return launch_pdl("skv_linear(bfloat16)", skinny_linear_bf16_kernel<TG, U, true, MAX_WARPS>, grid,
-                          dim3(warps * 32), smem, stream, (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N,
-                          K, mode, act, norm);
-    return launch_pdl("skv_linear(bfloat16)", skinny_linear_bf16_kernel<TG, U, false, MAX_WARPS>, grid,
-                      dim3(warps * 32), smem, stream, (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K,
-                      mode, act, norm);
+template <int TG, int XSTEPS, int DEPTH>
+static int launch_ring_as(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, const NormArgs& norm,
+                          int per_sm, cudaStream_t stream) {
+    constexpr int smem = ring_smem<TG, XSTEPS, DEPTH>();
+    if (int code = reserve_shared_once<skinny_ring_bf16_kernel<TG, XSTEPS, DEPTH>>("skv_linear(bfloat16)", smem)) return code;
+    const int tiles = (N + 15) / 16, slots = per_sm * sm_count();
+    return launch_pdl("skv_linear(bfloat16)", skinny_ring_bf16_kernel<TG, XSTEPS, DEPTH>, dim3(tiles < slots ? tiles : slots),
+                      dim3(RING_WARPS * 32), smem, stream, (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K, mode, act, norm);
 }
 
-static int launch_walk(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, const NormArgs& norm,
+// Slots and blocks an SM by the inner size and the tiles, us a decode step (Llama 2,048 x 22 unless said otherwise).
+// At most 8 tokens: two blocks of four slots fit an SM and overlap each other's ends, and where a projection has one an SM the next
+// one's blocks are resident beside them (a single block of six or eight slots: 2,048 rows at 1 / 8 tokens 570 / 650 against 542 /
+// 636, 2,560 rows 589 / 650, gate and up 556 / 648).  Inner sizes of 2,049 to 4,096 over more tiles than those two blocks hold:
+// one block of eight, half the activations' reads (22,016 x 4,096 at 8 tokens, 4 layers and head 396 -> 380; 256 tiles are
+// faster in twos, 474 against 479 at 1 token).  Longer: six slots with their activations, 144 KB (2,048 x 5,632: 542, five 544, four
+// 548; two blocks of three 583).
+// 9 to 16 tokens take twice the registers for activations, so one block an SM (16 tokens, two blocks of four slots 910 against 750).
+template <int TG>
+static int launch_ring(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, const NormArgs& norm,
                        cudaStream_t stream) {
-    const size_t smem = ((size_t)WALK_WARPS * 16 * 9 + 8 + (size_t)8 * (norm.partials_in ? (norm.n_partials_in + 3) & ~3 : 0)) * sizeof(float);
-    if (smem > 48 * 1024) return fail("skv_linear(bfloat16)", "too many partial sums for the consumer to stage: let the producer finish them");
-    return launch_pdl("skv_linear(bfloat16)", skinny_walk_bf16_kernel, dim3(2 * sm_count()), dim3(WALK_WARPS * 32), smem, stream,
-                      (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K, mode, act, norm);
+    // (each block adds up all of its tokens' partial sums: wider rows are finished by their writer)
+    if (norm.partials_in && (4 * 16 * (8 * TG + 1) + 8 * TG + 8 * TG * ((norm.n_partials_in + 3) & ~3)) * sizeof(float) > 48 * 1024)
+        return fail("skv_linear(bfloat16)", "too many partial sums for the consumer: let the producer finish them");
+    const int steps = (K + 31) / 32;
+    if (TG == 1) {
+        if (steps <= 4 * RING_WARPS) return launch_ring_as<1, 4, 4>(a, w, out, M, N, K, mode, act, norm, 2, stream);
+        if (steps <= 8 * RING_WARPS) {
+            if ((N + 15) / 16 <= 2 * sm_count()) return launch_ring_as<1, 8, 4>(a, w, out, M, N, K, mode, act, norm, 2, stream);
+            return launch_ring_as<1, 8, 8>(a, w, out, M, N, K, mode, act, norm, 1, stream);
+        }
+        return launch_ring_as<1, 0, 6>(a, w, out, M, N, K, mode, act, norm, 1, stream);
+    }
+    if (steps <= 4 * RING_WARPS) return launch_ring_as<2, 4, 6>(a, w, out, M, N, K, mode, act, norm, 1, stream);
+    if (steps <= 8 * RING_WARPS) return launch_ring_as<2, 8, 8>(a, w, out, M, N, K, mode, act, norm, 1, stream);
+    return launch_ring_as<2, 0, 4>(a, w, out, M, N, K, mode, act, norm, 1, stream);
 }
 
-// Warps per block.  Four to five row tiles per SM: 4 warps, compiled to fit 5 blocks on an SM so that
-// e.g. 704 tiles run as one wave.  Fewer row tiles, or more than one such wave holds: 8 warps (two blocks fit on an
-// SM, so the next kernel's weight loads overlap this one's end; with many tiles, blocks of 8 warps that come and go
-// keep the memory pipe fuller than two waves of 4-warp blocks: 22,016 x 4,096 at 8 tokens 44.2 -> 35.9 us, 32,000 x
-// 2,048 31.6 -> 28.3 us), or 16 when the inner size is so long that 8 warps would need more than two rounds of loads
-// each and the tiles are no more than the SMs (a block of 16 warps has an SM to itself; 256 tiles of 8 warps run as
-// one wave, of 16 warps as two).  Never more warps than k steps.
-template <int TG, int U, int MAX_WARPS>
+template <int TG, int U>
 static int launch_skinny(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act,
                          const NormArgs& norm, cudaStream_t stream) {
-    const int row_tiles = (N + 15) / 16, chunks = (M + 8 * TG - 1) / (8 * TG);
-    const int steps = (K + 31) / 32;
-    const long long blocks = (long long)row_tiles * chunks;
-    const int sms = sm_count();
-    int warps = (blocks >= sms * 4 && blocks <= sms * 5) ? 4 : 8;
-    // (Blocks of 3 warps, of which 7 fit on an SM, were once used for a few more tiles than five blocks of 4 warps per SM
-    // hold, 768 at hidden size 4096; blocks of 8 warps measured faster there too: 12,288 x 4,096 at 8 tokens 27.9 -> 22.5 us.)
-    if (warps == 8 && MAX_WARPS >= 16 && steps > 8 * U * 2 && blocks <= sms) warps = 16;   // (16 warps: one block per SM)
-    if (warps > MAX_WARPS) warps = MAX_WARPS;
-    while (warps > 1 && warps > steps) warps >>= 1;
-    if (TG == 1 && warps == WALK_WARPS && row_tiles > 2 * sms && chunks == 1 && steps <= 12 * WALK_WARPS && !norm.partials)
-        return launch_walk(a, w, out, M, N, K, mode, act, norm, stream);
-    if (warps <= 4) return launch_skinny_as<TG, U, 4>(a, w, out, M, N, K, mode, act, warps, norm, stream);
-    if (warps <= 8 || MAX_WARPS < 16) return launch_skinny_as<TG, U, 8>(a, w, out, M, N, K, mode, act, warps, norm, stream);
-    return launch_skinny_as<TG, U, 16>(a, w, out, M, N, K, mode, act, warps, norm, stream);
+    int warps = 8;
+    while (warps > 1 && warps > (K + 31) / 32) warps >>= 1;          // never more warps than k steps
+    const size_t smem = ((size_t)warps * 16 * (8 * TG + 1) + 8 * TG + (size_t)8 * TG * (norm.partials_in ? (norm.n_partials_in + 3) & ~3 : 0)) * sizeof(float);
+    if (smem > 48 * 1024) return fail("skv_linear(bfloat16)", "too many partial sums for the consumer to stage: let the producer finish them");
+    return launch_pdl("skv_linear(bfloat16)", skinny_linear_bf16_kernel<TG, U>, dim3((N + 15) / 16), dim3(warps * 32), smem, stream,
+                      (const __nv_bfloat16*)w, (const __nv_bfloat16*)a, out, M, N, K, mode, act, norm);
 }
 
 // gemm_tcgen05.cu: the tensor-memory GEMM that serves steps with many tokens
@@ -767,12 +868,10 @@ static int launch_linear(const void* a, const void* w, void* out, int M, int N, 
     // each: relative to float64 21e-7 against 4.7e-7, and 21e-7 against 2.4e-7 with an inner size of 2,048)
     if (M > 16 && !norm.row_scale && !norm.partials_in && !norm.partials)
         return linear_tcgen05(a, w, out, M, N, K, mode, act, flag, stream);
-    // at most 8 warps and under 100 registers a thread: two blocks fit on an SM, so the next
-    // kernel's weight loads are in flight while this one finishes
-    if (M <= 8) return launch_skinny<1, 8, 16>(a, w, out, M, N, K, mode, act, norm, stream);
-    if (M <= 16) return launch_skinny<2, 8, 16>(a, w, out, M, N, K, mode, act, norm, stream);
-    if (M <= 32) return launch_skinny<4, 4, 8>(a, w, out, M, N, K, mode, act, norm, stream);
-    return launch_skinny<8, 4, 8>(a, w, out, M, N, K, mode, act, norm, stream);
+    if (M <= 8) return launch_ring<1>(a, w, out, M, N, K, mode, act, norm, stream);
+    if (M <= 16) return launch_ring<2>(a, w, out, M, N, K, mode, act, norm, stream);
+    if (M <= 32) return launch_skinny<4, 4>(a, w, out, M, N, K, mode, act, norm, stream);
+    return launch_skinny<8, 4>(a, w, out, M, N, K, mode, act, norm, stream);
 }
 #endif
 

@@ -62,7 +62,7 @@ class ResidualStats:
 
     @property
     def consumer_sums(self) -> bool:
-        # (the consumer stages rows x partial sums in shared memory beside its reduction area: 24 KB at most)
+        # (every block of the consumer adds up rows x partial sums: 24 KB at most)
         rows, width = self.partials.shape
         return rows <= CONSUMER_SUMS_ROWS and rows * width <= 6144
 

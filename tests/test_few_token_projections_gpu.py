@@ -1,5 +1,4 @@
-"""Projections of at most 16 tokens where blocks walk the weight's tiles (at most 8 tokens), and of 8 to 16 tokens over weights around
-48 MB, against float64."""
+"""Projections of at most 16 tokens, whose blocks walk the weight's tiles, against float64."""
 import math
 
 import pytest
@@ -20,6 +19,36 @@ def test_tiles_are_walked(M, N, K):
 @pytest.mark.parametrize("M,N,K", [(8, 6146, 4096), (9, 6144, 4096), (16, 6146, 4096), (16, 6142, 4096), (13, 3072, 12288), (12, 40000, 648)])
 def test_up_to_sixteen_tokens_over_large_weights(M, N, K):
     check(M, N, K)
+
+
+# tiles of 16 rows around one and two blocks an SM of 148 and beyond; inner sizes around what a warp's activations in registers and its
+# slots hold (4, 8 steps of 16 warps), and shorter than a warp's first step
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N", [16, 2368, 2384, 4736, 4768])
+@pytest.mark.parametrize("K", [24, 512, 2048, 2056, 4096, 4104, 5632])
+def test_blocks_walk_and_slots_wrap(M, N, K):
+    check(M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 6416, 512), (8, 12304, 4104)])
+def test_the_last_block_finishes_wide_rows(M, N, K):
+    """Rows too wide for every consumer to add their partial sums up: the writer's last block leaves the factors, and the counter at zero."""
+    from types import SimpleNamespace
+    from stratakv_b200 import ops
+    from stratakv_b200.residual import ResidualStats
+    k = ops.kernels_for(torch.bfloat16, 64, verbose=False)
+    stats = ResidualStats.allocate(lambda name, shape, dtype, zero=False: torch.zeros(shape, dtype=dtype, device="cuda"), M, N, torch.bfloat16)
+    norm = SimpleNamespace(gamma=1 + 0.2 * torch.randn(N, device="cuda"), spec=SimpleNamespace(eps=1e-5))
+    for _ in range(2):
+        a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
+        x, plain = torch.ones(M, N, device="cuda"), torch.ones(M, N, device="cuda")
+        stats.expect(norm)
+        k.linear(a, w, x, ops.MODE_ADD_F32, stats=stats)
+        k.linear(a, w, plain, ops.MODE_ADD_F32)
+        assert stats.n_partials == 0 and int(stats.counter) == 0 and torch.equal(x, plain)
+        assert torch.equal(stats.scaled, (x * norm.gamma).bfloat16())
+        want = torch.rsqrt((x.double() ** 2).mean(-1) + 1e-5)
+        assert ((stats.row_scale.double() - want).abs() <= 1e-5 * want).all()
 
 
 def check(M, N, K):
