@@ -816,7 +816,9 @@ static int launch_ring_as(const void* a, const void* w, void* out, int M, int N,
 // one's blocks are resident beside them (a single block of six or eight slots: 2,048 rows at 1 / 8 tokens 570 / 650 against 542 /
 // 636, 2,560 rows 589 / 650, gate and up 556 / 648).  Inner sizes of 2,049 to 4,096 over more tiles than those two blocks hold:
 // one block of eight, half the activations' reads (22,016 x 4,096 at 8 tokens, 4 layers and head 396 -> 380; 256 tiles are
-// faster in twos, 474 against 479 at 1 token).  Longer: six slots with their activations, 144 KB (2,048 x 5,632: 542, five 544, four
+// faster in twos, 474 against 479 at 1 token).  Where no norm is folded, kernels that stream through L1 stand between projections, and two
+// blocks' slots leave them little of it: up to a tile an SM one block of six (Fidolix at 4 tokens 416 -> 386, Kedelorn at 8 364 -> 349,
+// Vekanex at 1 213 -> 206).  Longer: six slots with their activations, 144 KB (2,048 x 5,632: 542, five 544, four
 // 548; two blocks of three 583).
 // 9 to 16 tokens take twice the registers for activations, so one block an SM (16 tokens, two blocks of four slots 910 against 750).
 template <int TG>
@@ -827,7 +829,11 @@ static int launch_ring(const void* a, const void* w, void* out, int M, int N, in
         return fail("skv_linear(bfloat16)", "too many partial sums for the consumer: let the producer finish them");
     const int steps = (K + 31) / 32;
     if (TG == 1) {
-        if (steps <= 4 * RING_WARPS) return launch_ring_as<1, 4, 4>(a, w, out, M, N, K, mode, act, norm, 2, stream);
+        if (steps <= 4 * RING_WARPS) {
+            const bool folded = norm.partials || norm.partials_in || norm.row_scale;
+            if (!folded && (N + 15) / 16 <= sm_count()) return launch_ring_as<1, 4, 6>(a, w, out, M, N, K, mode, act, norm, 1, stream);
+            return launch_ring_as<1, 4, 4>(a, w, out, M, N, K, mode, act, norm, 2, stream);
+        }
         if (steps <= 8 * RING_WARPS) {
             if ((N + 15) / 16 <= 2 * sm_count()) return launch_ring_as<1, 8, 4>(a, w, out, M, N, K, mode, act, norm, 2, stream);
             return launch_ring_as<1, 8, 8>(a, w, out, M, N, K, mode, act, norm, 1, stream);
