@@ -4,25 +4,30 @@
 // It does the arithmetic of attention_prefill.cu (src/layers/attention.cpp:261-338 in the
 // reference, which has no prefill kernel at all) with another division of labour.  A block takes
 // 128 queries of one head; keys and values come in tiles of 64 positions:
-//   warp 0   keys and scores: TMA loads of the Q tile (once) and of K tiles into a ring of four stages (a tile
+//   warp 0   keys and scores: TMA loads of the Q tile (once) and of K tiles into two stages (a tile
 //            is gathered from the cache blocks the sequence's block table names, whose entries the warp holds 32
-//            at a time in registers), and S = Q.K^T (128 x 64 x head_dim) into one of two score buffers in
-//            tensor memory, a tile ahead of the softmax;
-//   warp 1   values and output: TMA loads of V tiles into a ring of three stages, and O += P.V
+//            at a time in registers), and S = Q.K^T (128 x 64 x head_dim) into tensor memory, as soon as the softmax
+//            has taken the scores of the tile before;
+//   warp 1   values and output: TMA loads of V tiles into two stages, and O += P.V
 //            (128 x head_dim x 64) into the output accumulator, also in tensor memory; V is used as it lies
 //            in the cache (positions x head_dim), as an MN-major operand.
 //            Both warps walk their loops whole, and one elected lane issues.  A single issuing thread for
 //            both products measured as the limit of the kernel: its four waits and sixteen small tcgen05
 //            instructions a tile took 1,800 cycles, more than the softmax of the tile;
-//   warps 2-5  one thread per query row: read the scores with tcgen05.ld, mask, 2^x on the
-//            special-function unit (scores carry log2 e), row sums, probabilities as bfloat16 into
-//            one of two swizzled shared-memory tiles (the A operand of P.V).  The maximum the
+//   warps 4-7  one thread per query row: read the scores with tcgen05.ld, mask, 2^x on the
+//            special-function unit (scores carry log2 e; scale, offset and sums two numbers an instruction), row sums,
+//            probabilities as bfloat16 into tensor memory (the A operand of P.V).  The maximum the
 //            exponentials are taken against is raised only when a tile exceeds it by 2^8; only then
 //            is the accumulated output rescaled (tcgen05.ld / st), so most tiles never touch it.
 //            At the end the output is read once, divided by the row sum and stored.
-// The softmax is the long pole, so a block uses only half of the SM's tensor memory and shared
-// memory and (for head size 64) two blocks share an SM.  Every mbarrier
-// wait is bounded; on time-out bit 2 (value 4) of the flag word is raised and the block drains.
+// The softmax is the long pole (the special-function unit is busy 62 % of the cycles at 2,048 queries behind 6,144 tokens), so what
+// counts is that two blocks share an SM and hide each other's waits.  Products that take both operands from shared memory read the
+// 128 rows of A again for every 64 columns: with probabilities in shared memory too, and for head size 128 one block an SM, a
+// tile took 1,150 cycles of shared memory alone.  Probabilities in tensor memory, one buffer of them and of scores and two stages of keys and
+// values leave room for two blocks of either head size.  Before and now, us: 32 heads of 64 over 4 key heads, 2,048 tokens 43.4 and 40.1, behind 6,144
+// others 227 and 207, 8 x 870 tokens 87 and 79; of 128 over 8, 64 x 384 tokens 358 and 229, 2,048 74.5 and 44.6, behind 6,144 426 and 223
+// (1,070 TFLOP/s).  (A block that walks several query tiles measured slower, 8 x 870 tokens 107 against 87.)
+// Every mbarrier wait is bounded; on time-out bit 2 (value 4) of the flag word is raised and the block drains.
 #include "head_size.cuh"
 
 #if SKV_DTYPE == SKV_BF16 && (SKV_HEAD_DIM == 64 || SKV_HEAD_DIM == 128)
@@ -38,7 +43,7 @@ namespace skv {
 constexpr int AHD = SKV_HEAD_DIM;
 constexpr int ACH = AHD / 64;                       // 64-wide (128-byte) chunks of a head
 constexpr int ABM = 128, ABN = 64;                  // queries and keys per tile
-constexpr int ATHREADS = 192;
+constexpr int ATHREADS = 256;
 constexpr uint32_t AWAIT = 1u << 20;
 constexpr uint32_t TILE_BYTES = 128 * 128;          // one 128-row x 128-byte swizzled tile
 constexpr uint32_t KV_TILE_BYTES = ABN * 128;       // one 64-row tile of keys or values
@@ -90,6 +95,12 @@ __device__ __forceinline__ void a_mma(uint32_t d, uint64_t a, uint64_t b, uint32
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
         ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// The same with A in tensor memory: a lane a row, two bfloat16 a column
+__device__ __forceinline__ void a_mma_tmem(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
 __device__ __forceinline__ void a_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -110,10 +121,49 @@ __device__ __forceinline__ float a_exp2(float x) {
     return y;
 }
 
+// Two floats as one operand: one instruction multiplies and adds, or adds, both
+__device__ __forceinline__ uint64_t a_pair(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void a_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t a_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t a_add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 __device__ __forceinline__ float a_max3(float a, float b, float c) {
     float y;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
+}
+
+__device__ __forceinline__ void a_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void a_cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address, in the cluster's shared window, of what lies at `local` in block `rank` of the cluster
+__device__ __forceinline__ uint32_t a_remote(uint32_t local, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void a_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
 __device__ __forceinline__ void a_st32(uint32_t taddr, const uint32_t (&v)[32]) {
@@ -128,13 +178,18 @@ __device__ __forceinline__ void a_st32(uint32_t taddr, const uint32_t (&v)[32]) 
         : "memory");
 }
 
-// Keys come through a ring of four tiles and values through one of three, both asked for two tiles ahead (a stage of
-// keys is known to be free when the softmax has taken the scores of its tile, a stage of values when the product after
-// it has been seen complete); scores and probabilities have two buffers each.
-constexpr int K_STAGES = 4, V_STAGES = 3;
-// barriers: Q; K full and V full for each stage of the rings; S full/empty and P full/empty for each buffer
-enum { B_Q = 0, B_KF = 1, B_VF = B_KF + K_STAGES, B_SF = B_VF + V_STAGES, B_SE = B_SF + 2, B_PF = B_SE + 2, B_PE = B_PF + 2,
-       B_COUNT = B_PE + 2 };
+// Keys and values come through two stages each, the scores and the probabilities through one buffer.  A stage of keys is free when
+// the softmax has taken the scores of its tile, a stage of values (and the buffer of probabilities) when the product after it is complete.
+// barriers: Q; K full and V full for each stage; S full/empty, P full/empty
+enum { B_Q = 0, B_KF = 1, B_VF = 3, B_SF = 5, B_SE, B_PF, B_PE, B_COUNT };
+// Tensor memory, in columns: 64 of scores, AHD of output, 32 of probabilities (two bfloat16 a column); handed out in powers of two.
+constexpr uint32_t A_TMEM = 256;
+// Two blocks an SM (three of head size 64 fit with 80 registers a thread: 2,048 tokens 48.1 us against 40.1, behind 6,144 others 216 against 207).
+// Registers a thread: at launch (what two blocks leave each of their 8 warps), of the issuing warpgroup, of the softmax's.
+constexpr int A_BLOCKS = 2, A_REGS = 128, A_REGS_ISSUE = 88, A_REGS_SOFTMAX = 2 * A_REGS - A_REGS_ISSUE;
+// The blocks of a cluster may share a query tile's keys; what they tell each other lies where queries, keys and values were.
+constexpr int A_MAX_SPLITS = 4, A_INBOX_AT = A_MAX_SPLITS * ABM * 8;
+static_assert(A_INBOX_AT + ABM * (AHD + 4 * A_MAX_SPLITS) * 4 <= ACH * TILE_BYTES + 4 * ACH * KV_TILE_BYTES, "the merge takes the place of the queries, keys and values");
 
 // The running maximum a row's exponentials are taken against is only raised when a tile's maximum
 // exceeds it by more than this many powers of two; until then the accumulated output (in tensor
@@ -143,20 +198,18 @@ constexpr float RESCALE_MARGIN = 8.0f;
 
 // EXTRAS false: the instantiation without the bias table and the gate (nothing of them is compiled in).
 template <bool EXTRAS>
-__global__ void __launch_bounds__(ATHREADS, AHD <= 64 ? 2 : 1)
+__global__ void __launch_bounds__(ATHREADS, A_BLOCKS)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                             int table_width, const int* __restrict__ cu_q, const int* __restrict__ ctx_after,
                             __nv_bfloat16* __restrict__ out, int num_heads, int num_kv_heads, int block_size,
                             int rows_per_load, float scale, int window, int tiles_per_seq, int* __restrict__ flag,
                             const AttentionExtras extras) {
-    extern __shared__ uint8_t a_raw[];
-    uint8_t* base = (uint8_t*)(((uintptr_t)a_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* q_tile = base;                                        // ACH tiles of 128 rows
-    uint8_t* k_ring = q_tile + ACH * TILE_BYTES;                   // K_STAGES stages x ACH tiles of 64 rows
-    uint8_t* v_ring = k_ring + K_STAGES * ACH * KV_TILE_BYTES;     // V_STAGES stages x ACH tiles of 64 rows
-    uint8_t* p_ring = v_ring + V_STAGES * ACH * KV_TILE_BYTES;            // 2 tiles of 128 rows (64 keys = 128 bytes a row)
-    uint64_t* bars = (uint64_t*)(p_ring + 2 * TILE_BYTES);
+    extern __shared__ __align__(1024) uint8_t a_raw[];             // (swizzled tiles start at 1024 bytes)
+    uint8_t* q_tile = a_raw;                                       // ACH tiles of 128 rows
+    uint8_t* k_ring = q_tile + ACH * TILE_BYTES;                   // 2 stages x ACH tiles of 64 rows
+    uint8_t* v_ring = k_ring + 2 * ACH * KV_TILE_BYTES;            // the same
+    uint64_t* bars = (uint64_t*)(v_ring + 2 * ACH * KV_TILE_BYTES);
     uint32_t* tmem_slot = (uint32_t*)(bars + B_COUNT);
     const uint32_t bar0 = a_smem(bars);
     auto bar = [&](int which, int index = 0) { return bar0 + 8u * (uint32_t)(which + index); };
@@ -170,33 +223,40 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int head = blockIdx.x;
     const int kv_head = head / (num_heads / num_kv_heads);
     pdl_launch_dependents();
+    if (a_smem(a_raw) & 1023) {
+        if (threadIdx.x == 0 && flag) atomicOr(flag, 4);
+        return;
+    }
     const int q_begin = cu_q[seq], q_len = cu_q[seq + 1] - q_begin;
     if (tile * ABM >= q_len) return;                               // the whole block leaves together
     const int ctx = ctx_after[seq], ctx_before = ctx - q_len;
     const int last_query = min(q_len, tile * ABM + ABM) - 1;
     const int kv_end = ctx_before + last_query + 1;
     const int kv_lo = window > 0 ? max(0, ctx_before + tile * ABM - window + 1) : 0;
-    const int first_tile = kv_lo / ABN, n_tiles = (kv_end + ABN - 1) / ABN - first_tile;
+    // The blocks of a cluster share the keys of the query tile.
+    const int splits = gridDim.z, split = blockIdx.z;
+    const int all_first = kv_lo / ABN, all_tiles = (kv_end + ABN - 1) / ABN - all_first;
+    const int first_tile = all_first + all_tiles * split / splits, n_tiles = all_first + all_tiles * (split + 1) / splits - first_tile;
 
     if (threadIdx.x == 0) {
         a_init(bar(B_Q), 1);
-        for (int i = 0; i < K_STAGES; ++i) a_init(bar(B_KF, i), 1);
-        for (int i = 0; i < V_STAGES; ++i) a_init(bar(B_VF, i), 1);
-        for (int i = 0; i < 2; ++i) {
-            a_init(bar(B_SF, i), 1); a_init(bar(B_SE, i), 4); a_init(bar(B_PF, i), 4); a_init(bar(B_PE, i), 1);
-        }
+        for (int i = 0; i < 2; ++i) { a_init(bar(B_KF, i), 1); a_init(bar(B_VF, i), 1); }
+        a_init(bar(B_SF), 1); a_init(bar(B_SE), 4); a_init(bar(B_PF), 4); a_init(bar(B_PE), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2 && a_elect()) {
+        for (const CUtensorMap* map : {&map_q, &map_k, &map_v}) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(a_smem(tmem_slot)), "r"(256u) : "memory");
+                     ::"r"(a_smem(tmem_slot)), "r"(A_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_s = tmem, tmem_o = tmem + 128;             // S: 2 x 64 columns; O: AHD columns
+    const uint32_t tmem_s = tmem, tmem_o = tmem + 64, tmem_p = tmem_o + AHD;
     pdl_wait();                                                    // q and the cache rows come from the kernels before
 
     // Cache rows of a tile of 64 keys, for the copies of either warp below: the block table's entries come 32 at a time
@@ -214,7 +274,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         return (block * num_kv_heads + kv_head) * block_size + (key % block_size);
     };
     auto load_tile = [&](int which, int t) {                           // 0: keys, 1: values; tile t of this block
-        const int st = which ? t % V_STAGES : t % K_STAGES;
+        const int st = t & 1;
         const uint32_t full = bar(which ? B_VF : B_KF, st);
         uint8_t* dst = (which ? v_ring : k_ring) + (size_t)st * ACH * KV_TILE_BYTES;
         const int key0 = (first_tile + t) * ABN;
@@ -229,79 +289,77 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
         __syncwarp();
     };
-    if (warp == 0) {
-        // ---- keys and scores: the whole warp walks the loop, one elected lane issues -----------------------
-        // For tile i: wait until softmax i - 2 has taken its scores out of the buffer (which also says that the
-        // product of tile i - 2 is complete and its keys' stage free), and for the keys of tile i; issue
-        // S[i & 1] = Q . K_i^T; then ask for the keys of tile i + 2, into the stage of tile i - 2.
-        if (a_elect()) {
-            a_expect(bar(B_Q), ACH * TILE_BYTES);
-            for (int c = 0; c < ACH; ++c)
-                a_tma(a_smem(q_tile + c * TILE_BYTES), &map_q, head * AHD + 64 * c, q_begin + tile * ABM, bar(B_Q));
-        }
-        __syncwarp();
-        for (int t = 0; t < 2 && t < n_tiles; ++t) load_tile(0, t);
-        constexpr uint32_t idesc_s = a_idesc(ABM, ABN, 0);
-        bool ok = a_wait(bar(B_Q), 0, flag);
-        for (int i = 0; i < n_tiles && ok; ++i) {
-            const int s = i & 1, ks = i % K_STAGES;
-            if (i >= 2) ok = a_wait(bar(B_SE, s), ((i >> 1) - 1) & 1, flag);
-            if (ok) ok = a_wait(bar(B_KF, ks), (i / K_STAGES) & 1, flag);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(A_REGS_ISSUE));
+        if (warp == 0) {
+            // ---- keys and scores: the whole warp walks the loop, one elected lane issues -----------------------
+            // For tile i: wait until softmax i - 1 has taken its scores (which also says that its product is complete and its keys' stage
+            // free), and for the keys of tile i; issue S = Q . K_i^T; then ask for the keys of tile i + 1.
             if (a_elect()) {
-#pragma unroll
-                for (int c = 0; c < ACH; ++c) {
-                    const uint64_t qd = a_desc(a_smem(q_tile + c * TILE_BYTES));
-                    const uint64_t kd = a_desc(a_smem(k_ring + (size_t)(ks * ACH + c) * KV_TILE_BYTES));
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) a_mma(tmem_s + 64u * s, qd + 2 * k, kd + 2 * k, idesc_s, (c | k) ? 1u : 0u);
-                }
-                a_commit(bar(B_SF, s));
+                a_expect(bar(B_Q), ACH * TILE_BYTES);
+                for (int c = 0; c < ACH; ++c)
+                    a_tma(a_smem(q_tile + c * TILE_BYTES), &map_q, head * AHD + 64 * c, q_begin + tile * ABM, bar(B_Q));
             }
             __syncwarp();
-            if (i + 2 < n_tiles) load_tile(0, i + 2);
-        }
-        if (!ok) {
-            // a wait gave up: let the copies in flight land (microseconds) before the block may leave
-            for (int t = 0; t < 64; ++t) __nanosleep(1000);
-        }
-    } else if (warp == 1) {
-        // ---- values and output products: O += P_j . V_j once the probabilities and the values are in shared
-        // memory; then the values of tile j + 2 are asked for, into the stage of tile j - 1, whose product (issued
-        // a round ago) has to be complete.
-        constexpr uint32_t idesc_o = a_idesc(ABM, 64, 1);
-        for (int t = 0; t < 2 && t < n_tiles; ++t) load_tile(1, t);
-        bool ok = true;
-        for (int j = 0; j < n_tiles && ok; ++j) {
-            const int s = j & 1, vs = j % V_STAGES;
-            ok = a_wait(bar(B_VF, vs), (j / V_STAGES) & 1, flag) && a_wait(bar(B_PF, s), (j >> 1) & 1, flag);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (a_elect()) {
-#pragma unroll
-                for (int kk = 0; kk < ABN / 16; ++kk) {               // 16 keys per instruction
-                    const uint64_t pd = a_desc(a_smem(p_ring + s * TILE_BYTES)) + 2 * kk;
+            for (int t = 0; t < 2 && t < n_tiles; ++t) load_tile(0, t);
+            constexpr uint32_t idesc_s = a_idesc(ABM, ABN, 0);
+            bool ok = a_wait(bar(B_Q), 0, flag);
+            for (int i = 0; i < n_tiles && ok; ++i) {
+                const int ks = i & 1;
+                if (i >= 1) ok = a_wait(bar(B_SE), (i - 1) & 1, flag);
+                if (ok) ok = a_wait(bar(B_KF, ks), (i >> 1) & 1, flag);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (a_elect()) {
 #pragma unroll
                     for (int c = 0; c < ACH; ++c) {
-                        // V tile rows are keys: 16 keys further is 16 x 128 bytes = 128 descriptor units
-                        const uint64_t vd = a_desc(a_smem(v_ring + (size_t)(vs * ACH + c) * KV_TILE_BYTES)) + 128 * kk;
-                        a_mma(tmem_o + (uint32_t)(64 * c), pd, vd, idesc_o, (j | kk) ? 1u : 0u);
+                        const uint64_t qd = a_desc(a_smem(q_tile + c * TILE_BYTES));
+                        const uint64_t kd = a_desc(a_smem(k_ring + (size_t)(ks * ACH + c) * KV_TILE_BYTES));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) a_mma(tmem_s, qd + 2 * k, kd + 2 * k, idesc_s, (c | k) ? 1u : 0u);
                     }
+                    a_commit(bar(B_SF));
                 }
-                a_commit(bar(B_PE, s));                               // the output holds tiles 0..j; V_j and P_j are free
+                __syncwarp();
+                if (i >= 1 && i + 1 < n_tiles) load_tile(0, i + 1);
             }
-            __syncwarp();
-            if (j + 2 < n_tiles) {
-                if (j >= 1) ok = a_wait(bar(B_PE, (j - 1) & 1), ((j - 1) >> 1) & 1, flag);
+            if (!ok) {
+                // a wait gave up: let the copies in flight land (microseconds) before the block may leave
+                for (int t = 0; t < 64; ++t) __nanosleep(1000);
+            }
+        } else if (warp == 1) {
+            // ---- values and output products: O += P_j . V_j once the probabilities and the values are in shared memory; then
+            // the values of tile j + 1 are asked for, into the stage of tile j - 1: its product is complete, or the softmax could
+            // not have written the probabilities of tile j where those of j - 1 lay.
+            constexpr uint32_t idesc_o = a_idesc(ABM, 64, 1);
+            for (int t = 0; t < 2 && t < n_tiles; ++t) load_tile(1, t);
+            bool ok = true;
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                const int vs = j & 1;
+                ok = a_wait(bar(B_VF, vs), (j >> 1) & 1, flag) && a_wait(bar(B_PF), j & 1, flag);
                 if (!ok) break;
-                load_tile(1, j + 2);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (a_elect()) {
+#pragma unroll
+                    for (int kk = 0; kk < ABN / 16; ++kk) {               // 16 keys per instruction
+#pragma unroll
+                        for (int c = 0; c < ACH; ++c) {
+                            // V tile rows are keys: 16 keys further is 16 x 128 bytes = 128 descriptor units
+                            const uint64_t vd = a_desc(a_smem(v_ring + (size_t)(vs * ACH + c) * KV_TILE_BYTES)) + 128 * kk;
+                            a_mma_tmem(tmem_o + (uint32_t)(64 * c), tmem_p + (uint32_t)(8 * kk), vd, idesc_o, (j | kk) ? 1u : 0u);
+                        }
+                    }
+                    a_commit(bar(B_PE));                                  // the output holds tiles 0..j; V_j and P_j are free
+                }
+                __syncwarp();
+                if (j >= 1 && j + 1 < n_tiles) load_tile(1, j + 1);
+            }
+            if (!ok) {
+                for (int t = 0; t < 64; ++t) __nanosleep(1000);
             }
         }
-        if (!ok) {
-            for (int t = 0; t < 64; ++t) __nanosleep(1000);
-        }
-    } else if (warp >= 2) {
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(A_REGS_SOFTMAX));
         // ---- softmax and output: one thread per query row -----------------------------------------
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                          // row of the tile = TMEM lane
@@ -319,9 +377,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         float used_max = -INFINITY, row_sum = 0.0f;                   // in units of log2, after the scale
         bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
-            const int s = j & 1;
             const int key0 = (first_tile + j) * ABN;
-            ok = a_wait(bar(B_SF, s), (j >> 1) & 1, flag);
+            ok = a_wait(bar(B_SF), j & 1, flag);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // a row needs masks only in tiles that reach past its own position, past the sequence's end or
@@ -329,12 +386,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             const bool plain = key0 + ABN - 1 <= pos && key0 + ABN - 1 < ctx && (window == 0 || key0 > pos - window);
             auto visible = [&](int key) { return key <= pos && key < ctx && (window == 0 || key > pos - window); };
             uint32_t v0[32], v1[32];                                  // the row's 64 scores
-            a_ld32(tmem_s + lane_bits + (uint32_t)(64 * s), v0);
-            a_ld32(tmem_s + lane_bits + (uint32_t)(64 * s + 32), v1);
+            a_ld32(tmem_s + lane_bits, v0);
+            a_ld32(tmem_s + lane_bits + 32u, v1);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) a_arrive(bar(B_SE, s));                     // the scores are in registers
+            if (lane == 0) a_arrive(bar(B_SE));                     // the scores are in registers
             float sc[ABN];
             if (plain) {
 #pragma unroll
@@ -378,10 +435,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             const float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * unit;   // scale > 0
             // raise the maximum in use (and rescale what has been accumulated) only when it matters
             const bool raise = tile_max > used_max + RESCALE_MARGIN;
+            // once the product of the previous tile has finished the output accumulator may be touched and the probabilities
+            // rewritten
+            if (j > 0) ok = a_wait(bar(B_PE), (j - 1) & 1, flag);
+            if (!ok) break;
             if (j > 0 && __any_sync(0xffffffffu, raise)) {
-                // the output accumulator may be touched once the product of the previous tile has finished
-                ok = a_wait(bar(B_PE, (j - 1) & 1), ((j - 1) >> 1) & 1, flag);
-                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const float corr = raise ? a_exp2(used_max - tile_max) : 1.0f;     // 0 if nothing was seen before
 #pragma unroll 1
@@ -398,80 +456,147 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
             if (raise) used_max = tile_max;
             const float offset = used_max == -INFINITY ? 0.0f : used_max;      // nothing visible yet: every p is 0
-            // the probability buffer may be rewritten once the product two tiles back has read it
-            if (j >= 2) ok = a_wait(bar(B_PE, s), ((j >> 1) - 1) & 1, flag);
-            if (!ok) break;
-            uint8_t* p_tile = p_ring + s * TILE_BYTES;
-            float s4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const uint64_t unit2 = a_pair(unit, unit), offset2 = a_pair(-offset, -offset);
+            uint64_t sums[2] = {0ull, 0ull};                            // four running sums, two an addition
 #pragma unroll
-            for (int piece = 0; piece < ABN / 8; ++piece) {             // 8 keys = one 16-byte piece
-                float p[8];
+            for (int piece = 0; piece < ABN / 16; ++piece) {            // 16 keys = 8 columns
+                uint32_t packed[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     // (a masked score is -infinity, the offset is finite and the scale positive: 2^-infinity = 0)
-                    p[e] = a_exp2(fmaf(sc[8 * piece + e], unit, -offset));
-                    s4[e & 3] += p[e];
-                }
-                uint32_t packed[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const __nv_bfloat162 pair = __floats2bfloat162_rn(p[2 * e], p[2 * e + 1]);
+                    float lo, hi;
+                    a_split(a_fma2(a_pair(sc[16 * piece + 2 * e], sc[16 * piece + 2 * e + 1]), unit2, offset2), lo, hi);
+                    lo = a_exp2(lo);
+                    hi = a_exp2(hi);
+                    sums[e & 1] = a_add2(sums[e & 1], a_pair(lo, hi));
+                    const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, hi);
                     packed[e] = *(const uint32_t*)&pair;
                 }
-                *(uint4*)(p_tile + row * 128 + ((piece ^ (row & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                a_st8(tmem_p + lane_bits + (uint32_t)(8 * piece), packed);
             }
+            float s4[4];
+            a_split(sums[0], s4[0], s4[1]);
+            a_split(sums[1], s4[2], s4[3]);
             row_sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) a_arrive(bar(B_PF, s));                     // probabilities in place (and any rescale done)
+            if (lane == 0) a_arrive(bar(B_PF));                     // probabilities in place (and any rescale done)
         }
         // the last product has finished: read the output once, normalise, store
-        if (ok && n_tiles > 0) ok = a_wait(bar(B_PE, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, flag);
-        if (ok && n_tiles > 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // (a sink has no key and no value and is not scaled; the sums are in units of log2 below used_max)
-            const float sunk = EXTRAS && extras.sink ? a_exp2(fmaf(extras.sink[head], 1.4426950408889634f, -used_max)) : 0.0f;
-            const float inverse = (EXTRAS ? gate_factor(extras, q_begin + min(q_row, q_len - 1), head) : 1.0f) / (row_sum + sunk);
-            __nv_bfloat16* dst = out + ((size_t)(q_begin + min(q_row, q_len - 1)) * num_heads + head) * AHD;
-            const float* gate_row = EXTRAS && extras.gate && extras.gate_per_element
-                ? extras.gate + (size_t)(q_begin + min(q_row, q_len - 1)) * extras.gate_stride + (size_t)head * AHD : nullptr;
-#pragma unroll 1
-            for (int c = 0; c < AHD; c += 32) {
-                uint32_t v[32];
-                a_ld32(tmem_o + lane_bits + (uint32_t)c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (EXTRAS && gate_row) {                              // a gate for every number of the output
+        if (ok && n_tiles > 0) ok = a_wait(bar(B_PE), (n_tiles - 1) & 1, flag);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int token = q_begin + min(q_row, q_len - 1);
+        // (a sink has no key and no value and is not scaled; the sums are in units of log2 below used_max)
+        const float sink_log2 = EXTRAS && extras.sink ? extras.sink[head] * 1.4426950408889634f : 0.0f;
+        const float* gate_row = EXTRAS && extras.gate && extras.gate_per_element
+            ? extras.gate + (size_t)token * extras.gate_stride + (size_t)head * AHD : nullptr;
+        __nv_bfloat16* dst = out + ((size_t)token * num_heads + head) * AHD;
+        const float gate = EXTRAS ? gate_factor(extras, token, head) : 1.0f;
+        // eight numbers of the row from column d on, times `by`
+        auto store = [&](float (&v)[8], int d, float by) {
+            if (EXTRAS && gate_row) {                                  // a gate for every number of the output
 #pragma unroll
-                    for (int d = 0; d < 32; d += 4) {
-                        const float4 logit = *(const float4*)(gate_row + c + d);
-                        v[d] = __float_as_uint(__fdividef(__uint_as_float(v[d]), 1.0f + __expf(-logit.x)));
-                        v[d + 1] = __float_as_uint(__fdividef(__uint_as_float(v[d + 1]), 1.0f + __expf(-logit.y)));
-                        v[d + 2] = __float_as_uint(__fdividef(__uint_as_float(v[d + 2]), 1.0f + __expf(-logit.z)));
-                        v[d + 3] = __float_as_uint(__fdividef(__uint_as_float(v[d + 3]), 1.0f + __expf(-logit.w)));
-                    }
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 logit = *(const float4*)(gate_row + d + e);
+                    v[e] = __fdividef(v[e], 1.0f + __expf(-logit.x));
+                    v[e + 1] = __fdividef(v[e + 1], 1.0f + __expf(-logit.y));
+                    v[e + 2] = __fdividef(v[e + 2], 1.0f + __expf(-logit.z));
+                    v[e + 3] = __fdividef(v[e + 3], 1.0f + __expf(-logit.w));
                 }
-                if (q_row < q_len) {
+            }
+            uint32_t packed[4];
 #pragma unroll
-                    for (int d = 0; d < 32; d += 8) {
-                        uint32_t packed[4];
+            for (int e = 0; e < 4; ++e) {
+                const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * e] * by, v[2 * e + 1] * by);
+                packed[e] = *(const uint32_t*)&pair;
+            }
+            *(uint4*)(dst + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        };
+        if (splits == 1) {
+            if (ok && n_tiles > 0) {
+                const float sunk = EXTRAS && extras.sink ? a_exp2(sink_log2 - used_max) : 0.0f;
+                const float inverse = gate / (row_sum + sunk);
+#pragma unroll 1
+                for (int c = 0; c < AHD; c += 32) {
+                    uint32_t v[32];
+                    a_ld32(tmem_o + lane_bits + (uint32_t)c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (q_row < q_len) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const __nv_bfloat162 pair = __floats2bfloat162_rn(__uint_as_float(v[d + 2 * e]) * inverse,
-                                                                              __uint_as_float(v[d + 2 * e + 1]) * inverse);
-                            packed[e] = *(const uint32_t*)&pair;
+                        for (int d = 0; d < 32; d += 8) {
+                            float x[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[d + e]);
+                            store(x, c + d, inverse);
                         }
-                        *(uint4*)(dst + c + d) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                     }
                 }
             }
+        } else {
+            // Each block tells the others its rows' maxima and sums, then brings its output to the common maximum and pushes it, by
+            // columns, to the blocks that own them (AHD / splits columns each), which add up in rank order and store.  All of it
+            // lies where the queries, keys and values were: the first barrier is passed when every block's products are complete.
+            float2* rows = (float2*)a_raw;                                // [splits][128] (maximum, sum)
+            const uint32_t rows_at = a_smem(rows);
+            a_cluster_barrier();                                          // nobody's products read shared memory any more
+            for (int to = 0; to < splits; ++to) {
+                const uint32_t at = a_remote(rows_at + (uint32_t)(split * ABM + row) * 8u, (uint32_t)to);
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at), "f"(ok ? used_max : -INFINITY), "f"(ok ? row_sum : 0.0f) : "memory");
+            }
+            a_cluster_barrier();
+            float top = -INFINITY, total = 0.0f;
+            for (int from = 0; from < splits; ++from) top = fmaxf(top, rows[from * ABM + row].x);
+            for (int from = 0; from < splits; ++from) {
+                const float2 r = rows[from * ABM + row];
+                if (r.x != -INFINITY) total += a_exp2(r.x - top) * r.y;
+            }
+            const float weight = ok && used_max != -INFINITY ? a_exp2(used_max - top) : 0.0f;
+            const int columns = AHD / splits, pitch = columns + 4;        // (the pitch spreads a warp's rows over the banks)
+            float* inbox = (float*)(a_raw + A_INBOX_AT);                  // [splits][128][pitch]
+            const uint32_t inbox_at = a_smem(inbox);
+            for (int c = 0; c < AHD; c += 16) {
+                uint32_t v[16];
+                if (n_tiles > 0) {                                         // (with no keys the output was never written)
+                    a_ld16(tmem_o + lane_bits + (uint32_t)c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                }
+                const uint32_t at = a_remote(inbox_at + (uint32_t)((split * ABM + row) * pitch + c % columns) * 4u, (uint32_t)(c / columns));
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) {
+                    float x[4];
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) x[f] = weight > 0.0f ? __uint_as_float(v[e + f]) * weight : 0.0f;
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * e), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
+                }
+            }
+            a_cluster_barrier();
+            if (q_row < q_len) {
+                const float sunk = EXTRAS && extras.sink ? a_exp2(sink_log2 - top) : 0.0f;
+                const float inverse = gate / (total + sunk);
+                for (int d = 0; d < columns; d += 8) {
+                    float x[8] = {};
+                    for (int from = 0; from < splits; ++from) {
+                        const float* at = inbox + (from * ABM + row) * pitch + d;
+                        const float4 lo = *(const float4*)at, hi = *(const float4*)(at + 4);
+                        x[0] += lo.x; x[1] += lo.y; x[2] += lo.z; x[3] += lo.w;
+                        x[4] += hi.x; x[5] += hi.y; x[6] += hi.z; x[7] += hi.w;
+                    }
+                    store(x, split * columns + d, inverse);
+                }
+            }
         }
+    }
+    if (splits > 1 && warp < 4) {
+        a_cluster_barrier();
+        a_cluster_barrier();
+        a_cluster_barrier();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A_TMEM) : "memory");
     }
 }
 
@@ -555,20 +680,44 @@ SKV_EXPORT int skv_attention_prefill_tc_extras(const void* q, const void* k_cach
     const int tiles_per_seq = (max_q_len + ABM - 1) / ABM;
     const long long blocks = (long long)n_seqs * tiles_per_seq;
     if (blocks > 65535) return fail("skv_attention_prefill_tc", "too many query tiles in one step (65,535 at most)");
-    const size_t smem = (size_t)(ACH + 2) * TILE_BYTES + (size_t)(K_STAGES + V_STAGES) * ACH * KV_TILE_BYTES + B_COUNT * 8 + 16 + 1024;
+    const size_t smem = (size_t)ACH * TILE_BYTES + (size_t)4 * ACH * KV_TILE_BYTES + B_COUNT * 8 + 16;
     static bool configured = false;
     if (!configured) {
         for (auto kernel : {prefill_attention_tc_kernel<false>, prefill_attention_tc_kernel<true>}) {
             const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (status != cudaSuccess) return fail("skv_attention_prefill_tc", cudaGetErrorString(status));
+            cudaFuncAttributes attributes;
+            if (status != cudaSuccess || cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess)
+                return fail("skv_attention_prefill_tc", cudaGetErrorString(status));
+            // (the softmax's share is taken from what the block was launched with)
+            if (attributes.numRegs != A_REGS) return fail("skv_attention_prefill_tc", "built with another number of registers than the warpgroups share out");
         }
         configured = true;
     }
-    return launch_pdl("skv_attention_prefill_tc", bias || gate || sink || softcap > 0.0f ? prefill_attention_tc_kernel<true> : prefill_attention_tc_kernel<false>,
-                      dim3(num_heads, (unsigned)blocks),
-                      dim3(ATHREADS), smem, stream, map_q, map_k, map_v, block_table, table_width, cu_q, ctx_after,
-                      (__nv_bfloat16*)out, num_heads, num_kv_heads, block_size, rows_per_load, scale, window,
-                      tiles_per_seq, flag, extras);
+    // Fewer query tiles than SMs over long contexts: their keys are shared out, which starts every block for less work and ends in a
+    // merge (512 queries behind 4,096 others, 32 heads of 64, 128 blocks: 68.2 -> 44.0 us; 512 blocks 207 -> 212).
+    const long long most_keys = (long long)table_width * block_size, keys = window > 0 && window + ABM < most_keys ? window + ABM : most_keys;
+    const long long tiles = blocks * num_heads;
+    int splits = 1;
+    while (splits < A_MAX_SPLITS && tiles * 2 * splits <= A_BLOCKS * sm_count() && keys >= 1024 * splits) splits *= 2;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(num_heads, (unsigned)blocks, splits);
+    config.blockDim = dim3(ATHREADS);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = pdl_enabled();
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = splits;
+    config.attrs = attributes;
+    config.numAttrs = splits > 1 ? 2 : 1;
+    auto kernel = bias || gate || sink || softcap > 0.0f ? prefill_attention_tc_kernel<true> : prefill_attention_tc_kernel<false>;
+    const cudaError_t status = cudaLaunchKernelEx(&config, kernel, map_q, map_k, map_v, block_table, table_width, cu_q, ctx_after,
+                                                  (__nv_bfloat16*)out, num_heads, num_kv_heads, block_size, rows_per_load, scale, window,
+                                                  tiles_per_seq, flag, extras);
+    if (status != cudaSuccess) return fail("skv_attention_prefill_tc", cudaGetErrorString(status));
+    return 0;
 }
 
 SKV_EXPORT int skv_attention_prefill_tc(const void* q, const void* k_cache, const void* v_cache, int cache_blocks,
