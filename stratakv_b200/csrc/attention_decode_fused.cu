@@ -10,7 +10,10 @@
 // rounded to bfloat16 once, scores / softmax / output accumulate in float.
 //
 // The kernel is built around its latency chain, since a decode step gives it little else to
-// win: at batch 8 and 2,048 keys a block reads 64 KB.
+// win: at batch 8 and 2,048 keys a block reads 64 KB.  Over long contexts a warp's own chain counts as much: it copies its own 16 keys
+// and values of a chunk and waits for them alone (no block-wide barrier in the loop), looks the cache block up once a group (its rows lie one behind the
+// other), keeps two chains of score products and rescales its output only where a maximum was raised.  Before and now, us over caches beyond L2:
+// 8 sequences x 32 heads of 128 over 400 / 1,600 keys 16.5 / 47.7 and 12.6 / 34.0 (6.2 TB/s), 64 x 8 shared by 4 35.8 / 97.9 and 29.3 / 72.5.
 //  * Keys and values of earlier positions cannot change during the step, so a block starts
 //    streaming its piece of the context into shared memory (cp.async, two stages of 128 keys)
 //    as soon as it is resident, before it waits for the q|k|v projection in front of it.
@@ -47,7 +50,7 @@ __device__ __forceinline__ uint32_t f_staged(int row, int piece) {          // b
 constexpr int FPIECES = FHD / 8;                    // 16-byte pieces per row
 constexpr int FWARP_BYTES = 2 * 16 * FROW;            // what 16 keys and 16 values, one group per warp, take of a stage
 constexpr int FPITCH = FHD + 2;                     // floats per partial row: outputs, max, sum
-constexpr int FINBOX_ROWS = 24;                     // >= ceil(16 / blocks) * blocks for 1..8 blocks
+constexpr int FINBOX_ROWS = 24;                     // >= ceil(16 / blocks) * blocks for 1..8 and 16 blocks
 
 // shared memory, in bytes from the start
 constexpr int F_Q_AT = 0;                                           // [16][FQROW] rotated queries
@@ -197,23 +200,22 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
     };
     auto row_in_block = [&](int key) { return block_shift >= 0 ? key & (block_size - 1) : key % block_size; };
 
-    // Stage chunk c (groups my_first + 8c ...) of this block's keys and values.  Rows past the context are
-    // zero-filled: a masked key has weight 0, and 0 times whatever lay in shared memory need not be 0.
+    // Stage this warp's 16 keys and values of chunk c (groups my_first + FWARPS c ...): a warp waits for its own copies alone.  Rows past
+    // the context are zero-filled: a masked key has weight 0, and 0 times whatever lay in shared memory need not be 0.
+    // A group's rows lie in one cache block, one behind the other: one look-up, and every piece is at a constant distance.
     auto issue_chunk = [&](int c) {
-        if (c < n_chunks) {
-            const int key0 = (my_first + c * FWARPS) << 4;
-            const int key_end = min(ctx, my_end << 4);
-            const uint32_t stage = smem + F_STAGES_AT + (c % stages) * FSTAGE_BYTES;
-            for (int i = threadIdx.x; i < FCHUNK * FPIECES; i += FTHREADS) {
-                const int row = i / FPIECES, piece = i - row * FPIECES;
-                const int key = key0 + row;
-                const bool live = key < key_end;
-                size_t at = 0;
-                if (live)
-                    at = ((size_t)(block_of(key) * num_kv_heads + kv_head) * block_size + row_in_block(key)) * FHD + piece * 8;
+        const int group = my_first + c * FWARPS + warp;
+        if (group < my_end) {
+            const int key0 = group << 4, live = ctx - key0;
+            const size_t base = ((size_t)(block_of(key0) * num_kv_heads + kv_head) * block_size + row_in_block(key0)) * FHD;
+            const __nv_bfloat16 *k_from = k_cache + base + lane * 8, *v_from = v_cache + base + lane * 8;
+            const uint32_t stage = smem + F_STAGES_AT + (c % stages) * FSTAGE_BYTES + warp * 16 * FROW;
+#pragma unroll
+            for (int it = 0; it < FHD / 16; ++it) {
+                const int i = lane + 32 * it, row = i / FPIECES, piece = i - row * FPIECES;
                 const uint32_t dst = stage + f_staged(row, piece);
-                f_copy16(dst, k_cache + at, live ? 16 : 0);
-                f_copy16(dst + FCHUNK * FROW, v_cache + at, live ? 16 : 0);
+                f_copy16(dst, k_from + 256 * it, row < live ? 16 : 0);
+                f_copy16(dst + FCHUNK * FROW, v_from + 256 * it, row < live ? 16 : 0);
             }
         }
         f_commit();
@@ -344,50 +346,56 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
     for (int j = 0; j < FOTILES; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f; }
     float row_max[2] = {-INFINITY, -INFINITY}, row_sum[2] = {0.0f, 0.0f};
 
+    const float *bias_top = nullptr, *bias_bottom = nullptr;     // what the distance takes off the scores of rows g and g + 8
+    if (EXTRAS && extras.bias) {
+        bias_top = extras.bias + (size_t)(head0 + min(g, rows - 1)) * extras.bias_len;
+        bias_bottom = extras.bias + (size_t)(head0 + min(g + 8, rows - 1)) * extras.bias_len;
+    }
     for (int c = 0; c < n_chunks; ++c) {
-        float bias[2][4];                             // what the distance takes off each score: on its way while the chunk lands
+        float bias[2][4];                             // on its way while the chunk lands
         if (EXTRAS && extras.bias) {
-            const int j0 = (my_first + c * FWARPS + warp) << 4;
+            const int away = pos - ((my_first + c * FWARPS + warp) << 4) - 2 * tig;
 #pragma unroll
             for (int t = 0; t < 2; ++t)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int key = j0 + 8 * t + 2 * tig + (e & 1), row = g + 8 * (e >> 1);
-                    bias[t][e] = key < ctx && key >= lo && row < rows
-                        ? __ldg(extras.bias + (size_t)(head0 + row) * extras.bias_len + min(pos - key, extras.bias_len - 1)) : 0.0f;
+                for (int e = 0; e < 2; ++e) {
+                    const int at = min(max(away - 8 * t - e, 0), extras.bias_len - 1);
+                    bias[t][e] = g < rows ? __ldg(bias_top + at) : 0.0f;
+                    bias[t][e + 2] = rows > 8 ? __ldg(bias_bottom + at) : 0.0f;
                 }
         }
         // chunk c has landed (this thread's part) once all but the stages - 1 groups committed after it are complete
         if (stages == 2) f_wait_copies<1>();
         else if (stages == 3) f_wait_copies<2>();
         else f_wait_copies<3>();
-        __syncthreads();                              // ... and everybody's
+        __syncwarp();                                 // ... and the warp's
         const int group0 = my_first + c * FWARPS;
         const uint32_t stage = smem + F_STAGES_AT + (c % stages) * FSTAGE_BYTES;
-        if (owns_newest && newest_group >= group0 && newest_group < group0 + FWARPS) {
+        if (newest_group == group0 + warp && newest_group < my_end) {
             // the newest position's row, which the copy fetched as the cache had it before this step
             const int row = pos - (group0 << 4);
             unsigned char* base = fused_smem + F_STAGES_AT + (c % stages) * FSTAGE_BYTES;
-            for (int i = threadIdx.x; i < 2 * FPIECES; i += FTHREADS) {
+            for (int i = lane; i < 2 * FPIECES; i += 32) {
                 const int which = i / FPIECES, piece = i - which * FPIECES;
                 *(uint4*)(base + which * FCHUNK * FROW + f_staged(row, piece)) =
                     *(const uint4*)(fused_smem + F_NEW_AT + which * FQROW + piece * 16);
             }
-            __syncthreads();
+            __syncwarp();
         }
         const int group = group0 + warp;
         if (group < my_end) {
             const int j0 = group << 4;
             const uint32_t k_rows = stage + warp * 16 * FROW, v_rows = k_rows + FCHUNK * FROW;
-            float s[2][4];
-            s[0][0] = s[0][1] = s[0][2] = s[0][3] = s[1][0] = s[1][1] = s[1][2] = s[1][3] = 0.0f;
+            float s[2][4] = {}, odd[2][4] = {};           // (two chains of products each: every second step)
 #pragma unroll
             for (int step = 0; step < FKSTEPS; ++step) {
                 uint32_t kb[4];                       // keys 0-7: dims 0-7, 8-15 of the step; keys 8-15 likewise
                 f_ldmatrix(kb, k_rows + f_staged((lane & 7) + (lane >> 4) * 8, 2 * step + ((lane >> 3) & 1)));
-                mma_bf16_16816(s[0], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
-                mma_bf16_16816(s[1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
+                mma_bf16_16816(step & 1 ? odd[0] : s[0], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[0], kb[1]);
+                mma_bf16_16816(step & 1 ? odd[1] : s[1], qa[step][0], qa[step][1], qa[step][2], qa[step][3], kb[2], kb[3]);
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { s[0][e] += odd[0][e]; s[1][e] += odd[1][e]; }
             float tile_max[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
@@ -395,7 +403,7 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
                 for (int e = 0; e < 4; ++e) {
                     const int key = j0 + 8 * t + 2 * tig + (e & 1);
                     float v = (key < ctx && key >= lo) ? s[t][e] * scale_log2 : -INFINITY;
-                    if (EXTRAS && extras.bias) v -= bias[t][e];
+                    if (EXTRAS && extras.bias && v != -INFINITY) v -= bias[t][e];
                     // (capped: in units of log2; a masked score stays -infinity)
                     if (EXTRAS && extras.softcap > 0.0f && v != -INFINITY) v = cap_log2 * tanh_by_exp2(v * inverse_cap_log2);
                     s[t][e] = v;
@@ -424,9 +432,11 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
 #pragma unroll
             for (int r = 0; r < 2; ++r)
                 row_sum[r] = row_sum[r] * corr[r] + p[0][2 * r] + p[0][2 * r + 1] + p[1][2 * r] + p[1][2 * r + 1];
+            if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {       // (a maximum was raised)
 #pragma unroll
-            for (int j = 0; j < FOTILES; ++j) {
-                o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
+                for (int j = 0; j < FOTILES; ++j) {
+                    o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
+                }
             }
             const uint32_t a0 = f_pack(p[0][0], p[0][1]), a1 = f_pack(p[0][2], p[0][3]);
             const uint32_t a2 = f_pack(p[1][0], p[1][1]), a3 = f_pack(p[1][2], p[1][3]);
@@ -438,7 +448,7 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
                 mma_bf16_16816(o[j + 1], a0, a1, a2, a3, vb[2], vb[3]);
             }
         }
-        __syncthreads();                              // the stage is free
+        __syncwarp();                                 // the stage is free
         issue_chunk(c + stages);
     }
     f_wait_copies<0>();
@@ -559,6 +569,7 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
         return fail("skv_attention_decode_fused", "operands must be 16-byte aligned");
     const int group_size = num_heads / num_kv_heads;
     const int m_tiles = (group_size + 15) / 16;
+    const long long most_keys = (long long)table_width * block_size;
     int block_shift = -1;                             // log2 of block_size where it is a power of two
     for (int bit = 4; bit < 31; ++bit)
         if (block_size == (1 << bit)) block_shift = bit;
@@ -570,7 +581,8 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
             return fail("skv_attention_decode_fused", "cannot read the number of SMs");
         for (auto kernel : {decode_attention_fused_kernel<false, FWIDE>, decode_attention_fused_kernel<true, FWIDE>,
                             decode_attention_fused_kernel<false, FNARROW>, decode_attention_fused_kernel<true, FNARROW>}) {
-            const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM_LIMIT);
+            cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM_LIMIT);
+            if (status == cudaSuccess) status = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (status != cudaSuccess) return fail("skv_attention_decode_fused", cudaGetErrorString(status));
         }
         sm_count = count;
@@ -579,12 +591,11 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
     // piece of the longest context is at most four stages, fetches the whole piece ahead instead (measured: batch 8 at
     // 2,048 keys gains 3 % that way, while deeper staging of longer pieces loses 10 %).
     const long long blocks = (long long)n_seqs * num_kv_heads * m_tiles * splits;
-    const int warps = fused_warps(blocks, (long long)table_width * block_size, splits, sm_count), stage_bytes = warps * FWARP_BYTES;
+    const int warps = fused_warps(blocks, most_keys, splits, sm_count), stage_bytes = warps * FWARP_BYTES;
     const bool narrow = warps == FNARROW;
-    const long long piece_chunks = ((long long)table_width * block_size / splits + warps * 16 - 1) / (warps * 16);
+    const long long piece_chunks = (most_keys / splits + warps * 16 - 1) / (warps * 16);
     const int room = (F_SMEM_LIMIT - F_STAGES_AT) / stage_bytes;
-    // (a third stage for longer pieces, which two blocks of head size 64 could still share an SM with, measured
-    // 7-12 % slower in the step at 8,100 and 16,200 keys)
+    // (a third stage for longer pieces, which two blocks of head size 64 could still share an SM with, gains nothing)
     int stages = 2;
     if (blocks <= sm_count && piece_chunks <= FMAX_STAGES && piece_chunks <= room) stages = (int)(piece_chunks < 2 ? 2 : piece_chunks);
     const size_t smem = (size_t)F_STAGES_AT + (size_t)stages * stage_bytes;
@@ -606,6 +617,28 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
                             qk_norm || q_temp_every > 0 || softcap > 0.0f;
     auto kernel = narrow ? (any_extras ? decode_attention_fused_kernel<true, FNARROW> : decode_attention_fused_kernel<false, FNARROW>)
                          : (any_extras ? decode_attention_fused_kernel<true, FWIDE> : decode_attention_fused_kernel<false, FWIDE>);
+    // Eight pieces of a long context over few heads leave most of the GPU idle: sixteen, where as many clusters of sixteen run at once as
+    // there are (1 sequence of 8,100 tokens, 32 heads over 4: 14 -> 8 us, the step of 22 layers 699 -> 575).
+    const long long clusters = (long long)n_seqs * num_kv_heads * m_tiles;
+    if (splits == 8 && 16 * clusters <= sm_count && most_keys >= 4096 && (window <= 0 || window >= 4096)) {
+        cudaLaunchConfig_t wider = config;
+        cudaLaunchAttribute cluster = attributes[0];
+        cluster.val.clusterDim.z = 16;
+        wider.gridDim.z = 16;
+        wider.attrs = &cluster;
+        wider.numAttrs = 1;
+        const long long chunks = (most_keys / 16 + warps * 16 - 1) / (warps * 16);
+        wider.dynamicSmemBytes = (size_t)F_STAGES_AT + (size_t)(chunks <= FMAX_STAGES && chunks <= room ? (chunks < 2 ? 2 : chunks) : 2) * stage_bytes;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, kernel, &wider) == cudaSuccess && fit >= clusters) {
+            splits = 16;
+            stages = (int)((wider.dynamicSmemBytes - F_STAGES_AT) / stage_bytes);
+            config.gridDim.z = attributes[0].val.clusterDim.z = 16;
+            config.dynamicSmemBytes = wider.dynamicSmemBytes;
+        } else {
+            cudaGetLastError();                       // (a refusal is an answer, not an error of the caller's)
+        }
+    }
     const cudaError_t status = cudaLaunchKernelEx(
         &config, kernel, qkv, (const float2*)cos_sin, (__nv_bfloat16*)k_cache,
         (__nv_bfloat16*)v_cache, block_table, table_width, ctx_after, (__nv_bfloat16*)out, num_heads, num_kv_heads,

@@ -1,4 +1,5 @@
-"""Fused decode attention where blocks of a wide head outnumber the SMs (four warps a block, stages of 64 keys)."""
+"""Fused decode attention where blocks of a wide head outnumber the SMs (four warps a block, stages of 64 keys), and where few blocks share
+a long context (sixteen pieces)."""
 import math
 
 import pytest
@@ -26,6 +27,20 @@ def test_more_blocks_than_sms(heads, kv_heads, head_dim, block_size, lengths, wi
     k.attention_decode_fused(qkv, table, setup["k_cache"], setup["v_cache"], setup["table"],
                              torch.tensor(lengths, dtype=torch.int32, device="cuda"), out, heads, kv_heads, head_dim,
                              block_size, scale, window, splits, True)
+    close(out, attention_reference(setup, dtype, heads, kv_heads, scale, window).view(n, -1), dtype)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,block_size,lengths,window", [
+    (32, 4, 64, 64, [8100], 0), (32, 4, 64, 16, [4096], 0), (8, 2, 64, 64, [4100, 1, 300], 0),    # pieces without keys, a piece of one
+    (20, 1, 128, 64, [9000, 64], 4097), (1, 1, 80, 32, [5000], 0), (8, 1, 192, 64, [4500], 0)])   # a window, more than 16 heads a key head
+def test_a_long_context_in_sixteen_pieces(heads, kv_heads, head_dim, block_size, lengths, window):
+    dtype, n, scale = torch.bfloat16, len(lengths), 0.5 / math.sqrt(head_dim)
+    k = lib(dtype, head_dim)
+    setup, qkv, table, _ = _fused_decode_case(dtype, lengths, heads, kv_heads, head_dim, block_size, seed=heads + head_dim)
+    out = torch.full((n, heads * head_dim), float("nan"), device="cuda").to(dtype)
+    k.attention_decode_fused(qkv, table, setup["k_cache"], setup["v_cache"], setup["table"],
+                             torch.tensor(lengths, dtype=torch.int32, device="cuda"), out, heads, kv_heads, head_dim,
+                             block_size, scale, window, 8, True)
     close(out, attention_reference(setup, dtype, heads, kv_heads, scale, window).view(n, -1), dtype)
 
 
