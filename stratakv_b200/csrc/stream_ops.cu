@@ -329,7 +329,51 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * R;
     const int block_col = rank * SIDE_WARPS * COLS, col0 = block_col + warp * COLS;
-    if (MT == 1) {
+    // Few tokens: the chain of loads is all there is, so that everything which no kernel in front writes is in registers ahead of the
+    // wait: the table's numbers behind the ids, both weights, the norms' weights (in the step, width 32 on 2,048 at 8 tokens 9.0 -> 6.7 us, 64 at 4
+    // 10.5 -> 7.4).
+    constexpr bool EARLY = MT == 1 && COLS <= 64;
+    constexpr int EACH = R * DIM / (SIDE_WARPS * 32);                 // gated values a thread makes
+    static_assert(R * DIM % (SIDE_WARPS * 32) == 0, "gated values a thread");
+    float entry[EACH];
+    bool known[EACH];
+    auto load_entries = [&]() {
+#pragma unroll
+        for (int n = 0; n < EACH; ++n) {
+            const int i = tid + n * SIDE_WARPS * 32, id = ids[min(t0 + i / DIM, n_tokens - 1)];
+            known[n] = id >= 0 && id < vocab;                         // (the embedding has flagged an id outside the table)
+            entry[n] = known[n] ? __bfloat162float(table[(size_t)id * table_stride + offset + i % DIM]) : 0.0f;
+        }
+    };
+    auto load_gate = [&](int c, uint4 (&w)[DIM / 8]) {
+#pragma unroll
+        for (int n = 0; n < DIM / 8; ++n) w[n] = *(const uint4*)(gate_w + (size_t)(8 * n + g) * hidden + col0 + c + 8 * t);
+    };
+    auto load_proj = [&](int c, int k, uint32_t (&w)[4][TILES / 2]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat16* at = proj_t + (size_t)(k + 2 * t + (i & 1) + 8 * (i >> 1)) * hidden + col0 + c * CW + TILES * g;
+            if (TILES == 8) { const uint4 v = *(const uint4*)at; w[i][0] = v.x; w[i][1] = v.y; w[i][TILES / 2 - 2] = v.z; w[i][TILES / 2 - 1] = v.w; }
+            else { const uint2 v = *(const uint2*)at; w[i][0] = v.x; w[i][1] = v.y; }
+        }
+    };
+    uint4 gate_early[EARLY ? COLS / 32 : 1][DIM / 8];
+    uint32_t proj_early[EARLY ? DIM / 16 : 1][4][TILES / 2];
+    float4 norm_early[EARLY ? TILES / 2 : 1], next_early[EARLY ? TILES / 2 : 1];
+    if (EARLY) {
+        load_entries();
+        if (col0 < hidden) {
+#pragma unroll
+            for (int c = 0; c < COLS; c += 32) load_gate(c, gate_early[c / 32]);
+#pragma unroll
+            for (int k = 0; k < DIM; k += 16) load_proj(0, k, proj_early[k / 16]);
+#pragma unroll
+            for (int i = 0; i < TILES / 2; ++i) {
+                norm_early[i] = *(const float4*)(norm_w + col0 + 2 * TILES * t + 4 * i);
+                if (next_out) next_early[i] = *(const float4*)(next_gamma + col0 + 2 * TILES * t + 4 * i);
+            }
+        }
+    } else if (MT == 1) {
         constexpr int LINES = SIDE_WARPS * COLS * 2 / 128;             // 128-byte lines of a weight row in this block's columns
         for (int i = tid; i < 2 * DIM * LINES; i += SIDE_WARPS * 32) {
             const int c = block_col + (i % LINES) * 64, row = (i / LINES) % DIM;
@@ -349,13 +393,12 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     // of 16 is the same for both operands)
     {
         float acc[MT][DIM / 8][4] = {};
-#pragma unroll (MT == 1 ? 2 : 1)
+#pragma unroll (EARLY ? COLS / 32 : MT == 1 ? 2 : 1)
         for (int c = 0; c < COLS; c += 32) {
             const int k = col0 + c + 8 * t;
             if (col0 + c >= hidden) break;
             uint4 w[DIM / 8];
-#pragma unroll
-            for (int n = 0; n < DIM / 8; ++n) w[n] = *(const uint4*)(gate_w + (size_t)(8 * n + g) * hidden + k);
+            if (!EARLY) load_gate(c, w);
             uint32_t a[MT][2][3][4];
 #pragma unroll
             for (int m = 0; m < MT; ++m)
@@ -375,8 +418,9 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
             for (int n = 0; n < DIM / 8; ++n)
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
-                    mma_bf16_add<3>(acc[m][n], a[m][0], w[n].x, w[n].y);
-                    mma_bf16_add<3>(acc[m][n], a[m][1], w[n].z, w[n].w);
+                    const uint4 of = EARLY ? gate_early[c / 32 % (EARLY ? COLS / 32 : 1)][n] : w[n];
+                    mma_bf16_add<3>(acc[m][n], a[m][0], of.x, of.y);
+                    mma_bf16_add<3>(acc[m][n], a[m][1], of.z, of.w);
                 }
         }
 #pragma unroll
@@ -395,18 +439,17 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         for (int w = 1; w < SIDE_WARPS; ++w) sum += part[w * R * DIM + i];
         own[i] = sum;
     }
+    if (!EARLY) load_entries();
     side_cluster_sync();
-    for (int i = tid; i < R * DIM; i += SIDE_WARPS * 32) {
-        const int row = i / DIM, j = i % DIM;
-        const int id = ids[min(t0 + row, n_tokens - 1)];
-        const bool known = id >= 0 && id < vocab;                     // (the embedding has flagged an id outside the table)
-        const float e = known ? __bfloat162float(table[(size_t)id * table_stride + offset + j]) : 0.0f;
+#pragma unroll
+    for (int n = 0; n < EACH; ++n) {
+        const int i = tid + n * SIDE_WARPS * 32;
         float sum = 0.0f;
         for (int r = 0; r < ranks; ++r) sum += side_remote(own + i, r);
         uint32_t parts[3];
-        split3(known ? gelu_tanh(sum) * e : 0.0f, 0.0f, parts);
+        split3(known[n] ? gelu_tanh(sum) * entry[n] : 0.0f, 0.0f, parts);
 #pragma unroll
-        for (int s = 0; s < 3; ++s) gated[(s * R + row) * PITCH + j] = __ushort_as_bfloat16((unsigned short)parts[s]);
+        for (int s = 0; s < 3; ++s) gated[(s * R + i / DIM) * PITCH + i % DIM] = __ushort_as_bfloat16((unsigned short)parts[s]);
     }
     __syncthreads();
 
@@ -419,13 +462,9 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         if (col0 + c * CW >= hidden) continue;
 #pragma unroll
         for (int k = 0; k < DIM; k += 16) {
-            uint32_t w[4][TILES / 2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const __nv_bfloat16* at = proj_t + (size_t)(k + 2 * t + (i & 1) + 8 * (i >> 1)) * hidden + col0 + c * CW + TILES * g;
-                if (TILES == 8) { const uint4 v = *(const uint4*)at; w[i][0] = v.x; w[i][1] = v.y; w[i][TILES / 2 - 2] = v.z; w[i][TILES / 2 - 1] = v.w; }
-                else { const uint2 v = *(const uint2*)at; w[i][0] = v.x; w[i][1] = v.y; }
-            }
+            uint32_t loaded[4][TILES / 2];
+            if (!EARLY) load_proj(c, k, loaded);
+            const uint32_t (&w)[4][TILES / 2] = EARLY ? proj_early[k / 16 % (EARLY ? DIM / 16 : 1)] : loaded;
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 uint32_t a[3][4];
@@ -475,6 +514,13 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         }
         __syncthreads();
     };
+    float4 old[EARLY ? 2 : 1][EARLY ? TILES / 2 : 1];
+    if (EARLY && col0 < hidden) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < TILES / 2; ++i) old[h][i] = *(const float4*)(rows[0][h] + col0 + 2 * TILES * t + 4 * i);
+    }
     make_factor(0, eps);
 #pragma unroll
     for (int m = 0; m < MT; ++m)
@@ -491,8 +537,8 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
                 float* at = x + (size_t)(t0 + row) * hidden + col;
 #pragma unroll
                 for (int i = 0; i < 2 * TILES; i += 4) {
-                    float4 v = *(const float4*)(at + i);
-                    const float4 n = *(const float4*)(norm_w + col + i);
+                    float4 v = EARLY ? old[EARLY ? h : 0][EARLY ? i / 4 : 0] : *(const float4*)(at + i);
+                    const float4 n = EARLY ? norm_early[EARLY ? i / 4 : 0] : *(const float4*)(norm_w + col + i);
                     const int half = i / TILES, j = i % TILES;
                     v.x += y[c][m][j][2 * h + half] * inverse * n.x; v.y += y[c][m][j + 1][2 * h + half] * inverse * n.y;
                     v.z += y[c][m][j + 2][2 * h + half] * inverse * n.z; v.w += y[c][m][j + 3][2 * h + half] * inverse * n.w;
@@ -524,7 +570,8 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             const int e = i + 2 * q, half = e / TILES, j = e % TILES;
-                            const float2 n = *(const float2*)(next_gamma + col + e);
+                            const float4 four = next_early[EARLY ? e / 4 : 0];
+                            const float2 n = EARLY ? (e & 2 ? make_float2(four.z, four.w) : make_float2(four.x, four.y)) : *(const float2*)(next_gamma + col + e);
                             const __nv_bfloat162 v = __floats2bfloat162_rn(y[c][m][j][2 * h + half] * inverse * n.x,
                                                                            y[c][m][j + 1][2 * h + half] * inverse * n.y);
                             packed[q] = *(const uint32_t*)&v;
