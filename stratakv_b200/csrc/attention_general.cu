@@ -315,10 +315,10 @@ attention_general_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
 
 // The parts of a (token, head) that attention_general_kernel or latent_attention_kernel left with splits > 1, put together:
 // the largest maximum, the sums and outputs brought to it, the sink, the gate.  A block per (token, head): the first warp
-// makes the parts' weights, then a thread adds up its numbers of the parts with four loads on their way.  (A warp per
-// (token, head) that walked the parts one after the other took 20 us for 256 of them over 16 parts of 256 numbers,
-// with this one and the kernel below a decode step of 8 sequences over 780 cached rows takes 14 us in place of 69.)
-constexpr int MERGE_THREADS = 128, MERGE_MAX_SPLITS = 1024;
+// makes the parts' weights while the numbers of the first 16 parts are on their way, then a thread adds up its numbers (in the step, 256
+// (token, head) of 256 numbers: 6.0 -> 3.8 us).  (A warp per (token, head) that walked the parts one after the other took 20 us for 256 of
+// them over 16 parts.)
+constexpr int MERGE_THREADS = 256, MERGE_MAX_SPLITS = 1024, MERGE_AHEAD = 16;
 template <typename T>
 __global__ void __launch_bounds__(MERGE_THREADS)
 attention_general_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
@@ -330,6 +330,12 @@ attention_general_merge_kernel(const float* __restrict__ partial_o, const float*
     pdl_wait();
     const long long item = blockIdx.x;
     const int t = (int)(item / num_heads), head = (int)(item % num_heads);
+    // the first numbers of the first parts are on their way while their weights are made (a part without keys left nothing: what is
+    // read of it is not used)
+    const float* o_parts = partial_o + (size_t)item * splits * vdim;
+    float ahead[MERGE_AHEAD];
+#pragma unroll
+    for (int s = 0; s < MERGE_AHEAD; ++s) ahead[s] = s < splits && (int)threadIdx.x < vdim ? o_parts[(size_t)s * vdim + threadIdx.x] : 0.0f;
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         const float* ml = partial_ml + (size_t)item * splits * 2;
@@ -351,10 +357,17 @@ attention_general_merge_kernel(const float* __restrict__ partial_o, const float*
     __syncthreads();
     const float* gate_row = gate && gate_per_element ? gate + (size_t)t * gate_stride + (size_t)head * vdim : nullptr;
     T* out_row = out + (size_t)t * out_stride + (size_t)head * vdim;
-    const float* o_parts = partial_o + (size_t)item * splits * vdim;
     for (int d = threadIdx.x; d < vdim; d += MERGE_THREADS) {
         float value = 0.0f;
-        for (int s0 = 0; s0 < splits; s0 += 4) {
+        const bool first = d == (int)threadIdx.x;
+        if (first) {
+#pragma unroll
+            for (int s = 0; s < MERGE_AHEAD; ++s) {
+                const float w = s < splits ? weights[s] : 0.0f;
+                if (w != 0.0f) value = fmaf(ahead[s], w, value);
+            }
+        }
+        for (int s0 = first ? MERGE_AHEAD : 0; s0 < splits; s0 += 4) {
             float part[4], w[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {                              // (a part without keys left nothing to read)
