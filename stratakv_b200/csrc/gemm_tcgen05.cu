@@ -484,26 +484,29 @@ __device__ __forceinline__ void epilogue_tile_rope(uint32_t acc_tmem, int quarte
 // offsets[e] .. offsets[e + 1], and W holds one [N, K] matrix per group, one after the other.  A row tile starts at a
 // group's first row and at every 128th after it, so no tile spans two groups: what a tile computes for rows past its
 // group's last (they belong to the next group, or lie past the matrix) is not stored.  The counts stay on the device.
+// (Two blocks' tiles have 256 rows: TILE_ROWS.)
 struct GroupArgs {
     const int* offsets;                // [groups + 1], or null: the plain product
     int groups;
 };
 
+template <int TILE_ROWS>
 __device__ __forceinline__ int group_row_tiles(const GroupArgs& group) {
     int tiles = 0;
-    for (int e = 0; e < group.groups; ++e) tiles += (group.offsets[e + 1] - group.offsets[e] + TC_BM - 1) / TC_BM;
+    for (int e = 0; e < group.groups; ++e) tiles += (group.offsets[e + 1] - group.offsets[e] + TILE_ROWS - 1) / TILE_ROWS;
     return tiles;
 }
 
 // Row tile `row_tile` of the grouped form: its first row, the row after its group's last, and its group.
+template <int TILE_ROWS>
 __device__ __forceinline__ void group_tile(const GroupArgs& group, int row_tile, int& m0, int& m_end, int& owner) {
     int seen = 0;
     m0 = 0; m_end = 0; owner = 0;
     for (int e = 0; e < group.groups; ++e) {
         const int lo = group.offsets[e], hi = group.offsets[e + 1];
-        const int tiles = (hi - lo + TC_BM - 1) / TC_BM;
+        const int tiles = (hi - lo + TILE_ROWS - 1) / TILE_ROWS;
         if (row_tile < seen + tiles) {
-            m0 = lo + (row_tile - seen) * TC_BM;
+            m0 = lo + (row_tile - seen) * TILE_ROWS;
             m_end = hi;
             owner = e;
             return;
@@ -553,7 +556,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                                   // A (and the groups' offsets) are earlier kernels' output
-    const int m_tiles = grouped ? group_row_tiles(group) : (M + TC_BM - 1) / TC_BM;
+    const int m_tiles = grouped ? group_row_tiles<TC_BM>(group) : (M + TC_BM - 1) / TC_BM;
     const int total_tiles = m_tiles * n_tiles;
 
     // A block walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ...; neighbouring tiles share their
@@ -567,7 +570,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (grouped) {
                 int m_end, owner;
                 n_tile = tile / m_tiles;
-                group_tile(group, tile - n_tile * m_tiles, m0, m_end, owner);
+                group_tile<TC_BM>(group, tile - n_tile * m_tiles, m0, m_end, owner);
                 w0 = owner * N + n_tile * BN;     // the group's own matrix among the stacked ones
             } else {
                 tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
@@ -639,7 +642,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (grouped) {
                 int owner;
                 n_tile = tile / m_tiles;
-                group_tile(group, tile - n_tile * m_tiles, m0, rows_end, owner);
+                group_tile<TC_BM>(group, tile - n_tile * m_tiles, m0, rows_end, owner);
             } else {
                 tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
                 m0 = m_tile * TC_BM;
@@ -650,7 +653,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     epilogue_tile_rope<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, rope,
                                            M, N, m0, n0);
             } else {
-                epilogue_tile<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, tma_out, out,
+                // (a slab that reaches into the next group's rows is stored by the threads)
+                const int by_copy = tma_out && (rows_end == M || m0 + quarter * 32 + 32 <= rows_end);
+                epilogue_tile<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, by_copy, out,
                                   rows_end, N, mode, act, m0, n0);
             }
             // the accumulator has been read out: hand it back to the issuer
@@ -725,7 +730,7 @@ template <int STAGES>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                          const __grid_constant__ CUtensorMap map_out, int tma_out, void* __restrict__ out, int M,
-                         int N, int K, int mode, act_t act, int* __restrict__ flag, const RopeArgs rope) {
+                         int N, int K, int mode, act_t act, int* __restrict__ flag, const RopeArgs rope, const GroupArgs group) {
     constexpr int BN = 256;                                  // the pair's tile: 256 rows (128 per block) x 256 columns
     constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, W_BYTES = (BN / 2) * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     constexpr uint32_t TMEM_COLS = 512, ACC_STRIDE = 256;
@@ -739,9 +744,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t rank = cluster_rank();                   // 0: the block that issues the pair's MMAs
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int k_iters = (K + TC_BK - 1) / TC_BK;
-    const int m_tiles = (M + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (N + BN - 1) / BN;
-    const int total_tiles = m_tiles * n_tiles;
+    const int n_tiles = (N + BN - 1) / BN;
     const int band = tile_band(2 * TC_BM, K);
+    const bool grouped = group.offsets != nullptr;
     const uint32_t full0 = smem_addr(bars), empty0 = smem_addr(bars + STAGES);
     const uint32_t acc_full0 = smem_addr(bars + 2 * STAGES), acc_empty0 = smem_addr(bars + 2 * STAGES + 2);
 
@@ -765,7 +770,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_wait();
+    pdl_wait();                                    // A (and the groups' offsets) are earlier kernels' output
+    const int m_tiles = grouped ? group_row_tiles<2 * TC_BM>(group) : (M + 2 * TC_BM - 1) / (2 * TC_BM);
+    const int total_tiles = m_tiles * n_tiles;
 
     if (warp == 0) {
         // ---- loader: this block's rows of A and its half of the W rows (the warp walks, an elected lane issues) ----
@@ -773,10 +780,16 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         int it = 0;
         const uint32_t first_full0 = cluster_address(full0, 0);
         for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
-            int m_tile, n_tile;
-            tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
-            const int m0 = m_tile * 2 * TC_BM + (int)rank * TC_BM;
-            const int w0 = n_tile * BN + (int)rank * (BN / 2);
+            int m_tile, n_tile, m0, m_end, owner = 0;
+            if (grouped) {
+                n_tile = tile / m_tiles;
+                group_tile<2 * TC_BM>(group, tile - n_tile * m_tiles, m0, m_end, owner);
+            } else {
+                tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
+                m0 = m_tile * 2 * TC_BM;
+            }
+            m0 += (int)rank * TC_BM;
+            const int w0 = owner * N + n_tile * BN + (int)rank * (BN / 2);
             for (int i = 0; i < k_iters; ++i, ++it) {
                 const int s = it % STAGES;
                 if (it >= STAGES) ok = mbar_wait(empty0 + 8 * s, ((it / STAGES) - 1) & 1, flag);
@@ -838,15 +851,25 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             ok = mbar_wait(acc_full0 + 8 * buf, (local >> 1) & 1, flag);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            int m_tile, n_tile;
-            tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
-            const int m0 = m_tile * 2 * TC_BM + (int)rank * TC_BM, n0 = n_tile * BN;
+            int m_tile, n_tile, m0, rows_end = M;
+            if (grouped) {
+                int owner;
+                n_tile = tile / m_tiles;
+                group_tile<2 * TC_BM>(group, tile - n_tile * m_tiles, m0, rows_end, owner);
+            } else {
+                tile_coordinates(tile, m_tiles, n_tiles, band, m_tile, n_tile);
+                m0 = m_tile * 2 * TC_BM;
+            }
+            m0 += (int)rank * TC_BM;
+            const int n0 = n_tile * BN;
             if (mode == TC_MODE_QKV_ROPE) {
                 epilogue_tile_rope<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, rope,
                                        M, N, m0, n0);
             } else {
-                epilogue_tile<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, tma_out, out,
-                                  M, N, mode, act, m0, n0);
+                // (a slab that reaches into the next group's rows is stored by the threads)
+                const int by_copy = tma_out && (rows_end == M || m0 + quarter * 32 + 32 <= rows_end);
+                epilogue_tile<BN>(tmem_base + (uint32_t)buf * ACC_STRIDE, quarter, lane, slabs, buffer, &map_out, by_copy, out,
+                                  rows_end, N, mode, act, m0, n0);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -1228,15 +1251,26 @@ static int launch_tc(const void* a, const void* w, void* out, int M, int N, int 
                       map_a, map_w, map_out, tma_out, out, M, N, K, mode, act, flag, rope, GroupArgs{nullptr, 0});
 }
 
+// Where the grouped form's result goes: through the copy engine where its rows are whole 16 bytes, except at the groups' ends.  (A thread
+// that stores its own row touches 32 lines with every instruction of its warp: 9,300 rows x 2816 x 2048 118 -> 89 us, 4,800 x 14,336 x 4096
+// 537 -> 505, 6,900 x 5632 x 2048 187 -> 147.)
+static int grouped_out_map(void* out, int out_is_float, int rows, int N, int gated, const CUtensorMap& unused, CUtensorMap* map, int* use) {
+    const int cols = gated ? N / 2 : N, elem = out_is_float ? 4 : 2;
+    *map = unused;
+    *use = ((size_t)cols * elem) % 16 == 0 && ((uintptr_t)out & 15) == 0;
+    return *use ? tensor_map(out, rows, cols, elem, 32, out_is_float ? 32 : 64, map) : 0;
+}
+
 // The grouped form of the kernel above: `a` [rows, K] sorted by group, `w` [groups, N, K], `out` [rows, N] (bfloat16
-// with the activation, or float).  The threads store their rows themselves (a tile's rows past its group are another
-// group's).  Blocks beyond the tiles there turn out to be leave at once.
+// with the activation, or float).  Blocks beyond the tiles there turn out to be leave at once.
 template <int BN, int STAGES>
 static int launch_grouped(const void* a, const void* w, const int* offsets, void* out, int out_is_float, int rows,
                           int groups, int N, int K, act_t act, int gated, int* flag, cudaStream_t stream) {
-    CUtensorMap map_a, map_w;
+    CUtensorMap map_a, map_w, map_out;
     if (int code = tensor_map(a, rows, K, 2, TC_BM, TC_BK, &map_a)) return code;
     if (int code = tensor_map(w, groups * N, K, 2, BN, TC_BK, &map_w)) return code;
+    int tma_out = 0;
+    if (int code = grouped_out_map(out, out_is_float, rows, N, gated, map_a, &map_out, &tma_out)) return code;
     constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 4 * 2 * 4096 +
                             (2 * STAGES + 4) * 8 + 16 + 1024;
     static bool configured = false;
@@ -1253,25 +1287,7 @@ static int launch_grouped(const void* a, const void* w, const int* offsets, void
     dim3 grid((unsigned)(tiles < sms ? tiles : sms));
     const int mode = gated ? TC_MODE_GATED : (out_is_float ? TC_MODE_STORE_F32 : TC_MODE_STORE);
     return launch_pdl("skv_expert_linear(tcgen05)", gemm_tcgen05_kernel<BN, STAGES>, grid, dim3(TC_THREADS), smem, stream,
-                      map_a, map_w, map_a, 0, out, rows, N, K, mode, act, flag, RopeArgs{}, GroupArgs{offsets, groups});
-}
-
-// gated: every group's matrix holds N rows in tiles of 16 (8 gate rows, then their 8 up rows) and out is [rows, N / 2]
-// bfloat16, act(gate) * up; act is then the plain activation code.
-int grouped_linear_tcgen05(const void* a, const void* w, const int* offsets, void* out, int out_is_float, int rows,
-                           int groups, int N, int K, act_t act, int gated, int* flag, cudaStream_t stream) {
-    if (gated && (N % 16 != 0 || out_is_float || (act & 0xff) == ACT_RELU2))
-        return fail("skv_expert_linear(tcgen05)", "a gated weight needs whole tiles of 16 rows, a bfloat16 result and a gate's activation");
-    if (K % 8 != 0) return fail("skv_expert_linear(tcgen05)", "the inner size must be a multiple of 8 (16-byte rows)");
-    if (((uintptr_t)a | (uintptr_t)w) & 15) return fail("skv_expert_linear(tcgen05)", "operands must be 16-byte aligned");
-    if ((long long)groups * N > 0x7fffffffLL) return fail("skv_expert_linear(tcgen05)", "too many weight rows");
-    // Tiles 256 columns wide keep the tensor pipe busier (wider MMAs, half the epilogues a FLOP) where the groups have
-    // rows for them; few rows (a decode step) are bound by streaming the weights, and narrow tiles spread those over
-    // more blocks.
-    const long long wide_tiles = ((long long)(rows + TC_BM - 1) / TC_BM + groups) * ((N + 255) / 256);
-    if (N >= 256 && rows >= 2 * TC_BM * groups && wide_tiles >= tc_sm_count())
-        return launch_grouped<256, 4>(a, w, offsets, out, out_is_float, rows, groups, N, K, act, gated, flag, stream);
-    return launch_grouped<128, 4>(a, w, offsets, out, out_is_float, rows, groups, N, K, act, gated, flag, stream);
+                      map_a, map_w, map_out, tma_out, out, rows, N, K, mode, act, flag, RopeArgs{}, GroupArgs{offsets, groups});
 }
 
 // The two-block form: clusters of two blocks, as many as the GPU runs at once (74 on 148 SMs), walk the 256 x 256 tiles.
@@ -1339,9 +1355,54 @@ static int launch_pair(const void* a, const void* w, void* out, int M, int N, in
     config.gridDim = dim3(2u * (unsigned)(tiles < slots ? tiles : slots));
     config.numAttrs = pdl_enabled() ? 2 : 1;
     const cudaError_t status = cudaLaunchKernelEx(&config, gemm_tcgen05_pair_kernel<PAIR_STAGES>, map_a, map_w, map_out,
-                                                  tma_out, out, M, N, K, mode, act, flag, rope);
+                                                  tma_out, out, M, N, K, mode, act, flag, rope, GroupArgs{nullptr, 0});
     if (status != cudaSuccess) return fail("skv_linear(tcgen05 pair)", cudaGetErrorString(status));
     return 0;
+}
+
+// The grouped form of pairs of blocks.
+static int launch_grouped_pair(const void* a, const void* w, const int* offsets, void* out, int out_is_float, int rows, int groups, int N,
+                               int K, act_t act, int gated, int* flag, cudaStream_t stream) {
+    CUtensorMap map_a, map_w, map_out;
+    if (int code = tensor_map(a, rows, K, 2, TC_BM, TC_BK, &map_a)) return code;
+    if (int code = tensor_map(w, groups * N, K, 2, 128, TC_BK, &map_w)) return code;
+    int tma_out = 0;
+    if (int code = grouped_out_map(out, out_is_float, rows, N, gated, map_a, &map_out, &tma_out)) return code;
+    cudaLaunchConfig_t config;
+    cudaLaunchAttribute attributes[2];
+    pair_launch_config(&config, attributes, stream);
+    const long long tiles = ((long long)(rows + 2 * TC_BM - 1) / (2 * TC_BM) + groups) * ((N + 255) / 256);
+    config.gridDim = dim3(2u * (unsigned)(tiles < pair_slots() ? tiles : pair_slots()));
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    const int mode = gated ? TC_MODE_GATED : (out_is_float ? TC_MODE_STORE_F32 : TC_MODE_STORE);
+    const cudaError_t status = cudaLaunchKernelEx(&config, gemm_tcgen05_pair_kernel<PAIR_STAGES>, map_a, map_w, map_out, tma_out, out, rows, N, K,
+                                                  mode, act, flag, RopeArgs{}, GroupArgs{offsets, groups});
+    if (status != cudaSuccess) return fail("skv_expert_linear(tcgen05 pair)", cudaGetErrorString(status));
+    return 0;
+}
+
+// gated: every group's matrix holds N rows in tiles of 16 (8 gate rows, then their 8 up rows) and out is [rows, N / 2]
+// bfloat16, act(gate) * up; act is then the plain activation code.
+int grouped_linear_tcgen05(const void* a, const void* w, const int* offsets, void* out, int out_is_float, int rows,
+                           int groups, int N, int K, act_t act, int gated, int* flag, cudaStream_t stream) {
+    if (gated && (N % 16 != 0 || out_is_float || (act & 0xff) == ACT_RELU2))
+        return fail("skv_expert_linear(tcgen05)", "a gated weight needs whole tiles of 16 rows, a bfloat16 result and a gate's activation");
+    if (K % 8 != 0) return fail("skv_expert_linear(tcgen05)", "the inner size must be a multiple of 8 (16-byte rows)");
+    if (((uintptr_t)a | (uintptr_t)w) & 15) return fail("skv_expert_linear(tcgen05)", "operands must be 16-byte aligned");
+    if ((long long)groups * N > 0x7fffffffLL) return fail("skv_expert_linear(tcgen05)", "too many weight rows");
+    // Tiles 256 columns wide keep the tensor pipe busier (wider MMAs, half the epilogues a FLOP) where the groups have
+    // rows for them; few rows (a decode step) are bound by streaming the weights, and narrow tiles spread those over
+    // more blocks.
+    const long long wide_tiles = ((long long)(rows + TC_BM - 1) / TC_BM + groups) * ((N + 255) / 256);
+    if (N >= 256 && rows >= 2 * TC_BM * groups && wide_tiles >= tc_sm_count()) {
+        // Pairs of blocks fetch a third less for the same products (as for plain projections), but a group leaves up to 256 rows of a tile
+        // empty in place of 128: from four tiles of 256 a group on.  8 groups, us on single blocks / pairs: 9,300 rows x 2816 x 2048 88.6 / 84.3, x
+        // 2048 x 2816 105 / 96; 6,900 rows x 5632 x 2048 147 / 157; 4,000 rows x 2048 x 1408 40 / 48.
+        if (pair_slots() > 0 && rows >= 4 * 256 * groups && wide_tiles >= 2 * pair_slots())
+            return launch_grouped_pair(a, w, offsets, out, out_is_float, rows, groups, N, K, act, gated, flag, stream);
+        return launch_grouped<256, 4>(a, w, offsets, out, out_is_float, rows, groups, N, K, act, gated, flag, stream);
+    }
+    return launch_grouped<128, 4>(a, w, offsets, out, out_is_float, rows, groups, N, K, act, gated, flag, stream);
 }
 
 // Whether the two-block kernel is the cheaper one, in the units of the cost of a width below (rounds x 256 columns):
