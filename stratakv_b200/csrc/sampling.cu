@@ -96,6 +96,12 @@ __device__ __forceinline__ unsigned long long sort_key(float v, int index) {
     return ((unsigned long long)orderable(v) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)index);
 }
 
+// The value in such a key.
+__device__ __forceinline__ float value_of(unsigned long long key) {
+    const uint32_t high = (uint32_t)(key >> 32);
+    return __uint_as_float((high & 0x80000000u) ? high & 0x7fffffffu : ~high);
+}
+
 __device__ __forceinline__ unsigned long long fixed_mass(float v, float max_value) {
     // exp(v - max) in (0, 1] as 40-bit fixed point; never below 1 so that every kept token can be drawn.  (The
     // special-function unit's exponential, a few units in the last place of a float off libm's: a row is walked up to
@@ -292,7 +298,10 @@ __device__ unsigned long long radix_select(const float* __restrict__ row, const 
 // 253 for k = 200.  Their order, the top-p cut and the draw come from counting: a thread per element counts the keys
 // above its own.  The masses, the cuts and the drawn number are those of the general path, integer for integer.
 // Bound by the two walks (the row comes from L2 or HBM once each, 16 bytes a load, no division but for what reaches
-// the bound).  64 rows of 128,256 logits with k = 40, p = 0.95: the general path's fourteen passes took 389 us.
+// the bound), which the blocks of a cluster share out where rows are few, and by about 6 us of short steps one behind the
+// other.  64 rows of 128,256 logits with k = 40, p = 0.95: the general path's fourteen passes took 389 us, one block a row that
+// counted 512 maxima 29.0, now 19.8 (1 row 24.2 and 12.7; 8 rows of 32,000 17.0 and 10.3; 8 of 50,257, whose rows lie off 16-byte
+// boundaries and were read 4 bytes at a time, 35.6 and 10.9).
 // Returns false where the list would not hold the candidates (more than SAMPLE_THREADS equal values at the bound) or
 // where the quotients lie so near zero that they lose bits (then the bound on x says nothing about x / temperature).
 constexpr int FEW_K = 256;
@@ -306,8 +315,35 @@ __host__ __device__ inline bool sample_few_serves(int vocab, int top_k, float to
     return top_k > 0 && top_k <= FEW_K && vocab >= (top_p < 1.0f ? 4 * top_k : 2000 + 10 * top_k);
 }
 
+// Blocks that share a row: while the GPU has an SM for each (a tenth fewer: clusters do not fill every partition of it), what they list
+// fits, and a block's part is long enough to pay for the exchange of bounds, which takes about 2 us.  One row of 128,256 logits (top-k
+// 40, top-p 0.95) 12.7 us over eight blocks, 64 rows 19.8 over two each; 100 rows, one block each, 22.8.  64 rows of 16,384 took 9.8 us
+// over two blocks each and 8.6 over one.
+__host__ __device__ inline int sample_few_ranks(int rows, int vocab, int top_k, int slots) {
+    int ranks = 1;
+    while (ranks < 8 && rows * ranks * 2 <= slots - slots / 10 && 2 * ranks * top_k <= SAMPLE_THREADS / 8 * 5 && vocab / (2 * ranks) >= 12000) ranks *= 2;
+    return ranks;
+}
+
+// What a block of a cluster found in its part of the row.
+struct SamplePart {
+    float bound, most, largest;
+    int at_bound, bad, unused[3];
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t in_rank(const void* p, int rank) {
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return at;
+}
+
+// With `ranks` > 1 the blocks of a cluster share the row out; rank 0 goes on alone behind the second walk, and the other ranks
+// return true whatever becomes of the row.
 __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out, int vocab, float temperature, int top_k, float top_p,
-                           unsigned long long seed, uint32_t stream, uint32_t counter, int* __restrict__ flag, unsigned char* smem) {
+                           unsigned long long seed, uint32_t stream, uint32_t counter, int* __restrict__ flag, unsigned char* smem,
+                           int ranks, int part) {
     float* maxima = (float*)smem;                                                          // [threads]
     unsigned long long* keys = (unsigned long long*)(smem + SAMPLE_THREADS * 4);            // [threads], in list order
     unsigned long long* sorted = keys + SAMPLE_THREADS;                                     // [threads], largest first
@@ -316,11 +352,18 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
     int* listed = (int*)(drawn + FEW_K);                                                    // [threads]
     int* drawn_index = listed + SAMPLE_THREADS;                                             // [FEW_K]
     __shared__ float bound, extent[2];                      // extent: the largest logit, and the largest magnitude
-    __shared__ int count, bad_row, kept, at_bound;
+    __shared__ int count, bad_row, kept, at_bound, total, first;
+    __shared__ __align__(16) SamplePart parts[8];
     const int tid = threadIdx.x, lane = tid & 31;
-    if (tid == 0) { count = 0; bad_row = 0; extent[0] = -INFINITY; extent[1] = 0.0f; }
-    const bool wide = ((uintptr_t)row & 15) == 0;
-    const int quads = wide ? vocab >> 2 : 0;
+    if (tid == 0) { count = 0; bad_row = 0; total = 0; extent[0] = -INFINITY; extent[1] = 0.0f; }
+    if (ranks > 1) cluster_arrive();                        // (waited for ahead of the first access to another block's memory)
+    // Whole quads of the row, counted from its first 16-byte boundary, are shared out; the elements ahead of that boundary go to the
+    // first part, those behind the last quad to the last.
+    const int head = min(vocab, (int)((16 - ((uintptr_t)row & 15)) & 15) >> 2), all_quads = (vocab - head) >> 2;
+    const int share = (all_quads + ranks - 1) / ranks, first_quad = min(all_quads, part * share), quads = min(all_quads, first_quad + share);
+    const float4* row4 = (const float4*)(row + head);
+    const int odd = tid < head ? tid : head + 4 * all_quads + tid - head;                   // (seven such elements at most)
+    const bool has_odd = tid < head ? part == 0 : odd < vocab && part == ranks - 1;
     float most = -INFINITY, largest = 0.0f;
     bool bad = false;
     auto look = [&](float x) {
@@ -328,39 +371,68 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
         most = fmaxf(most, x);
         largest = fmaxf(largest, fabsf(x));
     };
-    for (int q0 = tid; q0 < quads; q0 += FEW_LOADS * SAMPLE_THREADS) {
+    for (int q0 = first_quad + tid; q0 < quads; q0 += FEW_LOADS * SAMPLE_THREADS) {
         float4 x[FEW_LOADS];
 #pragma unroll
         for (int u = 0; u < FEW_LOADS; ++u)
-            x[u] = q0 + u * SAMPLE_THREADS < quads ? ((const float4*)row)[q0 + u * SAMPLE_THREADS] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            x[u] = q0 + u * SAMPLE_THREADS < quads ? row4[q0 + u * SAMPLE_THREADS] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int u = 0; u < FEW_LOADS; ++u)
             if (q0 + u * SAMPLE_THREADS < quads) { look(x[u].x); look(x[u].y); look(x[u].z); look(x[u].w); }
     }
-    for (int i = 4 * quads + tid; i < vocab; i += SAMPLE_THREADS) look(row[i]);
-    maxima[tid] = most;
+    if (has_odd) look(row[odd]);
+    // A bound is the k-th largest of the maxima of groups of neighbouring threads: one thread of 512 a group, two of 256 or four of
+    // 128: the smallest number of which at least twice top_k hold something (40 of 128 list 48 candidates, of 512 42).
+    // The lanes of a group share the counting out: 512 groups are 512 comparisons a thread, 6.5 us of a call's 15; 128 are 32.
+    const int holding = min(all_quads / ranks, SAMPLE_THREADS);
+    const int lanes = holding >= 8 * top_k ? 4 : holding >= 4 * top_k ? 2 : 1, groups = SAMPLE_THREADS / lanes;
+    if (lanes > 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1));
+    if (lanes > 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
+    if ((tid & (lanes - 1)) == 0) maxima[tid / lanes] = most;
     __syncthreads();
     if (bad) bad_row = 1;
     const float warp_largest = warp_max(largest);
     if (lane == 0) atomicMax((unsigned int*)&extent[1], __float_as_uint(warp_largest));     // (not negative: ordered as integers)
-    // the k-th largest of the maxima
     int above = 0, not_below = 0;
-    for (int i = 0; i < SAMPLE_THREADS; i += 4) {
+    for (int i = 4 * (tid & (lanes - 1)); i < groups; i += 4 * lanes) {
         const float4 o = *(const float4*)(maxima + i);
         above += (o.x > most) + (o.y > most) + (o.z > most) + (o.w > most);
         not_below += (o.x >= most) + (o.y >= most) + (o.z >= most) + (o.w >= most);
     }
+    if (lanes > 1) { above += __shfl_xor_sync(0xffffffffu, above, 1); not_below += __shfl_xor_sync(0xffffffffu, not_below, 1); }
+    if (lanes > 2) { above += __shfl_xor_sync(0xffffffffu, above, 2); not_below += __shfl_xor_sync(0xffffffffu, not_below, 2); }
     if (above < top_k && not_below >= top_k) { bound = most; at_bound = not_below - above; }    // (all who write write the same)
     if (above == 0) extent[0] = most;
     __syncthreads();
+    if (ranks > 1) {
+        // The largest of the parts' bounds is a bound of the row: k logits of that part reach it.
+        cluster_wait();
+        if (tid < ranks) {
+            const uint32_t at = in_rank(parts + part, tid);
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(__float_as_uint(bound)), "r"(__float_as_uint(extent[0])),
+                         "r"(__float_as_uint(extent[1])), "r"(at_bound) : "memory");
+            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at + 16u), "r"(bad_row) : "memory");
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (tid == 0) {
+            for (int r = 0; r < ranks; ++r) {
+                if (r == 0 || parts[r].bound > bound) { bound = parts[r].bound; at_bound = parts[r].at_bound; }
+                extent[0] = r == 0 ? parts[r].most : fmaxf(extent[0], parts[r].most);
+                extent[1] = r == 0 ? parts[r].largest : fmaxf(extent[1], parts[r].largest);
+                bad_row |= parts[r].bad;
+            }
+        }
+        __syncthreads();
+    }
     if (bad_row || !isfinite(extent[1] / temperature)) {
-        if (tid == 0) { if (flag) atomicOr(flag, 2); *out = 0; }
+        if (tid == 0 && part == 0) { if (flag) atomicOr(flag, 2); *out = 0; }
         return true;
     }
     const float max_value = extent[0] / temperature, x_bound = bound, v_bound = x_bound / temperature;
-    if (fabsf(v_bound) < 1e-30f) return false;
-    // equal values at the bound in three threads of four: fewer than k logits stand out of a row of the mask's value, say
-    if (at_bound > SAMPLE_THREADS / 4 * 3 && x_bound > -INFINITY) return false;
+    if (fabsf(v_bound) < 1e-30f) return part != 0;
+    // equal values at the bound in three groups of four: fewer than k logits stand out of a row of the mask's value, say
+    if (at_bound > groups / 4 * 3 && x_bound > -INFINITY) return part != 0;
     const float x_low = x_bound - fabsf(x_bound) * 9.5367431640625e-7f;                     // (2^-20: 16 roundings of a quotient)
     auto collect = [&](float x, int i) {
         if (x >= x_low && x / temperature >= v_bound) {
@@ -368,33 +440,55 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
             if (at < SAMPLE_THREADS) listed[at] = i;
         }
     };
-    for (int q0 = tid; q0 < quads && *(volatile int*)&count <= SAMPLE_THREADS; q0 += FEW_LOADS * SAMPLE_THREADS) {   // (no further once it overflows)
+    for (int q0 = first_quad + tid; q0 < quads && *(volatile int*)&count <= SAMPLE_THREADS; q0 += FEW_LOADS * SAMPLE_THREADS) {   // (no further once it overflows)
         float4 x[FEW_LOADS];
 #pragma unroll
         for (int u = 0; u < FEW_LOADS; ++u)
-            x[u] = q0 + u * SAMPLE_THREADS < quads ? ((const float4*)row)[q0 + u * SAMPLE_THREADS] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            x[u] = q0 + u * SAMPLE_THREADS < quads ? row4[q0 + u * SAMPLE_THREADS] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
 #pragma unroll
         for (int u = 0; u < FEW_LOADS; ++u) {
-            const int i = 4 * (q0 + u * SAMPLE_THREADS);
-            if (i >= 4 * quads || fmaxf(fmaxf(x[u].x, x[u].y), fmaxf(x[u].z, x[u].w)) < x_low) continue;
+            const int i = head + 4 * (q0 + u * SAMPLE_THREADS);
+            if (q0 + u * SAMPLE_THREADS >= quads || fmaxf(fmaxf(x[u].x, x[u].y), fmaxf(x[u].z, x[u].w)) < x_low) continue;
             collect(x[u].x, i); collect(x[u].y, i + 1); collect(x[u].z, i + 2); collect(x[u].w, i + 3);
         }
     }
-    for (int i = 4 * quads + tid; i < vocab; i += SAMPLE_THREADS) collect(row[i], i);
+    if (has_odd) collect(row[odd], odd);
     __syncthreads();
-    const int n = count;
-    if (n > SAMPLE_THREADS) return false;
+    int n = count;
     unsigned long long key = 0ull, mass = 0ull;
+    if (ranks > 1) {
+        // the ranks' lists go one behind the other into rank 0's (in any order: what follows counts)
+        if (tid == 0)
+            asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(first) : "r"(in_rank(&total, 0)), "r"(n) : "memory");
+        __syncthreads();
+        if (tid < n && first + tid < SAMPLE_THREADS) {
+            const int i = listed[tid];
+            key = sort_key(row[i] / temperature, i);
+            asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(in_rank(keys + first + tid, 0)), "l"(key) : "memory");
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (part != 0) return true;
+        n = total;
+        key = 0ull;
+    }
+    if (n > SAMPLE_THREADS) return false;
     if (tid < n) {
-        const int i = listed[tid];
-        const float v = row[i] / temperature;
-        key = sort_key(v, i);
-        mass = fixed_mass(v, max_value);
-        keys[tid] = key;
+        if (ranks > 1) {
+            key = keys[tid];
+            mass = fixed_mass(value_of(key), max_value);
+        } else {
+            const int i = listed[tid];
+            const float v = row[i] / temperature;
+            key = sort_key(v, i);
+            mass = fixed_mass(v, max_value);
+            keys[tid] = key;
+        }
     }
     __syncthreads();
     int rank = 0;
-    for (int i = 0; i < n; ++i) rank += keys[i] > key;
+    if (tid - lane < n)
+        for (int i = 0; i < n; ++i) rank += keys[i] > key;
     if (tid < n) { sorted[rank] = key; masses[rank] = mass; }
     __syncthreads();
     // the top-p cut: lane l of the first warp walks ranks 8l to 8l + 7
@@ -461,7 +555,7 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab, float temperature, int top_k,
               float top_p, unsigned long long seed, const int* __restrict__ streams,
-              const int* __restrict__ counters, int* __restrict__ flag, int staged) {
+              const int* __restrict__ counters, int* __restrict__ flag, int staged, int ranks) {
     // `staged`: the row divided by the temperature is kept in (dynamic) shared memory after the first walk, and the
     // later walks read it there; rows too long for that are read and divided again each time, with the same results
     extern __shared__ __align__(16) unsigned char sample_smem[];
@@ -477,11 +571,12 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     __shared__ int bad_flag;
     pdl_launch_dependents();
     pdl_wait();
-    const float* row = logits + (size_t)blockIdx.x * vocab;
+    const int at = blockIdx.x / ranks;                     // (blocks of a cluster share a row)
+    const float* row = logits + (size_t)at * vocab;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (sample_few_serves(vocab, top_k, top_p) &&
-        sample_few(row, out + blockIdx.x, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[blockIdx.x],
-                   (uint32_t)counters[blockIdx.x], flag, sample_smem))
+        sample_few(row, out + at, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[at], (uint32_t)counters[at], flag, sample_smem,
+                   ranks, (int)blockIdx.x - at * ranks))
         return;
     if (threadIdx.x == 0) bad_flag = 0;
     __syncthreads();
@@ -516,7 +611,7 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     __syncthreads();
     const float max_value = scratch[32];
     if (bad_flag) {
-        if (threadIdx.x == 0) { if (flag) atomicOr(flag, 2); out[blockIdx.x] = 0; }
+        if (threadIdx.x == 0) { if (flag) atomicOr(flag, 2); out[at] = 0; }
         return;
     }
 
@@ -559,7 +654,7 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     if (threadIdx.x == 0) {
         unsigned long long total = 0ull;
         for (int w = 0; w < SAMPLE_WARPS; ++w) total += warp_total[w];
-        const uint32_t r = philox_first_word(seed, (uint32_t)streams[blockIdx.x], (uint32_t)counters[blockIdx.x]);
+        const uint32_t r = philox_first_word(seed, (uint32_t)streams[at], (uint32_t)counters[at]);
         // target in [0, total): floor(total * r / 2^32) with a 96-bit product
         const unsigned long long target = __umul64hi(total, (unsigned long long)r << 32);
         unsigned long long run = 0ull;
@@ -594,7 +689,7 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
                 run += fixed_mass(v, max_value);
                 if (remaining < run) { chosen = i; break; }
             }
-            out[blockIdx.x] = chosen >= 0 ? chosen : max(last_allowed, 0);
+            out[at] = chosen >= 0 ? chosen : max(last_allowed, 0);
         }
     }
 }
@@ -634,9 +729,29 @@ SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, fl
         if (status != cudaSuccess) return fail("skv_sample", cudaGetErrorString(status));
         configured = true;
     }
+    const size_t smem = histograms + (staged ? row_bytes : 0), alone = 116 * 1024;
+    const int ranks = sample_few_serves(vocab, top_k, top_p) ? sample_few_ranks(rows, vocab, top_k, sm_count()) : 1;
+    if (ranks > 1) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3((unsigned)(rows * ranks));
+        config.blockDim = dim3(SAMPLE_THREADS);
+        config.dynamicSmemBytes = smem;
+        config.stream = stream;
+        cudaLaunchAttribute attributes[2];
+        attributes[0].id = cudaLaunchAttributeClusterDimension;
+        attributes[0].val.clusterDim.x = (unsigned)ranks;
+        attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+        attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attributes[1].val.programmaticStreamSerializationAllowed = 1;
+        config.attrs = attributes;
+        config.numAttrs = pdl_enabled() ? 2 : 1;
+        const cudaError_t status = cudaLaunchKernelEx(&config, sample_kernel, logits, out, vocab, temperature, top_k, top_p, (unsigned long long)seed,
+                                                      streams, counters, flag, staged, ranks);
+        if (status != cudaSuccess) return fail("skv_sample", cudaGetErrorString(status));
+        return 0;
+    }
     // Rows that fit the GPU's SMs one by one take more than half of an SM's memory each: blocks of this launch that start while the one
     // in front still runs would share SMs and leave others idle (128 rows of 50,257, top-k 40 and top-p 45 us, 36 so).
-    const size_t smem = histograms + (staged ? row_bytes : 0), alone = 116 * 1024;
     return launch_pdl("skv_sample", sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), rows <= sm_count() && smem < alone ? alone : smem, stream, logits, out,
-                      vocab, temperature, top_k, top_p, (unsigned long long)seed, streams, counters, flag, staged);
+                      vocab, temperature, top_k, top_p, (unsigned long long)seed, streams, counters, flag, staged, 1);
 }

@@ -174,3 +174,41 @@ def test_masked_rows_with_few_logits_left(vocab, allowed):
 def test_two_blocks_of_the_kernel_share_an_sm():
     """More rows than SMs: with one block an SM they take half as long again."""
     assert kernels().lib.skv_sample_blocks_per_sm() >= 2
+
+
+@pytest.mark.parametrize("vocab,top_k", [(16384, 1), (32000, 40), (50257, 40), (65539, 97), (128256, 40), (128256, 256)])
+@pytest.mark.parametrize("kind", ["plain", "ties", "masked", "one_part"])
+def test_blocks_that_share_a_row_draw_what_one_block_draws(vocab, top_k, kind):
+    """A row of a small batch is walked by two, four or eight blocks, a row of a large one by one: the tokens are the same,
+    whatever part the largest logits lie in, and a logit that is not finite is found in every part."""
+    rng = np.random.default_rng(vocab + top_k)
+    rows = 300
+    logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
+    if kind == "ties":
+        logits = np.round(logits * 8) / 8
+    elif kind == "masked":
+        logits[:, 100:] = -1e30
+        logits[::2, -30:] = 1.0
+    elif kind == "one_part":
+        for r in range(rows):
+            logits[r, (r * 997) % (vocab - 600):][:600] += 30.0
+    k = kernels()
+    streams = torch.arange(rows, dtype=torch.int32, device="cuda")
+    device = torch.tensor(logits, device="cuda")
+
+    def tokens(first, count):
+        out = torch.full((count,), -1, dtype=torch.int32, device="cuda")
+        k.sample(device[first:first + count], out, 0.9, top_k, 0.95, 7, streams[first:first + count], streams[first:first + count])
+        return out
+
+    whole = tokens(0, rows)
+    for count in (1, 3, 16, 17, 60, 130):
+        assert torch.equal(tokens(rows - count, count), whole[rows - count:]), count
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for place in (0, vocab // 2 - 1, vocab // 2 + 1, vocab - 1):
+        row = device[:1].clone()
+        row[0, place] = float("nan")
+        out = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+        flag.zero_()
+        k.sample(row, out, 0.9, top_k, 0.95, 7, streams[:1], streams[:1], flag)
+        assert int(flag) == 2 and int(out) == 0, place
