@@ -308,9 +308,10 @@ constexpr int FEW_K = 256;
 constexpr int FEW_LOADS = 8;           // 16-byte loads a thread keeps on its way in a walk (4: 44 us for those 64 rows out of HBM, 8: 28)
 
 // The rows it is taken for: a thread walks four neighbouring logits at a time, so that rows shorter than 4 x top_k leave fewer maxima
-// than k and all of the row on the list, and counting costs more than passes over a short row: top-k 20 / 100 / 256 alone 13.5 / 15.6 /
-// 22 us over 1,000 logits here (11.3 in passes), 13.7 / 15.6 / 20 over 2,000 (13.9), 14.5 / 16.6 / 22 over 5,000 (22).  With a top-p the
-// passes go on for the cut: top-k 20 / 200 14 / 19 us over 1,000 (21 and 23), but 256 35 (23).
+// than k and all of the row on the list, and counting costs more than passes over a short row.  Eight rows, in us, with a top-p of 0.95
+// and top-k 20 / 100 / 200 / 256: 6.0 / 16.2 / 19.0 / 23 (in passes) over 1,000 logits, 6.3 / 9.4 / 17.8 / 19.4 over 2,000, 6.8 / 10.1 / 19.6 /
+// 20.9 over 5,000; in passes, without a top-p, 11 over 1,000 and 13.5 over 2,000.  (Where one thread is a group, from a top-k of 128 on,
+// the sharing of the counting costs about 1 us: 17.5 / 16.7 / 18.5 before for 200.  20 and 100: 13.5 to 14 and 15 to 16 before.)
 __host__ __device__ inline bool sample_few_serves(int vocab, int top_k, float top_p) {
     return top_k > 0 && top_k <= FEW_K && vocab >= (top_p < 1.0f ? 4 * top_k : 2000 + 10 * top_k);
 }
