@@ -329,21 +329,23 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * R;
     const int block_col = rank * SIDE_WARPS * COLS, col0 = block_col + warp * COLS;
-    // Few tokens: the chain of loads is all there is, so that everything which no kernel in front writes is in registers ahead of the
-    // wait: the table's numbers behind the ids, both weights, the norms' weights (in the step, width 32 on 2,048 at 8 tokens 9.0 -> 6.7 us, 64 at 4
-    // 10.5 -> 7.4).
+    // Few tokens: the chain of loads is all there is, so that the weights and the norms' weights, which no kernel in front writes, are in
+    // registers ahead of the wait.  The ids are not: a kernel in front may be the one that chooses them.  They are asked for first
+    // behind the wait, and their table entries as soon as the first products have been issued, two barriers ahead of their use.
     constexpr bool EARLY = MT == 1 && COLS <= 64;
     constexpr int EACH = R * DIM / (SIDE_WARPS * 32);                 // gated values a thread makes
     static_assert(R * DIM % (SIDE_WARPS * 32) == 0, "gated values a thread");
+    int id[EACH];
     float entry[EACH];
-    bool known[EACH];
+    auto known = [&](int n) { return id[n] >= 0 && id[n] < vocab; };  // (the embedding has flagged an id outside the table)
+    auto load_ids = [&]() {
+#pragma unroll
+        for (int n = 0; n < EACH; ++n) id[n] = ids[min(t0 + (tid + n * SIDE_WARPS * 32) / DIM, n_tokens - 1)];
+    };
     auto load_entries = [&]() {
 #pragma unroll
-        for (int n = 0; n < EACH; ++n) {
-            const int i = tid + n * SIDE_WARPS * 32, id = ids[min(t0 + i / DIM, n_tokens - 1)];
-            known[n] = id >= 0 && id < vocab;                         // (the embedding has flagged an id outside the table)
-            entry[n] = known[n] ? __bfloat162float(table[(size_t)id * table_stride + offset + i % DIM]) : 0.0f;
-        }
+        for (int n = 0; n < EACH; ++n)
+            entry[n] = known(n) ? __bfloat162float(table[(size_t)id[n] * table_stride + offset + (tid + n * SIDE_WARPS * 32) % DIM]) : 0.0f;
     };
     auto load_gate = [&](int c, uint4 (&w)[DIM / 8]) {
 #pragma unroll
@@ -360,20 +362,17 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     uint4 gate_early[EARLY ? COLS / 32 : 1][DIM / 8];
     uint32_t proj_early[EARLY ? DIM / 16 : 1][4][TILES / 2];
     float4 norm_early[EARLY ? TILES / 2 : 1], next_early[EARLY ? TILES / 2 : 1];
-    if (EARLY) {
-        load_entries();
-        if (col0 < hidden) {
+    if (EARLY && col0 < hidden) {
 #pragma unroll
-            for (int c = 0; c < COLS; c += 32) load_gate(c, gate_early[c / 32]);
+        for (int c = 0; c < COLS; c += 32) load_gate(c, gate_early[c / 32]);
 #pragma unroll
-            for (int k = 0; k < DIM; k += 16) load_proj(0, k, proj_early[k / 16]);
+        for (int k = 0; k < DIM; k += 16) load_proj(0, k, proj_early[k / 16]);
 #pragma unroll
-            for (int i = 0; i < TILES / 2; ++i) {
-                norm_early[i] = *(const float4*)(norm_w + col0 + 2 * TILES * t + 4 * i);
-                if (next_out) next_early[i] = *(const float4*)(next_gamma + col0 + 2 * TILES * t + 4 * i);
-            }
+        for (int i = 0; i < TILES / 2; ++i) {
+            norm_early[i] = *(const float4*)(norm_w + col0 + 2 * TILES * t + 4 * i);
+            if (next_out) next_early[i] = *(const float4*)(next_gamma + col0 + 2 * TILES * t + 4 * i);
         }
-    } else if (MT == 1) {
+    } else if (!EARLY && MT == 1) {
         constexpr int LINES = SIDE_WARPS * COLS * 2 / 128;             // 128-byte lines of a weight row in this block's columns
         for (int i = tid; i < 2 * DIM * LINES; i += SIDE_WARPS * 32) {
             const int c = block_col + (i % LINES) * 64, row = (i / LINES) % DIM;
@@ -383,6 +382,7 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     }
     pdl_launch_dependents();
     pdl_wait();
+    if (EARLY) load_ids();
     const float* rows[MT][2];
 #pragma unroll
     for (int m = 0; m < MT; ++m)
@@ -432,6 +432,7 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
                 *(float2*)(at + 8 * DIM) = make_float2(acc[m][n][2], acc[m][n][3]);
             }
     }
+    if (EARLY) load_entries();
     __syncthreads();
     for (int i = tid; i < R * DIM; i += SIDE_WARPS * 32) {
         float sum = part[i];
@@ -439,7 +440,10 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         for (int w = 1; w < SIDE_WARPS; ++w) sum += part[w * R * DIM + i];
         own[i] = sum;
     }
-    if (!EARLY) load_entries();
+    if (!EARLY) {
+        load_ids();
+        load_entries();
+    }
     side_cluster_sync();
 #pragma unroll
     for (int n = 0; n < EACH; ++n) {
@@ -447,7 +451,7 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
         float sum = 0.0f;
         for (int r = 0; r < ranks; ++r) sum += side_remote(own + i, r);
         uint32_t parts[3];
-        split3(known[n] ? gelu_tanh(sum) * entry[n] : 0.0f, 0.0f, parts);
+        split3(known(n) ? gelu_tanh(sum) * entry[n] : 0.0f, 0.0f, parts);
 #pragma unroll
         for (int s = 0; s < 3; ++s) gated[(s * R + i / DIM) * PITCH + i % DIM] = __ushort_as_bfloat16((unsigned short)parts[s]);
     }

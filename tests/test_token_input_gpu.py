@@ -43,3 +43,40 @@ def test_token_side_skips_an_unknown_id():
     ids = torch.tensor([2, -1, 7], dtype=torch.int32, device="cuda")
     k.token_side(x, ids, torch.randn(7, 32, device="cuda").bfloat16(), 0, 32, w, w, torch.ones(128, device="cuda"), 1e-5)
     assert torch.equal(x[1:], before[1:]) and not torch.equal(x[0], before[0])
+
+
+@pytest.mark.parametrize("hidden", [256, 4096])
+@pytest.mark.parametrize("choose", ["argmax", "sample"])
+def test_ids_chosen_by_the_kernels_in_front(hidden, choose):
+    """The chooser, the embedding and the token input one behind the other on a stream: each may start before the one in front has
+    finished, and none may read the ids before they are there."""
+    from stratakv_b200.ops import kernels_for
+    k = kernels_for(torch.bfloat16, 64, verbose=False)
+    n, dim, vocab = 8, 32, 100000
+    g = torch.Generator(device="cuda").manual_seed(3)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    logits, embedding, table = normal(n, vocab), normal(vocab, hidden).bfloat16(), normal(vocab, dim).bfloat16()
+    gate, proj_t, norm = normal(dim, hidden).bfloat16(), normal(dim, hidden).bfloat16(), torch.ones(hidden, device="cuda")
+    counters = torch.zeros(n, dtype=torch.int32, device="cuda")
+
+    def step(ids):
+        x = torch.empty(n, hidden, device="cuda")
+        if ids is not settled:
+            if choose == "argmax":
+                k.argmax(logits, ids)
+            else:
+                k.sample(logits, ids, 1.0, 1, 1.0, 0, counters, counters)
+        k.embed(embedding, ids, x)
+        k.token_side(x, ids, table, 0, dim, gate, proj_t, norm, 1e-5)
+        return x
+
+    settled = logits.argmax(-1).int()
+    torch.cuda.synchronize()
+    want, stale = step(settled), ((settled + 1) % vocab).int()
+    busy = torch.empty(1 << 28, device="cuda")
+    for _ in range(10):
+        ids = stale.clone()
+        torch.cuda.synchronize()
+        busy.add_(1.0)                                   # (the three launches queue up behind it)
+        assert torch.equal(step(ids), want)
+        assert torch.equal(ids, settled)
