@@ -436,11 +436,13 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // raise the maximum in use (and rescale what has been accumulated) only when it matters
             const bool raise = tile_max > used_max + RESCALE_MARGIN;
             // once the product of the previous tile has finished the output accumulator may be touched and the probabilities
-            // rewritten
-            if (j > 0) ok = a_wait(bar(B_PE), (j - 1) & 1, flag);
-            if (!ok) break;
-            if (j > 0 && __any_sync(0xffffffffu, raise)) {
+            // rewritten, both in tensor memory: the fence orders either behind the wait
+            if (j > 0) {
+                ok = a_wait(bar(B_PE), (j - 1) & 1, flag);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            if (j > 0 && __any_sync(0xffffffffu, raise)) {
                 const float corr = raise ? a_exp2(used_max - tile_max) : 1.0f;     // 0 if nothing was seen before
 #pragma unroll 1
                 for (int c = 0; c < AHD; c += 32) {

@@ -94,3 +94,20 @@ def test_rows_that_are_sampled_from_a_short_list(call, serves):
         pytest.skip("not compiled yet")
     vocab, top_k, top_p = call
     assert bool(ctypes.CDLL(str(path)).skv_sample_few_serves(vocab, top_k, ctypes.c_float(top_p))) == serves
+
+
+def test_tensor_memory_is_touched_behind_a_fence():
+    """What a barrier's phase tells of another thread's tensor-core work is ordered with this thread's accesses to tensor memory by a fence
+    on every path between the two: not one inside a branch.  (A missing one shows in no result: program order has held so far.)"""
+    text = re.sub(r"//[^\n]*", "", (build.CSRC / "attention_prefill_tc.cu").read_text().split("prefill_attention_tc_kernel(")[1])
+    waits = 0
+    for wait in re.finditer(r"a_wait\(bar\(", text):
+        depth = 0
+        for token in re.finditer(r"[{}]|tcgen05\.fence::after_thread_sync|a_wait\(|\ba_(?:ld|st|mma)\w*\(", text[wait.end():]):
+            word = token.group()
+            depth += (word == "{") - (word == "}")
+            if word == "a_wait(" or (word.startswith("tcgen05") and depth <= 0):
+                waits += word != "a_wait("
+                break
+            assert not re.match(r"a_(ld|st|mma)", word), text[wait.start():wait.end() + token.end()]
+    assert waits >= 5                                   # scores, probabilities, the products' ends
