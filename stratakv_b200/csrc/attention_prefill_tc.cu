@@ -549,17 +549,20 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             a_cluster_barrier();
             float top = -INFINITY, total = 0.0f;
             for (int from = 0; from < splits; ++from) top = fmaxf(top, rows[from * ABM + row].x);
+            // (a block none of whose keys the row sees has a sum of zero; one whose visible scores are all NaN has no maximum either, and its
+            // sum is NaN, which must reach the result.  So must a value that is not finite, however little it weighs)
             for (int from = 0; from < splits; ++from) {
                 const float2 r = rows[from * ABM + row];
-                if (r.x != -INFINITY) total += a_exp2(r.x - top) * r.y;
+                total += r.x != -INFINITY ? a_exp2(r.x - top) * r.y : r.y;
             }
-            const float weight = ok && used_max != -INFINITY ? a_exp2(used_max - top) : 0.0f;
+            const float weight = a_exp2(used_max - top);
+            const bool sees = ok && used_max != -INFINITY;                // (with no keys the output was never written)
             const int columns = AHD / splits, pitch = columns + 4;        // (the pitch spreads a warp's rows over the banks)
             float* inbox = (float*)(a_raw + A_INBOX_AT);                  // [splits][128][pitch]
             const uint32_t inbox_at = a_smem(inbox);
             for (int c = 0; c < AHD; c += 16) {
                 uint32_t v[16];
-                if (n_tiles > 0) {                                         // (with no keys the output was never written)
+                if (n_tiles > 0) {
                     a_ld16(tmem_o + lane_bits + (uint32_t)c, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 }
@@ -568,7 +571,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 for (int e = 0; e < 16; e += 4) {
                     float x[4];
 #pragma unroll
-                    for (int f = 0; f < 4; ++f) x[f] = weight > 0.0f ? __uint_as_float(v[e + f]) * weight : 0.0f;
+                    for (int f = 0; f < 4; ++f) x[f] = sees ? __uint_as_float(v[e + f]) * weight : 0.0f;
                     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * e), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
                 }
             }

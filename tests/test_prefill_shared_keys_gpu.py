@@ -53,3 +53,39 @@ def test_keys_shared_by_a_cluster(sequences, heads, kv_heads, dim, extras):
         # every probability is rounded to bfloat16 once (by up to 2^-8 of it), and so is the result; scores err by float sums of order one
         assert ((out[rows].double().view_as(want) - want).abs() <= 2.0 ** -8 * (want.abs() + size) * 1.01 + 1e-5).all()
     assert int(k.error_flag) == 0
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("fault", ["key", "query with a sink", "value beyond reach"])
+def test_what_is_not_finite_is_not_lost_in_a_merge(dim, fault):
+    """Four pieces a query tile.  A NaN key is the only one that its own row sees of its piece (the pieces of the first two tiles are
+    single tiles of 64 keys); a NaN query makes all pieces' scores NaN; a value of infinity is reached with weights that vanish."""
+    from stratakv_b200.ops import kernels_for
+    k, block, n, heads, kv_heads = kernels_for(torch.bfloat16, dim, verbose=False), 64, 2100, 2, 1
+    blocks = -(-n // block)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda").bfloat16()
+    keys, values, q = normal(blocks, kv_heads, block, dim), normal(blocks, kv_heads, block, dim), normal(n, heads * dim)
+    table = torch.arange(blocks, dtype=torch.int32, device="cuda")[None]
+    cu_q, after = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, n], [n]))
+    sink = None
+    if fault == "key":
+        first = 192
+        keys[first // block, 0, first % block] = math.nan
+        bad = slice(first, n)
+    elif fault == "query with a sink":
+        first, sink = 300, torch.zeros(heads, device="cuda")
+        q[first] = math.nan
+        bad = slice(first, first + 1)
+    else:
+        first = 0                                            # (0 x infinity spoils the rows ahead of it in its tile as well)
+        q.fill_(1.0)
+        keys.fill_(1.0)
+        keys[0].fill_(-1.0)                                  # the first piece's weights are 2^-180 and less beyond its own tile
+        values[0, 0, first] = math.inf
+        bad = slice(first, n)
+    out = torch.zeros(n, heads * dim, device="cuda").bfloat16()
+    k.attention_prefill_tc(q, keys, values, table, cu_q, after, out, n, heads, kv_heads, dim, block, 1.0, sink=sink)
+    wrong = torch.ones(n, dtype=torch.bool, device="cuda")
+    wrong[bad] = False
+    assert not out[bad].isfinite().all(-1).any() and out[wrong].isfinite().all()
