@@ -420,14 +420,13 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
                 corr[r] = new_max == -INFINITY ? 1.0f : f_exp2(row_max[r] - new_max);
                 row_max[r] = new_max;
             }
+            // (nothing seen yet: a score of -infinity weighs nothing against any offset, and one that is NaN stays NaN)
+            const float offset[2] = {row_max[0] == -INFINITY ? 0.0f : row_max[0], row_max[1] == -INFINITY ? 0.0f : row_max[1]};
             float p[2][4];
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float m = row_max[e >> 1];
-                    p[t][e] = m == -INFINITY ? 0.0f : f_exp2(s[t][e] - m);
-                }
+                for (int e = 0; e < 4; ++e) p[t][e] = f_exp2(s[t][e] - offset[e >> 1]);
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r)
@@ -479,7 +478,8 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
     f_cluster_wait();                                 // every block of the cluster runs: its shared memory may be written
 
     // Merge the warps, and push each row to the block that owns it: row r belongs to block r % blocks and
-    // lands in that block's inbox at [(r / blocks) * blocks + this block's rank].
+    // lands in that block's inbox at [(r / blocks) * blocks + this block's rank].  What has no maximum has a weight of zero and sums of
+    // zero, or sums of NaN, where all of its scores are NaN: those go on into the result.
     const int rank = (int)f_cluster_rank(), blocks = (int)f_cluster_size();
     const uint32_t inbox_local = smem + F_INBOX_AT;
     for (int idx = threadIdx.x; idx < rows * FPITCH; idx += FTHREADS) {
@@ -490,12 +490,11 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
         float value = m;
         if (d != FHD) {
             value = 0.0f;
-            if (m != -INFINITY) {
+            const float top = m == -INFINITY ? 0.0f : m;
 #pragma unroll
-                for (int w = 0; w < FWARPS; ++w) {
-                    const float* tile = partial + ((size_t)w * 16 + r) * FPITCH;
-                    value += f_exp2(tile[FHD] - m) * tile[d];      // column FHD+1 (the sums) is weighted the same way
-                }
+            for (int w = 0; w < FWARPS; ++w) {
+                const float* tile = partial + ((size_t)w * 16 + r) * FPITCH;
+                value += f_exp2(tile[FHD] - top) * tile[d];        // column FHD+1 (the sums) is weighted the same way
             }
         }
         const int slot = (r / blocks) * blocks + rank;
@@ -510,11 +509,10 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
         const float* slots = inbox + (size_t)mine_index * blocks * FPITCH;
         float m = -INFINITY;
         for (int b = 0; b < blocks; ++b) m = fmaxf(m, slots[b * FPITCH + FHD]);
+        const float top = m == -INFINITY ? 0.0f : m;
         float total = 0.0f, sum = 0.0f;
         for (int b = 0; b < blocks; ++b) {
-            const float mb = slots[b * FPITCH + FHD];
-            if (mb == -INFINITY) continue;
-            const float weight = f_exp2(mb - m);
+            const float weight = f_exp2(slots[b * FPITCH + FHD] - top);
             total += weight * slots[b * FPITCH + d];
             sum += weight * slots[b * FPITCH + FHD + 1];
         }

@@ -59,3 +59,16 @@ def test_bias_by_distance(heads, kv_heads, lengths, window, reach, splits):
     k.attention_decode(setup["q"].view(n, -1), setup["k_cache"], setup["v_cache"], setup["table"], ctx, other, heads, kv_heads, head_dim, 64,
                        scale, window, 1, bias=bias)
     close(out, other, dtype)
+
+
+@pytest.mark.parametrize("head_dim,length", [(64, 4097), (64, 4200), (128, 4097)])
+def test_a_nan_is_not_lost_among_sixteen_pieces(head_dim, length):
+    """The newest key alone makes its warp's scores of a piece, and it is NaN: so is the result."""
+    dtype, heads, kv_heads, block_size = torch.bfloat16, 8, 2, 64
+    k = lib(dtype, head_dim)
+    setup, qkv, table, _ = _fused_decode_case(dtype, [length], heads, kv_heads, head_dim, block_size, seed=1)
+    qkv[0, heads * head_dim:(heads + 1) * head_dim] = math.nan                    # the key of the first key head
+    out = torch.zeros(1, heads, head_dim, device="cuda").to(dtype)
+    k.attention_decode_fused(qkv, table, setup["k_cache"], setup["v_cache"], setup["table"], torch.tensor([length], dtype=torch.int32, device="cuda"),
+                             out.view(1, -1), heads, kv_heads, head_dim, block_size, 0.1, 0, 8, True)
+    assert out[0, :heads // 2].isnan().all() and out[0, heads // 2:].isfinite().all()
