@@ -311,8 +311,8 @@ __device__ __forceinline__ float side_remote(const float* p, int rank) {
     return v;
 }
 
-template <int DIM, int COLS, int MT>
-__global__ void __launch_bounds__(SIDE_WARPS * 32)
+template <int DIM, int COLS, int MT, bool ROOMY>
+__global__ void __launch_bounds__(SIDE_WARPS * 32, ROOMY && (MT == 2 || DIM * COLS >= 32 * 64) ? 1 : 2)
 token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                       int table_stride, int offset, int vocab, const __nv_bfloat16* __restrict__ gate_w,
                       const __nv_bfloat16* __restrict__ proj_t, const float* __restrict__ norm_w, float eps,
@@ -329,10 +329,10 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * R;
     const int block_col = rank * SIDE_WARPS * COLS, col0 = block_col + warp * COLS;
-    // Few tokens: the chain of loads is all there is, so that the weights and the norms' weights, which no kernel in front writes, are in
-    // registers ahead of the wait.  The ids are not: a kernel in front may be the one that chooses them.  They are asked for first
+    // Few tokens: the chain of loads is all there is, so that the weights and the norms' weights, which no kernel in front writes,
+    // are in registers ahead of the wait.  The ids are not: a kernel in front may be the one that chooses them.  They are asked for first
     // behind the wait, and their table entries as soon as the first products have been issued, two barriers ahead of their use.
-    constexpr bool EARLY = MT == 1 && COLS <= 64;
+    constexpr bool EARLY = ROOMY && MT == 1 && COLS <= 64;
     constexpr int EACH = R * DIM / (SIDE_WARPS * 32);                 // gated values a thread makes
     static_assert(R * DIM % (SIDE_WARPS * 32) == 0, "gated values a thread");
     int id[EACH];
@@ -588,15 +588,15 @@ token_side_mma_kernel(float* __restrict__ x, const int* __restrict__ ids, const 
     side_cluster_sync();                                              // no block leaves while another reads its sums
 }
 
-template <int DIM, int COLS, int MT>
+template <int DIM, int COLS, int MT, bool ROOMY>
 static int launch_token_side_mma(float* x, const int* ids, const void* table, int table_stride, int offset, int vocab,
                                  const void* gate_w, const void* proj_t, const float* norm_w, float eps,
                                  const float* next_gamma, float next_eps, void* next_out, int n_tokens, int hidden,
                                  cudaStream_t stream) {
     constexpr int R = 16 * MT;
     constexpr size_t smem = (size_t)((SIDE_WARPS + 1) * R * DIM + (SIDE_WARPS + 3) * R) * 4 + (size_t)3 * R * (DIM + 8) * 2;
-    auto kernel = token_side_mma_kernel<DIM, COLS, MT>;
-    if (int code = reserve_shared_once<token_side_mma_kernel<DIM, COLS, MT>>("skv_token_side", smem)) return code;
+    auto kernel = token_side_mma_kernel<DIM, COLS, MT, ROOMY>;
+    if (int code = reserve_shared_once<token_side_mma_kernel<DIM, COLS, MT, ROOMY>>("skv_token_side", smem)) return code;
     const int ranks = (hidden + SIDE_WARPS * COLS - 1) / (SIDE_WARPS * COLS);
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(ranks * ((n_tokens + R - 1) / R)));
@@ -617,6 +617,24 @@ static int launch_token_side_mma(float* x, const int* ids, const void* table, in
                                                   next_eps, (__nv_bfloat16*)next_out, n_tokens, hidden, ranks);
     if (status != cudaSuccess) return fail("skv_token_side", cudaGetErrorString(status));
     return 0;
+}
+
+// At most 256 tokens.  With as many registers as they ask for (they hold weights ahead of the wait) the forms below take up to 128, and two
+// blocks share an SM, or up to 255 and have it to themselves.  The latter are the faster ones while all clusters run at once, which fifteen of eight
+// blocks do and sixteen don't (a partition of the GPU leaves some of its SMs over): 240 tokens with / with at most 128 registers, width 64 on
+// 2,048 10.4 / 14.1 us, 32 on 8,192 17.9 / 23.5; 256 tokens 19.5 / 13.6 and 34.6 / 24.4.  (Width 64 on more than 4,096 takes more than 128 without such weights.)
+template <int DIM, int COLS>
+static int launch_token_side_few(float* x, const int* ids, const void* table, int table_stride, int offset, int vocab,
+                                 const void* gate_w, const void* proj_t, const float* norm_w, float eps,
+                                 const float* next_gamma, float next_eps, void* next_out, int n_tokens, int hidden,
+                                 cudaStream_t stream) {
+    const int ranks = (hidden + SIDE_WARPS * COLS - 1) / (SIDE_WARPS * COLS), clusters = (n_tokens + 15) / 16;
+    if constexpr (DIM * COLS >= 32 * 64 && DIM * COLS < 64 * 128)
+        if (ranks * clusters > sm_count() - sm_count() / 6)
+            return launch_token_side_mma<DIM, COLS, 1, false>(x, ids, table, table_stride, offset, vocab, gate_w, proj_t, norm_w, eps,
+                                                              next_gamma, next_eps, next_out, n_tokens, hidden, stream);
+    return launch_token_side_mma<DIM, COLS, 1, true>(x, ids, table, table_stride, offset, vocab, gate_w, proj_t, norm_w, eps, next_gamma,
+                                                     next_eps, next_out, n_tokens, hidden, stream);
 }
 #endif
 
@@ -664,13 +682,13 @@ SKV_EXPORT int skv_token_side(float* x, const int* ids, const void* table, int t
     // 16-byte rows, nothing to add first
     if (!branch && (dim == 16 || dim == 32 || dim == 64) && hidden % 64 == 0 && hidden <= 8 * SIDE_WARPS * 128 &&
         (((uintptr_t)x | (uintptr_t)gate_w | (uintptr_t)proj_t | (uintptr_t)norm_w | (uintptr_t)next_gamma | (uintptr_t)next_out) & 15) == 0) {
-#define SKV_SIDE_MMA(DIM, COLS, MT) launch_token_side_mma<DIM, COLS, MT>(x, ids, table, table_stride, offset, vocab, gate_w, proj_t, norm_w, \
-                                                                       eps, next_gamma, next_eps, next_out, n_tokens, hidden, stream)
-#define SKV_SIDE_DIM(DIM) (n_tokens > 256 ? SKV_SIDE_MMA(DIM, 128, 2) : hidden <= 8 * SIDE_WARPS * 32 ? SKV_SIDE_MMA(DIM, 32, 1) : \
-                           hidden <= 8 * SIDE_WARPS * 64 ? SKV_SIDE_MMA(DIM, 64, 1) : SKV_SIDE_MMA(DIM, 128, 1))
+#define SKV_SIDE_ARGS x, ids, table, table_stride, offset, vocab, gate_w, proj_t, norm_w, eps, next_gamma, next_eps, next_out, n_tokens, hidden, stream
+#define SKV_SIDE_DIM(DIM) (n_tokens > 256 ? launch_token_side_mma<DIM, 128, 2, true>(SKV_SIDE_ARGS) :                       \
+                           hidden <= 8 * SIDE_WARPS * 32 ? launch_token_side_few<DIM, 32>(SKV_SIDE_ARGS) :                  \
+                           hidden <= 8 * SIDE_WARPS * 64 ? launch_token_side_few<DIM, 64>(SKV_SIDE_ARGS) : launch_token_side_few<DIM, 128>(SKV_SIDE_ARGS))
         return dim == 64 ? SKV_SIDE_DIM(64) : dim == 32 ? SKV_SIDE_DIM(32) : SKV_SIDE_DIM(16);
 #undef SKV_SIDE_DIM
-#undef SKV_SIDE_MMA
+#undef SKV_SIDE_ARGS
     }
 #endif
     const bool vec = hidden % 4 == 0 && (((uintptr_t)x | (uintptr_t)gate_w) & 15) == 0 && sizeof(skv_t) * hidden % 8 == 0;

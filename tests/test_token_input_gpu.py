@@ -34,6 +34,13 @@ def test_token_side_on_tensor_cores(dim, hidden, n, next_norm):
         assert ((out.double() - normed).abs() <= 2.0 ** -8 * normed.abs() + 2e-5).all()
 
 
+# the last count whose clusters all have SMs to themselves, the first that takes the form of fewer registers, and the most
+@pytest.mark.parametrize("dim,hidden", [(64, 2048), (32, 4096), (32, 8192), (64, 4096)])
+@pytest.mark.parametrize("n", [240, 241, 256])
+def test_token_side_where_two_blocks_share_an_sm(dim, hidden, n):
+    test_token_side_on_tensor_cores(dim, hidden, n, True)
+
+
 def test_token_side_skips_an_unknown_id():
     from stratakv_b200.ops import kernels_for
     k = kernels_for(torch.bfloat16, 64, verbose=False)
