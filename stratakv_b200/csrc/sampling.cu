@@ -6,6 +6,8 @@
 // equals (src/generation/sampler.cpp:58-62).
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace skv {
 
 // One block per row.  flag |= 2 if a logit of the row is NaN or infinite
@@ -293,36 +295,36 @@ __device__ unsigned long long radix_select(const float* __restrict__ row, const 
 }
 
 // A top-k of at most FEW_K: the row is walked twice and the rest happens on a short list.
-// The k-th largest of the threads' own maxima is a bound below which none of the k largest logits can lie (k threads
-// hold one that is not below it), so the second walk writes down what reaches the bound: about 43 elements for k = 40,
-// 253 for k = 200.  Their order, the top-p cut and the draw come from counting: a thread per element counts the keys
+// The k-th largest of the maxima of groups of threads is a bound below which none of the k largest logits can lie (k groups
+// hold one that is not below it), so the second walk writes down what reaches the bound: about 48 elements for k = 40 (128 groups),
+// 253 for k = 200 (a thread a group).  Their order, the top-p cut and the draw come from counting: a thread per element counts the keys
 // above its own.  The masses, the cuts and the drawn number are those of the general path, integer for integer.
 // Bound by the two walks (the row comes from L2 or HBM once each, 16 bytes a load, no division but for what reaches
 // the bound), which the blocks of a cluster share out where rows are few, and by about 6 us of short steps one behind the
 // other.  64 rows of 128,256 logits with k = 40, p = 0.95: the general path's fourteen passes took 389 us, one block a row that
-// counted 512 maxima 29.0, now 19.8 (1 row 24.2 and 12.7; 8 rows of 32,000 17.0 and 10.3; 8 of 50,257, whose rows lie off 16-byte
-// boundaries and were read 4 bytes at a time, 35.6 and 10.9).
+// counted 512 maxima 25.3, now 16.4 (1 row 24.2 and 12.7; 8 rows of 32,000 17.0 and 10.6; 8 of 50,257, whose rows lie off 16-byte
+// boundaries and were read 4 bytes at a time, 35.6 and 11.6).
 // Returns false where the list would not hold the candidates (more than SAMPLE_THREADS equal values at the bound) or
 // where the quotients lie so near zero that they lose bits (then the bound on x says nothing about x / temperature).
 constexpr int FEW_K = 256;
 constexpr int FEW_LOADS = 8;           // 16-byte loads a thread keeps on its way in a walk (4: 44 us for those 64 rows out of HBM, 8: 28)
 
 // The rows it is taken for: a thread walks four neighbouring logits at a time, so that rows shorter than 4 x top_k leave fewer maxima
-// than k and all of the row on the list, and counting costs more than passes over a short row.  Eight rows, in us, with a top-p of 0.95
-// and top-k 20 / 100 / 200 / 256: 6.0 / 16.2 / 19.0 / 23 (in passes) over 1,000 logits, 6.3 / 9.4 / 17.8 / 19.4 over 2,000, 6.8 / 10.1 / 19.6 /
-// 20.9 over 5,000; in passes, without a top-p, 11 over 1,000 and 13.5 over 2,000.  (Where one thread is a group, from a top-k of 128 on,
-// the sharing of the counting costs about 1 us: 17.5 / 16.7 / 18.5 before for 200.  20 and 100: 13.5 to 14 and 15 to 16 before.)
+// than k and all of the row on the list, and counting costs more than passes over a short row.  Eight rows, in us, with a top-p and
+// top-k 40 / 129 / 200: 7.7 / 15.3 / 17.4 over 1,000 logits (256: 23 in passes), 7.2 / 16.4 / 17.6 over 5,000; without a top-p, top-k 256, 11.2
+// over 1,000 in passes and 20.8 over 5,000 here (in passes 13.5 over 2,000).
 __host__ __device__ inline bool sample_few_serves(int vocab, int top_k, float top_p) {
     return top_k > 0 && top_k <= FEW_K && vocab >= (top_p < 1.0f ? 4 * top_k : 2000 + 10 * top_k);
 }
 
 // Blocks that share a row: while the GPU has an SM for each (a tenth fewer: clusters do not fill every partition of it), what they list
 // fits, and a block's part is long enough to pay for the exchange of bounds, which takes about 2 us.  One row of 128,256 logits (top-k
-// 40, top-p 0.95) 12.7 us over eight blocks, 64 rows 19.8 over two each; 100 rows, one block each, 22.8.  64 rows of 16,384 took 9.8 us
-// over two blocks each and 8.6 over one.
+// 40, top-p 0.95) 12.7 us over eight blocks, 64 rows 16.4 over two each; 100 rows, one block each, 22.8.  64 rows of 16,384 took 9.8 us
+// over two blocks each and 8.6 over one.  Not beyond a top-k of 128, where a bound takes all 512 maxima and the lists to be ordered are long: 64 rows
+// of 32,000, top-k 129, 23.1 us over two blocks each and 21.3 over one.
 __host__ __device__ inline int sample_few_ranks(int rows, int vocab, int top_k, int slots) {
     int ranks = 1;
-    while (ranks < 8 && rows * ranks * 2 <= slots - slots / 10 && 2 * ranks * top_k <= SAMPLE_THREADS / 8 * 5 && vocab / (2 * ranks) >= 12000) ranks *= 2;
+    while (ranks < 8 && top_k <= 128 && rows * ranks * 2 <= slots - slots / 10 && 2 * ranks * top_k <= SAMPLE_THREADS / 8 * 5 && vocab / (2 * ranks) >= 12000) ranks *= 2;
     return ranks;
 }
 
@@ -342,9 +344,11 @@ __device__ __forceinline__ uint32_t in_rank(const void* p, int rank) {
 
 // With `ranks` > 1 the blocks of a cluster share the row out; rank 0 goes on alone behind the second walk, and the other ranks
 // return true whatever becomes of the row.
+template <bool SHARED>
 __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out, int vocab, float temperature, int top_k, float top_p,
                            unsigned long long seed, uint32_t stream, uint32_t counter, int* __restrict__ flag, unsigned char* smem,
-                           int ranks, int part) {
+                           int of_cluster, int rank_of_cluster) {
+    const int ranks = SHARED ? of_cluster : 1, part = SHARED ? rank_of_cluster : 0;         // (known to the compiler where a block has the row alone)
     float* maxima = (float*)smem;                                                          // [threads]
     unsigned long long* keys = (unsigned long long*)(smem + SAMPLE_THREADS * 4);            // [threads], in list order
     unsigned long long* sorted = keys + SAMPLE_THREADS;                                     // [threads], largest first
@@ -395,13 +399,20 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
     const float warp_largest = warp_max(largest);
     if (lane == 0) atomicMax((unsigned int*)&extent[1], __float_as_uint(warp_largest));     // (not negative: ordered as integers)
     int above = 0, not_below = 0;
-    for (int i = 4 * (tid & (lanes - 1)); i < groups; i += 4 * lanes) {
-        const float4 o = *(const float4*)(maxima + i);
-        above += (o.x > most) + (o.y > most) + (o.z > most) + (o.w > most);
-        not_below += (o.x >= most) + (o.y >= most) + (o.z >= most) + (o.w >= most);
-    }
-    if (lanes > 1) { above += __shfl_xor_sync(0xffffffffu, above, 1); not_below += __shfl_xor_sync(0xffffffffu, not_below, 1); }
-    if (lanes > 2) { above += __shfl_xor_sync(0xffffffffu, above, 2); not_below += __shfl_xor_sync(0xffffffffu, not_below, 2); }
+    auto count_maxima = [&](auto of) {                      // (with the step known to the compiler: 1,000 logits, top-k 129, 17.2 us without and 16.0 so)
+        constexpr int LANES = decltype(of)::value;
+#pragma unroll 8
+        for (int i = 0; i < SAMPLE_THREADS / LANES; i += 4 * LANES) {
+            const float4 o = *(const float4*)(maxima + i + 4 * (tid & (LANES - 1)));
+            above += (o.x > most) + (o.y > most) + (o.z > most) + (o.w > most);
+            not_below += (o.x >= most) + (o.y >= most) + (o.z >= most) + (o.w >= most);
+        }
+#pragma unroll
+        for (int o = 1; o < LANES; o *= 2) { above += __shfl_xor_sync(0xffffffffu, above, o); not_below += __shfl_xor_sync(0xffffffffu, not_below, o); }
+    };
+    if (lanes == 4) count_maxima(std::integral_constant<int, 4>{});
+    else if (lanes == 2) count_maxima(std::integral_constant<int, 2>{});
+    else count_maxima(std::integral_constant<int, 1>{});
     if (above < top_k && not_below >= top_k) { bound = most; at_bound = not_below - above; }    // (all who write write the same)
     if (above == 0) extent[0] = most;
     __syncthreads();
@@ -553,6 +564,7 @@ __device__ bool sample_few(const float* __restrict__ row, int* __restrict__ out,
 
 // Two blocks an SM, where their rows fit its shared memory: left to itself the short list takes 93 registers a thread, and with one
 // block an SM 296 rows of 50,257 logits with top-p alone took 710 us in place of 439.
+template <bool SHARED>
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab, float temperature, int top_k,
               float top_p, unsigned long long seed, const int* __restrict__ streams,
@@ -572,11 +584,11 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
     __shared__ int bad_flag;
     pdl_launch_dependents();
     pdl_wait();
-    const int at = blockIdx.x / ranks;                     // (blocks of a cluster share a row)
+    const int at = SHARED ? blockIdx.x / ranks : blockIdx.x;                     // (blocks of a cluster share a row)
     const float* row = logits + (size_t)at * vocab;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (sample_few_serves(vocab, top_k, top_p) &&
-        sample_few(row, out + at, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[at], (uint32_t)counters[at], flag, sample_smem,
+        sample_few<SHARED>(row, out + at, vocab, temperature, top_k, top_p, seed, (uint32_t)streams[at], (uint32_t)counters[at], flag, sample_smem,
                    ranks, (int)blockIdx.x - at * ranks))
         return;
     if (threadIdx.x == 0) bad_flag = 0;
@@ -700,12 +712,17 @@ sample_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab
 // Whether such a call chooses from a short list.
 SKV_EXPORT int skv_sample_few_serves(int vocab, int top_k, float top_p) { return sample_few_serves(vocab, top_k, top_p); }
 
+// Blocks that share a row in such a call on a GPU of `slots` SMs (1 also where the call does not choose from a short list).
+SKV_EXPORT int skv_sample_few_ranks(int rows, int vocab, int top_k, float top_p, int slots) {
+    return sample_few_serves(vocab, top_k, top_p) ? sample_few_ranks(rows, vocab, top_k, slots) : 1;
+}
+
 // Blocks of the sampling kernel that an SM holds, with as much dynamic shared memory as rows too long to be staged take.
 SKV_EXPORT int skv_sample_blocks_per_sm() {
     const size_t histograms = (size_t)SAMPLE_WARPS * 256 * (sizeof(unsigned long long) + sizeof(unsigned int)) + (size_t)SAMPLE_CANDIDATES * sizeof(int);
     int blocks = 0;
-    if (cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(histograms + 152 * 1024)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, sample_kernel, SAMPLE_THREADS, histograms) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(sample_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(histograms + 152 * 1024)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, sample_kernel<false>, SAMPLE_THREADS, histograms) != cudaSuccess) return -1;
     return blocks;
 }
 
@@ -723,20 +740,20 @@ SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, fl
     const size_t histograms = (size_t)SAMPLE_WARPS * 256 * (sizeof(unsigned long long) + sizeof(unsigned int)) +
                               (size_t)SAMPLE_CANDIDATES * sizeof(int);      // 48 KB of histograms and 16 KB of indices
     const int staged = row_bytes <= 152 * 1024 ? 1 : 0;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t status = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        (int)(histograms + 152 * 1024));
-        if (status != cudaSuccess) return fail("skv_sample", cudaGetErrorString(status));
-        configured = true;
-    }
     const size_t smem = histograms + (staged ? row_bytes : 0), alone = 116 * 1024;
     const int ranks = sample_few_serves(vocab, top_k, top_p) ? sample_few_ranks(rows, vocab, top_k, sm_count()) : 1;
+    // Blocks that each have an SM take more than half of its memory: blocks of this launch that start while the one in front still runs would
+    // share SMs and leave others idle (128 rows of 50,257, top-k 40 and top-p 45 us, 36 so; 64 rows of 128,256 by two blocks each, top-k 129, 37.7
+    // and 29.2).  Sixteen clusters of eight do not fit the GPU so (16 rows of 128,256, top-k 40 16.9 us and 20.8): fifteen do.
+    const bool alone_fits = rows * ranks <= (ranks < 8 ? sm_count() : sm_count() - sm_count() / 6);
+    const size_t bytes = alone_fits && smem < alone ? alone : smem;
+    if (int code = reserve_shared_once<sample_kernel<false>>("skv_sample", histograms + 152 * 1024)) return code;
     if (ranks > 1) {
+        if (int code = reserve_shared_once<sample_kernel<true>>("skv_sample", histograms + 152 * 1024)) return code;
         cudaLaunchConfig_t config = {};
         config.gridDim = dim3((unsigned)(rows * ranks));
         config.blockDim = dim3(SAMPLE_THREADS);
-        config.dynamicSmemBytes = smem;
+        config.dynamicSmemBytes = bytes;
         config.stream = stream;
         cudaLaunchAttribute attributes[2];
         attributes[0].id = cudaLaunchAttributeClusterDimension;
@@ -746,13 +763,11 @@ SKV_EXPORT int skv_sample(const float* logits, int* out, int rows, int vocab, fl
         attributes[1].val.programmaticStreamSerializationAllowed = 1;
         config.attrs = attributes;
         config.numAttrs = pdl_enabled() ? 2 : 1;
-        const cudaError_t status = cudaLaunchKernelEx(&config, sample_kernel, logits, out, vocab, temperature, top_k, top_p, (unsigned long long)seed,
+        const cudaError_t status = cudaLaunchKernelEx(&config, sample_kernel<true>, logits, out, vocab, temperature, top_k, top_p, (unsigned long long)seed,
                                                       streams, counters, flag, staged, ranks);
         if (status != cudaSuccess) return fail("skv_sample", cudaGetErrorString(status));
         return 0;
     }
-    // Rows that fit the GPU's SMs one by one take more than half of an SM's memory each: blocks of this launch that start while the one
-    // in front still runs would share SMs and leave others idle (128 rows of 50,257, top-k 40 and top-p 45 us, 36 so).
-    return launch_pdl("skv_sample", sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), rows <= sm_count() && smem < alone ? alone : smem, stream, logits, out,
+    return launch_pdl("skv_sample", sample_kernel<false>, dim3(rows), dim3(SAMPLE_THREADS), bytes, stream, logits, out,
                       vocab, temperature, top_k, top_p, (unsigned long long)seed, streams, counters, flag, staged, 1);
 }

@@ -111,3 +111,15 @@ def test_tensor_memory_is_touched_behind_a_fence():
                 break
             assert not re.match(r"a_(ld|st|mma)", word), text[wait.start():wait.end() + token.end()]
     assert waits >= 5                                   # scores, probabilities, the products' ends
+
+
+# (rows, vocabulary, top-k): one row, as many as two blocks each leave SMs for, more; short rows; more than a shared list's top-k
+@pytest.mark.parametrize("call,ranks", [((1, 128256, 40), 8), ((1, 128256, 80), 4), ((1, 128256, 128), 2), ((1, 128256, 129), 1), ((64, 128256, 40), 2),
+                                        ((67, 128256, 40), 2), ((68, 128256, 40), 1), ((16, 128256, 40), 8), ((17, 128256, 40), 4), ((1, 23999, 1), 1), ((1, 24000, 1), 2),
+                                        ((1, 128256, 0), 1)])
+def test_blocks_that_share_a_row_of_logits(call, ranks):
+    path = build.find_built("bfloat16", 64)
+    if path is None:
+        pytest.skip("not compiled yet")
+    rows, vocab, top_k = call
+    assert ctypes.CDLL(str(path)).skv_sample_few_ranks(rows, vocab, top_k, ctypes.c_float(0.95), 148) == ranks

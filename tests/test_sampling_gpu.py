@@ -1,4 +1,5 @@
 """The sampling kernels against the distribution the reference's sampler draws from."""
+import ctypes
 import numpy as np
 import pytest
 import torch
@@ -176,7 +177,7 @@ def test_two_blocks_of_the_kernel_share_an_sm():
     assert kernels().lib.skv_sample_blocks_per_sm() >= 2
 
 
-@pytest.mark.parametrize("vocab,top_k", [(16384, 1), (32000, 40), (50257, 40), (65539, 97), (128256, 40), (128256, 256)])
+@pytest.mark.parametrize("vocab,top_k", [(24000, 1), (32000, 40), (50257, 40), (65539, 97), (128256, 40), (128256, 128)])
 @pytest.mark.parametrize("kind", ["plain", "ties", "masked", "one_part"])
 def test_blocks_that_share_a_row_draw_what_one_block_draws(vocab, top_k, kind):
     """A row of a small batch is walked by two, four or eight blocks, a row of a large one by one: the tokens are the same,
@@ -202,6 +203,8 @@ def test_blocks_that_share_a_row_draw_what_one_block_draws(vocab, top_k, kind):
         return out
 
     whole = tokens(0, rows)
+    ranks = lambda count: k.lib.skv_sample_few_ranks(count, vocab, top_k, ctypes.c_float(0.95), torch.cuda.get_device_properties(0).multi_processor_count)
+    assert ranks(rows) == 1 and ranks(1) > 1 and ranks(60) > 1
     for count in (1, 3, 16, 17, 60, 130):
         assert torch.equal(tokens(rows - count, count), whole[rows - count:]), count
     flag = torch.zeros(1, dtype=torch.int32, device="cuda")
