@@ -643,7 +643,15 @@ SKV_EXPORT int skv_attention_general(const void* q, const void* k_cache, const v
     }
 #endif
     auto kernel = vdim <= 256 ? attention_general_kernel<skv_t, 8> : attention_general_kernel<skv_t, 16>;
-    if (int code = launch_pdl("skv_attention_general", kernel, dim3((unsigned)blocks),
+    // A warp per (token, head) reads its keys straight through L1, where the heads of a key head find them: behind a projection whose weights wait
+    // in shared memory and whose blocks it overlapped it had 60 KB of L1 left.  8 sequences x 32 heads of 256 over 8 with their projection, 8 parts of 300
+    // / 2,000 keys: 92 / 304 us overlapping, 75 / 256 so; 32 heads of 96, 52 / 180 and 36 / 141.  (The float32 projections are as they were.)
+#if SKV_DTYPE == SKV_BF16
+    const auto launch = [&](auto... args) { return launch_alone(args...); };
+#else
+    const auto launch = [&](auto... args) { return launch_pdl(args...); };
+#endif
+    if (int code = launch("skv_attention_general", kernel, dim3((unsigned)blocks),
                               dim3(GEN_WARPS * 32), smem, stream, (const skv_t*)q, (const skv_t*)k_cache,
                               (const skv_t*)v_cache, block_table, table_width, positions, token_seq, (skv_t*)out, n_tokens,
                               num_heads, num_kv_heads, dim, vdim, block_size, scale, window, r1, r2, gate, gate_stride,

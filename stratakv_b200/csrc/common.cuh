@@ -82,6 +82,21 @@ inline int launch_pdl(const char* name, void (*kernel)(KernelArgs...), dim3 grid
     return 0;
 }
 
+// The same for a kernel that lives on L1: it starts when the kernel in front has left the SMs, whose shared memory then goes to L1.  Blocks that
+// start beside others find the division that those needed.
+template <typename... KernelArgs, typename... Args>
+inline int launch_alone(const char* name, void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem,
+                        cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    const cudaError_t status = cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+    if (status != cudaSuccess) return fail(name, cudaGetErrorString(status));
+    return 0;
+}
+
 // Number of SMs of the current device (asked once per process; a process drives one kind of GPU).
 inline int sm_count() {
     static const int count = [] {
