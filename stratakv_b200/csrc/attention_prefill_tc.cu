@@ -32,6 +32,7 @@
 
 #if SKV_DTYPE == SKV_BF16 && (SKV_HEAD_DIM == 64 || SKV_HEAD_DIM == 128)
 
+#include <atomic>
 #include <cuda.h>
 #include <mutex>
 #include <unordered_map>
@@ -622,6 +623,22 @@ static AEncode a_encoder() {
     return fn;
 }
 
+// Whether the compiler gave the kernels the registers that their warpgroups share out (the softmax's share is taken from what the block was
+// launched with): with another number its request would wait forever, and prompts go to attention_prefill.cu.  Without a GPU nobody can tell.
+static bool a_registers_fit() {
+    static std::atomic<int> known{-1};
+    if (known.load(std::memory_order_relaxed) < 0) {
+        cudaFuncAttributes plain, extras;
+        if (cudaFuncGetAttributes(&plain, prefill_attention_tc_kernel<false>) != cudaSuccess ||
+            cudaFuncGetAttributes(&extras, prefill_attention_tc_kernel<true>) != cudaSuccess) {
+            cudaGetLastError();
+            return true;
+        }
+        known.store(plain.numRegs == A_REGS && extras.numRegs == A_REGS, std::memory_order_relaxed);
+    }
+    return known.load(std::memory_order_relaxed) != 0;
+}
+
 // bfloat16 matrix [rows, cols] row-major, box of box_rows x 64 columns, 128-byte swizzle
 static int a_map(const void* base, long long rows, int cols, int box_rows, CUtensorMap* out) {
     struct Key { const void* base; long long rows; int cols, box; };
@@ -686,18 +703,9 @@ SKV_EXPORT int skv_attention_prefill_tc_extras(const void* q, const void* k_cach
     const long long blocks = (long long)n_seqs * tiles_per_seq;
     if (blocks > 65535) return fail("skv_attention_prefill_tc", "too many query tiles in one step (65,535 at most)");
     const size_t smem = (size_t)ACH * TILE_BYTES + (size_t)4 * ACH * KV_TILE_BYTES + B_COUNT * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        for (auto kernel : {prefill_attention_tc_kernel<false>, prefill_attention_tc_kernel<true>}) {
-            const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            cudaFuncAttributes attributes;
-            if (status != cudaSuccess || cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess)
-                return fail("skv_attention_prefill_tc", cudaGetErrorString(status));
-            // (the softmax's share is taken from what the block was launched with)
-            if (attributes.numRegs != A_REGS) return fail("skv_attention_prefill_tc", "built with another number of registers than the warpgroups share out");
-        }
-        configured = true;
-    }
+    if (!a_registers_fit()) return fail("skv_attention_prefill_tc", "built with another number of registers than the warpgroups share out");
+    if (int code = reserve_shared_once<prefill_attention_tc_kernel<false>>("skv_attention_prefill_tc", smem)) return code;
+    if (int code = reserve_shared_once<prefill_attention_tc_kernel<true>>("skv_attention_prefill_tc", smem)) return code;
     // Fewer query tiles than SMs over long contexts: their keys are shared out, which starts every block for less work and ends in a
     // merge (512 queries behind 4,096 others, 32 heads of 64, 128 blocks: 68.2 -> 44.0 us; 512 blocks 207 -> 212).
     const long long most_keys = (long long)table_width * block_size, keys = window > 0 && window + ABM < most_keys ? window + ABM : most_keys;
@@ -735,7 +743,7 @@ SKV_EXPORT int skv_attention_prefill_tc(const void* q, const void* k_cache, cons
                                            scale, window, nullptr, 0, nullptr, 0, 0.0f, 0, nullptr, flag, stream);
 }
 
-SKV_EXPORT int skv_has_attention_prefill_tc() { return 1; }
+SKV_EXPORT int skv_has_attention_prefill_tc() { return a_registers_fit(); }
 
 #else
 

@@ -1,8 +1,10 @@
 """What is compiled per head size, and that the libraries of one dtype share the rest."""
 import ctypes
 import re
+import subprocess
 
 import pytest
+import torch
 
 from stratakv_b200.csrc import build
 
@@ -111,6 +113,24 @@ def test_tensor_memory_is_touched_behind_a_fence():
                 break
             assert not re.match(r"a_(ld|st|mma)", word), text[wait.start():wait.end() + token.end()]
     assert waits >= 5                                   # scores, probabilities, the products' ends
+
+
+@pytest.mark.gpu
+def test_a_build_with_other_registers_leaves_prompts_to_the_other_kernel(tmp_path):
+    """The tensor-memory prompt kernel's warpgroups share out the registers that a block is launched with.  Where the compiler gives it another
+    number the library says that it has no such kernel, so that prompts go to the one without (nothing is launched here)."""
+    from stratakv_b200.ops import kernels_for
+    lib = kernels_for(torch.bfloat16, 64, verbose=False).lib
+    assert lib.skv_has_attention_prefill_tc() == 1
+    text = (build.CSRC / "attention_prefill_tc.cu").read_text()
+    assert text.count("A_REGS = 128") == 1
+    (tmp_path / "other.cu").write_text(text.replace("A_REGS = 128", "A_REGS = 120"))
+    folder = build.find_built("bfloat16", 64).parent
+    subprocess.run([build.find_nvcc(), *build.ARCH_FLAGS, *build.COMMON_FLAGS, "-shared", *build._defines("bfloat16", 64), f"-I{build.CSRC}",
+                    str(tmp_path / "other.cu"), "-o", str(tmp_path / "other.so"), "-L", str(folder),
+                    f"-l:{build.common_library_name('bfloat16')}", "-Xlinker", f"-rpath={folder}"], check=True)
+    other = ctypes.CDLL(str(tmp_path / "other.so"))
+    assert other.skv_has_attention_prefill_tc() == 0
 
 
 # (rows, vocabulary, top-k): one row, as many as two blocks each leave SMs for, more; short rows; more than a shared list's top-k
