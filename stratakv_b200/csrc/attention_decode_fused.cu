@@ -26,6 +26,8 @@
 //    scratch in global memory, no second kernel, no barrier after the merge.
 #include "head_size.cuh"
 
+#include <mutex>
+#include <vector>
 
 // Two stages of 128 keys and values must fit one block's shared memory, which holds for head sizes up
 // to 192; above that this kernel is not built and the separate kernels (elementwise.cu,
@@ -521,13 +523,34 @@ decode_attention_fused_kernel(const float* __restrict__ qkv, const float2* __res
     }
 }
 
+// How many clusters like this launch's the GPU runs at once.  A kernel, its shared memory and a device have one answer for good, so it is asked for
+// once (0.3 us of the host's time a launch otherwise) and an error of the caller's is not cleared with each launch.
+static int f_clusters_at_once(const void* kernel, const cudaLaunchConfig_t& config) {
+    struct Known { const void* kernel; size_t smem; int device, count; };
+    static std::mutex lock;
+    static std::vector<Known> known;                  // (two kernels, two to four stages)
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> guard(lock);
+    for (const Known& k : known)
+        if (k.kernel == kernel && k.smem == config.dynamicSmemBytes && k.device == device) return k.count;
+    int count = 0;
+    if (cudaOccupancyMaxActiveClusters(&count, kernel, &config) != cudaSuccess) {
+        cudaGetLastError();                           // (a refusal is an answer)
+        count = 0;
+    }
+    known.push_back({kernel, config.dynamicSmemBytes, device, count});
+    return count;
+}
+
 }  // namespace skv
 
 using namespace skv;
 
 // qkv: float [n_seqs, (heads + 2 kv_heads) * head_dim] (the q|k|v projection of each sequence's new
 // token); cos_sin: float [positions, head_dim/2, 2] or null; ctx_after[s]: keys cached for sequence s
-// once this token's key is in (so the token's position is ctx_after[s] - 1).  splits is 1..8.
+// once this token's key is in (so the token's position is ctx_after[s] - 1).  splits is 1..8; of 8 the launcher
+// makes 16 where that is faster (below).
 // The _extras form: rows of qkv are row_stride floats apart (0: exactly queries, keys and values); biases, the
 // value norm (value_norm != 0, head sizes up to 128), a bias table by distance and a gate as NewTokenFinish and
 // AttentionExtras say, each off when null or 0.
@@ -627,14 +650,11 @@ SKV_EXPORT int skv_attention_decode_fused_extras(const float* qkv, int row_strid
         wider.numAttrs = 1;
         const long long chunks = (most_keys / 16 + warps * 16 - 1) / (warps * 16);
         wider.dynamicSmemBytes = (size_t)F_STAGES_AT + (size_t)(chunks <= FMAX_STAGES && chunks <= room ? (chunks < 2 ? 2 : chunks) : 2) * stage_bytes;
-        int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, kernel, &wider) == cudaSuccess && fit >= clusters) {
+        if (f_clusters_at_once((const void*)kernel, wider) >= clusters) {
             splits = 16;
             stages = (int)((wider.dynamicSmemBytes - F_STAGES_AT) / stage_bytes);
             config.gridDim.z = attributes[0].val.clusterDim.z = 16;
             config.dynamicSmemBytes = wider.dynamicSmemBytes;
-        } else {
-            cudaGetLastError();                       // (a refusal is an answer, not an error of the caller's)
         }
     }
     const cudaError_t status = cudaLaunchKernelEx(
