@@ -430,7 +430,7 @@ struct NormArgs {
 
 // The three steps that the kernels below share.  First, what a folded norm's factors will be made from is sent for.
 template <int COLS>
-__device__ __forceinline__ void skinny_send_for_norm(float* staged, const NormArgs& norm, int m0, int M) {
+__device__ __forceinline__ void skinny_send_for_norm(float* staged, const NormArgs& norm, int M) {
     if (norm.partials_in) {
         // the partial sums are wanted after the main loop: they travel to shared memory meanwhile, 16 bytes
         // at a time where the rows allow it (the row in shared memory is `pitch` floats)
@@ -439,8 +439,8 @@ __device__ __forceinline__ void skinny_send_for_norm(float* staged, const NormAr
         const int pieces = wide ? pitch >> 2 : norm.n_partials_in;
         for (int i = threadIdx.x; i < COLS * pieces; i += blockDim.x) {
             const int m = i / pieces, piece = i - m * pieces;
-            if (m0 + m < M) {
-                const float* row = norm.partials_in + (size_t)(norm.rows ? norm.rows[m0 + m] : m0 + m) * norm.stride_in;
+            if (m < M) {
+                const float* row = norm.partials_in + (size_t)(norm.rows ? norm.rows[m] : m) * norm.stride_in;
                 if (wide)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(staged + m * pitch + 4 * piece)),
                                  "l"(row + 4 * piece) : "memory");
@@ -495,7 +495,7 @@ __device__ __forceinline__ void skinny_finish_partials(const NormArgs& norm, int
 // Last, the warps' partial tiles are added up and the result stored, rows n0 .. n0 + 15 of the weight.
 template <int TG>
 __device__ __forceinline__ void skinny_store(float* red, const float* factor, const float (&acc)[TG][4], void* __restrict__ out, int M,
-                                             int N, int n0, int m0, int mode, act_t act, const NormArgs& norm, int warps, int warp, int lane) {
+                                             int N, int n0, int mode, act_t act, const NormArgs& norm, int warps, int warp, int lane) {
     constexpr int COLS = 8 * TG, PITCH = COLS + 1;
     const int g = lane >> 2, tig = lane & 3;
     float* mine = red + (size_t)warp * 16 * PITCH;
@@ -512,7 +512,7 @@ __device__ __forceinline__ void skinny_store(float* red, const float* factor, co
         float sum = 0.0f;
         for (int w = 0; w < warps; ++w) sum += red[((size_t)w * 16 + r) * PITCH + m];
         if (norm.partials_in) sum *= factor[m];
-        else if (norm.row_scale && m0 + m < M) sum *= norm.row_scale[norm.rows ? norm.rows[m0 + m] : m0 + m];
+        else if (norm.row_scale && m < M) sum *= norm.row_scale[norm.rows ? norm.rows[m] : m];
         red[(size_t)r * PITCH + m] = sum;          // warp 0's tile becomes the total
         // (each (r, m) is read and written by this thread only)
     }
@@ -521,10 +521,10 @@ __device__ __forceinline__ void skinny_store(float* red, const float* factor, co
         const int half_n = N >> 1;
         for (int idx = threadIdx.x; idx < 8 * COLS; idx += blockDim.x) {
             const int r = idx & 7, m = idx >> 3;
-            const int o = (n0 >> 1) + r, gm = m0 + m;
-            if (gm < M && o < half_n) {
+            const int o = (n0 >> 1) + r;
+            if (m < M && o < half_n) {
                 const float gate = red[(size_t)r * PITCH + m], up = red[(size_t)(r + 8) * PITCH + m];
-                ((__nv_bfloat16*)out)[(size_t)gm * half_n + o] = __float2bfloat16_rn(gated_product(gate, up, act));
+                ((__nv_bfloat16*)out)[(size_t)m * half_n + o] = __float2bfloat16_rn(gated_product(gate, up, act));
             }
         }
     } else if (mode == MODE_ADD_F32 && norm.partials) {
@@ -532,22 +532,22 @@ __device__ __forceinline__ void skinny_store(float* red, const float* factor, co
         for (int idx = threadIdx.x; idx < 16 * COLS; idx += blockDim.x) {        // whole warps stay together
             const int r = idx & 15, m = idx >> 4;
             float updated = 0.0f;
-            if (m0 + m < M && n0 + r < N) {
-                float* at = (float*)out + (size_t)(m0 + m) * N + n0 + r;
+            if (m < M && n0 + r < N) {
+                float* at = (float*)out + (size_t)m * N + n0 + r;
                 updated = *at + red[(size_t)r * PITCH + m];
                 *at = updated;
-                norm.scaled_out[(size_t)(m0 + m) * N + n0 + r] = __float2bfloat16_rn(updated * norm.gamma_next[n0 + r]);
+                norm.scaled_out[(size_t)m * N + n0 + r] = __float2bfloat16_rn(updated * norm.gamma_next[n0 + r]);
             }
             float square = updated * updated;
 #pragma unroll
             for (int offset = 8; offset > 0; offset >>= 1) square += __shfl_xor_sync(0xffffffffu, square, offset);
-            if (r == 0 && m0 + m < M) norm.partials[(size_t)(m0 + m) * norm.partial_stride + blockIdx.x] = square;
+            if (r == 0 && m < M) norm.partials[(size_t)m * norm.partial_stride + blockIdx.x] = square;
         }
         if (norm.counter) skinny_finish_partials(norm, M, N, gridDim.x, warps, warp, lane);      // (one chunk of tokens: M <= 8*TG)
     } else {
         for (int idx = threadIdx.x; idx < 16 * COLS; idx += blockDim.x) {
             const int r = idx & 15, m = idx >> 4;
-            epilogue_store<__nv_bfloat16>(out, mode, M, N, m0 + m, n0 + r, red[(size_t)r * PITCH + m], act);
+            epilogue_store<__nv_bfloat16>(out, mode, M, N, m, n0 + r, red[(size_t)r * PITCH + m], act);
         }
     }
 }
@@ -567,7 +567,7 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tig = lane & 3;
-    const int n0 = blockIdx.x * 16, m0 = 0;
+    const int n0 = blockIdx.x * 16;
     const int steps = (K + 31) >> 5;
 
     const int row_a = min(n0 + g, N - 1), row_b = min(n0 + g + 8, N - 1);
@@ -593,14 +593,14 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
     bool has_x[TG];
 #pragma unroll
     for (int t = 0; t < TG; ++t) {
-        const int m = m0 + t * 8 + g;
+        const int m = t * 8 + g;
         has_x[t] = m < M;
         const int safe = min(m, M - 1);
         x_ptr[t] = X + (size_t)(norm.rows ? norm.rows[safe] : safe) * K + tig * 8;
     }
     float* factor = red + (size_t)warps * 16 * PITCH;
     float* staged = factor + COLS;
-    skinny_send_for_norm<COLS>(staged, norm, m0, M);
+    skinny_send_for_norm<COLS>(staged, norm, M);
     float acc[TG][4];
 #pragma unroll
     for (int t = 0; t < TG; ++t) { acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f; }
@@ -620,7 +620,7 @@ skinny_linear_bf16_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat
         }
     }
     skinny_norm_factors<COLS>(factor, staged, norm, K, warps, warp, lane);
-    skinny_store<TG>(red, factor, acc, out, M, N, n0, m0, mode, act, norm, warps, warp, lane);
+    skinny_store<TG>(red, factor, acc, out, M, N, n0, mode, act, norm, warps, warp, lane);
 }
 
 // At most 16 tokens: the weights stream by once, and on their way they wait in shared memory.  Such a projection is bound by HBM
@@ -824,9 +824,6 @@ static int launch_ring_as(const void* a, const void* w, void* out, int M, int N,
 template <int TG>
 static int launch_ring(const void* a, const void* w, void* out, int M, int N, int K, int mode, act_t act, const NormArgs& norm,
                        cudaStream_t stream) {
-    // (each block adds up all of its tokens' partial sums: wider rows are finished by their writer)
-    if (norm.partials_in && (4 * 16 * (8 * TG + 1) + 8 * TG + 8 * TG * ((norm.n_partials_in + 3) & ~3)) * sizeof(float) > 48 * 1024)
-        return fail("skv_linear(bfloat16)", "too many partial sums for the consumer: let the producer finish them");
     const int steps = (K + 31) / 32;
     if (TG == 1) {
         if (steps <= 4 * RING_WARPS) {

@@ -76,3 +76,18 @@ def check(M, N, K):
         want = torch.nn.functional.silu(g) * u
         assert ((gated.double() - want).abs() <= 1.2 * eg * u.abs() + torch.nn.functional.silu(g).abs() * eu + 2.0 ** -8 * want.abs() + 1e-6).all()
     assert int(k.error_flag) == 0
+
+
+@pytest.mark.parametrize("M,partials", [(1, 1464), (8, 2000), (8, 2001), (16, 1403)])
+def test_any_number_of_partial_sums(M, partials):
+    """A folded norm's factors from more partial sums than a block could stage: they are added up as they are read."""
+    from stratakv_b200 import ops
+    from stratakv_b200.residual import NormedRows
+    k, N, K, eps = ops.kernels_for(torch.bfloat16, 64, verbose=False), 2400, 1024, 1e-5
+    a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
+    sums = torch.rand(M, partials, device="cuda")
+    out = torch.full((M, N), float("nan"), device="cuda")
+    k.linear(NormedRows(a, torch.ones(M, device="cuda"), partials=sums, n_partials=partials, eps=eps), w, out, ops.MODE_STORE_F32)
+    factor = torch.rsqrt(sums.double().sum(-1, keepdim=True) / K + eps)
+    ref, bound = a.double() @ w.double().T * factor, a.double().abs() @ w.double().abs().T * factor
+    assert ((out.double() - ref).abs() <= 2e-6 * (1 + bound)).all()
