@@ -329,7 +329,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 for (int t = 0; t < 64; ++t) __nanosleep(1000);
             }
         } else if (warp == 1) {
-            // ---- values and output products: O += P_j . V_j once the probabilities and the values are in shared memory; then
+            // ---- values and output products: O += P_j . V_j once the probabilities are in tensor and the values in shared memory; then
             // the values of tile j + 1 are asked for, into the stage of tile j - 1: its product is complete, or the softmax could
             // not have written the probabilities of tile j where those of j - 1 lay.
             constexpr uint32_t idesc_o = a_idesc(ABM, 64, 1);
@@ -639,6 +639,16 @@ static bool a_registers_fit() {
     return known.load(std::memory_order_relaxed) != 0;
 }
 
+// Blocks that share a query tile's keys.  Fewer query tiles than SMs over long contexts (as long as the block tables have room for): their keys are shared
+// out, which starts every block for less work and ends in a merge (512 queries behind 4,096 others, 32 heads of 64, 128 blocks: 68.2 -> 44.0 us; 512
+// blocks 207 -> 212; from 512 keys on 200 queries behind 800, 24 heads of 128, 16.3 -> 21.7).
+static int a_splits(long long query_tiles, int heads, int table_width, int block_size, int window, int sms) {
+    const long long most_keys = (long long)table_width * block_size, keys = window > 0 && window + ABM < most_keys ? window + ABM : most_keys;
+    int splits = 1;
+    while (splits < A_MAX_SPLITS && query_tiles * heads * 2 * splits <= A_BLOCKS * sms && keys >= 1024 * splits) splits *= 2;
+    return splits;
+}
+
 // bfloat16 matrix [rows, cols] row-major, box of box_rows x 64 columns, 128-byte swizzle
 static int a_map(const void* base, long long rows, int cols, int box_rows, CUtensorMap* out) {
     struct Key { const void* base; long long rows; int cols, box; };
@@ -706,12 +716,7 @@ SKV_EXPORT int skv_attention_prefill_tc_extras(const void* q, const void* k_cach
     if (!a_registers_fit()) return fail("skv_attention_prefill_tc", "built with another number of registers than the warpgroups share out");
     if (int code = reserve_shared_once<prefill_attention_tc_kernel<false>>("skv_attention_prefill_tc", smem)) return code;
     if (int code = reserve_shared_once<prefill_attention_tc_kernel<true>>("skv_attention_prefill_tc", smem)) return code;
-    // Fewer query tiles than SMs over long contexts: their keys are shared out, which starts every block for less work and ends in a
-    // merge (512 queries behind 4,096 others, 32 heads of 64, 128 blocks: 68.2 -> 44.0 us; 512 blocks 207 -> 212).
-    const long long most_keys = (long long)table_width * block_size, keys = window > 0 && window + ABM < most_keys ? window + ABM : most_keys;
-    const long long tiles = blocks * num_heads;
-    int splits = 1;
-    while (splits < A_MAX_SPLITS && tiles * 2 * splits <= A_BLOCKS * sm_count() && keys >= 1024 * splits) splits *= 2;
+    const int splits = a_splits(blocks, num_heads, table_width, block_size, window, sm_count());
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(num_heads, (unsigned)blocks, splits);
     config.blockDim = dim3(ATHREADS);
@@ -744,6 +749,11 @@ SKV_EXPORT int skv_attention_prefill_tc(const void* q, const void* k_cache, cons
 }
 
 SKV_EXPORT int skv_has_attention_prefill_tc() { return a_registers_fit(); }
+
+// Blocks that share the keys of a query tile of such a call (`query_tiles`: sequences x tiles of 128 of the longest) on a GPU of `sms` SMs.
+SKV_EXPORT int skv_attention_prefill_tc_splits(int query_tiles, int heads, int table_width, int block_size, int window, int sms) {
+    return a_splits(query_tiles, heads, table_width, block_size, window, sms);
+}
 
 #else
 

@@ -143,3 +143,13 @@ def test_blocks_that_share_a_row_of_logits(call, ranks):
         pytest.skip("not compiled yet")
     rows, vocab, top_k = call
     assert ctypes.CDLL(str(path)).skv_sample_few_ranks(rows, vocab, top_k, ctypes.c_float(0.95), 148) == ranks
+
+
+# (query tiles, heads, table width, block size, window): few tiles over long tables, short tables, windows, more tiles
+@pytest.mark.parametrize("call,splits", [((1, 32, 32, 64, 0), 4), ((1, 32, 31, 64, 0), 2), ((1, 32, 15, 64, 0), 1), ((1, 32, 128, 64, 700), 1), ((1, 32, 128, 64, 896), 2),
+                                         ((1, 32, 128, 64, 1920), 4), ((4, 32, 128, 64, 0), 2), ((5, 32, 128, 64, 0), 1), ((2, 37, 128, 64, 0), 4), ((3, 25, 128, 64, 0), 2)])
+def test_blocks_that_share_a_query_tiles_keys(call, splits):
+    path = build.find_built("bfloat16", 64)
+    if path is None:
+        pytest.skip("not compiled yet")
+    assert ctypes.CDLL(str(path)).skv_attention_prefill_tc_splits(*call, 148) == splits

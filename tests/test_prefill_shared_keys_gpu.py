@@ -8,10 +8,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# (new tokens, context after) of the sequences: a cluster of two and of four (head counts below), contexts shorter than the pieces are many
+# (new tokens, context after) of the sequences: clusters of two and of four, contexts shorter than the pieces are many; windows that end inside tiles,
+# of two pieces and of four (whole pieces that a row does not see)
 @pytest.mark.parametrize("sequences", [[(100, 3100)], [(40, 1100), (33, 33)], [(200, 5000), (130, 130), (1, 64)]])
-@pytest.mark.parametrize("heads,kv_heads,dim", [(2, 1, 64), (40, 8, 64), (2, 2, 128), (40, 8, 128)])
-@pytest.mark.parametrize("extras", ["plain", "window", "sink cap gate", "bias gate per number"])
+@pytest.mark.parametrize("heads,kv_heads,dim", [(2, 1, 64), (20, 4, 64), (2, 2, 128), (20, 4, 128)])
+@pytest.mark.parametrize("extras", ["plain", "window 1001", "window 2101", "sink cap gate", "bias gate per number"])
 def test_keys_shared_by_a_cluster(sequences, heads, kv_heads, dim, extras):
     from stratakv_b200.ops import kernels_for
     k, block = kernels_for(torch.bfloat16, dim, verbose=False), 64
@@ -24,7 +25,10 @@ def test_keys_shared_by_a_cluster(sequences, heads, kv_heads, dim, extras):
     cu_q = torch.tensor([0] + [sum(q for q, _ in sequences[:i + 1]) for i in range(len(sequences))], dtype=torch.int32, device="cuda")
     after = torch.tensor([c for _, c in sequences], dtype=torch.int32, device="cuda")
     q, out = normal(n, heads * dim).bfloat16(), torch.full((n, heads * dim), float("nan"), device="cuda").bfloat16()
-    scale, window = 1.3 / math.sqrt(dim), 700 if extras == "window" else 0
+    scale, window = 1.3 / math.sqrt(dim), int(extras.split()[1]) if extras.startswith("window") else 0
+    tiles = len(sequences) * -(-max(t for t, _ in sequences) // 128)
+    splits = k.lib.skv_attention_prefill_tc_splits(tiles, heads, width, block, window, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert splits > 1 and (splits == 4 or tiles * heads > 74 or min(width * block, window + 128 if window else math.inf) < 2048)
     more, sink, gate, bias, cap = {}, None, None, None, 0.0
     if extras == "sink cap gate":
         sink, gate, cap = normal(heads), normal(n, heads), 20.0
