@@ -52,13 +52,15 @@ def fused_decode_splits(n_seqs: int, blocks_per_seq: int, max_ctx: int, sms: int
     return wanted
 
 
-def wants_more_pieces(n_seqs: int, blocks_per_seq: int, max_ctx: int, cluster_splits: int, sms: int) -> bool:
-    """A cluster holds at most 8 pieces of a context.  Few long sequences want more: when the fused kernel's
-    grid leaves SMs idle, its pieces are 2,048 keys or longer and the path through scratch memory would cut
-    at least twice as many (batch 1 at 32,000 keys: 1.14 ms a step with 64 pieces and a combine kernel,
-    1.72 ms with 8 pieces in one cluster)."""
-    return (n_seqs * blocks_per_seq * cluster_splits < sms and max_ctx >= 2048 * cluster_splits
-            and decode_splits(n_seqs, blocks_per_seq, max_ctx, sms) >= 2 * cluster_splits)
+def wants_more_pieces(n_seqs: int, blocks_per_seq: int, max_ctx: int, cluster_splits: int, sms: int, head_dim: int = 64) -> bool:
+    """A cluster holds at most 16 pieces of a context (8 where clusters of sixteen would not all run at once).  One or a few long
+    sequences over few key heads want more, through scratch memory and a combine kernel: while sixteen pieces each leave SMs
+    idle, from 2,048 keys a piece on.  Heads of 64, 4 key heads, a step of four layers with the pieces in one cluster / through scratch,
+    us: batch 1 at 33,000 / 64,000 / 128,000 keys 193 / 217, 247 / 246 and 353 / 313, batch 2 202 / 242, 260 / 302 and 376 / 411 (the kernels
+    alone at 131,072 keys, 1 key head 46 / 29, 4 50 / 43, 8 66 / 67); batch 4 at 33,000, where eight pieces fill half of the GPU, 258 / 379.  Heads of
+    128 stay in the cluster: the split kernel reads them at 2.0 TB/s, heads of 64 at 3.1 (8 key heads, 120,000 keys 855 / 1,315, 24 key heads,
+    60,000 keys 651 / 1,905)."""
+    return (head_dim < 128 and cluster_splits == 8 and 16 * n_seqs * blocks_per_seq <= sms and max_ctx >= 16 * 2048)
 
 
 def _residual_mode(step):
@@ -263,7 +265,7 @@ class PagedAttention(Mixer):
 
     def _decode_fused(self, step, fused, ctx, k_cache, v_cache, table, writes_cache) -> bool:
         """One token a sequence, in one kernel straight from the fused projection: biases, value norm, cache write,
-        attention with the bias table over up to 8 pieces of the context, their merge, the gate.  False where
+        attention with the bias table over up to 16 pieces of the context, their merge, the gate.  False where
         that kernel does not serve (then ``qkv_finish`` and the split kernel do)."""
         s, rt = self.spec, self.rt
         ops = rt.kernels(s.head_dim)
@@ -276,7 +278,7 @@ class PagedAttention(Mixer):
         blocks_per_seq = s.num_kv_heads * (-(-(s.num_heads // s.num_kv_heads) // 16))
         keys = min(step.max_ctx, s.window) if s.window > 0 else step.max_ctx
         splits = fused_decode_splits(n, blocks_per_seq, keys, rt.sm_count, per_sm=2 if s.head_dim <= 64 else 1)
-        if wants_more_pieces(n, blocks_per_seq, keys, splits, rt.sm_count):
+        if wants_more_pieces(n, blocks_per_seq, keys, splits, rt.sm_count, s.head_dim):
             return False
         ops.attention_decode_fused(fused, None, k_cache, v_cache, table, step.ctx_after, ctx, s.num_heads, s.num_kv_heads,
                                    s.head_dim, block_size, s.scale, s.window, splits, writes_cache and not s.shares_kv,
@@ -358,9 +360,9 @@ class PagedAttention(Mixer):
                  and ops.has_attention_decode_fused())
         if fused:
             splits = fused_decode_splits(n, blocks_per_seq, step.max_ctx, rt.sm_count, per_sm=2 if s.head_dim <= 64 else 1)
-            fused = not wants_more_pieces(n, blocks_per_seq, step.max_ctx, splits, rt.sm_count)
+            fused = not wants_more_pieces(n, blocks_per_seq, step.max_ctx, splits, rt.sm_count, s.head_dim)
         if fused:
-            # one kernel: rotation, cache write, attention over the context in up to 8 pieces, merge
+            # one kernel: rotation, cache write, attention over the context in up to 16 pieces, merge
             ops.attention_decode_fused(qkv, self.position.fusion_table(step.max_ctx), k_cache, v_cache, table,
                                        step.ctx_after, ctx, s.num_heads, s.num_kv_heads, s.head_dim,
                                        step.cache.block_size, s.scale, s.window, splits, writes_cache)

@@ -2,6 +2,7 @@
 ``residual.ResidualStats`` and of the ``pre_norm`` arrangement, with stand-in parts (no GPU)."""
 from types import SimpleNamespace
 
+import pytest
 import torch
 
 from stratakv_b200.parts.attention import decode_splits, fused_decode_splits, wants_more_pieces
@@ -120,3 +121,12 @@ def test_only_few_long_sequences_leave_the_cluster_kernel():
     assert not leaves(1, 4, 8192) and not leaves(8, 4, 2048) and not leaves(8, 4, 16384)
     assert not leaves(8, 32, 2048, per_sm=1)              # many heads fill the GPU with one piece each
     assert not leaves(64, 4, 32768)
+
+
+# where sixteen pieces each still leave SMs idle, and only heads that the split kernel reads at its rate
+@pytest.mark.parametrize("step,leaves", [((1, 1, 32768, 64), True), ((9, 1, 32768, 80), True), ((10, 1, 131072, 64), False), ((4, 4, 131072, 64), False),
+                                         ((1, 4, 32767, 64), False), ((1, 8, 131072, 128), False), ((1, 24, 65536, 128), False), ((1, 4, 131072, 112), True)])
+def test_who_leaves_a_cluster_of_sixteen(step, leaves):
+    batch, groups, ctx, head_dim = step
+    splits = fused_decode_splits(batch, groups, ctx, SMS, per_sm=2 if head_dim <= 64 else 1)
+    assert wants_more_pieces(batch, groups, ctx, splits, SMS, head_dim) is leaves

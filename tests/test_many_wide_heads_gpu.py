@@ -32,7 +32,8 @@ def test_more_blocks_than_sms(heads, kv_heads, head_dim, block_size, lengths, wi
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim,block_size,lengths,window", [
     (32, 4, 64, 64, [8100], 0), (32, 4, 64, 16, [4096], 0), (8, 2, 64, 64, [4100, 1, 300], 0),    # pieces without keys, a piece of one
-    (20, 1, 128, 64, [9000, 64], 4097), (1, 1, 80, 32, [5000], 0), (8, 1, 192, 64, [4500], 0)])   # a window, more than 16 heads a key head
+    (20, 1, 128, 64, [9000, 64], 4097), (1, 1, 80, 32, [5000], 0), (8, 1, 192, 64, [4500], 0),
+    (8, 2, 128, 64, [40000], 0)])               # above: a window, more than 16 heads a key head; more blocks than a block keeps of the table
 def test_a_long_context_in_sixteen_pieces(heads, kv_heads, head_dim, block_size, lengths, window):
     dtype, n, scale = torch.bfloat16, len(lengths), 0.5 / math.sqrt(head_dim)
     k = lib(dtype, head_dim)
