@@ -20,7 +20,7 @@
 //            exponentials are taken against is raised only when a tile exceeds it by 2^8; only then
 //            is the accumulated output rescaled (tcgen05.ld / st), so most tiles never touch it.
 //            At the end the output is read once, divided by the row sum and stored.
-// The softmax is the long pole (the special-function unit is busy 62 % of the cycles at 2,048 queries behind 6,144 tokens), so what
+// The softmax is the long pole (at 2,048 queries behind 6,144 tokens the special-function unit takes an instruction in 55 % of the cycles at head size 64, 50 % at 128), so what
 // counts is that two blocks share an SM and hide each other's waits.  Products that take both operands from shared memory read the
 // 128 rows of A again for every 64 columns: with probabilities in shared memory too, and for head size 128 one block an SM, a
 // tile took 1,150 cycles of shared memory alone.  Probabilities in tensor memory, one buffer of them and of scores and two stages of keys and
